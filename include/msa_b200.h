@@ -514,6 +514,18 @@ int msa_add_rmsnorm(const void* x, const void* y, const void* weight, float eps,
                     void* x_out, void* h_out, void* stream);
 int msa_silu_mul(const void* gate_up, int64_t row_stride, int32_t n_rows, int32_t ffn, void* out, void* stream);
 
+/* The same two with operands of their own: q [n_rows, n_q_heads*128] and k [n_rows, n_kv_heads*128] with row strides, cos_table
+ * and sin_table [table_rows, 128] repeating over the rows (n_rows a multiple of table_rows); gate and up [n_rows, ffn]. */
+int msa_heads_norm_rope(const void* q, int64_t q_stride, const void* k, int64_t k_stride, int32_t n_rows, int32_t n_q_heads,
+                        int32_t n_kv_heads, int32_t head_dim, const void* q_weight, const void* k_weight, float eps,
+                        const void* cos_table, const void* sin_table, int32_t table_rows, void* q_out, void* k_out, void* stream);
+int msa_silu_mul_parts(const void* gate, int64_t gate_stride, const void* up, int64_t up_stride, int32_t n_rows, int32_t ffn,
+                       void* out, void* stream);
+
+/* cos_table / sin_table [n, 2*half] in bf16: scaling * cos / sin of positions[i] * inv_freq[j], both halves alike. */
+int msa_rope_table(const int64_t* positions, const float* inv_freq, int32_t n, int32_t half, float scaling, void* cos_table,
+                   void* sin_table, void* stream);
+
 /* ---------------------------------------------------------------------------------------
  * Decode attention without any allocation.  (No counterpart in the reference: this entry
  * point exists for hosts of this library that cannot allocate device memory when a decode

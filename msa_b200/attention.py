@@ -30,10 +30,26 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
-from transformers.models.qwen3.modeling_qwen3 import Qwen3Attention, apply_rotary_pos_emb
+from torch.nn.modules import module as nn_module
+from transformers.models.qwen3.modeling_qwen3 import Qwen3Attention, Qwen3RMSNorm, apply_rotary_pos_emb
 
 from . import _cabi as A
 from . import ops
+
+
+def fused_ops(*tensors) -> bool:
+    """Whether the fused kernels may stand in for eager operations on these: plain bf16 tensors on the GPU, aligned rows, and no
+    gradient to keep (the kernels know none)."""
+    return not torch.is_grad_enabled() and all(
+        type(t) in (torch.Tensor, nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0
+        for t in tensors)
+
+
+def plain_module(m, cls) -> bool:
+    """``m`` is exactly a ``cls`` that nobody hooked into, so that stepping over its call changes nothing."""
+    return (type(m) is cls and "forward" not in m.__dict__ and not nn_module._has_any_global_hook()
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
+
 
 class MemorySparseAttention(Qwen3Attention):
     #: extra cache positions reserved for tokens appended during decode
@@ -82,11 +98,18 @@ class MemorySparseAttention(Qwen3Attention):
                                                  position_embeddings=None, past_key_value=None, **kwargs):
         bsz, q_len, _ = hidden_states.shape
         hidden_shape = (bsz, q_len, -1, self.head_dim)
-        query_states = self.q_norm(self.q_proj(hidden_states).view(hidden_shape)).transpose(1, 2)
-        key_states = self.k_norm(self.k_proj(hidden_states).view(hidden_shape)).transpose(1, 2)
+        query_states, key_states = self.q_proj(hidden_states), self.k_proj(hidden_states)
         value_states = self.v_proj(hidden_states).view(hidden_shape).transpose(1, 2)
         cos, sin = position_embeddings
-        query_states, key_states = apply_rotary_pos_emb(query_states, key_states, cos, sin)
+        if self._takes_fused(query_states, key_states, cos, sin):
+            query_states, key_states = ops.heads_norm_rope(query_states.flatten(0, 1), key_states.flatten(0, 1), self.q_norm.weight,
+                                                           self.k_norm.weight, self.q_norm.variance_epsilon, cos, sin)
+            query_states = query_states.view(hidden_shape).transpose(1, 2)
+            key_states = key_states.view(hidden_shape).transpose(1, 2)
+        else:
+            query_states = self.q_norm(query_states.view(hidden_shape)).transpose(1, 2)
+            key_states = self.k_norm(key_states.view(hidden_shape)).transpose(1, 2)
+            query_states, key_states = apply_rotary_pos_emb(query_states, key_states, cos, sin)
         stage = past_key_value.cache_kwargs[self.layer_idx]["stage"]
         if stage == "prefill_stage1":
             return self._stage1(hidden_states, doc_ids, attention_mask, past_key_value, query_states, key_states,
@@ -95,6 +118,15 @@ class MemorySparseAttention(Qwen3Attention):
             return self._stage2(hidden_states, doc_ids, attention_mask, past_key_value, query_states, key_states,
                                 value_states)
         return self._decode(attention_mask, past_key_value, query_states, key_states, value_states)
+
+    def _takes_fused(self, q, k, cos, sin) -> bool:
+        """Head norm and rotation in one launch (``ops.heads_norm_rope``): bf16 heads of 128, angles per token."""
+        b, s, _ = q.shape
+        return (self.head_dim == 128 and plain_module(self.q_norm, Qwen3RMSNorm) and plain_module(self.k_norm, Qwen3RMSNorm)
+                and self.q_norm.variance_epsilon == self.k_norm.variance_epsilon
+                and fused_ops(q, k, cos, sin, self.q_norm.weight, self.k_norm.weight)
+                and q.stride(0) == s * q.stride(1) and k.stride(0) == s * k.stride(1) and q.stride(1) % 4 == 0 and k.stride(1) % 4 == 0
+                and cos.shape == sin.shape and tuple(cos.shape) in ((b, s, 128), (1, s, 128)))
 
     # ------------------------------------------------------------------------------------ stage 1
     def _bookkeeping(self, doc_ids, attention_mask, cache):
@@ -110,7 +142,7 @@ class MemorySparseAttention(Qwen3Attention):
     def _segments(self, doc_ids, attention_mask, cache):
         """Token lists and segment offsets of the document tokens and of the template tokens of this block
         (one segment per (row, document) run / per row), the longest segment and whether every segment is a
-        run of consecutive tokens; computed once and shared by every layer."""
+        run of consecutive tokens, and how many template tokens there are; computed once and shared by every layer."""
         prev = cache.meta.get("_msa_b200_attn_status")
         if prev is not None and int(prev[0].item()) != 0:
             raise A.MsaError("a bounded barrier wait ran out inside doc_attn_tc_kernel (stage-1 attention output invalid)")
@@ -135,9 +167,9 @@ class MemorySparseAttention(Qwen3Attention):
             spans = None
             if not docs[3] and docs[0].numel() > 0:      # masked tokens inside documents: spans + bitmap for the tcgen05 kernel
                 spans = ops.document_spans(docs[0], docs[1]) + (ops.token_bitmap(listed),)
-            hit = (key, docs, table((doc_ids == -2) & valid, torch.zeros_like(doc_ids)), spans)
+            hit = (key, docs, table((doc_ids == -2) & valid, torch.zeros_like(doc_ids)), spans, int((doc_ids == -2).sum()))
             cache.meta["_msa_b200_segments"] = hit
-        return hit[1], hit[2], hit[3]
+        return hit[1:]
 
     def _valid_runs(self, valid, cache):
         """Device flags ``[2]`` int32: whether the valid tokens of every row are one run of consecutive tokens (what the
@@ -167,9 +199,11 @@ class MemorySparseAttention(Qwen3Attention):
             raise A.MsaError("stage 1 pools one block per call (the reference's worker uses batch size 1)")
 
         # intra-document and template causal attention (:216-241)
-        attn_output = torch.zeros((bsz, q_len, n_heads * self.head_dim), device=device, dtype=dtype)
         pooled_k = pooled_v = pooled_rk = pooled_doc_ids = None
-        (tok_d, off_d, max_d, runs_d), (tok_t, off_t, max_t, _), spans = self._segments(doc_ids, attention_mask, cache)
+        (tok_d, off_d, max_d, runs_d), (tok_t, off_t, max_t, _), spans, n_template = self._segments(doc_ids, attention_mask, cache)
+        # rows that no segment lists stay zero; where every row is listed nothing has to be cleared
+        new = torch.empty if tok_d.numel() + tok_t.numel() == bsz * q_len else torch.zeros
+        attn_output = new((bsz, q_len, n_heads * self.head_dim), device=device, dtype=dtype)
         tc_ok = tensor_cores and max_d >= 128 and ops.doc_attention_tc_supported(query_states, key_states, value_states)
         if tc_ok and runs_d:
             # unmasked documents: attention on the tcgen05 kernel (K and V are pooled by the pooling kernel below)
@@ -205,7 +239,6 @@ class MemorySparseAttention(Qwen3Attention):
                 pooled_rk = ops.pool_chunks(r_k_raw, off, tok, l2_normalize=cosine, head_major_out=True)
             elif cosine:
                 pooled_rk = F.normalize(pooled_k, p=2, dim=-1)
-        n_template = int((doc_ids == -2).sum())
         kw = {"template_prefix_kcache": key_states[:, :, :n_template],
               "template_prefix_vcache": value_states[:, :, :n_template]}
         if self.is_router_layer:

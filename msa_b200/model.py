@@ -5,7 +5,9 @@ Only what the stage-1 worker and the generation loop call: embeddings, N pre-nor
 is this package's ``MemorySparseAttention`` (``doc_ids`` handed down to every layer), final norm, ``lm_head``.
 Module and parameter names follow the reference (``model.embed_tokens``, ``model.layers.<i>.self_attn.*``,
 ``model.layers.<i>.mlp.*``, ``model.norm``, ``lm_head``), so a reference checkpoint's state dict loads with
-``load_state_dict``.  MLP, RMSNorm and rotary embedding are transformers' Qwen3 modules, as in the reference.
+``load_state_dict``.  MLP, RMSNorm and rotary embedding are transformers' Qwen3 modules, as in the reference.  In bf16
+inference (``fused_ops``) what they do between the matrix products runs on this package's kernels: the projections are called
+as modules, the norms with the residual adds, ``act(gate) * up`` and the angles of the rotation are one launch each.
 The training losses of the reference's ``MSAForCausalLM.forward`` are out of scope.
 """
 from __future__ import annotations
@@ -14,10 +16,22 @@ from types import SimpleNamespace
 
 import torch
 import torch.nn as nn
+import torch.nn.functional as F
 from transformers.models.qwen3.modeling_qwen3 import Qwen3MLP, Qwen3RMSNorm, Qwen3RotaryEmbedding
 
-from .attention import MemorySparseAttention
+from . import ops
+from .attention import MemorySparseAttention, fused_ops, plain_module
 from .cache import create_cache
+
+
+def add_norm(x, branch, norm):
+    """``(x + branch, norm(x + branch))`` of ``[B, S, hidden]``, in one launch where the operands allow it."""
+    if not (fused_ops(x, norm.weight) and (branch is None or (fused_ops(branch) and branch.shape == x.shape))):
+        x = x if branch is None else x + branch
+        return x, norm(x)
+    flat = lambda t: t if t is None else t.reshape(-1, t.shape[-1]).contiguous()
+    x_new, h = ops.add_rmsnorm(flat(x), flat(branch), norm.weight, norm.variance_epsilon)
+    return x_new.view(x.shape), h.view(x.shape)
 
 
 class MSADecoderLayer(nn.Module):
@@ -28,6 +42,28 @@ class MSADecoderLayer(nn.Module):
         self.mlp = Qwen3MLP(config)
         self.input_layernorm = Qwen3RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
         self.post_attention_layernorm = Qwen3RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
+        self._silu = type(self.mlp.act_fn) if config.hidden_act == "silu" else None
+
+    def takes_fused(self, x) -> bool:
+        """Whether ``fused`` computes what ``forward`` does on ``x``: nobody watches or replaced the modules it steps over."""
+        norms, mlp = (self.input_layernorm, self.post_attention_layernorm), self.mlp
+        return (plain_module(self, MSADecoderLayer) and plain_module(mlp, Qwen3MLP) and plain_module(mlp.act_fn, self._silu)
+                and all(plain_module(n, Qwen3RMSNorm) and fused_ops(x, n.weight) for n in norms)
+                and x.shape[-1] % 2 == 0 and x.shape[-1] <= 12288)
+
+    def fused(self, x, pending, attention_mask, past_key_value, position_embeddings, doc_ids):
+        """``forward`` on the stream ``x`` with a branch ``pending`` (or None) that has not joined it yet; returns the same pair,
+        so that every residual add is part of the norm that follows it."""
+        x, h = add_norm(x, pending, self.input_layernorm)
+        attn, _ = self.self_attn(h, doc_ids, attention_mask=attention_mask, position_embeddings=position_embeddings,
+                                 past_key_value=past_key_value)
+        x, h = add_norm(x, attn, self.post_attention_layernorm)
+        gate, up = self.mlp.gate_proj(h), self.mlp.up_proj(h)
+        if fused_ops(gate) and fused_ops(up) and gate.shape == up.shape and gate.shape[-1] % 2 == 0:
+            act = ops.silu_mul_parts(gate.flatten(0, 1), up.flatten(0, 1)).view(gate.shape)
+        else:
+            act = F.silu(gate) * up
+        return x, self.mlp.down_proj(act)
 
     def forward(self, hidden_states, attention_mask=None, past_key_value=None, position_embeddings=None, doc_ids=None):
         attn, _ = self.self_attn(self.input_layernorm(hidden_states), doc_ids, attention_mask=attention_mask,
@@ -45,6 +81,14 @@ class MSAModel(nn.Module):
         self.norm = Qwen3RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
         self.rotary_emb = Qwen3RotaryEmbedding(config=config)
 
+    def _angles(self, hidden, position_ids):
+        rot = self.rotary_emb
+        if (plain_module(rot, Qwen3RotaryEmbedding) and rot.rope_type == "default" and fused_ops(hidden) and position_ids.is_cuda
+                and position_ids.device == hidden.device == rot.inv_freq.device and position_ids.dtype == torch.int64
+                and position_ids.dim() == 2 and rot.inv_freq.dtype == torch.float32):
+            return ops.rope_table(position_ids, rot.inv_freq, rot.attention_scaling)
+        return rot(hidden, position_ids)
+
     def forward(self, input_ids=None, attention_mask=None, position_ids=None, past_key_values=None, inputs_embeds=None,
                 use_cache=True, doc_ids=None, **unused):
         """Same call as the reference's ``MSAModel.forward`` (the flags it only forwards to outputs are accepted and
@@ -56,7 +100,13 @@ class MSAModel(nn.Module):
             past_key_values = create_cache()
         if position_ids is None:
             position_ids = torch.arange(hidden.shape[1], device=hidden.device).unsqueeze(0)
-        position_embeddings = self.rotary_emb(hidden, position_ids)
+        position_embeddings = self._angles(hidden, position_ids)
+        if plain_module(self.norm, Qwen3RMSNorm) and fused_ops(hidden, self.norm.weight) and all(layer.takes_fused(hidden) for layer in self.layers):
+            pending = None
+            for layer in self.layers:
+                hidden, pending = layer.fused(hidden, pending, attention_mask, past_key_values, position_embeddings, doc_ids)
+            _, hidden = add_norm(hidden, pending, self.norm)
+            return SimpleNamespace(last_hidden_state=hidden, past_key_values=past_key_values if use_cache else None)
         for layer in self.layers:
             hidden = layer(hidden, attention_mask=attention_mask, past_key_value=past_key_values,
                            position_embeddings=position_embeddings, doc_ids=doc_ids)

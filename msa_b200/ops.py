@@ -786,6 +786,49 @@ def silu_mul(gate_up: torch.Tensor, ffn: int) -> torch.Tensor:
     return out
 
 
+def heads_norm_rope(q: torch.Tensor, k: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, eps: float,
+                    cos: torch.Tensor, sin: torch.Tensor):
+    """``qk_norm_rope`` over projections of their own: q ``[rows, Hq*128]``, k ``[rows, Hkv*128]`` (bf16, contiguous last axis),
+    cos / sin ``[table_rows, 128]`` repeating over the rows.  Returns ``(q[rows, Hq*128], k[rows, Hkv*128])`` contiguous."""
+    A.need_cuda(q, k, q_weight, k_weight, cos, sin)
+    rows = q.shape[0]
+    if any(t.dtype != torch.bfloat16 or t.stride(-1) != 1 for t in (q, k, q_weight, k_weight)) or k.shape[0] != rows:
+        raise A.MsaError("heads_norm_rope: bf16 rows with a contiguous feature axis expected")
+    cos, sin = cos.reshape(-1, 128).contiguous(), sin.reshape(-1, 128).contiguous()
+    if cos.dtype != torch.bfloat16 or sin.dtype != torch.bfloat16 or cos.shape != sin.shape:
+        raise A.MsaError("heads_norm_rope: bf16 cos / sin tables of equal shape expected")
+    q_out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+    k_out = torch.empty(k.shape, dtype=k.dtype, device=k.device)
+    A.check(A.lib().msa_heads_norm_rope(A.ptr(q), q.stride(0), A.ptr(k), k.stride(0), rows, q.shape[1] // 128, k.shape[1] // 128, 128,
+                                        A.ptr(q_weight), A.ptr(k_weight), float(eps), A.ptr(cos), A.ptr(sin), cos.shape[0], A.ptr(q_out),
+                                        A.ptr(k_out), A.stream_ptr(q.device)), "msa_heads_norm_rope")
+    return q_out, k_out
+
+
+def silu_mul_parts(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    """``silu(gate) * up`` (bf16 rows ``[n, ffn]`` of separate products)."""
+    A.need_cuda(gate, up)
+    if gate.dtype != torch.bfloat16 or up.dtype != torch.bfloat16 or gate.shape != up.shape or gate.stride(1) != 1 or up.stride(1) != 1:
+        raise A.MsaError("silu_mul_parts: bf16 rows of equal shape with a contiguous feature axis expected")
+    out = torch.empty(gate.shape, dtype=gate.dtype, device=gate.device)
+    A.check(A.lib().msa_silu_mul_parts(A.ptr(gate), gate.stride(0), A.ptr(up), up.stride(0), gate.shape[0], gate.shape[1], A.ptr(out),
+                                       A.stream_ptr(gate.device)), "msa_silu_mul_parts")
+    return out
+
+
+def rope_table(position_ids: torch.Tensor, inv_freq: torch.Tensor, scaling: float = 1.0):
+    """``(cos, sin)`` bf16 ``[*position_ids.shape, 2 * len(inv_freq)]`` of int64 positions and fp32 frequencies."""
+    A.need_cuda(position_ids, inv_freq)
+    if position_ids.dtype != torch.int64 or inv_freq.dtype != torch.float32:
+        raise A.MsaError("rope_table: int64 positions and float32 frequencies expected")
+    position_ids, inv_freq = position_ids.contiguous(), inv_freq.contiguous()
+    half = inv_freq.numel()
+    both = torch.empty((2, *position_ids.shape, 2 * half), dtype=torch.bfloat16, device=position_ids.device)
+    A.check(A.lib().msa_rope_table(A.ptr(position_ids), A.ptr(inv_freq), position_ids.numel(), half, float(scaling), A.ptr(both[0]),
+                                   A.ptr(both[1]), A.stream_ptr(position_ids.device)), "msa_rope_table")
+    return both[0], both[1]
+
+
 def keys_to_scores(keys: torch.Tensor) -> torch.Tensor:
     """Decode a table of order-preserving keys (int32 storage) back to float32 scores."""
     u = keys.to(torch.int64) & 0xFFFFFFFF
