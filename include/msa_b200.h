@@ -165,6 +165,15 @@ int msa_route_scores(const void* q_folded, const float* row_bias, int32_t dtype,
                      int64_t table_stride, int32_t n_docs, float min_val, uint32_t flags,
                      int32_t* status, void* stream);
 
+/* The same with scratch for skipping padding (both may be NULL): the tensor-core kernel lists the 16-row blocks that hold a row
+ * whose bias is not -inf in live_blocks (device int32 [n_seq*s_pad/16 + 1]), copies them to packed_rows (as large as q_folded)
+ * and contracts those only.  Same results. */
+int msa_route_scores_live(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
+                     int32_t s_pad, const void* rk, int64_t rk_chunk_stride, int32_t n_chunks,
+                     int32_t kdim, const int32_t* chunk_doc, float alpha, uint32_t* score_keys,
+                     int64_t table_stride, int32_t n_docs, float min_val, uint32_t flags,
+                     int32_t* status, int32_t* live_blocks, void* packed_rows, void* stream);
+
 /* ---------------------------------------------------------------------------------------
  * Routing in the other reduce modes of Memory.prefill_stage2 (src/msa_service.py:740-745 head_reduce
  * "max", :794-812 chunk_reduce "mean").  Both go through a per-(sequence, chunk) table of keys,

@@ -289,11 +289,11 @@ extern "C" int msa_route_table_reset(uint32_t* score_keys, int64_t table_stride,
   return MSA_OK;
 }
 
-extern "C" int msa_route_scores(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
+extern "C" int msa_route_scores_live(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
                                 int32_t s_pad, const void* rk, int64_t rk_chunk_stride, int32_t n_chunks,
                                 int32_t kdim, const int32_t* chunk_doc, float alpha, uint32_t* score_keys,
                                 int64_t table_stride, int32_t n_docs, float min_val, uint32_t flags,
-                                int32_t* status, void* stream) {
+                                int32_t* status, int32_t* live_blocks, void* packed_rows, void* stream) {
   MSA_REQUIRE(dtype_ok(dtype), "route: unknown dtype %d", dtype);
   MSA_REQUIRE(score_keys && status, "route: null pointer");
   MSA_REQUIRE(n_seq >= 0 && s_pad >= 1 && n_chunks >= 0 && kdim > 0 && n_docs >= 0, "route: bad sizes");
@@ -312,7 +312,16 @@ extern "C" int msa_route_scores(const void* q_folded, const float* row_bias, int
               "route: tile-blocked router keys are read by the tensor-core kernel only (bf16, kdim %% 64 == 0)");
   if (dtype == MSA_BF16 && !(flags & MSA_ROUTE_FORCE_SIMT))
     return launch_route_tc(q_folded, row_bias, n_seq, s_pad, rk, rk_chunk_stride, n_chunks, kdim, chunk_doc, n_docs,
-                           alpha, min_val, score_keys, table_stride, status, blocked, st);
+                           alpha, min_val, score_keys, table_stride, status, blocked, live_blocks, packed_rows, st);
   return launch_route_simt(dtype, q_folded, row_bias, n_seq, s_pad, rk, rk_chunk_stride, n_chunks, kdim, chunk_doc,
                            n_docs, alpha, score_keys, table_stride, status, st);
+}
+
+extern "C" int msa_route_scores(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
+                                int32_t s_pad, const void* rk, int64_t rk_chunk_stride, int32_t n_chunks,
+                                int32_t kdim, const int32_t* chunk_doc, float alpha, uint32_t* score_keys,
+                                int64_t table_stride, int32_t n_docs, float min_val, uint32_t flags,
+                                int32_t* status, void* stream) {
+  return msa_route_scores_live(q_folded, row_bias, dtype, n_seq, s_pad, rk, rk_chunk_stride, n_chunks, kdim, chunk_doc, alpha,
+                               score_keys, table_stride, n_docs, min_val, flags, status, nullptr, nullptr, stream);
 }

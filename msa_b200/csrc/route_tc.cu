@@ -51,6 +51,7 @@ struct RouteTcParams {
   uint32_t* keys;
   long long table_stride;
   int32_t* status;
+  const int32_t* live;   // pair kernel: [count | numbers of the 16-row blocks that hold a valid token], or null
 };
 
 struct TileCoord { int ct, qt; };
@@ -173,6 +174,36 @@ __device__ __forceinline__ void epilogue_compute(const RouteTcParams& p, const S
       }
       if (si.publish) publish_score(run, (q0 + s0) / p.s_pad);
     }
+  }
+}
+
+// The same for a tile whose 16-column blocks are listed: `seqs[1 .. n]` are the blocks' sequences, seqs[0] and seqs[n + 1] those
+// of the list's neighbours (-1: none).  Columns of one sequence stand side by side; a sequence that goes on in another tile has
+// another writer.
+__device__ __forceinline__ void epilogue_blocks(const RouteTcParams& p, const SegInfo& si, const float* bias, uint32_t taddr,
+                                                const int* seqs, int n) {
+  float run = -INFINITY;
+  bool whole = seqs[0] != seqs[1];
+  for (int i = 1; i <= n; ++i) {
+    uint32_t r[16];
+    tmem_ld16(taddr + (i - 1) * 16, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) run = fmaxf(run, __uint_as_float(r[j]) + bias[(i - 1) * 16 + j]);
+    const int seq = seqs[i];
+    if (i < n && seqs[i + 1] == seq) continue;
+    for (int d = 1; d < si.max_len; d <<= 1) {
+      const float o = __shfl_up_sync(0xffffffffu, run, d);
+      if (si.dist >= d) run = fmaxf(run, o);
+    }
+    if (si.publish) {
+      const uint32_t key = float_to_key(run * p.alpha);
+      uint32_t* dst = p.keys + (long long)seq * p.table_stride + si.doc;
+      if (si.exclusive && whole && seqs[i + 1] != seq) *dst = max(key, p.min_key);
+      else atomicMax(dst, key);
+    }
+    run = -INFINITY;
+    whole = true;
   }
 }
 
@@ -369,17 +400,28 @@ __device__ __forceinline__ void tc_mma_bf16_pair(uint32_t d_tmem, uint64_t a_des
 
 constexpr int kPairBN = 256;  // query rows per cluster tile
 constexpr int kPairBM = 256;  // chunks per cluster tile (128 per CTA)
+constexpr int kBlockRows = 16, kTileBlocks = kPairBN / kBlockRows;
 
+// kLive: questions of one batch differ in length, so a fixed layout of s_pad rows per sequence holds padding (a quarter of the
+// rows when lengths spread over half to full).  The 16-row blocks that hold a valid token are listed and copied next to one
+// another first (pack_rows_kernel); the tiles run over those, any tile may hold several sequences, and the list's length is read
+// here, so the host never waits for it.  (Fetching the blocks in place, eight 16-row boxes per stage, is bound by the copy
+// engine: 2.95 ms for 48 x (100..200) tokens x 190,000 chunks, as slow as all 208-row tiles of the one-CTA kernel; over packed rows 2.16 ms.)
+template <bool kLive>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 route_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_q,
-                     const RouteTcParams p) {
+                     const RouteTcParams args) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ uint64_t s_full[kMaxStages], s_empty[kMaxStages], s_acc_full[2], s_acc_empty[2], s_drain;
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
   __shared__ float s_bias[kEpiThreads / 32][kRouteMaxN];
   __shared__ EpiScratch s_epi[kEpiThreads / 32];
+  __shared__ int s_seqs[kEpiThreads / 32][kTileBlocks + 2];
 
+  RouteTcParams p = args;
+  const int n_live = kLive ? args.live[0] : 0;
+  if (kLive) p.n_qtiles = (n_live + kTileBlocks - 1) / kTileBlocks;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -476,7 +518,19 @@ route_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
       const int q0 = tc.qt * kPairBN;
       float* bias = s_bias[warp];
       __syncwarp();
-      for (int j = lane; j < kPairBN; j += 32) bias[j] = (q0 + j < p.n_rows) ? p.row_bias[q0 + j] : -INFINITY;
+      if (kLive) {
+        const int first = tc.qt * kTileBlocks;
+        if (lane < kTileBlocks + 2) {
+          const int i = first + lane - 1;
+          s_seqs[warp][lane] = i >= 0 && i < n_live ? args.live[1 + i] * kBlockRows / p.s_pad : -1;
+        }
+        for (int j = lane; j < kPairBN; j += 32) {
+          const int i = first + j / kBlockRows;
+          bias[j] = i < n_live ? p.row_bias[args.live[1 + i] * kBlockRows + j % kBlockRows] : -INFINITY;
+        }
+      } else {
+        for (int j = lane; j < kPairBN; j += 32) bias[j] = (q0 + j < p.n_rows) ? p.row_bias[q0 + j] : -INFINITY;
+      }
       const SegInfo si = seg_info(p, tc.ct * kPairBM + (int)rank * kBM + (int)threadIdx.x, lane, s_epi[warp]);
       __syncwarp();
       ok = mbar_wait(&s_acc_full[buf], acc_phase, abort_flag, p.status, 4);
@@ -484,7 +538,8 @@ route_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)buf * kRouteMaxN;
-      epilogue_compute(p, si, bias, taddr, q0, s_epi[warp], lane);
+      if (kLive) epilogue_blocks(p, si, bias, taddr, s_seqs[warp], min(kTileBlocks, n_live - tc.qt * kTileBlocks));
+      else epilogue_compute(p, si, bias, taddr, q0, s_epi[warp], lane);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&s_acc_empty[buf]), 0));
@@ -498,6 +553,60 @@ route_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
   tc_fence_after();
   if (warp == 5)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+}
+
+// live[1 ..]: the 16-row blocks with a row whose bias is not -inf, in order; live[0]: their number.  One block of 1024 threads:
+// 624 blocks of 16 biases take one round.
+__global__ void __launch_bounds__(1024) live_blocks_kernel(const float* __restrict__ row_bias, int n_blocks, int32_t* __restrict__ live) {
+  __shared__ int s_count[32], s_base;
+  grid_launch_dependents();
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (threadIdx.x == 0) s_base = 0;
+  for (int first = 0; first < n_blocks; first += 1024) {
+    const int i = first + threadIdx.x;
+    bool on = false;
+    if (i < n_blocks)
+      for (int j = 0; j < kBlockRows; j += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(row_bias + (long long)i * kBlockRows + j);
+        on = on || b.x > -INFINITY || b.y > -INFINITY || b.z > -INFINITY || b.w > -INFINITY;
+      }
+    const uint32_t ballot = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) s_count[warp] = __popc(ballot);
+    __syncthreads();
+    int at = s_base, all = 0;
+    for (int w = 0; w < 32; ++w) { if (w < warp) at += s_count[w]; all += s_count[w]; }
+    if (on) live[1 + at + __popc(ballot & ((1u << lane) - 1u))] = i;
+    __syncthreads();
+    if (threadIdx.x == 0) s_base += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) live[0] = s_base;
+}
+
+// Listed block i of rows [.., kdim] -> block i of `packed`; one CTA per block of 16 rows, eight 16-byte loads in flight per
+// thread (7,700 rows of 2 KB: 5 us).
+__global__ void __launch_bounds__(256) pack_rows_kernel(const uint4* __restrict__ rows, const int32_t* __restrict__ live, int vecs,
+                                                        uint4* __restrict__ packed) {
+  grid_dependency_wait();
+  if ((int)blockIdx.x >= live[0]) return;
+  const uint4* src = rows + (long long)live[1 + blockIdx.x] * vecs;
+  uint4* dst = packed + (long long)blockIdx.x * vecs;
+  for (int first = threadIdx.x; first < vecs; first += 2048) {
+    uint4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) if (first + j * 256 < vecs) v[j] = src[first + j * 256];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) if (first + j * 256 < vecs) dst[first + j * 256] = v[j];
+  }
+}
+
+static int pack_live_rows(const void* rows, const float* row_bias, int n_blocks, int kdim, int32_t* live, void* packed, cudaStream_t stream) {
+  MSA_REQUIRE(aligned16(row_bias) && aligned16(packed), "route: the row bias and the scratch rows must be 16-byte aligned");
+  live_blocks_kernel<<<1, 1024, 0, stream>>>(row_bias, n_blocks, live);
+  MSA_LAUNCH_OK("live_blocks_kernel");
+  MSA_CUDA_OK(launch_kernel_pdl(pack_rows_kernel, dim3(n_blocks), dim3(256), 0, stream, true, (const uint4*)rows, (const int32_t*)live,
+                                kBlockRows * kdim / 8, (uint4*)packed));
+  return MSA_OK;
 }
 
 // The bounded wait on its own: one CTA waits on a barrier that nothing ever completes, with the
@@ -518,7 +627,7 @@ __global__ void wait_selftest_kernel(unsigned long long limit_ns, int32_t* statu
 // ---- host side ------------------------------------------------------------------------
 int launch_route_tc(const void* qf, const float* row_bias, int n_seq, int s_pad, const void* rk, int64_t rk_stride,
                     int n_chunks, int kdim, const int32_t* chunk_doc, int n_docs, float alpha, float min_val,
-                    uint32_t* keys, int64_t table_stride, int32_t* status, bool blocked, cudaStream_t stream) {
+                    uint32_t* keys, int64_t table_stride, int32_t* status, bool blocked, int32_t* live, void* packed, cudaStream_t stream) {
   MSA_REQUIRE(kdim % kBK == 0, "route (tensor-core path): kdim=%d must be a multiple of %d", kdim, kBK);
   MSA_REQUIRE(aligned16(qf) && aligned16(rk) && rk_stride % 8 == 0 && rk_stride >= kdim,
               "route (tensor-core path): rows must be 16-byte aligned");
@@ -570,27 +679,42 @@ int launch_route_tc(const void* qf, const float* row_bias, int n_seq, int s_pad,
 
   int n_sm = 0;
   MSA_OK_OR_RETURN(device_sm_count(&n_sm));
-  static DeviceSmem smem_set{}, smem_set_8{}, smem_set_16{}, pair_set{};
+  static DeviceSmem smem_set{}, smem_set_8{}, smem_set_16{}, pair_set{}, pair_live_set{};
   const size_t smem = (size_t)p.stages * stage_bytes + 1024;
   if (epi_warps == 16) MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_kernel<16>, smem, smem_set_16));
   else if (epi_warps == 8) MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_kernel<8>, smem, smem_set_8));
   else MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_kernel<4>, smem, smem_set));
   const long long n_tiles = (long long)p.n_ctiles * p.n_qtiles;
-  // Tensor-bound shapes (full 256-row query tiles, enough chunk tiles to fill the GPU) run on CTA pairs.
+  // Tensor-bound shapes (enough chunk tiles to fill the GPU) run on CTA pairs: over the blocks of valid rows where sequences
+  // have several rows each, else over full 256-row query tiles.
   static const bool pair_off = getenv("MSA_B200_ROUTE_NO_PAIR") != nullptr;
-  if (!pair_off && !blocked && p.bn == kPairBN && p.n_rows % kPairBN == 0 && n_tiles >= 2ll * n_sm) {
+  const bool by_blocks = live && packed && s_pad > 1;
+  const long long n_qtiles_256 = (p.n_rows + kPairBN - 1) / kPairBN;
+  if (!pair_off && !blocked && (by_blocks ? n_qtiles_256 * p.n_ctiles >= 2ll * n_sm
+                                          : p.bn == kPairBN && p.n_rows % kPairBN == 0 && n_tiles >= 2ll * n_sm)) {
     RouteTcParams p2 = p;
+    p2.bn = kPairBN;
     p2.n_ctiles = (n_chunks + kPairBM - 1) / kPairBM;
+    p2.n_qtiles = (int)n_qtiles_256;
+    p2.qgroup = (int)((32u << 20) / ((size_t)kPairBN * kdim * 2));
+    if (p2.qgroup < 1) p2.qgroup = 1;
+    if (p2.qgroup > p2.n_qtiles) p2.qgroup = p2.n_qtiles;
     p2.stages = 6;  // 6 x 32 KB
+    p2.live = by_blocks ? live : nullptr;
     CUtensorMap map_q2;
-    rc = make_map(&map_q2, qf, (uint64_t)p.n_rows, (uint64_t)kdim, (uint64_t)kdim, kBK, (uint32_t)(kPairBN / 2));
+    rc = make_map(&map_q2, by_blocks ? packed : qf, (uint64_t)p.n_rows, (uint64_t)kdim, (uint64_t)kdim, kBK, (uint32_t)(kPairBN / 2));
     if (rc != MSA_OK) return rc;
     const size_t smem2 = (size_t)p2.stages * 2 * kBM * kBK * 2 + 1024;
-    MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_pair_kernel, smem2, pair_set));
-    const long long tiles2 = (long long)p2.n_ctiles * p2.n_qtiles;
     long long clusters = n_sm / 2;
-    if (clusters > tiles2) clusters = tiles2;
-    route_tc_pair_kernel<<<(int)(2 * clusters), kTcThreads, smem2, stream>>>(map_k, map_q2, p2);
+    if (clusters > (long long)p2.n_ctiles * p2.n_qtiles) clusters = (long long)p2.n_ctiles * p2.n_qtiles;
+    if (by_blocks) {
+      MSA_OK_OR_RETURN(pack_live_rows(qf, row_bias, p.n_rows / kBlockRows, kdim, live, packed, stream));
+      MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_pair_kernel<true>, smem2, pair_live_set));
+      route_tc_pair_kernel<true><<<(int)(2 * clusters), kTcThreads, smem2, stream>>>(map_k, map_q2, p2);
+    } else {
+      MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_pair_kernel<false>, smem2, pair_set));
+      route_tc_pair_kernel<false><<<(int)(2 * clusters), kTcThreads, smem2, stream>>>(map_k, map_q2, p2);
+    }
     MSA_LAUNCH_OK("route_tc_pair_kernel");
     return MSA_OK;
   }

@@ -110,7 +110,8 @@ def fold_queries(q: torch.Tensor, query_mask: torch.Tensor, num_kv_groups: int, 
     b, hq, s, d = q.shape
     if q.stride(3) != 1:
         q = q.contiguous()
-    mask = query_mask.reshape(b, s).to(torch.uint8).contiguous()
+    mask = query_mask.reshape(b, s).contiguous()
+    mask = mask.view(torch.uint8) if mask.dtype == torch.bool else mask.to(torch.uint8)
     if s_pad is None:
         s_pad = route_s_pad(s, query_reduce)
     hkv = hq // num_kv_groups
@@ -190,10 +191,14 @@ def route_scores(q_folded: torch.Tensor, row_bias: torch.Tensor, n_seq: int, s_p
         keys = torch.empty((n_seq, n_docs + 1), dtype=torch.int32, device=dev)
     if status is None:
         status = torch.zeros(4, dtype=torch.int32, device=dev)
-    A.check(A.lib().msa_route_scores(A.ptr(q_folded), A.ptr(row_bias), A.dtype_code(rk.dtype), n_seq, s_pad,
-                                     A.ptr(rk2), rk2.stride(0) if c > 0 else kdim, c, kdim, A.ptr(chunk_doc),
-                                     float(alpha), A.ptr(keys), keys.stride(0), n_docs, float(min_val), flags,
-                                     A.ptr(status), A.stream_ptr(dev)), "msa_route_scores")
+    # questions of unequal length: scratch for the list of 16-row blocks that hold a valid token, and for those rows
+    live = packed = None
+    if s_pad > 1 and rk.dtype == torch.bfloat16 and not blocked and row_bias.data_ptr() % 16 == 0:
+        live, packed = torch.empty(n_seq * s_pad // 16 + 1, dtype=torch.int32, device=dev), torch.empty_like(q_folded)
+    A.check(A.lib().msa_route_scores_live(A.ptr(q_folded), A.ptr(row_bias), A.dtype_code(rk.dtype), n_seq, s_pad,
+                                          A.ptr(rk2), rk2.stride(0) if c > 0 else kdim, c, kdim, A.ptr(chunk_doc),
+                                          float(alpha), A.ptr(keys), keys.stride(0), n_docs, float(min_val), flags,
+                                          A.ptr(status), A.ptr(live), A.ptr(packed), A.stream_ptr(dev)), "msa_route_scores_live")
     return keys, status
 
 
