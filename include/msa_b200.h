@@ -325,6 +325,15 @@ int msa_gather_plan(const int64_t* sel_local, const int32_t* sel_rank, int32_t n
                     int64_t* plan, int64_t* n_sel, int64_t* total, int64_t* total_host_mapped,
                     int32_t* status, void* stream);
 
+/* The same, and what a host that sizes its buffers reads back arrives with it: report (device-visible host memory, 3 int64) =
+ * the total, status words 0 and 1, status words 2 and 3 as the plan leaves them (zeros without status). */
+int msa_gather_plan_report(const int64_t* sel_local, const int32_t* sel_rank, int32_t n_seq, int32_t k,
+                           int32_t world, const int64_t* shard_doc_base, int64_t n_dir_rows,
+                           const int64_t* doc_chunk_offset, const int32_t* doc_chunk_len,
+                           const uint64_t* shard_kv_base, int64_t chunk_bytes, int64_t sample_stride,
+                           int64_t* plan, int64_t* n_sel, int64_t* total, int64_t* report,
+                           int32_t* status, void* stream);
+
 /* msa_gather_plan_resident: msa_gather_plan for a decode loop that refreshes the same per-sample segment every step
  * (what a per-step doc_query, src/msa_service.py:1193-1283, would fetch again and again).  A sample's room is k
  * slots of slot_len entries; resident [n_seq, k] int64 (filled with -1 by the caller before the first call, then

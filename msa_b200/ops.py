@@ -397,12 +397,14 @@ def topk_merge(cand_scores: torch.Tensor, cand_local: torch.Tensor, cand_global:
 def gather_plan(sel_local: torch.Tensor, sel_rank: Optional[torch.Tensor], world: int, shard_doc_base: torch.Tensor,
                 doc_chunk_offset: torch.Tensor, doc_chunk_len: torch.Tensor, shard_kv_base: torch.Tensor,
                 chunk_bytes: int, total_host: Optional[torch.Tensor] = None, sample_stride: int = 0,
-                status: Optional[torch.Tensor] = None, resident: Optional[torch.Tensor] = None):
+                status: Optional[torch.Tensor] = None, resident: Optional[torch.Tensor] = None,
+                report: Optional[torch.Tensor] = None):
     """Plan the fetch of the winners ``sel_local[B, k]`` (owner ranks ``sel_rank``).  ``sample_stride`` 0 packs
     the samples one after another; > 0 gives every sample that many entries of room (see ``gather_run``).
     Winners outside the directory are dropped and counted in ``status[2]``.  ``resident`` ``[B, k]`` int64 (-1 =
     empty, updated in place; needs ``sample_stride`` = k slots of equal length): winners whose entries the sample's
-    segment already holds are not planned again, the others go into the slots that became free.
+    segment already holds are not planned again, the others go into the slots that became free.  ``report`` (pinned int64
+    ``[3]``): receives the total and the four status words when the plan has run.
     Returns ``(plan[B*k, 4], n_sel[B], total[1])``."""
     A.need_cuda(sel_local, sel_rank, shard_doc_base, doc_chunk_offset, doc_chunk_len, shard_kv_base, status)
     n_seq, k = sel_local.shape
@@ -426,11 +428,14 @@ def gather_plan(sel_local: torch.Tensor, sel_rank: Optional[torch.Tensor], world
             chunk_bytes, int(sample_stride) // k, A.ptr(resident), A.ptr(plan), A.ptr(n_sel), A.ptr(total), A.ptr(status),
             A.stream_ptr(dev)), "msa_gather_plan_resident")
         return plan, n_sel, total
-    A.check(A.lib().msa_gather_plan(A.ptr(sel_local.contiguous()), A.ptr(sel_rank.contiguous() if sel_rank is not None else None),
-                                    n_seq, k, world, A.ptr(shard_doc_base), doc_chunk_len.numel(), A.ptr(doc_chunk_offset),
-                                    A.ptr(doc_chunk_len), A.ptr(shard_kv_base), chunk_bytes, int(sample_stride),
-                                    A.ptr(plan), A.ptr(n_sel), A.ptr(total), A.ptr(total_host), A.ptr(status),
-                                    A.stream_ptr(dev)), "msa_gather_plan")
+    if report is not None and (total_host is not None or report.dtype != torch.int64 or report.numel() != 3 or not report.is_pinned()):
+        raise A.MsaError("gather_plan: report must be a pinned int64 [3] tensor, in place of total_host")
+    call = A.lib().msa_gather_plan if report is None else A.lib().msa_gather_plan_report
+    A.check(call(A.ptr(sel_local.contiguous()), A.ptr(sel_rank.contiguous() if sel_rank is not None else None),
+                 n_seq, k, world, A.ptr(shard_doc_base), doc_chunk_len.numel(), A.ptr(doc_chunk_offset),
+                 A.ptr(doc_chunk_len), A.ptr(shard_kv_base), chunk_bytes, int(sample_stride),
+                 A.ptr(plan), A.ptr(n_sel), A.ptr(total), A.ptr(total_host if report is None else report), A.ptr(status),
+                 A.stream_ptr(dev)), "msa_gather_plan")
     return plan, n_sel, total
 
 

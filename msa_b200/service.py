@@ -145,8 +145,7 @@ class MSAService(Memory, MemoryClientBase):
         self.shard_top_k = shard_top_k or self.model_config.doc_top_k
         self.uniform_seqlen = False   # set when every rank is known to pass queries of equal length
         self._directory = None
-        self._total_pinned = torch.zeros(1, dtype=torch.int64).pin_memory()
-        self._status_pinned = torch.zeros(4, dtype=torch.int32).pin_memory()
+        self._report = torch.zeros(3, dtype=torch.int64).pin_memory()      # total and status words of a plan, written by the kernel
 
     def setup_memory_client(self, model):
         """Inject this service into every module that has ``set_memory_client`` (:1057-1067)."""
@@ -318,16 +317,15 @@ class MSAService(Memory, MemoryClientBase):
         blk = self.blocks[layer_idx]
         chunk_bytes = 2 * g.num_key_value_heads * g.head_dim * blk.kv.element_size()
         plan, n_sel, total = ops.gather_plan(winner_local, winner_rank, self.world_size, base, offs, ln,
-                                             kv_base[layer_idx], chunk_bytes, total_host=None, status=self._status)
+                                             kv_base[layer_idx], chunk_bytes, status=self._status,
+                                             report=self._report if max_entries is None else None)
         if max_entries is not None:
             k, v = ops.gather_run(plan, blk.kv.dtype, g.num_key_value_heads, g.head_dim, max_entries, max_ctas)
             return k, v, n_sel, total
-        # one read-back sizes the result; the status words of this layer's routing and plan ride along
-        self._total_pinned.copy_(total, non_blocking=True)
-        self._status_pinned.copy_(self._status, non_blocking=True)
+        # the plan writes its total and the status words of this layer's routing to host memory; waiting for it sizes the result
         torch.cuda.current_stream(self.device).synchronize()
-        self._raise_on_status(self._status_pinned.tolist())
-        n = int(self._total_pinned.item())
+        self._raise_on_status(self._report[1:].view(torch.int32).tolist())
+        n = int(self._report[0])
         k, v = ops.gather_run(plan, blk.kv.dtype, g.num_key_value_heads, g.head_dim, n, max_ctas)
         return k, v, n_sel
 
