@@ -285,6 +285,19 @@ int msa_lm_moe_gemm_tc(const void* x, int64_t x_stride, int32_t x_rows, const in
                        const int32_t* off, const int32_t* tiles, int32_t max_tiles, int32_t n_out, int32_t k, int32_t act,
                        float limit, void* out, int64_t out_stride, int32_t* status, void* stream);
 
+/* ---- few rows -------------------------------------------------------------------------------------------------------
+ * out[b, i, f] = x[b, i] . w[b, f] for n <= 8 rows, bf16 operands, fp32 sums, out bf16 or fp32.  act: w holds gate rows and then
+ * as many up rows, out[f] = silu(gate_f) * up_f.  k and the strides of x and w are multiples of 8 elements, pointers 16-byte aligned.
+ * early: no kernel or copy that may still run in the stream writes w; its first part is then fetched before the previous
+ * kernel has ended. */
+typedef struct {
+  const void* x; int64_t x_stride, x_batch;
+  const void* w; int64_t w_stride, w_batch;
+  void* out; int64_t out_stride, out_batch;
+  int32_t n, w_rows, k, batch, act, early, out_dtype;
+} msa_lm_rows_gemm_args;
+int msa_lm_rows_gemm(const msa_lm_rows_gemm_args* args, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

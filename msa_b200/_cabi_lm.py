@@ -17,7 +17,8 @@ EXPORTS = ["msa_lm_residual_norm", "msa_lm_embed", "msa_lm_silu_mul", "msa_lm_so
            "msa_lm_wkv_scan", "msa_lm_wkv_chunk_supported", "msa_lm_wkv_chunk", "msa_lm_ssd_decode", "msa_lm_ssd_prep", "msa_lm_ssd_scan",
            "msa_lm_ssd_chunk_supported", "msa_lm_ssd_chunk", "msa_lm_part_norm", "msa_lm_latent_prep", "msa_lm_ring_store",
            "msa_lm_window_attn", "msa_lm_window_attn_tc_supported", "msa_lm_window_attn_tc", "msa_lm_latent_decode_supported", "msa_lm_latent_decode", "msa_lm_delta_decode", "msa_lm_delta_prep", "msa_lm_delta_prep_split", "msa_lm_delta_chunk_supported", "msa_lm_delta_chunk_workspace", "msa_lm_delta_chunk", "msa_lm_gather_rows", "msa_lm_delta_conv_store", "msa_lm_delta_scan",
-           "msa_lm_delta_out", "msa_lm_moe_topk", "msa_lm_moe_sort", "msa_lm_moe_gemm", "msa_lm_moe_gemm_tc"]
+           "msa_lm_delta_out", "msa_lm_moe_topk", "msa_lm_moe_sort", "msa_lm_moe_gemm", "msa_lm_moe_gemm_tc",
+           "msa_lm_rows_gemm"]
 
 vp, i32, i64, f32 = C.c_void_p, C.c_int32, C.c_int64, C.c_float
 
@@ -72,6 +73,13 @@ class SsdArgs(C.Structure):
                 ("dtype", i32)]
 
 
+class RowsGemmArgs(C.Structure):
+    """``msa_lm_rows_gemm_args``."""
+    _fields_ = [("x", vp), ("x_stride", i64), ("x_batch", i64), ("w", vp), ("w_stride", i64), ("w_batch", i64), ("out", vp),
+                ("out_stride", i64), ("out_batch", i64), ("n", i32), ("w_rows", i32), ("k", i32), ("batch", i32),
+                ("act", i32), ("early", i32), ("out_dtype", i32)]
+
+
 _lib = None
 
 
@@ -114,6 +122,7 @@ def lib() -> C.CDLL:
             "msa_lm_latent_decode_supported": [i32, i32],
             "msa_lm_latent_decode": [vp, i64, i64, vp, i64, i64, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp, vp, vp, vp],
             "msa_lm_moe_gemm_tc": [vp, i64, i32, vp, vp, i32, vp, vp, i32, i32, i32, i32, f32, vp, i64, vp, vp],
+            "msa_lm_rows_gemm": [C.POINTER(RowsGemmArgs), vp],
             "msa_lm_delta_decode": [dp, vp, i64, vp],
             "msa_lm_delta_prep": [dp, vp, vp, vp, vp],
             "msa_lm_delta_conv_store": [dp, vp],

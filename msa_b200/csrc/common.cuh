@@ -128,7 +128,8 @@ template <> struct Elem<__nv_bfloat16> {
 // Programmatic dependent launch (sm_90+): a kernel launched with `pdl` may start while the kernel before it in the
 // stream is still running; it must execute grid_dependency_wait() before it touches anything that kernel writes.
 // The earlier kernel lets dependents start early with grid_launch_dependents(); without that call they start when
-// it completes.  Both are no-ops in a kernel that was launched normally.
+// it completes.  Both are no-ops in a kernel that was launched normally.  What an earlier kernel writes is not read through a
+// `const __restrict__` parameter: such a load may be moved above the wait.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

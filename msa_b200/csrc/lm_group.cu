@@ -175,6 +175,7 @@ __device__ __forceinline__ void group_mma(float (&c)[4], const uint32_t (&a)[4],
 
 template <int D, int DV, bool FULL>
 __global__ void __launch_bounds__(kMmaWarps * 32, 2) group_decode_kernel(const GroupDecodeParams p) {
+  grid_launch_dependents();
   constexpr int kRows = FULL ? 16 : 8, NE = FULL ? 2 : 1;
   constexpr int kPk = D * 2 + 16, kPv = DV * 2 + 16, kStage = kMmaKeys * (kPk + kPv);
   constexpr int kVk = D / 8, kVv = DV / 8;               // 16-byte pieces of a key, of a value
@@ -201,7 +202,6 @@ __global__ void __launch_bounds__(kMmaWarps * 32, 2) group_decode_kernel(const G
       const int r = row + 8 * (e & 1);
       qa[j][e] = r < n_heads ? *reinterpret_cast<const uint32_t*>(p.q + b * p.q_row + (long long)(h0 + r) * D + 16 * j + 2 * quad + 8 * (e >> 1)) : 0u;
     }
-  grid_launch_dependents();
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem) + warp * kMmaStages * kStage;
   auto issue = [&](int blk, int stage) {
     const uint32_t kdst = base + stage * kStage, vdst = kdst + kMmaKeys * kPk;

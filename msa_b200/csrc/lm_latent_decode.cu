@@ -41,6 +41,7 @@ __device__ __forceinline__ void bulk_row(uint32_t dst, const void* src, uint32_t
 
 template <int MT, int NT, int KS>
 __global__ void __launch_bounds__(kLdThreads, 1) latent_decode_kernel(const LatentDecodeParams p) {
+  grid_launch_dependents();
   constexpr int KQ = 8 / MT, kRows = MT * 16, kPart = 72;            // slices of the reduction; floats per partial row
   constexpr int TPR = kLdThreads / kRows, KPT = kLdKeys / TPR;       // softmax: threads per row, keys per thread
   extern __shared__ __align__(16) unsigned char sm[];
@@ -80,7 +81,6 @@ __global__ void __launch_bounds__(kLdThreads, 1) latent_decode_kernel(const Late
   }
   __syncthreads();
   if (n_tiles > 0) load_tile(0);
-  grid_launch_dependents();
   const int mt = warp % MT, kq = warp / MT, ks0 = kq * KS;
   uint32_t q[KS][4];
 #pragma unroll

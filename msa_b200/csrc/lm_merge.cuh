@@ -15,11 +15,12 @@ struct MergeParams {
 // One block per (sequence, head).  Launched early (programmatic dependent launch): waits for the partial results before
 // it reads them.
 static __global__ void __launch_bounds__(128) merge_partials_kernel(const MergeParams p) {
+  grid_launch_dependents();
   const long long row = blockIdx.x;
   const int b = (int)(row / p.heads), h = (int)(row % p.heads);
   const int c = threadIdx.x * 4, splits = p.splits, cols = p.cols;
-  const float g = p.gate ? sigmoid_f(__bfloat162float(p.gate[b * p.gate_row + h])) : 1.f;   // older than the partial results
   grid_dependency_wait();
+  const float g = p.gate ? sigmoid_f(__bfloat162float(p.gate[b * p.gate_row + h])) : 1.f;
   float m = p.sink ? 0.f : -INFINITY, l = p.sink ? 1.f : 0.f;
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int s0 = 0; s0 < splits; s0 += 8) {               // eight partial results in flight; an empty one has weight 0

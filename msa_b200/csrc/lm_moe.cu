@@ -10,8 +10,10 @@ constexpr int kMoeMaxExperts = 1024;
 // PER: logits per lane.
 template <int PER>
 __global__ void __launch_bounds__(256)
-moe_topk_kernel(const float* __restrict__ logits, long long stride, const float* __restrict__ bias, int n_rows, int experts,
+moe_topk_kernel(const float* logits, long long stride, const float* __restrict__ bias, int n_rows, int experts,
                 int top, int32_t* __restrict__ idx, float* __restrict__ weight) {
+  grid_launch_dependents();
+  grid_dependency_wait();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= n_rows) return;
   float z[PER];
@@ -52,8 +54,10 @@ moe_topk_kernel(const float* __restrict__ logits, long long stride, const float*
 
 // One block: histogram, prefix sums, placement, tile list.
 __global__ void __launch_bounds__(1024)
-moe_sort_kernel(const int32_t* __restrict__ idx, int n, int top, int experts, int tile_rows, int32_t* __restrict__ src,
+moe_sort_kernel(const int32_t* idx, int n, int top, int experts, int tile_rows, int32_t* __restrict__ src,
                 int32_t* __restrict__ inv, int32_t* __restrict__ off, int32_t* __restrict__ tiles, int max_tiles) {
+  grid_launch_dependents();
+  grid_dependency_wait();
   __shared__ int s_cnt[kMoeMaxExperts], s_off[kMoeMaxExperts + 1], s_tile[kMoeMaxExperts + 1];
   for (int e = threadIdx.x; e < experts; e += blockDim.x) s_cnt[e] = 0;
   __syncthreads();
@@ -236,11 +240,11 @@ extern "C" int msa_lm_moe_topk(const float* logits, int64_t stride, const float*
   if (n_rows == 0) return MSA_OK;
   const unsigned blocks = (unsigned)((n_rows + 7) / 8);
   cudaStream_t st = (cudaStream_t)stream;
-  if (experts <= 32) moe_topk_kernel<1><<<blocks, 256, 0, st>>>(logits, stride, bias, n_rows, experts, top, idx, weight);
-  else if (experts <= 64) moe_topk_kernel<2><<<blocks, 256, 0, st>>>(logits, stride, bias, n_rows, experts, top, idx, weight);
-  else if (experts <= 128) moe_topk_kernel<4><<<blocks, 256, 0, st>>>(logits, stride, bias, n_rows, experts, top, idx, weight);
-  else if (experts <= 256) moe_topk_kernel<8><<<blocks, 256, 0, st>>>(logits, stride, bias, n_rows, experts, top, idx, weight);
-  else moe_topk_kernel<32><<<blocks, 256, 0, st>>>(logits, stride, bias, n_rows, experts, top, idx, weight);
+  if (experts <= 32) MSA_CUDA_OK(launch_kernel_pdl(moe_topk_kernel<1>, blocks, 256, 0, st, true, logits, stride, bias, n_rows, experts, top, idx, weight));
+  else if (experts <= 64) MSA_CUDA_OK(launch_kernel_pdl(moe_topk_kernel<2>, blocks, 256, 0, st, true, logits, stride, bias, n_rows, experts, top, idx, weight));
+  else if (experts <= 128) MSA_CUDA_OK(launch_kernel_pdl(moe_topk_kernel<4>, blocks, 256, 0, st, true, logits, stride, bias, n_rows, experts, top, idx, weight));
+  else if (experts <= 256) MSA_CUDA_OK(launch_kernel_pdl(moe_topk_kernel<8>, blocks, 256, 0, st, true, logits, stride, bias, n_rows, experts, top, idx, weight));
+  else MSA_CUDA_OK(launch_kernel_pdl(moe_topk_kernel<32>, blocks, 256, 0, st, true, logits, stride, bias, n_rows, experts, top, idx, weight));
   MSA_LAUNCH_OK("moe_topk_kernel");
   return MSA_OK;
 }
@@ -262,7 +266,7 @@ extern "C" int msa_lm_moe_sort(const int32_t* idx, int32_t n_rows, int32_t top, 
     MSA_LAUNCH_OK("moe_place_kernel");
     return MSA_OK;
   }
-  moe_sort_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(idx, (int)n, top, experts, tile_rows, src, inv, off, tiles, max_tiles);
+  MSA_CUDA_OK(launch_kernel_pdl(moe_sort_kernel, 1, 1024, 0, (cudaStream_t)stream, true, idx, (int)n, top, experts, tile_rows, src, inv, off, tiles, max_tiles));
   MSA_LAUNCH_OK("moe_sort_kernel");
   return MSA_OK;
 }

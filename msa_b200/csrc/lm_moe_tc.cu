@@ -58,6 +58,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  grid_launch_dependents();                       // after the allocation: no dependent takes the TMEM of a block still to come
+  grid_dependency_wait();
   const int n_work = p.max_tiles * p.n_nt;
 
   if (warp == 4) {
@@ -215,11 +217,11 @@ extern "C" int msa_lm_moe_gemm_tc(const void* x, int64_t x_stride, int32_t x_row
   if (act) {
     static DeviceSmem s1{};
     MSA_OK_OR_RETURN(ensure_dynamic_smem(moe_gemm_tc_kernel<true>, kMtSmem, s1));
-    moe_gemm_tc_kernel<true><<<grid, kMtThreads, kMtSmem, (cudaStream_t)stream>>>(mx, mw, p);
+    MSA_CUDA_OK(launch_kernel_pdl(moe_gemm_tc_kernel<true>, grid, kMtThreads, kMtSmem, (cudaStream_t)stream, true, mx, mw, p));
   } else {
     static DeviceSmem s0{};
     MSA_OK_OR_RETURN(ensure_dynamic_smem(moe_gemm_tc_kernel<false>, kMtSmem, s0));
-    moe_gemm_tc_kernel<false><<<grid, kMtThreads, kMtSmem, (cudaStream_t)stream>>>(mx, mw, p);
+    MSA_CUDA_OK(launch_kernel_pdl(moe_gemm_tc_kernel<false>, grid, kMtThreads, kMtSmem, (cudaStream_t)stream, true, mx, mw, p));
   }
   MSA_LAUNCH_OK("moe_gemm_tc_kernel");
   return MSA_OK;

@@ -117,6 +117,7 @@ __global__ void residual_norm_kernel(const ResNormParams p) {
 // before the first reduction): a decode step has few rows and waits for latency, not for bandwidth.
 template <typename T, typename TY>
 __global__ void __launch_bounds__(1024) residual_norm_once_kernel(const ResNormParams p) {
+  grid_launch_dependents();
   __shared__ float s_part[32];
   const long long r = blockIdx.x;
   const long long rb = p.rows ? p.rows[r] : r;
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(1024) residual_norm_once_kernel(const ResNormP
 // V = 4: rows and pointers are 4-element aligned; V = 1: any width.
 template <typename T, int V>
 __global__ void embed_kernel(const msa_lm_embed_args a) {
+  grid_launch_dependents();
   extern __shared__ float s_row[];
   __shared__ float s_part[32];
   const long long r = blockIdx.x;
@@ -245,6 +247,7 @@ __global__ void __launch_bounds__(256) softcap_kernel(float* x, long long n, flo
 // so that a product over both keeps 16 significant bits.
 template <typename T>
 __global__ void __launch_bounds__(256) tanh_split_kernel(const float* __restrict__ x, int cols, int parts, long long n, T* __restrict__ out) {
+  grid_launch_dependents();
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
     const long long r = i / cols;
     const int c = (int)(i - r * cols);
@@ -263,6 +266,7 @@ template <typename T, int V>
 __global__ void token_shift_kernel(const T* __restrict__ h, const float* __restrict__ mu, int n_mix, int n_tok, int width,
                                    const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ slot,
                                    const int32_t* __restrict__ start, const int32_t* __restrict__ cu, T* shift, T* __restrict__ out) {
+  grid_launch_dependents();
   const long long r = blockIdx.x;
   const int s = tok_seq[r], t = (int)r - cu[s];
   T* state = shift + (long long)slot[s] * width;

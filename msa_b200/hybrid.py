@@ -72,7 +72,7 @@ class Mixer:
     """``mix`` goes from the input projections (one product with ``w_in``) to the input of the output product (``w_o``)."""
 
     def forward(self, h: torch.Tensor, step, cache: SequenceStateCache, run: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        y = self.mix(K.matmul(h, self.w_in), step, cache, run)
+        y = self.mix(K.matmul(h, self.w_in, weight=True), step, cache, run)
         return y if out is None else out.copy_(y)
 
 
@@ -197,7 +197,7 @@ class GroupedAttention(Mixer):
         return RingSpec(s.kv_heads * (self.dim + self.vdim), s.window, s.channels, s.taps)
 
     def forward(self, h, step, cache, run, out=None):
-        return self.mix(K.matmul(h, self.w_in), step, cache, run, out)
+        return self.mix(K.matmul(h, self.w_in, weight=True), step, cache, run, out)
 
     def mix(self, proj: torch.Tensor, step, cache: SequenceStateCache, run: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         s, n, nd = self.spec, step.n_tok, step.n_decode
@@ -254,9 +254,9 @@ class Wkv(Mixer):
 
     def forward(self, h, step, cache, run, out=None):
         mixes = K.token_shift(h, self.mu, step, cache.shift[run])
-        rkvg = torch.bmm(mixes[:4], self.w_in.transpose(1, 2))
-        low = K.tanh_split(K.matmul(mixes[4], self.w1, torch.float32), h.dtype, self.parts)
-        decay = K.matmul(low, self.w2, torch.float32)
+        rkvg = K.bmm(mixes[:4], self.w_in)
+        low = K.tanh_split(K.matmul(mixes[4], self.w1, torch.float32, weight=True), h.dtype, self.parts)
+        decay = K.matmul(low, self.w2, torch.float32, weight=True)
         if out is None:
             out = torch.empty((h.shape[0], self.spec.inner), dtype=h.dtype, device=h.device)
         return K.wkv_mix(rkvg, decay, self.spec, self, cache.state[run], self.eps, step, out)
@@ -283,7 +283,7 @@ class Mamba2(Mixer):
     def forward(self, h, step, cache, run, out=None):
         if out is None:
             out = torch.empty((h.shape[0], self.spec.inner), dtype=h.dtype, device=h.device)
-        return K.ssd_mix(K.matmul(h, self.w_in), self.spec, self, cache.conv[run], cache.state[run], self.eps, step, out)
+        return K.ssd_mix(K.matmul(h, self.w_in, weight=True), self.spec, self, cache.conv[run], cache.state[run], self.eps, step, out)
 
 
 class DenseFeedForward:
@@ -293,10 +293,10 @@ class DenseFeedForward:
         self.w_down = w.matrix(prefix + "down", width, spec.ff)
 
     def activate(self, h: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        return K.silu_mul(K.matmul(h, self.w_gate_up), self.ff, out)
+        return K.matmul_silu(h, self.w_gate_up, self.ff, out)
 
     def branch(self, h: torch.Tensor) -> dict:
-        return dict(y=K.matmul(self.activate(h), self.w_down))
+        return dict(y=K.matmul(self.activate(h), self.w_down, weight=True))
 
 
 class MixtureFeedForward:
@@ -318,7 +318,7 @@ class MixtureFeedForward:
 
     def branch(self, h: torch.Tensor) -> dict:
         s, n = self.spec, h.shape[0]
-        idx, mix = K.moe_topk(K.matmul(h, self.router, torch.float32), self.bias, s.top)
+        idx, mix = K.moe_topk(K.matmul(h, self.router, torch.float32, weight=True), self.bias, s.top)
         if self.tc:
             src, inv, off, tiles = K.moe_sort(idx, s.experts, K.MOE_TC_TILE_ROWS)
             if n * s.top >= s.experts * K.MOE_GATHER_ROWS:
@@ -428,7 +428,7 @@ class HybridForCausalLM:
         """Runs the step's tokens from the states in ``cache`` and advances those; fp32 logits ``[wanted, vocab]``."""
         x = (self._run_sandwich if self.config.structure.block == "sandwich" else self._run_parallel)(step, cache)
         h = K.residual_norm(x, None, None, self.final_norm, self.config.eps, self.dtype, rows=step.want_rows)
-        logits = K.matmul(h, self.head, torch.float32)
+        logits = K.matmul(h, self.head, torch.float32, weight=True)
         return logits if self.config.logit_softcap is None else K.softcap(logits, self.config.logit_softcap)
 
     def _pair_args(self, step, cache) -> dict:
@@ -451,7 +451,7 @@ class HybridForCausalLM:
             layer.mixer.forward(h[0], step, cache, k, act[:, :layer.cols])
             if layer.ff is not None:
                 layer.ff.activate(h[1], act[:, layer.cols:])
-            y = K.matmul(act, layer.w_out)
+            y = K.matmul(act, layer.w_out, weight=True)
             w1, w2 = norms(k + 1)
             if self.on_layer is not None:
                 K.residual_norm(x, y, None, None, eps, dt, x_out=x, want_h=False)
@@ -468,12 +468,12 @@ class HybridForCausalLM:
         for k, (kind, run, i, t) in enumerate(self._program[:-1]):
             nxt = self._next_norm(k + 1)
             if kind == "enter":
-                y = K.matmul(cat, self.loop_in, torch.float32)
+                y = K.matmul(cat, self.loop_in, torch.float32, weight=True)
                 h = K.residual_norm(self.loop_step[t], y, None, nxt, eps, dt, x_out=x, broadcast=True)
                 continue
             layer = self.layers[i]
             if kind == "mix":
-                branch, wb = dict(y=K.matmul(layer.mixer.forward(h, step, cache, run), layer.mixer.w_o)), layer.norm1b
+                branch, wb = dict(y=K.matmul(layer.mixer.forward(h, step, cache, run), layer.mixer.w_o, weight=True)), layer.norm1b
             else:
                 branch, wb = layer.ff.branch(h), layer.norm2b
             left = cat if self._program[k + 1][0] == "enter" else None

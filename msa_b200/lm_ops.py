@@ -16,11 +16,53 @@ def _rows(t: torch.Tensor) -> int:
     return t.stride(0)
 
 
-def matmul(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """``x @ w.T`` with 32-bit accumulation; ``out_dtype`` float32 keeps the accumulator's precision."""
+ROWS_GEMM_MAX = 8            # rows of x the kernel takes (one tile); a decode step of 16 sequences is no faster by two tiles
+
+
+def few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``x @ w.T`` ([..., n, k] by [..., rows, k]) is a product for ``msa_lm_rows_gemm``: bf16, few rows, and rows on
+    16-byte boundaries."""
+    if not 0 < x.shape[-2] <= ROWS_GEMM_MAX:
+        return False
+    ok = lambda t: t.is_cuda and t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in t.stride()[:-1])
+    return x.shape[-1] % 8 == 0 and ok(x) and ok(w)
+
+
+def rows_gemm(x, w, out, *, act: bool) -> torch.Tensor:
+    """One launch of ``msa_lm_rows_gemm``.  ``w`` is a weight: no kernel of the running step writes it."""
+    batch = x.shape[0] if x.dim() == 3 else 1
+    step = lambda t: t.stride(0) if t.dim() == 3 else 0
+    args = A.RowsGemmArgs(x=x.data_ptr(), x_stride=x.stride(-2), x_batch=step(x), w=w.data_ptr(), w_stride=w.stride(-2), w_batch=step(w),
+                          out=out.data_ptr(), out_stride=out.stride(-2), out_batch=step(out), n=x.shape[-2], w_rows=w.shape[-2], k=w.shape[-1],
+                          batch=batch, act=1 if act else 0, early=1, out_dtype=A.dtype_code(out.dtype))
+    A.call("msa_lm_rows_gemm", C.byref(args), A.stream_ptr(x.device))
+    return out
+
+
+def matmul(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, weight: bool = False) -> torch.Tensor:
+    """``x @ w.T`` with 32-bit accumulation; ``out_dtype`` float32 keeps the accumulator's precision.  ``weight``: nothing still in
+    the stream writes ``w``; few rows then take the package's own kernel."""
+    if weight and few_rows(x, w):
+        return rows_gemm(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device), act=False)
     if out_dtype is None or out_dtype == x.dtype:
         return torch.mm(x, w.t())
     return torch.mm(x, w.t(), out_dtype=out_dtype)
+
+
+def matmul_silu(x: torch.Tensor, w: torch.Tensor, ff: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``silu(x @ gate.T) * (x @ up.T)``; ``w``, a weight, holds the ``ff`` gate rows and then the up rows."""
+    if few_rows(x, w):
+        if out is None:
+            out = torch.empty((x.shape[0], ff), dtype=x.dtype, device=x.device)
+        return rows_gemm(x, w, out, act=True)
+    return silu_mul(matmul(x, w), ff, out)
+
+
+def bmm(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``x[b] @ w[b].T``; ``w`` is a weight."""
+    if few_rows(x, w):
+        return rows_gemm(x, w, torch.empty(x.shape[:2] + w.shape[1:2], dtype=x.dtype, device=x.device), act=False)
+    return torch.bmm(x, w.transpose(1, 2))
 
 
 def embed(table, token, w_next, eps, cat: Optional[torch.Tensor] = None, cat_both: bool = False, status=None, *, w_next2=None,
