@@ -38,8 +38,8 @@ __device__ __forceinline__ float branch1(const ResNormParams& p, long long r, in
   return a;
 }
 
-// V = 4: every row pointer is 4-element aligned and width % 4 == 0; V = 1: any width.
-template <typename T, typename TY, int V>
+// Any width and alignment, one element at a time.
+template <typename T, typename TY>
 __global__ void residual_norm_kernel(const ResNormParams p) {
   extern __shared__ float s_row[];   // [width]
   __shared__ float s_part[32];
@@ -52,64 +52,28 @@ __global__ void residual_norm_kernel(const ResNormParams p) {
   float scale_b = 1.f;
   if (p.y && p.w_branch) {
     float ss = 0.f;
-    for (int i = threadIdx.x * V; i < p.width; i += nt * V) {
-      if constexpr (V == 4) {
-        const float4 b = branch4<TY>(p, r, i);
-        store4(s_row + i, b);
-        ss += b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
-      } else {
-        const float b = branch1<TY>(p, r, i);
-        s_row[i] = b;
-        ss += b * b;
-      }
+    for (int i = threadIdx.x; i < p.width; i += nt) {
+      const float b = branch1<TY>(p, r, i);
+      s_row[i] = b;
+      ss += b * b;
     }
     scale_b = 1.f / sqrtf(block_sum(ss, s_part) / (float)p.width + p.eps);
   }
   float ss = 0.f;
-  for (int i = threadIdx.x * V; i < p.width; i += nt * V) {   // every thread revisits the elements it stored above
-    if constexpr (V == 4) {
-      float4 x = p.base ? load4(p.base + rb * p.base_stride + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (p.y) {
-        if (p.w_branch) {
-          const float4 b = load4(s_row + i), w = load4(p.w_branch + i);
-          x.x += b.x * scale_b * w.x; x.y += b.y * scale_b * w.y; x.z += b.z * scale_b * w.z; x.w += b.w * scale_b * w.w;
-        } else {
-          const float4 b = branch4<TY>(p, r, i);
-          x.x += b.x; x.y += b.y; x.z += b.z; x.w += b.w;
-        }
-      }
-      if (p.add) {
-        const float4 b = load4(p.add + r * p.width + i);
-        x.x += b.x; x.y += b.y; x.z += b.z; x.w += b.w;
-      }
-      if (p.x_out) store4(p.x_out + r * p.width + i, x);
-      if (cat) store4(cat + r * p.cat_stride + i, x);
-      store4(s_row + i, x);
-      ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
-    } else {
-      float x = p.base ? p.base[rb * p.base_stride + i] : 0.f;
-      if (p.y) x += p.w_branch ? s_row[i] * scale_b * p.w_branch[i] : branch1<TY>(p, r, i);
-      if (p.add) x += p.add[r * p.width + i];
-      if (p.x_out) p.x_out[r * p.width + i] = x;
-      if (cat) cat[r * p.cat_stride + i] = from_f<T>(x);
-      s_row[i] = x;
-      ss += x * x;
-    }
+  for (int i = threadIdx.x; i < p.width; i += nt) {   // every thread revisits the elements it stored above
+    float x = p.base ? p.base[rb * p.base_stride + i] : 0.f;
+    if (p.y) x += p.w_branch ? s_row[i] * scale_b * p.w_branch[i] : branch1<TY>(p, r, i);
+    if (p.add) x += p.add[r * p.width + i];
+    if (p.x_out) p.x_out[r * p.width + i] = x;
+    if (cat) cat[r * p.cat_stride + i] = from_f<T>(x);
+    s_row[i] = x;
+    ss += x * x;
   }
   if (!h_out) return;
   const float inv = 1.f / sqrtf(block_sum(ss, s_part) / (float)p.width + p.eps);
-  for (int i = threadIdx.x * V; i < p.width; i += nt * V) {
-    if constexpr (V == 4) {
-      const float4 x = load4(s_row + i), w = load4(p.w_next + i);
-      store4(h_out + r * p.width + i, make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w));
-      if (h_out2) {
-        const float4 w2 = load4(p.w_next2 + i);
-        store4(h_out2 + r * p.width + i, make_float4(x.x * inv * w2.x, x.y * inv * w2.y, x.z * inv * w2.z, x.w * inv * w2.w));
-      }
-    } else {
-      h_out[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next[i]);
-      if (h_out2) h_out2[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next2[i]);
-    }
+  for (int i = threadIdx.x; i < p.width; i += nt) {
+    h_out[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next[i]);
+    if (h_out2) h_out2[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next2[i]);
   }
 }
 
@@ -165,6 +129,75 @@ __global__ void __launch_bounds__(1024) residual_norm_once_kernel(const ResNormP
   if (on) store4(reinterpret_cast<T*>(p.h_out) + r * p.width + i, make_float4(x.x * inv * wn.x, x.y * inv * wn.y, x.z * inv * wn.z, x.w * inv * wn.w));
   if (on && p.h_out2)
     store4(reinterpret_cast<T*>(p.h_out2) + r * p.width + i, make_float4(x.x * inv * wn2.x, x.y * inv * wn2.y, x.z * inv * wn2.z, x.w * inv * wn2.w));
+}
+
+// The same for many rows: 128 threads per 2048 columns, four vectors each.  Bound by HBM (base and stream in 32 bits, branch and
+// norm in 16: 12 bytes per element), so as many loads as possible are in flight: all of a row's are issued before the first
+// reduction, and rows need few enough threads and registers for ten of them on an SM.  One row per 256 threads through shared memory,
+// one vector at a time, took 47.1 us for 6236 x 2048 from a cold L2 (bytes at HBM rate: 23), this takes 34.8.
+template <typename T, typename TY>
+__global__ void __launch_bounds__(768, 1) residual_norm_rows_kernel(const ResNormParams p) {
+  constexpr int E = 4;
+  __shared__ float s_part[2][32];
+  const long long r = blockIdx.x;
+  const long long rb = p.rows ? p.rows[r] : r;
+  const int nt = blockDim.x, lane = threadIdx.x & 31, warps = nt >> 5;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto at = [&](int e) { return (e * nt + (int)threadIdx.x) * 4; };
+  auto sum = [&](float v, float* part) {             // every thread gets it; the two reductions have a buffer each
+    v = warp_sum_f(v);
+    if (lane == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float t = 0.f;
+    for (int i = 0; i < warps; ++i) t += part[i];
+    return t;
+  };
+  float4 x[E], b[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) x[e] = p.base && at(e) < p.width ? load4(p.base + rb * p.base_stride + at(e)) : zero;
+  if (p.y) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) b[e] = at(e) < p.width ? branch4<TY>(p, r, at(e)) : zero;
+    if (p.w_branch) {
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < E; ++e) ss += b[e].x * b[e].x + b[e].y * b[e].y + b[e].z * b[e].z + b[e].w * b[e].w;
+      const float sc = 1.f / sqrtf(sum(ss, s_part[0]) / (float)p.width + p.eps);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const float4 w = at(e) < p.width ? load4(p.w_branch + at(e)) : zero;
+        x[e].x += b[e].x * sc * w.x; x[e].y += b[e].y * sc * w.y; x[e].z += b[e].z * sc * w.z; x[e].w += b[e].w * sc * w.w;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) { x[e].x += b[e].x; x[e].y += b[e].y; x[e].z += b[e].z; x[e].w += b[e].w; }
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    if (at(e) >= p.width) continue;
+    if (p.add) {
+      const float4 a = load4(p.add + r * p.width + at(e));
+      x[e].x += a.x; x[e].y += a.y; x[e].z += a.z; x[e].w += a.w;
+    }
+    if (p.x_out) store4(p.x_out + r * p.width + at(e), x[e]);
+    if (p.cat_out) store4(reinterpret_cast<T*>(p.cat_out) + r * p.cat_stride + at(e), x[e]);
+    ss += x[e].x * x[e].x + x[e].y * x[e].y + x[e].z * x[e].z + x[e].w * x[e].w;
+  }
+  if (!p.h_out) return;
+  const float inv = 1.f / sqrtf(sum(ss, s_part[1]) / (float)p.width + p.eps);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    if (at(e) >= p.width) continue;
+    const float4 w = load4(p.w_next + at(e));
+    store4(reinterpret_cast<T*>(p.h_out) + r * p.width + at(e), make_float4(x[e].x * inv * w.x, x[e].y * inv * w.y, x[e].z * inv * w.z, x[e].w * inv * w.w));
+    if (p.h_out2) {
+      const float4 w2 = load4(p.w_next2 + at(e));
+      store4(reinterpret_cast<T*>(p.h_out2) + r * p.width + at(e),
+             make_float4(x[e].x * inv * w2.x, x[e].y * inv * w2.y, x[e].z * inv * w2.z, x[e].w * inv * w2.w));
+    }
+  }
 }
 
 // V = 4: rows and pointers are 4-element aligned; V = 1: any width.
@@ -292,19 +325,47 @@ __global__ void token_shift_kernel(const T* __restrict__ h, const float* __restr
   }
 }
 
+// V = 8: 16-byte loads, two rows' in flight per thread (bf16); V = 4: 8- or 16-byte ones; V = 1: any alignment.  A block takes
+// 256 * V columns of two rows.  Bound by HBM; with 8-byte loads, an index division by a run-time number and full-accuracy
+// exponentials in front of the rounding to bf16 6236 x 6144 took 63.5 us from a cold L2 (bytes at HBM rate: 34.6), now 41.0.
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-lm_silu_mul_kernel(const T* __restrict__ gu, long long stride, int ff, long long n_rows, T* __restrict__ out, long long out_stride) {
-  const int per_row = ff / V;
-  const long long total = n_rows * per_row;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / per_row;
-    const int j = (int)(i % per_row) * V;
-    if constexpr (V == 4) {
-      const float4 g = load4(gu + r * stride + j), u = load4(gu + r * stride + ff + j);
-      store4(out + r * out_stride + j, make_float4(silu_f(g.x) * u.x, silu_f(g.y) * u.y, silu_f(g.z) * u.z, silu_f(g.w) * u.w));
-    } else {
-      out[r * out_stride + j] = from_f<T>(silu_f(to_f(gu[r * stride + j])) * to_f(gu[r * stride + ff + j]));
+lm_silu_mul_kernel(const T* __restrict__ gu, long long stride, int ff, int n_rows, T* __restrict__ out, long long out_stride) {
+  const int j = (blockIdx.x * 256 + threadIdx.x) * V;
+  if (j >= ff) return;
+  const long long r0 = 2ll * blockIdx.y;
+  const int rows = r0 + 1 < n_rows ? 2 : 1;
+  if constexpr (V == 8) {
+    uint4 g[2], u[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (k < rows) {
+        g[k] = *reinterpret_cast<const uint4*>(gu + (r0 + k) * stride + j);
+        u[k] = *reinterpret_cast<const uint4*>(gu + (r0 + k) * stride + ff + j);
+      }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (k < rows) {
+        const __nv_bfloat162 *a = reinterpret_cast<const __nv_bfloat162*>(&g[k]), *b = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
+        uint4 o;
+        __nv_bfloat162* c = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 x = __bfloat1622float2(a[i]), y = __bfloat1622float2(b[i]);
+          c[i] = __floats2bfloat162_rn(silu_act<T>(x.x) * y.x, silu_act<T>(x.y) * y.y);
+        }
+        *reinterpret_cast<uint4*>(out + (r0 + k) * out_stride + j) = o;
+      }
+  } else {
+    for (int k = 0; k < rows; ++k) {
+      const T *g = gu + (r0 + k) * stride + j, *u = g + ff;
+      T* o = out + (r0 + k) * out_stride + j;
+      if constexpr (V == 4) {
+        const float4 x = load4(g), y = load4(u);
+        store4(o, make_float4(silu_act<T>(x.x) * y.x, silu_act<T>(x.y) * y.y, silu_act<T>(x.z) * y.z, silu_act<T>(x.w) * y.w));
+      } else {
+        *o = from_f<T>(silu_act<T>(to_f(*g)) * to_f(*u));
+      }
     }
   }
 }
@@ -335,8 +396,6 @@ extern "C" int msa_lm_residual_norm(const float* base, int64_t base_stride, cons
   const bool v4 = width % 4 == 0 && base_stride % 4 == 0 && (!y || y_stride % 4 == 0) && (!cat_out || cat_stride % 4 == 0) &&
                   vec4_ok(base, 4) && vec4_ok(y, ey) && vec4_ok(w_branch, 4) && vec4_ok(w_next, 4) && vec4_ok(x_out, 4) &&
                   vec4_ok(h_out, e) && vec4_ok(cat_out, e) && vec4_ok(add, 4) && vec4_ok(w_next2, 4) && vec4_ok(h_out2, e);
-  const size_t smem = (size_t)width * 4;
-  const int threads = row_threads(width);
   cudaStream_t st = (cudaStream_t)stream;
   if (v4 && width <= 4096 && n_rows <= 512) {
     const int once = (width / 4 + 31) / 32 * 32;
@@ -347,14 +406,20 @@ extern "C" int msa_lm_residual_norm(const float* base, int64_t base_stride, cons
     MSA_LAUNCH_OK("residual_norm_once_kernel");
     return MSA_OK;
   }
+  if (v4) {                                            // width <= 12000: at most 24 warps
+    const int row = (width + 511) / 512 * 32;
+    MSA_LM_DISPATCH(dtype, {
+      if (y && y_dtype == MSA_BF16) residual_norm_rows_kernel<T, __nv_bfloat16><<<n_rows, row, 0, st>>>(p);
+      else residual_norm_rows_kernel<T, float><<<n_rows, row, 0, st>>>(p);
+    });
+    MSA_LAUNCH_OK("residual_norm_rows_kernel");
+    return MSA_OK;
+  }
+  const size_t smem = (size_t)width * 4;
+  const int threads = row_threads(width);
   MSA_LM_DISPATCH(dtype, {
-    if (y && y_dtype == MSA_BF16) {
-      if (v4) residual_norm_kernel<T, __nv_bfloat16, 4><<<n_rows, threads, smem, st>>>(p);
-      else residual_norm_kernel<T, __nv_bfloat16, 1><<<n_rows, threads, smem, st>>>(p);
-    } else {
-      if (v4) residual_norm_kernel<T, float, 4><<<n_rows, threads, smem, st>>>(p);
-      else residual_norm_kernel<T, float, 1><<<n_rows, threads, smem, st>>>(p);
-    }
+    if (y && y_dtype == MSA_BF16) residual_norm_kernel<T, __nv_bfloat16><<<n_rows, threads, smem, st>>>(p);
+    else residual_norm_kernel<T, float><<<n_rows, threads, smem, st>>>(p);
   });
   MSA_LAUNCH_OK("residual_norm_kernel");
   return MSA_OK;
@@ -426,12 +491,21 @@ extern "C" int msa_lm_silu_mul(const void* gu, int64_t gu_stride, int32_t n_rows
   if (n_rows == 0) return MSA_OK;
   const int e = (int)dtype_size(dtype);
   const bool v4 = ff % 4 == 0 && gu_stride % 4 == 0 && out_stride % 4 == 0 && vec4_ok(gu, e) && vec4_ok(out, e);
-  const long long total = (long long)n_rows * (v4 ? ff / 4 : ff);
-  const int grid = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-  MSA_LM_DISPATCH(dtype, {
-    if (v4) lm_silu_mul_kernel<T, 4><<<grid, 256, 0, (cudaStream_t)stream>>>((const T*)gu, gu_stride, ff, n_rows, (T*)out, out_stride);
-    else lm_silu_mul_kernel<T, 1><<<grid, 256, 0, (cudaStream_t)stream>>>((const T*)gu, gu_stride, ff, n_rows, (T*)out, out_stride);
-  });
+  const bool v8 = dtype == MSA_BF16 && ff % 8 == 0 && gu_stride % 8 == 0 && out_stride % 8 == 0 && aligned16(gu) && aligned16(out);
+  const int per = 256 * (v8 ? 8 : (v4 ? 4 : 1));
+  for (int r = 0; r < n_rows; r += 131070) {           // the second axis of a grid ends at 65535 pairs of rows
+    const int rows = n_rows - r < 131070 ? n_rows - r : 131070;
+    const dim3 grid((unsigned)((ff + per - 1) / per), (unsigned)((rows + 1) / 2));
+    MSA_LM_DISPATCH(dtype, {
+      const T* from = (const T*)gu + r * gu_stride;
+      T* to = (T*)out + r * out_stride;
+      if constexpr (sizeof(T) == 2) {
+        if (v8) { lm_silu_mul_kernel<T, 8><<<grid, 256, 0, (cudaStream_t)stream>>>(from, gu_stride, ff, rows, to, out_stride); continue; }
+      }
+      if (v4) lm_silu_mul_kernel<T, 4><<<grid, 256, 0, (cudaStream_t)stream>>>(from, gu_stride, ff, rows, to, out_stride);
+      else lm_silu_mul_kernel<T, 1><<<grid, 256, 0, (cudaStream_t)stream>>>(from, gu_stride, ff, rows, to, out_stride);
+    });
+  }
   MSA_LAUNCH_OK("lm_silu_mul_kernel");
   return MSA_OK;
 }
