@@ -60,6 +60,8 @@ int msa_lm_silu_mul(const void* gu, int64_t gu_stride, int32_t n_rows, int32_t f
 
 /* x = cap * tanh(x / cap) in place. */
 int msa_lm_softcap(float* x, int64_t n, float cap, void* stream);
+/* out[r] = place of the largest of the cols entries of row r (NaN counts as the largest, equals go to the lowest place). */
+int msa_lm_argmax(const float* x, int64_t stride, int32_t n_rows, int32_t cols, int32_t* out, void* stream);
 
 /* out [n_rows, parts, cols]: tanh(x [n_rows, cols]) as a sum of `parts` numbers of type dtype. */
 int msa_lm_tanh_split(const float* x, int32_t n_rows, int32_t cols, int32_t parts, void* out, int32_t dtype, void* stream);

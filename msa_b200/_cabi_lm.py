@@ -18,7 +18,7 @@ EXPORTS = ["msa_lm_residual_norm", "msa_lm_embed", "msa_lm_silu_mul", "msa_lm_so
            "msa_lm_ssd_chunk_supported", "msa_lm_ssd_chunk", "msa_lm_part_norm", "msa_lm_latent_prep", "msa_lm_ring_store",
            "msa_lm_window_attn", "msa_lm_window_attn_tc_supported", "msa_lm_window_attn_tc", "msa_lm_latent_decode_supported", "msa_lm_latent_decode", "msa_lm_delta_decode", "msa_lm_delta_prep", "msa_lm_delta_prep_split", "msa_lm_delta_chunk_supported", "msa_lm_delta_chunk_workspace", "msa_lm_delta_chunk", "msa_lm_gather_rows", "msa_lm_delta_conv_store", "msa_lm_delta_scan",
            "msa_lm_delta_out", "msa_lm_moe_topk", "msa_lm_moe_sort", "msa_lm_moe_gemm", "msa_lm_moe_gemm_tc",
-           "msa_lm_rows_gemm"]
+           "msa_lm_rows_gemm", "msa_lm_argmax"]
 
 vp, i32, i64, f32 = C.c_void_p, C.c_int32, C.c_int64, C.c_float
 
@@ -97,6 +97,7 @@ def lib() -> C.CDLL:
             "msa_lm_embed": [C.POINTER(EmbedArgs), vp],
             "msa_lm_silu_mul": [vp, i64, i32, i32, vp, i64, i32, vp],
             "msa_lm_softcap": [vp, i64, f32, vp],
+            "msa_lm_argmax": [vp, i64, i32, i32, vp, vp],
             "msa_lm_tanh_split": [vp, i32, i32, i32, vp, i32, vp],
             "msa_lm_token_shift": [vp, vp, i32, i32, i32, vp, vp, vp, vp, vp, vp, i32, vp],
             "msa_lm_group_prep": [C.POINTER(GroupArgs), vp],

@@ -541,7 +541,7 @@ class GraphedDecode:
 
         def body():
             logits = model.step(self.tables, cache)
-            return logits, logits.argmax(dim=-1).to(torch.int32)
+            return logits, K.argmax(logits)
         self.tables.fill([0] * n, [0] * n, [cache.scratch] * n)
         with torch.cuda.stream(side):
             for _ in range(2):

@@ -128,6 +128,14 @@ def softcap(logits: torch.Tensor, cap: float) -> torch.Tensor:
     return logits
 
 
+def argmax(logits: torch.Tensor) -> torch.Tensor:
+    """``logits.argmax(-1)`` of fp32 rows as int32."""
+    A.need_cuda(logits)
+    out = torch.empty(logits.shape[0], dtype=torch.int32, device=logits.device)
+    A.call("msa_lm_argmax", A.ptr(logits), _rows(logits), logits.shape[0], logits.shape[1], A.ptr(out), A.stream_ptr(logits.device))
+    return out
+
+
 def token_shift(h, mu, step, shift):
     """``[mixes, n, width]``: every row of ``h`` mixed with its sequence's previous one (``shift`` keeps the last rows)."""
     A.need_cuda(h, mu)

@@ -63,3 +63,16 @@ def test_silu_mul(rows, ff, offset, dtype):
     tiny = 2.0 ** -100          # where 1 + e^-z passes 2^126 (z < -87) the quotient may be 0: less than 2^-118 of the other factor
     assert near(K.silu_mul(gu, ff, out[:, offset:offset + ff]), want, want.abs() + tiny, dtype == BF16)
     assert (out[:, :offset] == 7).all() and (out[:, offset + ff:] == 7).all()
+
+
+@pytest.mark.parametrize("rows,cols,pad", [(1, 1, 0), (3, 31, 0), (2, 4097, 3), (8, 32768, 0), (2, 32768, 1), (3, 151936, 0), (2, 36868, 4)])
+def test_argmax(rows, cols, pad):
+    from msa_b200 import lm_ops as K
+    x = randn(rows, cols + pad, seed=cols)[:, :cols]
+    assert torch.equal(K.argmax(x), x.argmax(-1).to(torch.int32))
+    top = x.max() + 1
+    x[:, cols // 3] = x[:, cols // 2] = x[:, cols - 1] = top              # equals: the lowest place
+    assert K.argmax(x).tolist() == [cols // 3] * rows
+    x[-1, cols // 2], x[-1, cols - 1] = float("nan"), float("nan")
+    assert K.argmax(x).tolist() == [cols // 3] * (rows - 1) + [cols // 2]
+    assert K.argmax(torch.full_like(x, -float("inf"))).tolist() == [0] * rows
