@@ -544,6 +544,18 @@ int msa_silu_mul_parts(const void* gate, int64_t gate_stride, const void* up, in
 int msa_rope_table(const int64_t* positions, const float* inv_freq, int32_t n, int32_t half, float scaling, void* cos_table,
                    void* sin_table, void* stream);
 
+/* Before a batch of questions is assembled: kv_lengths[b] = t_len + n_sel[b] + number of valid tokens of row b; report = {longest,
+ * whether every row's valid tokens are consecutive, status[0] (0 without status)}.  valid: bytes [n_rows, row_len]. */
+int msa_question_plan(const uint8_t* valid, int32_t n_rows, int32_t row_len, const int64_t* n_sel, int32_t t_len, const int32_t* status,
+                      int64_t* kv_lengths, int32_t* report, void* stream);
+
+/* Segments of a block of documents [n_rows, row_len]: the valid tokens with doc_ids > 0 in segments of consecutive listed tokens of one
+ * row and id, and those with doc_ids == -2 in one segment per row.  tok_*: n_rows * row_len places, off_*: one more; report =
+ * {tokens, segments, longest, every segment a run of memory} of the documents, {tokens, segments, longest} of the template, and the
+ * number of tokens with doc_ids == -2, valid or not. */
+int msa_segments(const int64_t* doc_ids, const uint8_t* valid, int32_t n_rows, int32_t row_len, int32_t* tok_docs, int32_t* off_docs,
+                 int32_t* tok_template, int32_t* off_template, int32_t* report, void* stream);
+
 /* ---------------------------------------------------------------------------------------
  * Decode attention without any allocation.  (No counterpart in the reference: this entry
  * point exists for hosts of this library that cannot allocate device memory when a decode

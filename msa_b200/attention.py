@@ -149,25 +149,12 @@ class MemorySparseAttention(Qwen3Attention):
         key = (doc_ids.data_ptr(), attention_mask.data_ptr(), tuple(doc_ids.shape))
         hit = cache.meta.get("_msa_b200_segments")
         if hit is None or hit[0] != key:
-            s = doc_ids.shape[1]
             valid = attention_mask == 1
-
-            def table(mask, ids):
-                tok = torch.nonzero(mask.flatten()).flatten()
-                if tok.numel() == 0:
-                    return tok.to(torch.int32), torch.zeros(1, dtype=torch.int32, device=tok.device), 0, True
-                gid = (tok // s) * (int(ids.max().item()) + 2) + ids.flatten()[tok]
-                _, counts = torch.unique_consecutive(gid, return_counts=True)
-                off = F.pad(counts.cumsum(0), (1, 0))
-                first, last = tok[off[:-1]], tok[off[1:] - 1]
-                runs = bool(((last - first == counts - 1) & (first // s == last // s)).all().item())
-                return tok.to(torch.int32), off.to(torch.int32), int(counts.max().item()), runs
-            listed = (doc_ids > 0) & valid
-            docs = table(listed, doc_ids)
+            docs, template, n_template = ops.segments(doc_ids, valid)
             spans = None
             if not docs[3] and docs[0].numel() > 0:      # masked tokens inside documents: spans + bitmap for the tcgen05 kernel
-                spans = ops.document_spans(docs[0], docs[1]) + (ops.token_bitmap(listed),)
-            hit = (key, docs, table((doc_ids == -2) & valid, torch.zeros_like(doc_ids)), spans, int((doc_ids == -2).sum()))
+                spans = ops.document_spans(docs[0], docs[1]) + (ops.token_bitmap((doc_ids > 0) & valid),)
+            hit = (key, docs, template, spans, n_template)
             cache.meta["_msa_b200_segments"] = hit
         return hit[1:]
 
@@ -180,8 +167,15 @@ class MemorySparseAttention(Qwen3Attention):
         first = torch.where(valid, idx, s).amin(dim=1)
         last = torch.where(valid, idx, -1).amax(dim=1)
         runs = (((last - first + 1) == valid.sum(dim=1)) | (last < 0)).all().to(torch.int32)
-        status = cache.meta.setdefault("_msa_b200_attn_status", torch.zeros(4, dtype=torch.int32, device=valid.device))
-        return torch.stack([runs, status[0]])
+        return torch.stack([runs, MemorySparseAttention._attn_status(cache, valid.device)[0]])
+
+    @staticmethod
+    def _attn_status(cache, device):
+        """The status words of the tensor-core attention launches of this cache."""
+        status = cache.meta.get("_msa_b200_attn_status")
+        if status is None:
+            status = cache.meta["_msa_b200_attn_status"] = torch.zeros(4, dtype=torch.int32, device=device)
+        return status
 
     @staticmethod
     def _check_attn_status(word):
@@ -207,13 +201,13 @@ class MemorySparseAttention(Qwen3Attention):
         tc_ok = tensor_cores and max_d >= 128 and ops.doc_attention_tc_supported(query_states, key_states, value_states)
         if tc_ok and runs_d:
             # unmasked documents: attention on the tcgen05 kernel (K and V are pooled by the pooling kernel below)
-            status = cache.meta.setdefault("_msa_b200_attn_status", torch.zeros(4, dtype=torch.int32, device=device))
+            status = self._attn_status(cache, device)
             ops.doc_attention_tc(query_states, key_states, value_states, tok_d, off_d, max_d, out=attn_output,
                                  scale=self.scaling, status=status)
         elif tc_ok and spans is not None:
             # masked tokens inside documents: the same kernel over each document's span of memory with a bitmap of
             # the tokens that take part (masked rows of attn_output stay zero)
-            status = cache.meta.setdefault("_msa_b200_attn_status", torch.zeros(4, dtype=torch.int32, device=device))
+            status = self._attn_status(cache, device)
             ops.doc_attention_tc_masked(query_states, key_states, value_states, spans[0], spans[1], spans[2], spans[3],
                                         out=attn_output, scale=self.scaling, status=status)
         elif tensor_cores and self.is_router_layer and self.pooling_kernel_size % 32 == 0:
@@ -267,12 +261,13 @@ class MemorySparseAttention(Qwen3Attention):
             template_v = cache_kwargs["template_prefix_vcache"].to(device)
 
         final_k = final_v = None
+        valid_q = attention_mask == 1
         if self.is_router_layer:
             routing_q = (self.router_q_proj(hidden_states).view(hidden_shape).transpose(1, 2)
                          if self.decouple_router else query_states)
             if self.aux_loss_method == "INFONCE":
                 routing_q = F.normalize(routing_q, p=2, dim=-1)
-            query_mask = (doc_ids == 0) & (attention_mask == 1)
+            query_mask = (doc_ids == 0) & valid_q
             final_k, final_v, final_scores, n_sel, final_ids = self.memory_client.doc_query(routing_q, query_mask,
                                                                                           self.layer_idx)
             if cache.meta.get("require_recall_topk", False):
@@ -283,17 +278,13 @@ class MemorySparseAttention(Qwen3Attention):
 
         # One kernel builds the left-padded compact cache (reference :299-351) in storage with room to
         # append decode tokens; attention then reads it in place (bf16 / head_dim 128: own kernel).
-        valid_q = attention_mask == 1
-        num_q = valid_q.sum(dim=1)
         t_len = template_k.shape[2]
-        kv_lengths = t_len + n_sel + num_q
         tc = dtype == torch.bfloat16 and d == 128
-        if tc:   # one read-back for the cache size, the run check and the status of earlier launches
-            max_kv, runs, word = torch.cat([kv_lengths.max().reshape(1).to(torch.int32), self._valid_runs(valid_q, cache)]).tolist()
-            self._check_attn_status(word)
-            tc = bool(runs)
-        else:
-            max_kv = int(kv_lengths.max())
+        # one read-back for the cache size, the run check and the status of earlier launches
+        kv_lengths, report = ops.question_plan(valid_q, n_sel, t_len, self._attn_status(cache, device) if tc else None)
+        max_kv, runs, word = report.tolist()
+        self._check_attn_status(word)
+        tc = tc and bool(runs)
         reserve = int(cache.meta.get("max_generate_tokens", self.decode_reserve))
         k_store, v_store, kv_start, kv_len, q_tok, n_valid, _ = ops.assemble_context(
             template_k, template_v, final_k, None if final_v is None else final_v.to(device), n_sel, key_states,

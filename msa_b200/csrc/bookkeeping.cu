@@ -229,6 +229,151 @@ bk_emit_kernel(const int64_t* __restrict__ doc_ids, const int64_t* __restrict__ 
 
 }  // namespace msa
 
+namespace msa {
+
+// What a batch of questions needs on the host before its context is assembled, in one launch of one block (a warp per row): lengths of
+// the compact caches, the longest, and whether the valid tokens of every row are one run.  Bound by latency; as 20 tensor
+// operations it cost 6 us of host time each, twice per pair of layers: 2.05 -> 1.69 ms for 16 questions in two layers (with the head's
+// product on contiguous rows).
+__global__ void __launch_bounds__(1024)
+question_plan_kernel(const uint8_t* __restrict__ valid, int n_rows, int row_len, const int64_t* __restrict__ n_sel, int t_len,
+                     const int32_t* __restrict__ status, int64_t* __restrict__ kv_lengths, int32_t* __restrict__ report) {
+  __shared__ int s_max, s_runs;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) { s_max = 0; s_runs = 1; }
+  __syncthreads();
+  for (int b = warp; b < n_rows; b += 32) {
+    int count = 0, first = row_len, last = -1;
+    for (int i = lane; i < row_len; i += 32)
+      if (valid[(long long)b * row_len + i]) { ++count; first = min(first, i); last = i; }
+    count = __reduce_add_sync(0xffffffffu, count);
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) {
+      const int64_t n = t_len + n_sel[b] + count;
+      kv_lengths[b] = n;
+      atomicMax(&s_max, (int)n);
+      if (last >= 0 && last - first + 1 != count) s_runs = 0;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) { report[0] = s_max; report[1] = s_runs; report[2] = status ? status[0] : 0; }
+}
+
+// Token lists and segment offsets of a block's documents and templates (tables 0 and 1): a document's segment is a stretch of listed
+// tokens of one row and id, a template's all listed tokens of a row.  One block walks tiles of 4096 tokens with two scans each
+// (places in the list, starts of segments), so that nothing but the eight words of the report has to reach the host: as
+// tensor operations the tables took thirteen read-backs, during which the GPU waited; this takes 71 us for 32,002 tokens (11 for 4000).
+struct SegmentTables {
+  int32_t *tok[2], *off[2];
+  int32_t* report;            // per table: tokens, segments, longest, whether every segment is a run; the last word of table 1:
+};                            // tokens of the template, listed or not
+
+constexpr int kSegThreads = 1024, kSegPer = 4;
+
+__global__ void __launch_bounds__(kSegThreads)
+segments_kernel(const int64_t* __restrict__ doc_ids, const uint8_t* __restrict__ valid, int n, int row_len, const SegmentTables t) {
+  __shared__ int s_scan[2][32];             // listed tokens and starts of segments of every warp
+  __shared__ int s_last_tok[32];            // last listed token of a warp's stretch, -1: none
+  __shared__ int s_runs, s_longest, s_template;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_template = 0;
+  for (int k = 0; k < 2; ++k) {
+    int n_tok = 0, n_seg = 0, before = -1;  // so far: listed tokens, segments, the last listed token (the same in every thread)
+    if (threadIdx.x == 0) { s_runs = 1; s_longest = 0; }
+    __syncthreads();
+    for (int base = 0; base < n; base += kSegThreads * kSegPer) {
+      const int i0 = base + threadIdx.x * kSegPer;
+      int64_t id[kSegPer];
+      bool on[kSegPer];
+      int count = 0, last = -1, templ = 0;
+#pragma unroll
+      for (int j = 0; j < kSegPer; ++j) {
+        const int i = i0 + j;
+        id[j] = i < n ? doc_ids[i] : 0;
+        on[j] = i < n && valid[i] && (k == 0 ? id[j] > 0 : id[j] == -2);
+        templ += i < n && id[j] == -2;
+        if (on[j]) { ++count; last = i; }
+      }
+      if (k == 1) {
+        templ = __reduce_add_sync(0xffffffffu, templ);
+        if (lane == 0 && templ) atomicAdd(&s_template, templ);
+      }
+      // the listed token before this thread's first one
+      int upto = last;                      // last listed token of the warp's lanes up to this one
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto = max(upto, x);
+      }
+      int prev = __shfl_up_sync(0xffffffffu, upto, 1);
+      if (lane == 0) prev = -1;
+      if (lane == 31) s_last_tok[warp] = upto;
+      __syncthreads();
+      if (prev < 0) {
+        prev = before;
+        for (int w = 0; w < warp; ++w) prev = max(prev, s_last_tok[w]);
+      }
+      bool start[kSegPer];
+      int starts = 0, p = prev;
+      bool runs = true;
+#pragma unroll
+      for (int j = 0; j < kSegPer; ++j) {
+        start[j] = false;
+        if (!on[j]) continue;
+        const int i = i0 + j;
+        const bool same = p >= 0 && p / row_len == i / row_len && (k == 1 || doc_ids[p] == id[j]);
+        start[j] = !same;
+        if (same && p != i - 1) runs = false;
+        starts += start[j];
+        p = i;
+      }
+      if (!runs) s_runs = 0;
+      int tok_at = count, seg_at = starts;  // exclusive prefixes over the block
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, tok_at, o), y = __shfl_up_sync(0xffffffffu, seg_at, o);
+        if (lane >= o) { tok_at += x; seg_at += y; }
+      }
+      if (lane == 31) { s_scan[0][warp] = tok_at; s_scan[1][warp] = seg_at; }
+      __syncthreads();
+      int tok0 = 0, seg0 = 0, tok_all = 0, seg_all = 0, end = before;
+      for (int w = 0; w < 32; ++w) {
+        if (w == warp) { tok0 = tok_all; seg0 = seg_all; }
+        tok_all += s_scan[0][w];
+        seg_all += s_scan[1][w];
+        end = max(end, s_last_tok[w]);
+      }
+      tok_at += n_tok + tok0 - count;
+      seg_at += n_seg + seg0 - starts;
+#pragma unroll
+      for (int j = 0; j < kSegPer; ++j)
+        if (on[j]) {
+          if (start[j]) t.off[k][seg_at++] = tok_at;
+          t.tok[k][tok_at++] = i0 + j;
+        }
+      n_tok += tok_all;
+      n_seg += seg_all;
+      before = end;
+      __syncthreads();                      // the shared words are free again
+    }
+    if (threadIdx.x == 0) t.off[k][n_seg] = n_tok;
+    __syncthreads();                        // this block's offsets are there for all of its threads
+    int longest = 0;
+    for (int i = threadIdx.x; i < n_seg; i += kSegThreads) longest = max(longest, t.off[k][i + 1] - t.off[k][i]);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (lane == 0 && longest) atomicMax(&s_longest, longest);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      t.report[4 * k] = n_tok; t.report[4 * k + 1] = n_seg; t.report[4 * k + 2] = s_longest;
+      t.report[4 * k + 3] = k == 0 ? s_runs : s_template;
+    }
+    __syncthreads();
+  }
+}
+
+}  // namespace msa
+
 using namespace msa;
 
 extern "C" int64_t msa_bookkeeping_workspace_bytes(int32_t n_rows, int32_t row_len) {
@@ -266,5 +411,25 @@ extern "C" int msa_chunk_bookkeeping(const int64_t* doc_ids, const int64_t* atte
                                                  pooled_doc_ids, max_chunks);
     MSA_LAUNCH_OK("bk_emit_kernel");
   }
+  return MSA_OK;
+}
+
+extern "C" int msa_question_plan(const uint8_t* valid, int32_t n_rows, int32_t row_len, const int64_t* n_sel, int32_t t_len,
+                                 const int32_t* status, int64_t* kv_lengths, int32_t* report, void* stream) {
+  MSA_REQUIRE(n_rows > 0 && row_len >= 0 && t_len >= 0, "question_plan: bad sizes");
+  MSA_REQUIRE((valid || row_len == 0) && n_sel && kv_lengths && report, "question_plan: null pointer");
+  question_plan_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(valid, n_rows, row_len, n_sel, t_len, status, kv_lengths, report);
+  MSA_LAUNCH_OK("question_plan_kernel");
+  return MSA_OK;
+}
+
+extern "C" int msa_segments(const int64_t* doc_ids, const uint8_t* valid, int32_t n_rows, int32_t row_len, int32_t* tok_docs, int32_t* off_docs,
+                            int32_t* tok_template, int32_t* off_template, int32_t* report, void* stream) {
+  MSA_REQUIRE(n_rows >= 0 && row_len >= 0 && (int64_t)n_rows * row_len < (1ll << 31) - 8192, "segments: bad sizes");
+  MSA_REQUIRE(tok_docs && off_docs && tok_template && off_template && report, "segments: null pointer");
+  MSA_REQUIRE((doc_ids && valid) || (int64_t)n_rows * row_len == 0, "segments: null pointer");
+  const SegmentTables t{{tok_docs, tok_template}, {off_docs, off_template}, report};
+  segments_kernel<<<1, kSegThreads, 0, (cudaStream_t)stream>>>(doc_ids, valid, n_rows * row_len, row_len > 0 ? row_len : 1, t);
+  MSA_LAUNCH_OK("segments_kernel");
   return MSA_OK;
 }

@@ -124,5 +124,6 @@ class MSAForCausalLM(nn.Module):
                 use_cache=True, logits_to_keep: int = 0, **unused):
         out = self.model(input_ids=input_ids, attention_mask=attention_mask, position_ids=position_ids,
                          past_key_values=past_key_values, use_cache=use_cache, doc_ids=doc_ids)
-        hidden = out.last_hidden_state[:, -logits_to_keep:] if logits_to_keep else out.last_hidden_state
+        # contiguous: as a batch of strided rows the product would read the head's weights once per sequence
+        hidden = out.last_hidden_state[:, -logits_to_keep:].contiguous() if logits_to_keep else out.last_hidden_state
         return SimpleNamespace(logits=self.lm_head(hidden), past_key_values=out.past_key_values)

@@ -552,6 +552,35 @@ def assemble_context(template_k, template_v, sel_k, sel_v, n_sel, key_states, va
     return k_store, v_store, kv_start, kv_len, q_tok, num_q, err
 
 
+def question_plan(valid: torch.Tensor, n_sel: torch.Tensor, t_len: int, status: Optional[torch.Tensor] = None):
+    """``(kv_lengths[B] int64, report int32[3])`` of questions with the valid tokens ``valid`` [B, S] (bool): template, selected and valid
+    tokens of every row; the longest, whether every row's valid tokens are one run, ``status[0]``."""
+    A.need_cuda(valid, n_sel, status)
+    b, s = valid.shape
+    vmask = valid.contiguous().view(torch.uint8)
+    if n_sel.dtype != torch.int64 or not n_sel.is_contiguous():
+        n_sel = n_sel.to(torch.int64).contiguous()
+    kv_lengths = torch.empty(b, dtype=torch.int64, device=valid.device)
+    report = torch.empty(3, dtype=torch.int32, device=valid.device)
+    A.check(A.lib().msa_question_plan(A.ptr(vmask), b, s, A.ptr(n_sel), t_len, A.ptr(status), A.ptr(kv_lengths), A.ptr(report),
+                                      A.stream_ptr(valid.device)), "msa_question_plan")
+    return kv_lengths, report
+
+
+def segments(doc_ids: torch.Tensor, valid: torch.Tensor):
+    """Segment tables of a block ``[rows, len]`` of documents and of its template tokens: ``((tok, off, longest, runs), (tok, off, longest,
+    True), template_tokens)``, lists on the device as int32.  One read-back."""
+    A.need_cuda(doc_ids, valid)
+    doc_ids, vmask = doc_ids.to(torch.int64).contiguous(), valid.expand(doc_ids.shape).contiguous().view(torch.uint8)
+    n, dev = doc_ids.numel(), doc_ids.device
+    room = (n + 4) // 4 * 4                                       # every table starts on 16 bytes
+    tok_d, off_d, tok_t, off_t, report = torch.empty(4 * room + 8, dtype=torch.int32, device=dev).split([room] * 4 + [8])
+    A.check(A.lib().msa_segments(A.ptr(doc_ids), A.ptr(vmask), doc_ids.shape[0], doc_ids.shape[1], A.ptr(tok_d), A.ptr(off_d), A.ptr(tok_t),
+                                 A.ptr(off_t), A.ptr(report), A.stream_ptr(dev)), "msa_segments")
+    n_d, s_d, max_d, runs, n_t, s_t, max_t, n_template = report.tolist()
+    return (tok_d[:n_d], off_d[:s_d + 1], max_d, bool(runs)), (tok_t[:n_t], off_t[:s_t + 1], max_t, True), n_template
+
+
 def append_segment(key_states: torch.Tensor, value_states: torch.Tensor, valid: torch.Tensor, k_store: torch.Tensor,
                    v_store: torch.Tensor, kv_start: Optional[torch.Tensor], kv_len: torch.Tensor):
     """Append the valid tokens of a segment ``[B, Hkv, S, D]`` to every sequence's store ``[B, Hkv, L, D]`` in place;
