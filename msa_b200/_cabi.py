@@ -132,7 +132,9 @@ def ptr(t) -> int:
 
 
 def stream_ptr(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The handle of the current stream of ``device`` (a torch.device, an index or None), without a stream object around it."""
+    index = device.index if isinstance(device, torch.device) else device
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def need_cuda(*tensors) -> None:

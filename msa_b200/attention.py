@@ -40,9 +40,13 @@ from . import ops
 def fused_ops(*tensors) -> bool:
     """Whether the fused kernels may stand in for eager operations on these: plain bf16 tensors on the GPU, aligned rows, and no
     gradient to keep (the kernels know none)."""
-    return not torch.is_grad_enabled() and all(
-        type(t) in (torch.Tensor, nn.Parameter) and t.is_cuda and t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0
-        for t in tensors)
+    if torch.is_grad_enabled():
+        return False
+    for t in tensors:
+        if not ((type(t) is torch.Tensor or type(t) is nn.Parameter) and t.dtype == torch.bfloat16 and t.is_cuda and t.stride(-1) == 1
+                and t.data_ptr() % 16 == 0):
+            return False
+    return True
 
 
 def plain_module(m, cls) -> bool:
