@@ -70,6 +70,11 @@ __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + lo
 template <typename T> __device__ __forceinline__ float silu_act(float z) { return silu_f(z); }
 template <> __device__ __forceinline__ float silu_act<__nv_bfloat16>(float z) { return __fdividef(z, 1.f + __expf(-z)); }
 
+// Rows up to which the product behind a kernel may be rows_gemm_kernel, which fetches its weights early.  The library's products gain
+// nothing by it: behind a part_norm of 6236 rows they crowded it out (39 -> 53 us).
+constexpr int kEarlyRows = 8;
+__device__ __forceinline__ void let_product_start(int rows) { if (rows <= kEarlyRows) grid_launch_dependents(); }
+
 // Index of the sequence that owns position `i` of a prefix-sum table off[0 .. n].
 __device__ __forceinline__ int owner_of(const int32_t* off, int n, int i) {
   int lo = 0, hi = n - 1;

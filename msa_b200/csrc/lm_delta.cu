@@ -320,7 +320,7 @@ constexpr int kDdThreads = 256;
 template <typename T, int V, bool STAGE>
 __global__ void __launch_bounds__(kDdThreads)
 delta_decode_kernel(const msa_lm_delta_args a, T* __restrict__ out, long long out_stride, int groups) {
-  grid_launch_dependents();
+  let_product_start(gridDim.y);
   extern __shared__ float sm[];
   __shared__ float s_part[32];
   const DeltaLayout L(a);

@@ -82,7 +82,7 @@ inline int pass_groups(int dv, int v) { return dv / v >= kLinThreads ? 1 : kLinT
 // One block per (head, sequence).
 template <typename T, int V>
 __global__ void __launch_bounds__(kLinThreads, 4) wkv_decode_kernel(const msa_lm_wkv_args a, T* __restrict__ out, long long out_stride) {
-  grid_launch_dependents();
+  let_product_start(gridDim.y);
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_part[32];
   const int h = blockIdx.x, b = blockIdx.y, dim = a.dim, pad = (dim + 3) / 4 * 4;
@@ -122,7 +122,7 @@ struct SsdLayout {
 
 template <typename T, int V>
 __global__ void __launch_bounds__(kLinThreads, 4) ssd_decode_kernel(const msa_lm_ssd_args a) {
-  grid_launch_dependents();
+  let_product_start(gridDim.y);
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_part[32];
   const SsdLayout L(a);
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(256) wkv_out_kernel(const msa_lm_wkv_args a, c
 template <typename T, int V>
 __global__ void __launch_bounds__(256) part_norm_kernel(const float* __restrict__ x, long long x_stride, const float* __restrict__ w,
                                                         int size, float eps, T* __restrict__ out, long long out_stride) {
-  grid_launch_dependents();
+  let_product_start(gridDim.x);
   __shared__ float s_part[32];
   const long long row = blockIdx.x;
   const int c0 = blockIdx.y * size;

@@ -40,8 +40,8 @@ __device__ __forceinline__ float branch1(const ResNormParams& p, long long r, in
   return a;
 }
 
-// Any width and alignment, one element at a time.
-template <typename T, typename TY>
+// Rows above 4096 columns and odd ones.  V = 4: every row pointer is 4-element aligned and width % 4 == 0; V = 1: any width.
+template <typename T, typename TY, int V>
 __global__ void residual_norm_kernel(const ResNormParams p) {
   extern __shared__ float s_row[];   // [width]
   __shared__ float s_part[32];
@@ -54,28 +54,64 @@ __global__ void residual_norm_kernel(const ResNormParams p) {
   float scale_b = 1.f;
   if (p.y && p.w_branch) {
     float ss = 0.f;
-    for (int i = threadIdx.x; i < p.width; i += nt) {
-      const float b = branch1<TY>(p, r, i);
-      s_row[i] = b;
-      ss += b * b;
+    for (int i = threadIdx.x * V; i < p.width; i += nt * V) {
+      if constexpr (V == 4) {
+        const float4 b = branch4<TY>(p, r, i);
+        store4(s_row + i, b);
+        ss += b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
+      } else {
+        const float b = branch1<TY>(p, r, i);
+        s_row[i] = b;
+        ss += b * b;
+      }
     }
     scale_b = 1.f / sqrtf(block_sum(ss, s_part) / (float)p.width + p.eps);
   }
   float ss = 0.f;
-  for (int i = threadIdx.x; i < p.width; i += nt) {   // every thread revisits the elements it stored above
-    float x = p.base ? p.base[rb * p.base_stride + i] : 0.f;
-    if (p.y) x += p.w_branch ? s_row[i] * scale_b * p.w_branch[i] : branch1<TY>(p, r, i);
-    if (p.add) x += p.add[r * p.width + i];
-    if (p.x_out) p.x_out[r * p.width + i] = x;
-    if (cat) cat[r * p.cat_stride + i] = from_f<T>(x);
-    s_row[i] = x;
-    ss += x * x;
+  for (int i = threadIdx.x * V; i < p.width; i += nt * V) {   // every thread revisits the elements it stored above
+    if constexpr (V == 4) {
+      float4 x = p.base ? load4(p.base + rb * p.base_stride + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.y) {
+        if (p.w_branch) {
+          const float4 b = load4(s_row + i), w = load4(p.w_branch + i);
+          x.x += b.x * scale_b * w.x; x.y += b.y * scale_b * w.y; x.z += b.z * scale_b * w.z; x.w += b.w * scale_b * w.w;
+        } else {
+          const float4 b = branch4<TY>(p, r, i);
+          x.x += b.x; x.y += b.y; x.z += b.z; x.w += b.w;
+        }
+      }
+      if (p.add) {
+        const float4 b = load4(p.add + r * p.width + i);
+        x.x += b.x; x.y += b.y; x.z += b.z; x.w += b.w;
+      }
+      if (p.x_out) store4(p.x_out + r * p.width + i, x);
+      if (cat) store4(cat + r * p.cat_stride + i, x);
+      store4(s_row + i, x);
+      ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+    } else {
+      float x = p.base ? p.base[rb * p.base_stride + i] : 0.f;
+      if (p.y) x += p.w_branch ? s_row[i] * scale_b * p.w_branch[i] : branch1<TY>(p, r, i);
+      if (p.add) x += p.add[r * p.width + i];
+      if (p.x_out) p.x_out[r * p.width + i] = x;
+      if (cat) cat[r * p.cat_stride + i] = from_f<T>(x);
+      s_row[i] = x;
+      ss += x * x;
+    }
   }
   if (!h_out) return;
   const float inv = 1.f / sqrtf(block_sum(ss, s_part) / (float)p.width + p.eps);
-  for (int i = threadIdx.x; i < p.width; i += nt) {
-    h_out[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next[i]);
-    if (h_out2) h_out2[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next2[i]);
+  for (int i = threadIdx.x * V; i < p.width; i += nt * V) {
+    if constexpr (V == 4) {
+      const float4 x = load4(s_row + i), w = load4(p.w_next + i);
+      store4(h_out + r * p.width + i, make_float4(x.x * inv * w.x, x.y * inv * w.y, x.z * inv * w.z, x.w * inv * w.w));
+      if (h_out2) {
+        const float4 w2 = load4(p.w_next2 + i);
+        store4(h_out2 + r * p.width + i, make_float4(x.x * inv * w2.x, x.y * inv * w2.y, x.z * inv * w2.z, x.w * inv * w2.w));
+      }
+    } else {
+      h_out[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next[i]);
+      if (h_out2) h_out2[r * p.width + i] = from_f<T>(s_row[i] * inv * p.w_next2[i]);
+    }
   }
 }
 
@@ -83,7 +119,7 @@ __global__ void residual_norm_kernel(const ResNormParams p) {
 // before the first reduction): a decode step has few rows and waits for latency, not for bandwidth.
 template <typename T, typename TY>
 __global__ void __launch_bounds__(1024) residual_norm_once_kernel(const ResNormParams p) {
-  grid_launch_dependents();
+  let_product_start(gridDim.x);
   __shared__ float s_part[32];
   const long long r = blockIdx.x;
   const long long rb = p.rows ? p.rows[r] : r;
@@ -133,20 +169,19 @@ __global__ void __launch_bounds__(1024) residual_norm_once_kernel(const ResNormP
     store4(reinterpret_cast<T*>(p.h_out2) + r * p.width + i, make_float4(x.x * inv * wn2.x, x.y * inv * wn2.y, x.z * inv * wn2.z, x.w * inv * wn2.w));
 }
 
-// The same for many rows: 128 threads per 2048 columns, four vectors each.  Bound by HBM (base and stream in 32 bits, branch and
-// norm in 16: 12 bytes per element), so as many loads as possible are in flight: all of a row's are issued before the first
-// reduction, and rows need few enough threads and registers for ten of them on an SM.  One row per 256 threads through shared memory,
-// one vector at a time, took 47.1 us for 6236 x 2048 from a cold L2 (bytes at HBM rate: 23), this takes 34.8.
-template <typename T, typename TY>
-__global__ void __launch_bounds__(768, 1) residual_norm_rows_kernel(const ResNormParams p) {
-  constexpr int E = 4;
+// The same for many rows, E vectors per thread in registers.  Bound by HBM (base and stream in 32 bits, branch and norm in 16: 12 bytes
+// per element), so all of a row's loads are in flight before the first reduction.  Threads and order of the sums are those of the
+// general kernel below, so that a position's experts do not hang on the number of rows beside it.  One vector at a time through
+// shared memory took 47.1 us for 6236 x 2048 from a cold L2 (bytes at HBM rate: 23), this takes 39.9.
+template <typename T, typename TY, int E>
+__global__ void __launch_bounds__(256) residual_norm_rows_kernel(const ResNormParams p) {
   __shared__ float s_part[2][32];
   const long long r = blockIdx.x;
   const long long rb = p.rows ? p.rows[r] : r;
   const int nt = blockDim.x, lane = threadIdx.x & 31, warps = nt >> 5;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   auto at = [&](int e) { return (e * nt + (int)threadIdx.x) * 4; };
-  auto sum = [&](float v, float* part) {             // every thread gets it; the two reductions have a buffer each
+  auto sum = [&](float v, float* part) {             // block_sum with a buffer for each of the two reductions
     v = warp_sum_f(v);
     if (lane == 0) part[threadIdx.x >> 5] = v;
     __syncthreads();
@@ -205,7 +240,7 @@ __global__ void __launch_bounds__(768, 1) residual_norm_rows_kernel(const ResNor
 // V = 4: rows and pointers are 4-element aligned; V = 1: any width.
 template <typename T, int V>
 __global__ void embed_kernel(const msa_lm_embed_args a) {
-  grid_launch_dependents();
+  let_product_start(gridDim.x);
   extern __shared__ float s_row[];
   __shared__ float s_part[32];
   const long long r = blockIdx.x;
@@ -355,7 +390,7 @@ template <typename T, int V>
 __global__ void token_shift_kernel(const T* __restrict__ h, const float* __restrict__ mu, int n_mix, int n_tok, int width,
                                    const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ slot,
                                    const int32_t* __restrict__ start, const int32_t* __restrict__ cu, T* shift, T* __restrict__ out) {
-  grid_launch_dependents();
+  let_product_start(gridDim.x);
   const long long r = blockIdx.x;
   const int s = tok_seq[r], t = (int)r - cu[s];
   T* state = shift + (long long)slot[s] * width;
@@ -382,8 +417,9 @@ __global__ void token_shift_kernel(const T* __restrict__ h, const float* __restr
 }
 
 // V = 8: 16-byte loads, two rows' in flight per thread (bf16); V = 4: 8- or 16-byte ones; V = 1: any alignment.  A block takes
-// 256 * V columns of two rows.  Bound by HBM; with 8-byte loads, an index division by a run-time number and full-accuracy
-// exponentials in front of the rounding to bf16 6236 x 6144 took 63.5 us from a cold L2 (bytes at HBM rate: 34.6), now 41.0.
+// 256 * V columns of two rows.  Bound by HBM; with 8-byte loads and an index division by a run-time number 6236 x 6144 took 63.5 us
+// from a cold L2 (bytes at HBM rate: 34.6), now 43.0 (41.0 with approximate exponentials, whose last bits decide between experts
+// that tie).
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
 lm_silu_mul_kernel(const T* __restrict__ gu, long long stride, int ff, int n_rows, T* __restrict__ out, long long out_stride) {
@@ -408,7 +444,7 @@ lm_silu_mul_kernel(const T* __restrict__ gu, long long stride, int ff, int n_row
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float2 x = __bfloat1622float2(a[i]), y = __bfloat1622float2(b[i]);
-          c[i] = __floats2bfloat162_rn(silu_act<T>(x.x) * y.x, silu_act<T>(x.y) * y.y);
+          c[i] = __floats2bfloat162_rn(silu_f(x.x) * y.x, silu_f(x.y) * y.y);
         }
         *reinterpret_cast<uint4*>(out + (r0 + k) * out_stride + j) = o;
       }
@@ -418,9 +454,9 @@ lm_silu_mul_kernel(const T* __restrict__ gu, long long stride, int ff, int n_row
       T* o = out + (r0 + k) * out_stride + j;
       if constexpr (V == 4) {
         const float4 x = load4(g), y = load4(u);
-        store4(o, make_float4(silu_act<T>(x.x) * y.x, silu_act<T>(x.y) * y.y, silu_act<T>(x.z) * y.z, silu_act<T>(x.w) * y.w));
+        store4(o, make_float4(silu_f(x.x) * y.x, silu_f(x.y) * y.y, silu_f(x.z) * y.z, silu_f(x.w) * y.w));
       } else {
-        *o = from_f<T>(silu_act<T>(to_f(*g)) * to_f(*u));
+        *o = from_f<T>(silu_f(to_f(*g)) * to_f(*u));
       }
     }
   }
@@ -462,20 +498,27 @@ extern "C" int msa_lm_residual_norm(const float* base, int64_t base_stride, cons
     MSA_LAUNCH_OK("residual_norm_once_kernel");
     return MSA_OK;
   }
-  if (v4) {                                            // width <= 12000: at most 24 warps
-    const int row = (width + 511) / 512 * 32;
+  const int threads = row_threads(width);
+  const int vectors = (width / 4 + threads - 1) / threads;
+  if (v4 && vectors <= 4) {                            // beyond, the registers leave too few rows in flight (8192: 33.8 us against 20.5)
     MSA_LM_DISPATCH(dtype, {
-      if (y && y_dtype == MSA_BF16) residual_norm_rows_kernel<T, __nv_bfloat16><<<n_rows, row, 0, st>>>(p);
-      else residual_norm_rows_kernel<T, float><<<n_rows, row, 0, st>>>(p);
+      const bool half = y && y_dtype == MSA_BF16;
+      auto launch = [&](auto with_half, auto with_float) { half ? with_half<<<n_rows, threads, 0, st>>>(p) : with_float<<<n_rows, threads, 0, st>>>(p); };
+      if (vectors <= 2) launch(residual_norm_rows_kernel<T, __nv_bfloat16, 2>, residual_norm_rows_kernel<T, float, 2>);
+      else launch(residual_norm_rows_kernel<T, __nv_bfloat16, 4>, residual_norm_rows_kernel<T, float, 4>);
     });
     MSA_LAUNCH_OK("residual_norm_rows_kernel");
     return MSA_OK;
   }
   const size_t smem = (size_t)width * 4;
-  const int threads = row_threads(width);
   MSA_LM_DISPATCH(dtype, {
-    if (y && y_dtype == MSA_BF16) residual_norm_kernel<T, __nv_bfloat16><<<n_rows, threads, smem, st>>>(p);
-    else residual_norm_kernel<T, float><<<n_rows, threads, smem, st>>>(p);
+    if (y && y_dtype == MSA_BF16) {
+      if (v4) residual_norm_kernel<T, __nv_bfloat16, 4><<<n_rows, threads, smem, st>>>(p);
+      else residual_norm_kernel<T, __nv_bfloat16, 1><<<n_rows, threads, smem, st>>>(p);
+    } else {
+      if (v4) residual_norm_kernel<T, float, 4><<<n_rows, threads, smem, st>>>(p);
+      else residual_norm_kernel<T, float, 1><<<n_rows, threads, smem, st>>>(p);
+    }
   });
   MSA_LAUNCH_OK("residual_norm_kernel");
   return MSA_OK;

@@ -16,7 +16,7 @@ def _rows(t: torch.Tensor) -> int:
     return t.stride(0)
 
 
-ROWS_GEMM_MAX = 8            # rows of x the kernel takes (one tile); a decode step of 16 sequences is no faster by two tiles
+ROWS_GEMM_MAX = 8            # rows of x the kernel takes (kRgMaxRows, kEarlyRows); a decode step of 16 sequences is no faster by two tiles
 
 
 def few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:

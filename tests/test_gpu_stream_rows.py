@@ -19,8 +19,8 @@ def near(got, want, scale, bf16):
     return bool(((got.double() - want).abs() <= 2.0 ** -18 * scale + (2.0 ** -8 * want.abs() if bf16 else 0.0)).all())
 
 
-# few rows (one pass) up to 512, then 128 threads per 2048 columns; widths around a warp's, a vector's and the limits
-@pytest.mark.parametrize("rows,width", [(513, 4), (513, 508), (600, 512), (513, 516), (700, 2048), (515, 2052), (3, 4100), (2, 12000), (514, 2050), (3, 4101)])
+# few rows (one pass) up to 512, then a row in registers up to 4096 columns, then through shared memory; widths around the limits
+@pytest.mark.parametrize("rows,width", [(513, 4), (513, 508), (600, 512), (513, 516), (700, 2048), (515, 2052), (514, 4096), (3, 4100), (2, 12000), (514, 2050), (3, 4101)])
 @pytest.mark.parametrize("dtype", [BF16, F32], ids=["bf16", "f32"])
 def test_residual_norm(rows, width, dtype):
     from msa_b200 import lm_ops as K
