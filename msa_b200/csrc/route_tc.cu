@@ -584,9 +584,9 @@ __global__ void __launch_bounds__(1024) live_blocks_kernel(const float* __restri
 }
 
 // Listed block i of rows [.., kdim] -> block i of `packed`; one CTA per block of 16 rows, eight 16-byte loads in flight per
-// thread (7,700 rows of 2 KB: 5 us).
-__global__ void __launch_bounds__(256) pack_rows_kernel(const uint4* __restrict__ rows, const int32_t* __restrict__ live, int vecs,
-                                                        uint4* __restrict__ packed) {
+// thread (7,700 rows of 2 KB: 5 us).  Launched early, while the list is still being written: it is read behind the wait, through
+// plain pointers.
+__global__ void __launch_bounds__(256) pack_rows_kernel(const uint4* rows, const int32_t* live, int vecs, uint4* __restrict__ packed) {
   grid_dependency_wait();
   if ((int)blockIdx.x >= live[0]) return;
   const uint4* src = rows + (long long)live[1 + blockIdx.x] * vecs;

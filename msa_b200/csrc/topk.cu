@@ -75,10 +75,11 @@ sort_topk_kernel(const uint32_t* __restrict__ keys, long long table_stride, int 
   }
 }
 
+// keys and cand are written by the kernel before this one, which may still run when this one starts: plain pointers.
 template <bool FROM_KEYS>
 __global__ void __launch_bounds__(kSortThreads)
-select_topk_kernel(const uint32_t* __restrict__ keys, long long table_stride, int n_cols, int slice,
-                   const unsigned long long* __restrict__ cand, int n_in, int n2, int keep,
+select_topk_kernel(const uint32_t* keys, long long table_stride, int n_cols, int slice,
+                   const unsigned long long* cand, int n_in, int n2, int keep,
                    unsigned long long* __restrict__ cand_out, const int64_t* __restrict__ doc_ids_table, float* __restrict__ out_scores,
                    int64_t* __restrict__ out_local, int64_t* __restrict__ out_global) {
   extern __shared__ unsigned long long s_items[];
