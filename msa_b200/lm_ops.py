@@ -21,15 +21,23 @@ ROWS_GEMM_MAX = 8            # rows of x the kernel takes (kRgMaxRows, kEarlyRow
 
 def few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether ``x @ w.T`` ([..., n, k] by [..., rows, k]) is a product for ``msa_lm_rows_gemm``: bf16, few rows, and rows on
-    16-byte boundaries."""
-    if not 0 < x.shape[-2] <= ROWS_GEMM_MAX:
+    16-byte boundaries.  Sizes that do not fit one another, and empty ones, are torch's to refuse or to answer."""
+    if x.dim() not in (2, 3) or not 0 < x.shape[-2] <= ROWS_GEMM_MAX:
+        return False
+    k = x.shape[-1]
+    if k == 0 or k % 8 or w.dim() != x.dim() or w.shape[-1] != k or w.shape[-2] == 0 or w.get_device() != x.get_device():
+        return False
+    if x.dim() == 3 and not 0 < x.shape[0] == w.shape[0] < 65536:
         return False
     ok = lambda t: t.is_cuda and t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 for s in t.stride()[:-1])
-    return x.shape[-1] % 8 == 0 and ok(x) and ok(w)
+    return ok(x) and ok(w)
 
 
-def rows_gemm(x, w, out, *, act: bool) -> torch.Tensor:
-    """One launch of ``msa_lm_rows_gemm``.  ``w`` is a weight: no kernel of the running step writes it."""
+def _takes_out(out: torch.Tensor, x: torch.Tensor, rows: int) -> bool:
+    return out.shape == (*x.shape[:-1], rows) and out.stride(-1) == 1 and out.get_device() == x.get_device()
+
+
+def _rows_gemm(x, w, out, act: bool) -> torch.Tensor:
     batch = x.shape[0] if x.dim() == 3 else 1
     step = lambda t: t.stride(0) if t.dim() == 3 else 0
     args = A.RowsGemmArgs(x=x.data_ptr(), x_stride=x.stride(-2), x_batch=step(x), w=w.data_ptr(), w_stride=w.stride(-2), w_batch=step(w),
@@ -39,29 +47,37 @@ def rows_gemm(x, w, out, *, act: bool) -> torch.Tensor:
     return out
 
 
+def rows_gemm(x, w, out, *, act: bool) -> torch.Tensor:
+    """One launch of ``msa_lm_rows_gemm``.  ``w`` is a weight: no kernel of the running step writes it."""
+    if not few_rows(x, w) or (act and w.shape[-2] % 2) or not _takes_out(out, x, w.shape[-2] // 2 if act else w.shape[-2]):
+        raise A.MsaError("rows_gemm: operands of another form, or sizes that do not fit one another")
+    return _rows_gemm(x, w, out, act)
+
+
 def matmul(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, weight: bool = False) -> torch.Tensor:
     """``x @ w.T`` with 32-bit accumulation; ``out_dtype`` float32 keeps the accumulator's precision.  ``weight``: nothing still in
     the stream writes ``w``; few rows then take the package's own kernel."""
-    if weight and few_rows(x, w):
-        return rows_gemm(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device), act=False)
+    if weight and x.dim() == 2 and out_dtype in (None, x.dtype, torch.float32) and few_rows(x, w):
+        return _rows_gemm(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device), act=False)
     if out_dtype is None or out_dtype == x.dtype:
         return torch.mm(x, w.t())
     return torch.mm(x, w.t(), out_dtype=out_dtype)
 
 
-def matmul_silu(x: torch.Tensor, w: torch.Tensor, ff: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``silu(x @ gate.T) * (x @ up.T)``; ``w``, a weight, holds the ``ff`` gate rows and then the up rows."""
-    if few_rows(x, w):
+def matmul_silu(x: torch.Tensor, w: torch.Tensor, ff: int, out: Optional[torch.Tensor] = None, weight: bool = True) -> torch.Tensor:
+    """``silu(x @ gate.T) * (x @ up.T)``; ``w`` holds the ``ff`` gate rows and then the up rows (``weight`` as in ``matmul``)."""
+    if (weight and x.dim() == 2 and w.shape[0] == 2 * ff and few_rows(x, w)
+            and (out is None or (out.dtype == x.dtype and _takes_out(out, x, ff)))):
         if out is None:
             out = torch.empty((x.shape[0], ff), dtype=x.dtype, device=x.device)
-        return rows_gemm(x, w, out, act=True)
+        return _rows_gemm(x, w, out, act=True)
     return silu_mul(matmul(x, w), ff, out)
 
 
-def bmm(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    """``x[b] @ w[b].T``; ``w`` is a weight."""
-    if few_rows(x, w):
-        return rows_gemm(x, w, torch.empty(x.shape[:2] + w.shape[1:2], dtype=x.dtype, device=x.device), act=False)
+def bmm(x: torch.Tensor, w: torch.Tensor, weight: bool = True) -> torch.Tensor:
+    """``x[b] @ w[b].T`` (``weight`` as in ``matmul``)."""
+    if weight and x.dim() == 3 and few_rows(x, w):
+        return _rows_gemm(x, w, torch.empty(x.shape[:2] + w.shape[1:2], dtype=x.dtype, device=x.device), act=False)
     return torch.bmm(x, w.transpose(1, 2))
 
 
