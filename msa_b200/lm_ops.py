@@ -145,8 +145,9 @@ def softcap(logits: torch.Tensor, cap: float) -> torch.Tensor:
 
 
 def argmax(logits: torch.Tensor) -> torch.Tensor:
-    """``logits.argmax(-1)`` of fp32 rows as int32."""
-    A.need_cuda(logits)
+    """``logits.argmax(-1)`` as int32; one launch for fp32 rows."""
+    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(-1) != 1 or not logits.is_cuda:
+        return logits.argmax(dim=-1).to(torch.int32)
     out = torch.empty(logits.shape[0], dtype=torch.int32, device=logits.device)
     A.call("msa_lm_argmax", A.ptr(logits), _rows(logits), logits.shape[0], logits.shape[1], A.ptr(out), A.stream_ptr(logits.device))
     return out

@@ -1,0 +1,42 @@
+"""What the wrappers refuse before anything is launched, and the forms of a device, on fake CUDA tensors."""
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+pytestmark = pytest.mark.filterwarnings("ignore:Accessing the data pointer of FakeTensor")
+
+
+class Library:
+    def __init__(self):
+        self.seen = []
+
+    def __getattr__(self, name):
+        return lambda *a: self.seen.append(name) or 0
+
+
+@pytest.fixture
+def library(monkeypatch):
+    from msa_b200 import _cabi as A
+    lib = Library()
+    monkeypatch.setattr(A, "lib", lambda: lib)
+    monkeypatch.setattr(A, "stream_ptr", lambda device=None: 0)
+    monkeypatch.setattr(A, "ptr", lambda t: 0)
+    return lib
+
+
+def new(*shape, dtype=torch.int64, device="cuda:0"):
+    return torch.empty(shape, dtype=dtype, device=device)
+
+
+def test_argmax_of_other_types(monkeypatch):
+    from msa_b200 import lm_ops as K
+    seen = []
+    monkeypatch.setattr(K.A, "call", lambda name, *a: seen.append(name))
+    monkeypatch.setattr(K.A, "stream_ptr", lambda device=None: 0)
+    monkeypatch.setattr(K.A, "ptr", lambda t: 0)
+    with FakeTensorMode():
+        for x in (new(3, 40, dtype=torch.bfloat16), new(3, 40, dtype=torch.float64), new(40, 3, dtype=torch.float32).t(), new(2, 3, 40, dtype=torch.float32)):
+            assert K.argmax(x).dtype == torch.int32 and K.argmax(x).shape == x.shape[:-1]
+        assert not seen
+        assert K.argmax(new(3, 41, dtype=torch.float32)[:, :40]).shape == (3,)
+    assert seen == ["msa_lm_argmax"]
