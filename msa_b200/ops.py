@@ -557,6 +557,8 @@ def question_plan(valid: torch.Tensor, n_sel: torch.Tensor, t_len: int, status: 
     tokens of every row; the longest, whether every row's valid tokens are one run, ``status[0]``."""
     A.need_cuda(valid, n_sel, status)
     b, s = valid.shape
+    if valid.dtype != torch.bool or n_sel.shape != (b,) or n_sel.device != valid.device or (status is not None and status.device != valid.device):
+        raise A.MsaError("question_plan: a bool mask [B, S] and B lengths on its device expected")
     vmask = valid.contiguous().view(torch.uint8)
     if n_sel.dtype != torch.int64 or not n_sel.is_contiguous():
         n_sel = n_sel.to(torch.int64).contiguous()
@@ -571,6 +573,8 @@ def segments(doc_ids: torch.Tensor, valid: torch.Tensor):
     """Segment tables of a block ``[rows, len]`` of documents and of its template tokens: ``((tok, off, longest, runs), (tok, off, longest,
     True), template_tokens)``, lists on the device as int32.  One read-back."""
     A.need_cuda(doc_ids, valid)
+    if valid.dtype != torch.bool or valid.device != doc_ids.device:
+        raise A.MsaError("segments: a bool mask on the documents' device expected")
     doc_ids, vmask = doc_ids.to(torch.int64).contiguous(), valid.expand(doc_ids.shape).contiguous().view(torch.uint8)
     n, dev = doc_ids.numel(), doc_ids.device
     room = (n + 4) // 4 * 4                                       # every table starts on 16 bytes

@@ -28,6 +28,35 @@ def new(*shape, dtype=torch.int64, device="cuda:0"):
     return torch.empty(shape, dtype=dtype, device=device)
 
 
+def test_question_plan_wants_a_length_for_every_row(library):
+    from msa_b200 import _cabi as A, ops
+    with FakeTensorMode():
+        valid = new(3, 10, dtype=torch.bool)
+        for n_sel in (new(2), new(1), new(3, 1), new(3, device="cuda:1")):
+            with pytest.raises(A.MsaError):
+                ops.question_plan(valid, n_sel, 5)
+        for bad in (new(3, 10, dtype=torch.uint8), new(3, 10, dtype=torch.float32)):
+            with pytest.raises(A.MsaError):
+                ops.question_plan(bad, new(3), 5)
+        with pytest.raises(A.MsaError):
+            ops.question_plan(valid, new(3), 5, new(4, dtype=torch.int32, device="cuda:1"))
+        assert not library.seen
+        ops.question_plan(valid, new(3), 5)
+        ops.question_plan(valid, new(6)[::2], 5, new(4, dtype=torch.int32))
+        assert library.seen == ["msa_question_plan"] * 2
+
+
+def test_segments_wants_a_mask(library):
+    from msa_b200 import _cabi as A, ops
+    with FakeTensorMode():
+        for valid in (new(3, 10), new(3, 10, dtype=torch.bool, device="cuda:1")):
+            with pytest.raises(A.MsaError):
+                ops.segments(new(3, 10), valid)
+        with pytest.raises(RuntimeError):
+            ops.segments(new(3, 10), new(3, 9, dtype=torch.bool))
+    assert not library.seen
+
+
 def test_argmax_of_other_types(monkeypatch):
     from msa_b200 import lm_ops as K
     seen = []
