@@ -413,6 +413,9 @@ def gather_plan(sel_local: torch.Tensor, sel_rank: Optional[torch.Tensor], world
         raise A.MsaError("gather_plan: shard_doc_base / shard_kv_base must have one entry per rank")
     if doc_chunk_offset.numel() != doc_chunk_len.numel():
         raise A.MsaError("gather_plan: doc_chunk_offset and doc_chunk_len differ in length")
+    if report is not None and (total_host is not None or resident is not None or report.dtype != torch.int64 or report.shape != (3,)
+                               or not report.is_contiguous() or not report.is_pinned()):
+        raise A.MsaError("gather_plan: report must be a pinned contiguous int64 [3] tensor, in place of total_host and without resident")
     plan = torch.empty((n_seq * k, 4), dtype=torch.int64, device=dev)
     n_sel = torch.empty((n_seq,), dtype=torch.int64, device=dev)
     total = torch.empty((1,), dtype=torch.int64, device=dev)
@@ -428,8 +431,6 @@ def gather_plan(sel_local: torch.Tensor, sel_rank: Optional[torch.Tensor], world
             chunk_bytes, int(sample_stride) // k, A.ptr(resident), A.ptr(plan), A.ptr(n_sel), A.ptr(total), A.ptr(status),
             A.stream_ptr(dev)), "msa_gather_plan_resident")
         return plan, n_sel, total
-    if report is not None and (total_host is not None or report.dtype != torch.int64 or report.numel() != 3 or not report.is_pinned()):
-        raise A.MsaError("gather_plan: report must be a pinned int64 [3] tensor, in place of total_host")
     call = A.lib().msa_gather_plan if report is None else A.lib().msa_gather_plan_report
     A.check(call(A.ptr(sel_local.contiguous()), A.ptr(sel_rank.contiguous() if sel_rank is not None else None),
                  n_seq, k, world, A.ptr(shard_doc_base), doc_chunk_len.numel(), A.ptr(doc_chunk_offset),

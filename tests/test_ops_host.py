@@ -57,6 +57,24 @@ def test_segments_wants_a_mask(library):
     assert not library.seen
 
 
+def test_a_report_is_written_or_refused(library):
+    """A resident plan writes no report; one that the kernel could not write whole is refused too."""
+    from msa_b200 import _cabi as A, ops
+    pinned = type("Pinned", (torch.Tensor,), {"is_pinned": lambda self: True})
+    reports = [torch.zeros(3, dtype=torch.int64).as_subclass(pinned), torch.zeros(6, dtype=torch.int64)[::2].as_subclass(pinned),
+               torch.zeros(3, dtype=torch.int32).as_subclass(pinned), torch.zeros(3, dtype=torch.int64)]
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        plan = lambda report, **kw: ops.gather_plan(new(2, 4), None, 1, new(1), new(9), new(9, dtype=torch.int32), new(1), 64, report=report, **kw)
+        with pytest.raises(A.MsaError):
+            plan(reports[0], resident=new(2, 4), sample_stride=16)
+        for report in reports[1:]:
+            with pytest.raises(A.MsaError):
+                plan(report)
+        assert not library.seen
+        plan(reports[0])
+    assert library.seen == ["msa_gather_plan_report"]
+
+
 def test_argmax_of_other_types(monkeypatch):
     from msa_b200 import lm_ops as K
     seen = []
