@@ -516,14 +516,17 @@ int msa_sparse_prefill_attn_tc(const void* q, int64_t q_stride_b, int64_t q_stri
  * Dense glue of a decode step (bf16).  No single reference function: they replace the chains of
  * elementwise torch kernels that transformers' Qwen3 modules issue between the GEMMs of a layer as
  * driven by src/msa/model.py:67-135 (Qwen3RMSNorm on q / k heads + apply_rotary_pos_emb; residual add
- * + Qwen3RMSNorm; SiLU(gate) * up).  Each computes in fp32 and rounds once per module boundary.
+ * + Qwen3RMSNorm; SiLU(gate) * up).  Each computes in fp32 and rounds its results once (x_out of
+ * msa_add_rmsnorm, the stream as it is stored, before its norm is taken).
  *
  * msa_qk_norm_rope: qkv row b = [n_q_heads*128 | n_kv_heads*128 | ...] (row_stride elements apart);
  *   q_out[b, h, :] = rope(rmsnorm(q head) * q_weight), k_out likewise; cos_table / sin_table: [n_seq, 128]
- *   (rotate-half convention, the sequence's position already applied).  head_dim must be 128.
+ *   (rotate-half convention, the sequence's position already applied).  head_dim must be 128; every pointer, the weights'
+ *   too, lies on 8 bytes and row_stride is a multiple of 4 elements, else the call is refused.
  * msa_add_rmsnorm: x_out = x + y (y, x_out may be NULL: no add), h_out = rmsnorm(x_out) * weight; rows of
  *   `hidden` contiguous elements.
  * msa_silu_mul: out[r, j] = silu(gate_up[r, j]) * gate_up[r, ffn + j], out rows contiguous.
+ * Both take even sizes and pointers on 4 bytes.
  */
 int msa_qk_norm_rope(const void* qkv, int64_t row_stride, int32_t n_seq, int32_t n_q_heads, int32_t n_kv_heads,
                      int32_t head_dim, const void* q_weight, const void* k_weight, float eps,

@@ -257,6 +257,7 @@ rope_table_kernel(const int64_t* __restrict__ pos, const float* __restrict__ inv
   sin_t[at] = sin_t[at + half] = sb;
 }
 
+static bool aligned4(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }
 static bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
 // Eight heads per warp once that fills the GPU's warp slots (148 SMs x 64), else one round of heads.
@@ -319,6 +320,7 @@ extern "C" int msa_add_rmsnorm(const void* x, const void* y, const void* weight,
                                int32_t hidden, void* x_out, void* h_out, void* stream) {
   MSA_REQUIRE(x && weight && h_out, "add_rmsnorm: null pointer");
   MSA_REQUIRE(n_rows >= 0 && hidden > 0 && hidden % 2 == 0 && hidden <= 12288, "add_rmsnorm: hidden must be even and <= 12288");
+  MSA_REQUIRE(aligned4(x) && aligned4(y) && aligned4(weight) && aligned4(x_out) && aligned4(h_out), "add_rmsnorm: pointers must be 4-byte aligned");
   if (n_rows == 0) return MSA_OK;
   const bool vec = hidden % 8 == 0 && aligned16(x) && aligned16(y) && aligned16(weight) && aligned16(x_out) && aligned16(h_out);
   // A warp per row from the row count on that gives every SM eight of them.
@@ -349,6 +351,7 @@ extern "C" int msa_silu_mul_parts(const void* gate, int64_t gate_stride, const v
                                   void* out, void* stream) {
   MSA_REQUIRE(gate && up && out, "silu_mul: null pointer");
   MSA_REQUIRE(n_rows >= 0 && ffn > 0 && ffn % 2 == 0 && gate_stride % 2 == 0 && up_stride % 2 == 0, "silu_mul: ffn and the row strides must be even");
+  MSA_REQUIRE(aligned4(gate) && aligned4(up) && aligned4(out), "silu_mul: pointers must be 4-byte aligned");
   if (n_rows == 0) return MSA_OK;
   const bool vec = ffn % 8 == 0 && gate_stride % 8 == 0 && up_stride % 8 == 0 && aligned16(gate) && aligned16(up) && aligned16(out);
   const long long grid = ((long long)n_rows * (ffn / (vec ? 8 : 2)) + 1023) / 1024;

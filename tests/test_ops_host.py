@@ -87,3 +87,31 @@ def test_argmax_of_other_types(monkeypatch):
         assert not seen
         assert K.argmax(new(3, 41, dtype=torch.float32)[:, :40]).shape == (3,)
     assert seen == ["msa_lm_argmax"]
+
+
+def test_rows_and_weights_of_unequal_sizes(library):
+    from msa_b200 import _cabi as A, ops
+    b16 = lambda *shape: new(*shape, dtype=torch.bfloat16)
+    with FakeTensorMode():
+        for x, y, w in (((4, 64), None, 32), ((4, 64), (4, 32), 64), ((4, 64), (2, 64), 64), ((4, 64), None, 128)):
+            with pytest.raises(A.MsaError):
+                ops.add_rmsnorm(b16(*x), None if y is None else b16(*y), b16(w), 1e-6)
+        for q, k, qw, kw in ((250, 128, 128, 128), (256, 100, 128, 128), (256, 128, 64, 128), (256, 128, 128, 256)):
+            with pytest.raises(A.MsaError):
+                ops.heads_norm_rope(b16(4, q), b16(4, k), b16(qw), b16(kw), 1e-6, b16(4, 128), b16(4, 128))
+        assert not library.seen
+        ops.add_rmsnorm(b16(4, 64), b16(4, 64), b16(64), 1e-6)
+        ops.heads_norm_rope(b16(4, 256), b16(4, 128), b16(128), b16(128), 1e-6, b16(2, 128), b16(2, 128))
+    assert library.seen == ["msa_add_rmsnorm", "msa_heads_norm_rope"]
+
+
+def test_pointers_off_the_pairs_are_refused():
+    """Two bf16 values are read at a time; a pointer between them is an error of the call, not of the GPU."""
+    from msa_b200 import _cabi as A
+    lib, at = A.lib(), 1 << 20
+    for shift in range(3):
+        gate, up, out = (at + 2 * (shift == i) for i in range(3))
+        assert lib.msa_silu_mul_parts(gate, 64, up, 64, 1, 64, out, 0) != 0 and b"4-byte aligned" in lib.msa_last_error()
+    for shift in range(5):
+        x, y, w, x_out, h = (at + 2 * (shift == i) for i in range(5))
+        assert lib.msa_add_rmsnorm(x, y, w, 1e-6, 1, 64, x_out, h, 0) != 0 and b"4-byte aligned" in lib.msa_last_error()
