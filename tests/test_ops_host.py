@@ -89,6 +89,17 @@ def test_argmax_of_other_types(monkeypatch):
     assert seen == ["msa_lm_argmax"]
 
 
+def test_forms_of_a_device(monkeypatch):
+    from msa_b200 import _cabi as A
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 1000 + index)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 5)
+    assert [A.stream_ptr(d) for d in (None, "cuda", torch.device("cuda"))] == [1005] * 3
+    assert [A.stream_ptr(d) for d in (2, "cuda:2", torch.device("cuda:2"))] == [1002] * 3
+    for d in ("cpu", torch.device("cpu")):
+        with pytest.raises(ValueError):
+            A.stream_ptr(d)
+
+
 def test_rows_and_weights_of_unequal_sizes(library):
     from msa_b200 import _cabi as A, ops
     b16 = lambda *shape: new(*shape, dtype=torch.bfloat16)
