@@ -45,9 +45,10 @@ class MSADecoderLayer(nn.Module):
         self._silu = type(self.mlp.act_fn) if config.hidden_act == "silu" else None
 
     def takes_fused(self, x) -> bool:
-        """Whether ``fused`` computes what ``forward`` does on ``x``: nobody watches or replaced the modules it steps over."""
+        """Whether ``fused`` computes what ``forward`` does on ``x``: nobody watches or replaced the modules it steps over (the
+        layer itself is asked about by the caller: a module in its place knows neither method)."""
         norms, mlp = (self.input_layernorm, self.post_attention_layernorm), self.mlp
-        return (plain_module(self, MSADecoderLayer) and plain_module(mlp, Qwen3MLP) and plain_module(mlp.act_fn, self._silu)
+        return (plain_module(mlp, Qwen3MLP) and plain_module(mlp.act_fn, self._silu)
                 and all(plain_module(n, Qwen3RMSNorm) and fused_ops(x, n.weight) for n in norms)
                 and x.shape[-1] % 2 == 0 and x.shape[-1] <= 12288)
 
@@ -101,7 +102,8 @@ class MSAModel(nn.Module):
         if position_ids is None:
             position_ids = torch.arange(hidden.shape[1], device=hidden.device).unsqueeze(0)
         position_embeddings = self._angles(hidden, position_ids)
-        if plain_module(self.norm, Qwen3RMSNorm) and fused_ops(hidden, self.norm.weight) and all(layer.takes_fused(hidden) for layer in self.layers):
+        if plain_module(self.norm, Qwen3RMSNorm) and fused_ops(hidden, self.norm.weight) and all(
+                plain_module(layer, MSADecoderLayer) and layer.takes_fused(hidden) for layer in self.layers):
             pending = None
             for layer in self.layers:
                 hidden, pending = layer.fused(hidden, pending, attention_mask, past_key_values, position_embeddings, doc_ids)

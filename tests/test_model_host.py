@@ -1,0 +1,48 @@
+"""When ``MSAModel`` steps over its modules' calls, on fake CUDA tensors: never where a module was replaced."""
+import pytest
+import torch
+import torch.nn as nn
+from torch._subclasses.fake_tensor import FakeTensorMode
+from transformers.models.qwen3.modeling_qwen3 import Qwen3MLP, Qwen3RMSNorm, Qwen3RotaryEmbedding
+
+pytestmark = pytest.mark.filterwarnings("ignore:Accessing the data pointer of FakeTensor")
+BF16 = torch.bfloat16
+
+
+class Wrapped(nn.Module):
+    """What an offload, quantisation or debug wrapper puts in a layer's place."""
+
+    def __init__(self, layer, seen):
+        super().__init__()
+        self.layer, self.seen = layer, seen
+
+    def forward(self, hidden_states, **kwargs):
+        self.seen.append(sorted(kwargs))
+        return hidden_states
+
+
+def small_model():
+    from msa_b200.configuration import MSAConfig
+    from msa_b200.model import MSAModel
+    cfg = MSAConfig(
+        msa_config=dict(router_layer_idx="1", aux_loss=False, aux_loss_method="INFONCE", decouple_router=True, top_k_docs=4, pooling_kernel_size=64,
+                        head_reduce_method="mean", query_reduce_method="max", chunk_reduce_method="max", decouple_pooling_mode="mean"),
+        hidden_size=256, num_attention_heads=4, num_key_value_heads=2, head_dim=128, num_hidden_layers=2, intermediate_size=520, vocab_size=64,
+        max_position_embeddings=4096, rms_norm_eps=1e-6)
+    cfg._attn_implementation = "eager"
+    return MSAModel(cfg).to(BF16).eval()
+
+
+def test_a_layer_in_another_layers_place_is_called(monkeypatch):
+    from msa_b200 import model as M
+    seen, fused = [], []
+    net = small_model()
+    for i in range(2):
+        net.layers[i] = Wrapped(net.layers[i], seen)
+    # a forward on the CPU, with the operands answered for as if they were on a GPU
+    monkeypatch.setattr(M, "fused_ops", lambda *t: True)
+    monkeypatch.setattr(M.ops, "add_rmsnorm", lambda *a: fused.append(a))
+    with torch.no_grad():
+        out = net(input_ids=torch.zeros(1, 3, dtype=torch.long), attention_mask=torch.ones(1, 3, dtype=torch.long))
+    assert seen == [["attention_mask", "doc_ids", "past_key_value", "position_embeddings"]] * 2 and not fused
+    assert out.last_hidden_state.shape == (1, 3, 256)
