@@ -50,8 +50,9 @@ def fused_ops(*tensors) -> bool:
 
 
 def plain_module(m, cls) -> bool:
-    """``m`` is exactly a ``cls`` that nobody hooked into, so that stepping over its call changes nothing."""
-    return (type(m) is cls and "forward" not in m.__dict__ and not nn_module._has_any_global_hook()
+    """``m`` is exactly a ``cls`` that nobody hooked into, with the class's own ``forward`` (not one that was put in its place), so
+    that stepping over its call changes nothing."""
+    return (type(m) is cls and "forward" not in m.__dict__ and cls.forward.__module__ == cls.__module__ and not nn_module._has_any_global_hook()
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
 
 

@@ -46,3 +46,13 @@ def test_a_layer_in_another_layers_place_is_called(monkeypatch):
         out = net(input_ids=torch.zeros(1, 3, dtype=torch.long), attention_mask=torch.ones(1, 3, dtype=torch.long))
     assert seen == [["attention_mask", "doc_ids", "past_key_value", "position_embeddings"]] * 2 and not fused
     assert out.last_hidden_state.shape == (1, 3, 256)
+
+
+@pytest.mark.parametrize("cls", [Qwen3RMSNorm, Qwen3MLP, Qwen3RotaryEmbedding])
+def test_a_forward_put_in_a_class_is_called(monkeypatch, cls):
+    from msa_b200.attention import plain_module
+    net = small_model()
+    m = {Qwen3RMSNorm: net.norm, Qwen3MLP: net.layers[0].mlp, Qwen3RotaryEmbedding: net.rotary_emb}[cls]
+    assert plain_module(m, cls)
+    monkeypatch.setattr(cls, "forward", lambda self, *a: a[0])
+    assert not plain_module(m, cls)
