@@ -38,13 +38,14 @@ from . import ops
 
 
 def fused_ops(*tensors) -> bool:
-    """Whether the fused kernels may stand in for eager operations on these: plain bf16 tensors on the GPU, aligned rows, and no
+    """Whether the fused kernels may stand in for eager operations on these: plain bf16 tensors on one GPU, aligned rows, and no
     gradient to keep (the kernels know none)."""
-    if torch.is_grad_enabled():
+    if torch.is_grad_enabled() or not tensors[0].is_cuda:
         return False
+    device = tensors[0].get_device()
     for t in tensors:
-        if not ((type(t) is torch.Tensor or type(t) is nn.Parameter) and t.dtype == torch.bfloat16 and t.is_cuda and t.stride(-1) == 1
-                and t.data_ptr() % 16 == 0):
+        if not ((type(t) is torch.Tensor or type(t) is nn.Parameter) and t.dtype == torch.bfloat16 and t.get_device() == device
+                and t.stride(-1) == 1 and t.data_ptr() % 16 == 0):
             return False
     return True
 

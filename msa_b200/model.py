@@ -26,7 +26,7 @@ from .cache import create_cache
 
 def add_norm(x, branch, norm):
     """``(x + branch, norm(x + branch))`` of ``[B, S, hidden]``, in one launch where the operands allow it."""
-    if not (fused_ops(x, norm.weight) and (branch is None or (fused_ops(branch) and branch.shape == x.shape))):
+    if not (fused_ops(x, norm.weight) if branch is None else fused_ops(x, norm.weight, branch) and branch.shape == x.shape):
         x = x if branch is None else x + branch
         return x, norm(x)
     flat = lambda t: t if t is None else t.reshape(-1, t.shape[-1]).contiguous()
@@ -60,7 +60,7 @@ class MSADecoderLayer(nn.Module):
                                  past_key_value=past_key_value)
         x, h = add_norm(x, attn, self.post_attention_layernorm)
         gate, up = self.mlp.gate_proj(h), self.mlp.up_proj(h)
-        if fused_ops(gate) and fused_ops(up) and gate.shape == up.shape and gate.shape[-1] % 2 == 0:
+        if fused_ops(gate, up) and gate.shape == up.shape and gate.shape[-1] % 2 == 0:
             act = ops.silu_mul_parts(gate.flatten(0, 1), up.flatten(0, 1)).view(gate.shape)
         else:
             act = F.silu(gate) * up

@@ -56,3 +56,17 @@ def test_a_forward_put_in_a_class_is_called(monkeypatch, cls):
     assert plain_module(m, cls)
     monkeypatch.setattr(cls, "forward", lambda self, *a: a[0])
     assert not plain_module(m, cls)
+
+
+def test_operands_on_two_devices_are_not_fused():
+    from msa_b200 import attention
+    with FakeTensorMode(), torch.no_grad():
+        at = lambda d: torch.empty(4, 64, dtype=BF16, device=d)
+        plain = type(at("cuda:0"))
+        real, attention.torch = attention.torch, type("T", (), {"Tensor": plain, "bfloat16": BF16, "is_grad_enabled": staticmethod(lambda: False)})
+        try:
+            assert attention.fused_ops(at("cuda:0"), at("cuda:0"))
+            assert not attention.fused_ops(at("cuda:0"), at("cuda:1")) and not attention.fused_ops(at("cuda:0"), at("cpu"))
+            assert not attention.fused_ops(at("cpu"), at("cuda:0"))
+        finally:
+            attention.torch = real
