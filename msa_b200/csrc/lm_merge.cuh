@@ -15,7 +15,7 @@ struct MergeParams {
 // One block per (sequence, head).  Launched early (programmatic dependent launch): waits for the partial results before
 // it reads them.
 static __global__ void __launch_bounds__(128) merge_partials_kernel(const MergeParams p) {
-  grid_launch_dependents();
+  let_product_start((int)(gridDim.x / (unsigned)p.heads));
   const long long row = blockIdx.x;
   const int b = (int)(row / p.heads), h = (int)(row % p.heads);
   const int c = threadIdx.x * 4, splits = p.splits, cols = p.cols;

@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ 
 // so that a product over both keeps 16 significant bits.
 template <typename T>
 __global__ void __launch_bounds__(256) tanh_split_kernel(const float* __restrict__ x, int cols, int parts, long long n, T* __restrict__ out) {
-  grid_launch_dependents();
+  if (n <= (long long)kEarlyRows * cols) grid_launch_dependents();
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
     const long long r = i / cols;
     const int c = (int)(i - r * cols);

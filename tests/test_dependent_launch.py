@@ -42,3 +42,15 @@ def test_what_earlier_kernels_write_is_read_behind_the_wait():
              for p in params.split(",") if "const" in p and "__restrict__" in p and (name, p.split()[-1]) not in CONSTANT]
     assert not early
     assert not [name for name, _, body in kernels() if "grid_dependency_wait()" in body and "__restrict__" in body]
+
+
+def test_a_library_product_is_not_let_in_early():
+    """Kernels in front of a product let it start while they run only where it is the few-row one, which has weights to fetch; those
+    that always let their dependents start stand in front of a kernel of this package."""
+    always = {"fold_kernel",                                        # route_dec_kernel (any other waits for its end)
+              "live_blocks_kernel",                                  # pack_rows_kernel
+              "moe_topk_kernel", "moe_sort_kernel", "moe_gemm_tc_kernel",
+              "group_decode_kernel", "latent_decode_kernel",         # merge_partials_kernel
+              "rows_gemm_kernel"}
+    assert {name for name, _, body in kernels() if re.search(r"(?<!\) )grid_launch_dependents\(\);", body)} <= always
+    assert "if (rows <= kEarlyRows) grid_launch_dependents();" in open(os.path.join(CSRC, "lm_common.cuh")).read()
