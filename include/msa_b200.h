@@ -167,7 +167,9 @@ int msa_route_scores(const void* q_folded, const float* row_bias, int32_t dtype,
 
 /* The same with scratch for skipping padding (both may be NULL): the tensor-core kernel lists the 16-row blocks that hold a row
  * whose bias is not -inf in live_blocks (device int32 [n_seq*s_pad/16 + 1]), copies them to packed_rows (as large as q_folded)
- * and contracts those only.  Same results. */
+ * unless all are listed, and contracts those only.  Same results.  msa_route_live_rows: the rows of q_folded where a call of these
+ * sizes (bf16, row-major keys) uses the scratch, 0 where it does not. */
+int msa_route_live_rows(int32_t n_seq, int32_t s_pad, int32_t n_chunks);
 int msa_route_scores_live(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
                      int32_t s_pad, const void* rk, int64_t rk_chunk_stride, int32_t n_chunks,
                      int32_t kdim, const int32_t* chunk_doc, float alpha, uint32_t* score_keys,

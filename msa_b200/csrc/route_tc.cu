@@ -405,12 +405,12 @@ constexpr int kBlockRows = 16, kTileBlocks = kPairBN / kBlockRows;
 // kLive: questions of one batch differ in length, so a fixed layout of s_pad rows per sequence holds padding (a quarter of the
 // rows when lengths spread over half to full).  The 16-row blocks that hold a valid token are listed and copied next to one
 // another first (pack_rows_kernel); the tiles run over those, any tile may hold several sequences, and the list's length is read
-// here, so the host never waits for it.  (Fetching the blocks in place, eight 16-row boxes per stage, is bound by the copy
+// here, so the host never waits for it; where every block is listed, the rows are read where they are and nothing is copied.  (Fetching the blocks in place, eight 16-row boxes per stage, is bound by the copy
 // engine: 2.95 ms for 48 x (100..200) tokens x 190,000 chunks, as slow as all 208-row tiles of the one-CTA kernel; over packed rows 2.16 ms.)
 template <bool kLive>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 route_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_q,
-                     const RouteTcParams args) {
+                     const __grid_constant__ CUtensorMap tmap_packed, const RouteTcParams args) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ uint64_t s_full[kMaxStages], s_empty[kMaxStages], s_acc_full[2], s_acc_empty[2], s_drain;
   __shared__ uint32_t s_tmem_base;
@@ -452,6 +452,7 @@ route_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
   if (warp == 4) {
     // ------------------------------- TMA producer (each CTA loads its halves) ----------
     if (lane == 0) {
+      const CUtensorMap* rows = kLive && n_live * kBlockRows < p.n_rows ? &tmap_packed : &tmap_q;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -463,7 +464,7 @@ route_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
           if (leader) mbar_expect_tx(&s_full[stage], 2 * stage_bytes);  // both CTAs' bytes land on this barrier
           const uint32_t bar = map_to_cta(smem_u32(&s_full[stage]), 0);
           tma_load_2d_pair(sa, &tmap_k, kb * kBK, tc.ct * kPairBM + (int)rank * kBM, bar);
-          tma_load_2d_pair(sa + half_bytes, &tmap_q, kb * kBK, tc.qt * kPairBN + (int)rank * (kPairBN / 2), bar);
+          tma_load_2d_pair(sa + half_bytes, rows, kb * kBK, tc.qt * kPairBN + (int)rank * (kPairBN / 2), bar);
           if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -583,12 +584,13 @@ __global__ void __launch_bounds__(1024) live_blocks_kernel(const float* __restri
   if (threadIdx.x == 0) live[0] = s_base;
 }
 
-// Listed block i of rows [.., kdim] -> block i of `packed`; one CTA per block of 16 rows, eight 16-byte loads in flight per
+// Listed block i of rows [.., kdim] -> block i of `packed`, unless every block is listed; one CTA per block of 16 rows, eight 16-byte loads in flight per
 // thread (7,700 rows of 2 KB: 5 us).  Launched early, while the list is still being written: it is read behind the wait, through
 // plain pointers.
 __global__ void __launch_bounds__(256) pack_rows_kernel(const uint4* rows, const int32_t* live, int vecs, uint4* __restrict__ packed) {
   grid_dependency_wait();
-  if ((int)blockIdx.x >= live[0]) return;
+  const int n_live = live[0];
+  if ((int)blockIdx.x >= n_live || n_live == (int)gridDim.x) return;      // beyond the list, or every block is on it
   const uint4* src = rows + (long long)live[1 + blockIdx.x] * vecs;
   uint4* dst = packed + (long long)blockIdx.x * vecs;
   for (int first = threadIdx.x; first < vecs; first += 2048) {
@@ -625,6 +627,13 @@ __global__ void wait_selftest_kernel(unsigned long long limit_ns, int32_t* statu
 }
 
 // ---- host side ------------------------------------------------------------------------
+// Sequences of several rows each run on CTA pairs over their blocks of valid rows where these fill the GPU: two 128-chunk tiles or
+// more for every SM and 256 rows.
+static bool pairs_by_blocks(long long n_rows, int s_pad, int n_chunks, int n_sm) {
+  static const bool off = getenv("MSA_B200_ROUTE_NO_PAIR") != nullptr;
+  return !off && s_pad > 1 && (n_rows + kPairBN - 1) / kPairBN * ((n_chunks + kBM - 1) / kBM) >= 2ll * n_sm;
+}
+
 int launch_route_tc(const void* qf, const float* row_bias, int n_seq, int s_pad, const void* rk, int64_t rk_stride,
                     int n_chunks, int kdim, const int32_t* chunk_doc, int n_docs, float alpha, float min_val,
                     uint32_t* keys, int64_t table_stride, int32_t* status, bool blocked, int32_t* live, void* packed, cudaStream_t stream) {
@@ -685,13 +694,12 @@ int launch_route_tc(const void* qf, const float* row_bias, int n_seq, int s_pad,
   else if (epi_warps == 8) MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_kernel<8>, smem, smem_set_8));
   else MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_kernel<4>, smem, smem_set));
   const long long n_tiles = (long long)p.n_ctiles * p.n_qtiles;
-  // Tensor-bound shapes (enough chunk tiles to fill the GPU) run on CTA pairs: over the blocks of valid rows where sequences
-  // have several rows each, else over full 256-row query tiles.
+  // Tensor-bound shapes (enough chunk tiles to fill the GPU) run on CTA pairs: over the blocks of valid rows where there is
+  // scratch for them, else over full 256-row query tiles.
   static const bool pair_off = getenv("MSA_B200_ROUTE_NO_PAIR") != nullptr;
-  const bool by_blocks = live && packed && s_pad > 1;
+  const bool by_blocks = live && packed && pairs_by_blocks(p.n_rows, s_pad, n_chunks, n_sm);
   const long long n_qtiles_256 = (p.n_rows + kPairBN - 1) / kPairBN;
-  if (!pair_off && !blocked && (by_blocks ? n_qtiles_256 * p.n_ctiles >= 2ll * n_sm
-                                          : p.bn == kPairBN && p.n_rows % kPairBN == 0 && n_tiles >= 2ll * n_sm)) {
+  if (!pair_off && !blocked && (by_blocks || (p.bn == kPairBN && p.n_rows % kPairBN == 0 && n_tiles >= 2ll * n_sm))) {
     RouteTcParams p2 = p;
     p2.bn = kPairBN;
     p2.n_ctiles = (n_chunks + kPairBM - 1) / kPairBM;
@@ -701,19 +709,20 @@ int launch_route_tc(const void* qf, const float* row_bias, int n_seq, int s_pad,
     if (p2.qgroup > p2.n_qtiles) p2.qgroup = p2.n_qtiles;
     p2.stages = 6;  // 6 x 32 KB
     p2.live = by_blocks ? live : nullptr;
-    CUtensorMap map_q2;
-    rc = make_map(&map_q2, by_blocks ? packed : qf, (uint64_t)p.n_rows, (uint64_t)kdim, (uint64_t)kdim, kBK, (uint32_t)(kPairBN / 2));
-    if (rc != MSA_OK) return rc;
+    CUtensorMap map_q2, map_packed;
+    MSA_OK_OR_RETURN(make_map(&map_q2, qf, (uint64_t)p.n_rows, (uint64_t)kdim, (uint64_t)kdim, kBK, (uint32_t)(kPairBN / 2)));
+    MSA_OK_OR_RETURN(make_map(&map_packed, by_blocks ? packed : qf, (uint64_t)p.n_rows, (uint64_t)kdim, (uint64_t)kdim, kBK,
+                              (uint32_t)(kPairBN / 2)));
     const size_t smem2 = (size_t)p2.stages * 2 * kBM * kBK * 2 + 1024;
     long long clusters = n_sm / 2;
     if (clusters > (long long)p2.n_ctiles * p2.n_qtiles) clusters = (long long)p2.n_ctiles * p2.n_qtiles;
     if (by_blocks) {
       MSA_OK_OR_RETURN(pack_live_rows(qf, row_bias, p.n_rows / kBlockRows, kdim, live, packed, stream));
       MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_pair_kernel<true>, smem2, pair_live_set));
-      route_tc_pair_kernel<true><<<(int)(2 * clusters), kTcThreads, smem2, stream>>>(map_k, map_q2, p2);
+      route_tc_pair_kernel<true><<<(int)(2 * clusters), kTcThreads, smem2, stream>>>(map_k, map_q2, map_packed, p2);
     } else {
       MSA_OK_OR_RETURN(ensure_dynamic_smem(route_tc_pair_kernel<false>, smem2, pair_set));
-      route_tc_pair_kernel<false><<<(int)(2 * clusters), kTcThreads, smem2, stream>>>(map_k, map_q2, p2);
+      route_tc_pair_kernel<false><<<(int)(2 * clusters), kTcThreads, smem2, stream>>>(map_k, map_q2, map_packed, p2);
     }
     MSA_LAUNCH_OK("route_tc_pair_kernel");
     return MSA_OK;
@@ -727,6 +736,13 @@ int launch_route_tc(const void* qf, const float* row_bias, int n_seq, int s_pad,
 }
 
 }  // namespace msa
+
+extern "C" int msa_route_live_rows(int32_t n_seq, int32_t s_pad, int32_t n_chunks) {
+  if (n_seq <= 0 || s_pad <= 0 || n_chunks <= 0) return 0;
+  int n_sm = 0;
+  if (msa::device_sm_count(&n_sm) != MSA_OK) return 0;
+  return msa::pairs_by_blocks((long long)n_seq * s_pad, s_pad, n_chunks, n_sm) ? n_seq * s_pad : 0;
+}
 
 extern "C" int msa_selftest_bounded_wait(int64_t limit_ns, int32_t* status, void* stream) {
   MSA_REQUIRE(status && limit_ns > 0 && limit_ns <= 1000000000ll, "selftest: limit must be in (0, 1e9] ns");

@@ -193,7 +193,8 @@ def route_scores(q_folded: torch.Tensor, row_bias: torch.Tensor, n_seq: int, s_p
         status = torch.zeros(4, dtype=torch.int32, device=dev)
     # questions of unequal length: scratch for the list of 16-row blocks that hold a valid token, and for those rows
     live = packed = None
-    if s_pad > 1 and rk.dtype == torch.bfloat16 and not blocked and row_bias.data_ptr() % 16 == 0:
+    if (s_pad > 1 and rk.dtype == torch.bfloat16 and not flags & (A.ROUTE_KEYS_BLOCKED | A.ROUTE_FORCE_SIMT) and row_bias.data_ptr() % 16 == 0
+            and A.lib().msa_route_live_rows(n_seq, s_pad, c)):
         live, packed = torch.empty(n_seq * s_pad // 16 + 1, dtype=torch.int32, device=dev), torch.empty_like(q_folded)
     A.check(A.lib().msa_route_scores_live(A.ptr(q_folded), A.ptr(row_bias), A.dtype_code(rk.dtype), n_seq, s_pad,
                                           A.ptr(rk2), rk2.stride(0) if c > 0 else kdim, c, kdim, A.ptr(chunk_doc),
