@@ -135,13 +135,16 @@ def ptr(t) -> int:
 def stream_ptr(device=None) -> int:
     """The handle of the current stream of ``device`` (as ``torch.cuda.current_stream`` takes it), without a stream object around it
     (a decode token of the memory model, some seventy calls: 791 us with the objects, 706 without and with a plainer check of operands)."""
-    if isinstance(device, str):
-        device = torch.device(device)
-    if isinstance(device, torch.device):
-        if device.type != "cuda":
-            raise ValueError(f"expected a CUDA device, got {device}")
-        device = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device is None else device)
+    index = device.index if isinstance(device, torch.device) else device
+    if not isinstance(index, int):                      # a name, a device without an index or nothing: the current one of its type
+        if device is not None:
+            device = torch.device(device)
+            if device.type != "cuda":
+                raise ValueError(f"expected a CUDA device, got {device}")
+            index = device.index
+        if index is None:
+            index = torch.cuda.current_device()
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 def need_cuda(*tensors) -> None:

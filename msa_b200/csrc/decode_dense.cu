@@ -260,12 +260,14 @@ rope_table_kernel(const int64_t* __restrict__ pos, const float* __restrict__ inv
 static bool aligned4(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }
 static bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
 
-// Eight heads per warp once that fills the GPU's warp slots (148 SMs x 64), else one round of heads.
+// Eight heads per warp once that fills the GPU's warp slots (64 an SM), else one round of heads.
 static int launch_heads_norm_rope(const HeadsNormRope& p, void* stream) {
   const int heads = p.n_q + p.n_kv;
   const bool wide = aligned16(p.q) && aligned16(p.k) && aligned16(p.q_w) && aligned16(p.k_w) && aligned16(p.cos_t) && aligned16(p.sin_t) &&
                     aligned16(p.q_out) && aligned16(p.k_out) && p.q_stride % 8 == 0 && p.k_stride % 8 == 0;
-  const bool many = (long long)p.n_rows * ((heads + 7) / 8) >= 148 * 64;
+  int n_sm = 0;
+  MSA_OK_OR_RETURN(device_sm_count(&n_sm));
+  const bool many = (long long)p.n_rows * ((heads + 7) / 8) >= 64ll * n_sm;
   const int per_warp = many ? 8 : wide ? 4 : 2;
   const unsigned grid = (unsigned)(((long long)p.n_rows * ((heads + per_warp - 1) / per_warp) + 7) / 8);
   cudaStream_t st = (cudaStream_t)stream;
@@ -324,7 +326,9 @@ extern "C" int msa_add_rmsnorm(const void* x, const void* y, const void* weight,
   if (n_rows == 0) return MSA_OK;
   const bool vec = hidden % 8 == 0 && aligned16(x) && aligned16(y) && aligned16(weight) && aligned16(x_out) && aligned16(h_out);
   // A warp per row from the row count on that gives every SM eight of them.
-  const bool many = n_rows >= 148 * 8;
+  int n_sm = 0;
+  MSA_OK_OR_RETURN(device_sm_count(&n_sm));
+  const bool many = n_rows >= 8 * n_sm;
 #define MSA_ADD_RMSNORM(T, NV) launch_add_rmsnorm<T, NV>(x, y, weight, eps, n_rows, hidden, x_out, h_out, stream)
   if (vec && many && hidden <= 4096) {
     if (hidden <= 1024) MSA_ADD_RMSNORM(32, 4);

@@ -811,8 +811,8 @@ def add_rmsnorm(x: torch.Tensor, y: Optional[torch.Tensor], weight: torch.Tensor
     if x.dtype != torch.bfloat16 or not x.is_contiguous() or (y is not None and not y.is_contiguous()):
         raise A.MsaError("add_rmsnorm: bf16 contiguous rows expected")
     n, hidden = x.shape
-    if weight.numel() != hidden or (y is not None and y.shape != x.shape):
-        raise A.MsaError("add_rmsnorm: a branch of the rows' shape and one weight per column expected")
+    if weight.numel() != hidden or (y is not None and y.numel() != n * hidden):
+        raise A.MsaError("add_rmsnorm: a branch of the rows' size and one weight per column expected")
     x_new = torch.empty_like(x) if y is not None else x
     h = torch.empty_like(x)
     A.check(A.lib().msa_add_rmsnorm(A.ptr(x), A.ptr(y), A.ptr(weight), float(eps), n, hidden,
@@ -841,14 +841,15 @@ def heads_norm_rope(q: torch.Tensor, k: torch.Tensor, q_weight: torch.Tensor, k_
     rows = q.shape[0]
     if any(t.dtype != torch.bfloat16 or t.stride(-1) != 1 for t in (q, k, q_weight, k_weight)) or k.shape[0] != rows:
         raise A.MsaError("heads_norm_rope: bf16 rows with a contiguous feature axis expected")
-    if q.shape[1] % 128 or k.shape[1] % 128 or q_weight.numel() != 128 or k_weight.numel() != 128:
+    q_cols, k_cols = q.shape[1], k.shape[1]
+    if q_cols % 128 or k_cols % 128 or q_weight.numel() != 128 or k_weight.numel() != 128:
         raise A.MsaError("heads_norm_rope: whole heads of 128 and one weight per dimension expected")
     cos, sin = cos.reshape(-1, 128).contiguous(), sin.reshape(-1, 128).contiguous()
     if cos.dtype != torch.bfloat16 or sin.dtype != torch.bfloat16 or cos.shape != sin.shape:
         raise A.MsaError("heads_norm_rope: bf16 cos / sin tables of equal shape expected")
     q_out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
     k_out = torch.empty(k.shape, dtype=k.dtype, device=k.device)
-    A.check(A.lib().msa_heads_norm_rope(A.ptr(q), q.stride(0), A.ptr(k), k.stride(0), rows, q.shape[1] // 128, k.shape[1] // 128, 128,
+    A.check(A.lib().msa_heads_norm_rope(A.ptr(q), q.stride(0), A.ptr(k), k.stride(0), rows, q_cols // 128, k_cols // 128, 128,
                                         A.ptr(q_weight), A.ptr(k_weight), float(eps), A.ptr(cos), A.ptr(sin), cos.shape[0], A.ptr(q_out),
                                         A.ptr(k_out), A.stream_ptr(q.device)), "msa_heads_norm_rope")
     return q_out, k_out
