@@ -260,115 +260,106 @@ question_plan_kernel(const uint8_t* __restrict__ valid, int n_rows, int row_len,
   if (threadIdx.x == 0) { report[0] = s_max; report[1] = s_runs; report[2] = status ? status[0] : 0; }
 }
 
-// Token lists and segment offsets of a block's documents and templates (tables 0 and 1): a document's segment is a stretch of listed
-// tokens of one row and id, a template's all listed tokens of a row.  One block walks tiles of 4096 tokens with two scans each
-// (places in the list, starts of segments), so that nothing but the eight words of the report has to reach the host: as
-// tensor operations the tables took thirteen read-backs, during which the GPU waited; this takes 71 us for 32,002 tokens (11 for 4000).
+// Token lists and segment offsets of a block's documents and templates (tables 0 and 1, a block of threads each): a document's segment
+// is a stretch of listed tokens of one row and id, a template's all listed tokens of a row.  The block walks tiles of 8192 tokens, 256 a
+// warp in eight rounds of neighbours: listed tokens and starts of segments are bit masks of a round, so that places and the token before come
+// from counting bits, and two barriers a tile join the warps.  Nothing but the eight words of the report has to reach the host: as
+// tensor operations the tables took thirteen read-backs, during which the GPU waited.  Bound by the chain of loads and barriers of a tile.
+// With its read-back, on the host's clock, and the tensor operations: 4000 tokens 56 and 639 us, 32,000 75 and 672, 500,000 355 and 679,
+// 1,000,000 (the largest block by default) 653 and 676.  A block for both tables with neighbours in one thread: 131 and 2219 us for 32,000 and
+// 1,000,000.
 struct SegmentTables {
   int32_t *tok[2], *off[2];
   int32_t* report;            // per table: tokens, segments, longest, whether every segment is a run; the last word of table 1:
 };                            // tokens of the template, listed or not
 
-constexpr int kSegThreads = 1024, kSegPer = 4;
+constexpr int kSegThreads = 1024, kSegRounds = 8;
 
 __global__ void __launch_bounds__(kSegThreads)
 segments_kernel(const int64_t* __restrict__ doc_ids, const uint8_t* __restrict__ valid, int n, int row_len, const SegmentTables t) {
-  __shared__ int s_scan[2][32];             // listed tokens and starts of segments of every warp
-  __shared__ int s_last_tok[32];            // last listed token of a warp's stretch, -1: none
+  __shared__ int s_tokens[32], s_last[32], s_starts[32];     // of every warp: listed tokens, the last of them (-1: none), starts of segments
   __shared__ int s_runs, s_longest, s_template;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) s_template = 0;
-  for (int k = 0; k < 2; ++k) {
-    int n_tok = 0, n_seg = 0, before = -1;  // so far: listed tokens, segments, the last listed token (the same in every thread)
-    if (threadIdx.x == 0) { s_runs = 1; s_longest = 0; }
-    __syncthreads();
-    for (int base = 0; base < n; base += kSegThreads * kSegPer) {
-      const int i0 = base + threadIdx.x * kSegPer;
-      int64_t id[kSegPer];
-      bool on[kSegPer];
-      int count = 0, last = -1, templ = 0;
+  const unsigned all = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = blockIdx.x;
+  const unsigned before_lane = (1u << lane) - 1u;
+  int32_t *tok = k == 0 ? t.tok[0] : t.tok[1], *off = k == 0 ? t.off[0] : t.off[1];
+  int n_tok = 0, n_seg = 0, last = -1;      // so far: listed tokens, segments, the last listed token (the same in every thread)
+  if (threadIdx.x == 0) { s_template = 0; s_runs = 1; s_longest = 0; }
+  __syncthreads();
+  for (int base = 0; base < n; base += kSegThreads * kSegRounds) {
+    const int first = base + warp * 32 * kSegRounds;
+    int64_t id[kSegRounds];
+    unsigned listed[kSegRounds];
+    int count = 0, mine = -1, templ = 0;
 #pragma unroll
-      for (int j = 0; j < kSegPer; ++j) {
-        const int i = i0 + j;
-        id[j] = i < n ? doc_ids[i] : 0;
-        on[j] = i < n && valid[i] && (k == 0 ? id[j] > 0 : id[j] == -2);
-        templ += i < n && id[j] == -2;
-        if (on[j]) { ++count; last = i; }
-      }
-      if (k == 1) {
-        templ = __reduce_add_sync(0xffffffffu, templ);
-        if (lane == 0 && templ) atomicAdd(&s_template, templ);
-      }
-      // the listed token before this thread's first one
-      int upto = last;                      // last listed token of the warp's lanes up to this one
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto = max(upto, x);
-      }
-      int prev = __shfl_up_sync(0xffffffffu, upto, 1);
-      if (lane == 0) prev = -1;
-      if (lane == 31) s_last_tok[warp] = upto;
-      __syncthreads();
-      if (prev < 0) {
-        prev = before;
-        for (int w = 0; w < warp; ++w) prev = max(prev, s_last_tok[w]);
-      }
-      bool start[kSegPer];
-      int starts = 0, p = prev;
-      bool runs = true;
-#pragma unroll
-      for (int j = 0; j < kSegPer; ++j) {
-        start[j] = false;
-        if (!on[j]) continue;
-        const int i = i0 + j;
-        const bool same = p >= 0 && p / row_len == i / row_len && (k == 1 || doc_ids[p] == id[j]);
-        start[j] = !same;
-        if (same && p != i - 1) runs = false;
-        starts += start[j];
-        p = i;
-      }
-      if (!runs) s_runs = 0;
-      int tok_at = count, seg_at = starts;  // exclusive prefixes over the block
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, tok_at, o), y = __shfl_up_sync(0xffffffffu, seg_at, o);
-        if (lane >= o) { tok_at += x; seg_at += y; }
-      }
-      if (lane == 31) { s_scan[0][warp] = tok_at; s_scan[1][warp] = seg_at; }
-      __syncthreads();
-      int tok0 = 0, seg0 = 0, tok_all = 0, seg_all = 0, end = before;
-      for (int w = 0; w < 32; ++w) {
-        if (w == warp) { tok0 = tok_all; seg0 = seg_all; }
-        tok_all += s_scan[0][w];
-        seg_all += s_scan[1][w];
-        end = max(end, s_last_tok[w]);
-      }
-      tok_at += n_tok + tok0 - count;
-      seg_at += n_seg + seg0 - starts;
-#pragma unroll
-      for (int j = 0; j < kSegPer; ++j)
-        if (on[j]) {
-          if (start[j]) t.off[k][seg_at++] = tok_at;
-          t.tok[k][tok_at++] = i0 + j;
-        }
-      n_tok += tok_all;
-      n_seg += seg_all;
-      before = end;
-      __syncthreads();                      // the shared words are free again
+    for (int j = 0; j < kSegRounds; ++j) {
+      const int i = first + 32 * j + lane;
+      id[j] = i < n ? doc_ids[i] : 0;
+      listed[j] = i < n && valid[i] ? 1u : 0u;
     }
-    if (threadIdx.x == 0) t.off[k][n_seg] = n_tok;
-    __syncthreads();                        // this block's offsets are there for all of its threads
-    int longest = 0;
-    for (int i = threadIdx.x; i < n_seg; i += kSegThreads) longest = max(longest, t.off[k][i + 1] - t.off[k][i]);
-    longest = __reduce_max_sync(0xffffffffu, longest);
-    if (lane == 0 && longest) atomicMax(&s_longest, longest);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      t.report[4 * k] = n_tok; t.report[4 * k + 1] = n_seg; t.report[4 * k + 2] = s_longest;
-      t.report[4 * k + 3] = k == 0 ? s_runs : s_template;
+#pragma unroll
+    for (int j = 0; j < kSegRounds; ++j) {
+      listed[j] = __ballot_sync(all, listed[j] != 0 && (k == 0 ? id[j] > 0 : id[j] == -2));
+      if (k == 1) templ += __popc(__ballot_sync(all, id[j] == -2));
+      count += __popc(listed[j]);
+      if (listed[j]) mine = first + 32 * j + 31 - __clz(listed[j]);
+    }
+    if (lane == 0) {
+      s_tokens[warp] = count;
+      s_last[warp] = mine;
+      if (templ) atomicAdd(&s_template, templ);
     }
     __syncthreads();
+    const int tokens = s_tokens[lane], lasts = s_last[lane];
+    int tok_at = n_tok + __reduce_add_sync(all, lane < warp ? tokens : 0);
+    n_tok += __reduce_add_sync(all, tokens);
+    int p = max(last, __reduce_max_sync(all, lane < warp ? lasts : -1));   // the listed token before this round
+    last = max(last, __reduce_max_sync(all, lasts));
+    int64_t pid = count > 0 && p >= 0 ? doc_ids[p] : 0;
+    unsigned starts[kSegRounds];
+    int n_start = 0;
+    bool runs = true;
+#pragma unroll
+    for (int j = 0; j < kSegRounds; ++j) {
+      const int i = first + 32 * j + lane, row0 = row_len == n ? 0 : i / row_len * row_len;
+      const unsigned below = listed[j] & before_lane;
+      const int64_t near_id = __shfl_sync(all, id[j], below ? 31 - __clz(below) : 0);
+      const int prev = below ? first + 32 * j + 31 - __clz(below) : p;
+      const bool on = listed[j] >> lane & 1u, same = prev >= 0 && prev >= row0 && (k == 1 || (below ? near_id : pid) == id[j]);
+      starts[j] = __ballot_sync(all, on && !same);
+      if (on && same && prev != i - 1) runs = false;
+      n_start += __popc(starts[j]);
+      const int64_t last_id = __shfl_sync(all, id[j], listed[j] ? 31 - __clz(listed[j]) : 0);
+      if (listed[j]) {
+        p = first + 32 * j + 31 - __clz(listed[j]);
+        pid = last_id;
+      }
+    }
+    if (!runs) s_runs = 0;
+    if (lane == 0) s_starts[warp] = n_start;
+    __syncthreads();                        // (s_tokens and s_last have been read, too: the next tile may write them)
+    const int of_warp = s_starts[lane];
+    int seg_at = n_seg + __reduce_add_sync(all, lane < warp ? of_warp : 0);
+    n_seg += __reduce_add_sync(all, of_warp);
+#pragma unroll
+    for (int j = 0; j < kSegRounds; ++j) {
+      const int at = tok_at + __popc(listed[j] & before_lane);
+      if (listed[j] >> lane & 1u) tok[at] = first + 32 * j + lane;
+      if (starts[j] >> lane & 1u) off[seg_at + __popc(starts[j] & before_lane)] = at;
+      tok_at += __popc(listed[j]);
+      seg_at += __popc(starts[j]);
+    }
+  }
+  if (threadIdx.x == 0) off[n_seg] = n_tok;
+  __syncthreads();                          // this block's offsets are there for all of its threads
+  int longest = 0;
+  for (int i = threadIdx.x; i < n_seg; i += kSegThreads) longest = max(longest, off[i + 1] - off[i]);
+  longest = __reduce_max_sync(all, longest);
+  if (lane == 0 && longest) atomicMax(&s_longest, longest);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    t.report[4 * k] = n_tok; t.report[4 * k + 1] = n_seg; t.report[4 * k + 2] = s_longest;
+    t.report[4 * k + 3] = k == 0 ? s_runs : s_template;
   }
 }
 
@@ -429,7 +420,7 @@ extern "C" int msa_segments(const int64_t* doc_ids, const uint8_t* valid, int32_
   MSA_REQUIRE(tok_docs && off_docs && tok_template && off_template && report, "segments: null pointer");
   MSA_REQUIRE((doc_ids && valid) || (int64_t)n_rows * row_len == 0, "segments: null pointer");
   const SegmentTables t{{tok_docs, tok_template}, {off_docs, off_template}, report};
-  segments_kernel<<<1, kSegThreads, 0, (cudaStream_t)stream>>>(doc_ids, valid, n_rows * row_len, row_len > 0 ? row_len : 1, t);
+  segments_kernel<<<2, kSegThreads, 0, (cudaStream_t)stream>>>(doc_ids, valid, n_rows * row_len, row_len > 0 ? row_len : 1, t);
   MSA_LAUNCH_OK("segments_kernel");
   return MSA_OK;
 }

@@ -1,5 +1,5 @@
 """The two small planning kernels of the attention layer (``ops.segments``, ``ops.question_plan``) against plain Python, at the edges
-of their tiles (4 tokens a thread, 4096 a tile) and of what they are given."""
+of their tiles (8 tokens a thread, 8192 a tile) and of what they are given."""
 import pytest
 import torch
 
@@ -27,7 +27,7 @@ def table(doc, listed, by_id):
 
 
 @pytest.mark.parametrize("masked", [0.0, 0.02, 0.6, 1.0])
-@pytest.mark.parametrize("rows,size", [(1, 1), (1, 3), (1, 4096), (1, 4097), (1, 20001), (3, 1365), (5, 4096), (40, 7)])
+@pytest.mark.parametrize("rows,size", [(1, 1), (1, 3), (1, 4096), (1, 4097), (1, 8192), (1, 8193), (1, 20001), (3, 1365), (5, 4096), (40, 7), (9000, 1)])
 def test_segments(rows, size, masked):
     from msa_b200 import ops
     g = torch.Generator().manual_seed(rows * size)
