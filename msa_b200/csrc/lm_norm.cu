@@ -416,49 +416,33 @@ __global__ void token_shift_kernel(const T* __restrict__ h, const float* __restr
   }
 }
 
-// V = 8: 16-byte loads, two rows' in flight per thread (bf16); V = 4: 8- or 16-byte ones; V = 1: any alignment.  A block takes
-// 256 * V columns of two rows.  Bound by HBM; with 8-byte loads and an index division by a run-time number 6236 x 6144 took 63.5 us
-// from a cold L2 (bytes at HBM rate: 34.6), now 43.0 (41.0 with approximate exponentials, whose last bits decide between experts
-// that tie).
+// V = 8: 16-byte loads (bf16); V = 4: 8- or 16-byte ones; V = 1: any alignment.  A block takes 256 * V columns of a row.  Bound by the issue of
+// instructions (74 % of the slots, DRAM 61 %): the exponential and the quotient are exact.  With 8-byte loads and an index division
+// by a run-time number 6236 x 6144 took 57.5 us from a cold L2, now 40.2; the bytes alone take 35.6 at HBM's rate.  (A chain of such
+// launches from a graph.)  Approximate exponentials gave 2 us more, but their last bits decide between experts that tie.
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-lm_silu_mul_kernel(const T* __restrict__ gu, long long stride, int ff, int n_rows, T* __restrict__ out, long long out_stride) {
+lm_silu_mul_kernel(const T* __restrict__ gu, long long stride, int ff, T* __restrict__ out, long long out_stride) {
   const int j = (blockIdx.x * 256 + threadIdx.x) * V;
   if (j >= ff) return;
-  const long long r0 = 2ll * blockIdx.y;
-  const int rows = r0 + 1 < n_rows ? 2 : 1;
+  const T *g = gu + blockIdx.y * stride + j, *u = g + ff;
+  T* o = out + blockIdx.y * out_stride + j;
   if constexpr (V == 8) {
-    uint4 g[2], u[2];
+    const uint4 gv = *reinterpret_cast<const uint4*>(g), uv = *reinterpret_cast<const uint4*>(u);
+    const __nv_bfloat162 *a = reinterpret_cast<const __nv_bfloat162*>(&gv), *b = reinterpret_cast<const __nv_bfloat162*>(&uv);
+    uint4 ov;
+    __nv_bfloat162* c = reinterpret_cast<__nv_bfloat162*>(&ov);
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-      if (k < rows) {
-        g[k] = *reinterpret_cast<const uint4*>(gu + (r0 + k) * stride + j);
-        u[k] = *reinterpret_cast<const uint4*>(gu + (r0 + k) * stride + ff + j);
-      }
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-      if (k < rows) {
-        const __nv_bfloat162 *a = reinterpret_cast<const __nv_bfloat162*>(&g[k]), *b = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
-        uint4 o;
-        __nv_bfloat162* c = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 x = __bfloat1622float2(a[i]), y = __bfloat1622float2(b[i]);
-          c[i] = __floats2bfloat162_rn(silu_f(x.x) * y.x, silu_f(x.y) * y.y);
-        }
-        *reinterpret_cast<uint4*>(out + (r0 + k) * out_stride + j) = o;
-      }
-  } else {
-    for (int k = 0; k < rows; ++k) {
-      const T *g = gu + (r0 + k) * stride + j, *u = g + ff;
-      T* o = out + (r0 + k) * out_stride + j;
-      if constexpr (V == 4) {
-        const float4 x = load4(g), y = load4(u);
-        store4(o, make_float4(silu_f(x.x) * y.x, silu_f(x.y) * y.y, silu_f(x.z) * y.z, silu_f(x.w) * y.w));
-      } else {
-        *o = from_f<T>(silu_f(to_f(*g)) * to_f(*u));
-      }
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = __bfloat1622float2(a[i]), y = __bfloat1622float2(b[i]);
+      c[i] = __floats2bfloat162_rn(silu_f(x.x) * y.x, silu_f(x.y) * y.y);
     }
+    *reinterpret_cast<uint4*>(o) = ov;
+  } else if constexpr (V == 4) {
+    const float4 x = load4(g), y = load4(u);
+    store4(o, make_float4(silu_f(x.x) * y.x, silu_f(x.y) * y.y, silu_f(x.z) * y.z, silu_f(x.w) * y.w));
+  } else {
+    *o = from_f<T>(silu_f(to_f(*g)) * to_f(*u));
   }
 }
 
@@ -592,6 +576,15 @@ extern "C" int msa_lm_token_shift(const void* h, const float* mu, int32_t n_mix,
   return MSA_OK;
 }
 
+template <int V, typename T>
+static void launch_silu_mul(const T* gu, int64_t gu_stride, int n_rows, int ff, T* out, int64_t out_stride, cudaStream_t stream) {
+  for (int64_t r = 0; r < n_rows; r += 65535) {        // the second axis of a grid ends there
+    const unsigned rows = (unsigned)(n_rows - r < 65535 ? n_rows - r : 65535);
+    lm_silu_mul_kernel<T, V><<<dim3((unsigned)((ff + 256 * V - 1) / (256 * V)), rows), 256, 0, stream>>>(
+        gu + r * gu_stride, gu_stride, ff, out + r * out_stride, out_stride);
+  }
+}
+
 extern "C" int msa_lm_silu_mul(const void* gu, int64_t gu_stride, int32_t n_rows, int32_t ff, void* out, int64_t out_stride,
                                int32_t dtype, void* stream) {
   MSA_REQUIRE(dtype_ok(dtype) && gu && out && n_rows >= 0 && ff > 0, "lm_silu_mul: bad arguments");
@@ -599,20 +592,21 @@ extern "C" int msa_lm_silu_mul(const void* gu, int64_t gu_stride, int32_t n_rows
   const int e = (int)dtype_size(dtype);
   const bool v4 = ff % 4 == 0 && gu_stride % 4 == 0 && out_stride % 4 == 0 && vec4_ok(gu, e) && vec4_ok(out, e);
   const bool v8 = dtype == MSA_BF16 && ff % 8 == 0 && gu_stride % 8 == 0 && out_stride % 8 == 0 && aligned16(gu) && aligned16(out);
-  const int per = 256 * (v8 ? 8 : (v4 ? 4 : 1));
-  for (int r = 0; r < n_rows; r += 131070) {           // the second axis of a grid ends at 65535 pairs of rows
-    const int rows = n_rows - r < 131070 ? n_rows - r : 131070;
-    const dim3 grid((unsigned)((ff + per - 1) / per), (unsigned)((rows + 1) / 2));
-    MSA_LM_DISPATCH(dtype, {
-      const T* from = (const T*)gu + r * gu_stride;
-      T* to = (T*)out + r * out_stride;
-      if constexpr (sizeof(T) == 2) {
-        if (v8) { lm_silu_mul_kernel<T, 8><<<grid, 256, 0, (cudaStream_t)stream>>>(from, gu_stride, ff, rows, to, out_stride); continue; }
-      }
-      if (v4) lm_silu_mul_kernel<T, 4><<<grid, 256, 0, (cudaStream_t)stream>>>(from, gu_stride, ff, rows, to, out_stride);
-      else lm_silu_mul_kernel<T, 1><<<grid, 256, 0, (cudaStream_t)stream>>>(from, gu_stride, ff, rows, to, out_stride);
-    });
-  }
+  cudaStream_t st = (cudaStream_t)stream;
+  int n_sm = 0;
+  MSA_OK_OR_RETURN(device_sm_count(&n_sm));
+  // Eight elements a thread where that still makes four blocks for every SM, else four: 32 x 3072 3.1 and 2.8 us, 512 x 3072 (768 blocks)
+  // 5.1 both, 1055 x 6144 9.5 and 11.3.
+  const bool many = (long long)n_rows * ((ff + 2047) / 2048) >= 4ll * n_sm;
+  MSA_LM_DISPATCH(dtype, {
+    const T* from = (const T*)gu;
+    T* to = (T*)out;
+    if constexpr (sizeof(T) == 2) {
+      if (v8 && many) { launch_silu_mul<8>(from, gu_stride, n_rows, ff, to, out_stride, st); break; }
+    }
+    if (v4) launch_silu_mul<4>(from, gu_stride, n_rows, ff, to, out_stride, st);
+    else launch_silu_mul<1>(from, gu_stride, n_rows, ff, to, out_stride, st);
+  });
   MSA_LAUNCH_OK("lm_silu_mul_kernel");
   return MSA_OK;
 }

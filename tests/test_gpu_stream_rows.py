@@ -51,7 +51,7 @@ def test_residual_norm_of_a_mixture_and_of_chosen_rows(width, top):
     assert near(h, rms(base.double()[rows.long()]), 4 * base.abs().double()[rows.long()] + 1, False)
 
 
-@pytest.mark.parametrize("rows,ff,offset", [(1, 8, 0), (3, 2048, 0), (2, 2056, 0), (5, 6144, 0), (3, 20, 0), (4, 13, 0), (3, 64, 4), (2, 64, 1)])
+@pytest.mark.parametrize("rows,ff,offset", [(1, 8, 0), (3, 2048, 0), (2, 2056, 0), (591, 2048, 0), (592, 2048, 0), (300, 2056, 0), (65537, 8, 0), (65536, 20, 0), (5, 6144, 0), (3, 20, 0), (4, 13, 0), (3, 64, 4), (2, 64, 1)])
 @pytest.mark.parametrize("dtype", [BF16, F32], ids=["bf16", "f32"])
 def test_silu_mul(rows, ff, offset, dtype):
     from msa_b200 import lm_ops as K
