@@ -65,7 +65,7 @@ def test_silu_mul(rows, ff, offset, dtype):
     assert (out[:, :offset] == 7).all() and (out[:, offset + ff:] == 7).all()
 
 
-@pytest.mark.parametrize("rows,cols,pad", [(1, 1, 0), (3, 31, 0), (2, 4097, 3), (8, 32768, 0), (2, 32768, 1), (3, 151936, 0), (2, 36868, 4)])
+@pytest.mark.parametrize("rows,cols,pad", [(1, 1, 0), (3, 31, 0), (2, 4097, 3), (8, 32768, 0), (2, 32768, 1), (3, 151936, 0), (9, 151936, 0), (4, 131072, 0), (4, 131073, 0), (2, 36868, 4)])
 def test_argmax(rows, cols, pad):
     from msa_b200 import lm_ops as K
     x = randn(rows, cols + pad, seed=cols)[:, :cols]
