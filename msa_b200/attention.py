@@ -45,7 +45,7 @@ def fused_ops(*tensors) -> bool:
     device = tensors[0].get_device()
     for t in tensors:
         if not ((type(t) is torch.Tensor or type(t) is nn.Parameter) and t.dtype == torch.bfloat16 and t.get_device() == device
-                and t.stride(-1) == 1 and t.data_ptr() % 16 == 0):
+                and (t.is_contiguous() or t.stride(-1) == 1) and t.data_ptr() % 16 == 0):
             return False
     return True
 

@@ -414,7 +414,7 @@ def gather_plan(sel_local: torch.Tensor, sel_rank: Optional[torch.Tensor], world
         raise A.MsaError("gather_plan: shard_doc_base / shard_kv_base must have one entry per rank")
     if doc_chunk_offset.numel() != doc_chunk_len.numel():
         raise A.MsaError("gather_plan: doc_chunk_offset and doc_chunk_len differ in length")
-    if report is not None and (total_host is not None or resident is not None or report.dtype != torch.int64 or report.shape != (3,)
+    if report is not None and (total_host is not None or resident is not None or report.dtype != torch.int64 or report.numel() != 3
                                or not report.is_contiguous() or not report.is_pinned()):
         raise A.MsaError("gather_plan: report must be a pinned contiguous int64 [3] tensor, in place of total_host and without resident")
     plan = torch.empty((n_seq * k, 4), dtype=torch.int64, device=dev)
@@ -559,7 +559,8 @@ def question_plan(valid: torch.Tensor, n_sel: torch.Tensor, t_len: int, status: 
     tokens of every row; the longest, whether every row's valid tokens are one run, ``status[0]``."""
     A.need_cuda(valid, n_sel, status)
     b, s = valid.shape
-    if valid.dtype != torch.bool or n_sel.shape != (b,) or n_sel.device != valid.device or (status is not None and status.device != valid.device):
+    on = valid.get_device()
+    if valid.dtype != torch.bool or n_sel.numel() != b or n_sel.get_device() != on or (status is not None and status.get_device() != on):
         raise A.MsaError("question_plan: a bool mask [B, S] and B lengths on its device expected")
     vmask = valid.contiguous().view(torch.uint8)
     if n_sel.dtype != torch.int64 or not n_sel.is_contiguous():

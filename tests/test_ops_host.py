@@ -32,7 +32,7 @@ def test_question_plan_wants_a_length_for_every_row(library):
     from msa_b200 import _cabi as A, ops
     with FakeTensorMode():
         valid = new(3, 10, dtype=torch.bool)
-        for n_sel in (new(2), new(1), new(3, 1), new(3, device="cuda:1")):
+        for n_sel in (new(2), new(1), new(3, 2), new(3, device="cuda:1")):
             with pytest.raises(A.MsaError):
                 ops.question_plan(valid, n_sel, 5)
         for bad in (new(3, 10, dtype=torch.uint8), new(3, 10, dtype=torch.float32)):
