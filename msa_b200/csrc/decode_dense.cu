@@ -5,6 +5,12 @@
 // Here each reads its inputs once, computes in fp32 and rounds once.
 //
 // All are bound by HBM on a block of documents and by launch latency in a decode step.
+//
+// Quotients, roots and exponentials are the fast ones (a few 2^-23 of themselves, subnormals flushed) where the eager modules take
+// the exact ones: the results are rounded to 8 bits once, the modules' two to four times, and that outweighs it.  silu(gate) * up over
+// every finite bf16 gate from -87 on and four values of up, against 64 bits: at most 1.00 x 2^-8 of the result and 0.43 x 2^-8 in the mean (root of
+// squares); silu and product as two modules 1.61 and 0.45.  Below -87 the sum 1 + e^-gate passes 2^126 and the result, 3e-36 at
+// most in size, is 0.  No choice between discrete things hangs on last bits here (the layered decoders' experts, which do, take exact ones).
 #include "common.cuh"
 
 namespace msa {

@@ -169,10 +169,13 @@ __global__ void __launch_bounds__(1024) residual_norm_once_kernel(const ResNormP
     store4(reinterpret_cast<T*>(p.h_out2) + r * p.width + i, make_float4(x.x * inv * wn2.x, x.y * inv * wn2.y, x.z * inv * wn2.z, x.w * inv * wn2.w));
 }
 
-// The same for many rows, E vectors per thread in registers.  Bound by HBM (base and stream in 32 bits, branch and norm in 16: 12 bytes
-// per element), so all of a row's loads are in flight before the first reduction.  Threads and order of the sums are those of the
-// general kernel below, so that a position's experts do not hang on the number of rows beside it.  One vector at a time through
-// shared memory took 47.1 us for 6236 x 2048 from a cold L2 (bytes at HBM rate: 23), this takes 39.9.
+// The same for many rows, E vectors per thread in registers, all of a row's loads in flight before the first reduction.  12 bytes per
+// element (base and stream in 32 bits, branch and norm in 16).  One vector at a time through shared memory took 47.1 us for 6236 x 2048
+// from a cold L2, this takes 39.9; the bytes alone take 24 at HBM's rate.  What bounds it is the issue of instructions (63 % of the slots, DRAM
+// 36 %): two sums over the block per row and four conversions per vector.
+// Threads and order of the sums are those of residual_norm_kernel above, bit for bit.  That holds from 513 rows on: up to 512 rows
+// residual_norm_once_kernel sums in another order, and products of up to 8 rows (rows_gemm_kernel) do too, so the last bits
+// of a position, and its experts where two of them tie, do depend on the number of rows beside it.
 template <typename T, typename TY, int E>
 __global__ void __launch_bounds__(256) residual_norm_rows_kernel(const ResNormParams p) {
   __shared__ float s_part[2][32];

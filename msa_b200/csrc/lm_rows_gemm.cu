@@ -162,6 +162,9 @@ extern "C" int msa_lm_rows_gemm(const msa_lm_rows_gemm_args* args, void* stream)
   if (a.act) return launch_rows_gemm<2, true>(p, a.batch, st);
   int n_sm = 0;
   MSA_OK_OR_RETURN(device_sm_count(&n_sm));
-  // Taller tiles halve what the rows of x take from L2; they pay once there are two blocks for every SM.
+  // Taller tiles halve what the rows of x take from L2.  Tiles of 16 and of 32 rows, 8 rows of x in a chain of products: 9472 x 2048 10.7 and 9.6 us,
+  // 12288 x 2048 16.4 and 12.9, 16384 x 4096 32.8 and 27.1, a vocabulary of 32768 x 2048 33.3 and 28.2, of 151936 x 2048 122.4 and 104.5.
+  // Below the line both read about the same (4736 x 2048 5.3 and 5.3, 6144 x 2048 7.9 and 7.5, 4096 x 4096 9.3 and 8.9), but for the
+  // smallest, where 32 rows were faster (2048 x 2048 3.9 and 3.0) and are not taken yet: they split K over other warps, which moves last bits.
   return (long long)a.w_rows * a.batch >= 64ll * n_sm ? launch_rows_gemm<2, false>(p, a.batch, st) : launch_rows_gemm<1, false>(p, a.batch, st);
 }
