@@ -17,11 +17,14 @@ from types import SimpleNamespace
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from transformers.activations import ACT2FN
 from transformers.models.qwen3.modeling_qwen3 import Qwen3MLP, Qwen3RMSNorm, Qwen3RotaryEmbedding
 
 from . import ops
 from .attention import MemorySparseAttention, fused_ops, plain_module
 from .cache import create_cache
+
+SILU = type(ACT2FN["silu"])
 
 
 def add_norm(x, branch, norm):
@@ -42,13 +45,12 @@ class MSADecoderLayer(nn.Module):
         self.mlp = Qwen3MLP(config)
         self.input_layernorm = Qwen3RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
         self.post_attention_layernorm = Qwen3RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
-        self._silu = type(self.mlp.act_fn) if config.hidden_act == "silu" else None
 
     def takes_fused(self, x) -> bool:
         """Whether ``fused`` computes what ``forward`` does on ``x``: nobody watches or replaced the modules it steps over (the
         layer itself is asked about by the caller: a module in its place knows neither method)."""
         norms, mlp = (self.input_layernorm, self.post_attention_layernorm), self.mlp
-        return (plain_module(mlp, Qwen3MLP) and plain_module(mlp.act_fn, self._silu)
+        return (plain_module(mlp, Qwen3MLP) and plain_module(mlp.act_fn, SILU)
                 and all(plain_module(n, Qwen3RMSNorm) and fused_ops(x, n.weight) for n in norms)
                 and x.shape[-1] % 2 == 0 and x.shape[-1] <= 12288)
 

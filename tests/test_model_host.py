@@ -21,14 +21,14 @@ class Wrapped(nn.Module):
         return hidden_states
 
 
-def small_model():
+def small_model(hidden_act="silu"):
     from msa_b200.configuration import MSAConfig
     from msa_b200.model import MSAModel
     cfg = MSAConfig(
         msa_config=dict(router_layer_idx="1", aux_loss=False, aux_loss_method="INFONCE", decouple_router=True, top_k_docs=4, pooling_kernel_size=64,
                         head_reduce_method="mean", query_reduce_method="max", chunk_reduce_method="max", decouple_pooling_mode="mean"),
         hidden_size=256, num_attention_heads=4, num_key_value_heads=2, head_dim=128, num_hidden_layers=2, intermediate_size=520, vocab_size=64,
-        max_position_embeddings=4096, rms_norm_eps=1e-6)
+        max_position_embeddings=4096, rms_norm_eps=1e-6, hidden_act=hidden_act)
     cfg._attn_implementation = "eager"
     return MSAModel(cfg).to(BF16).eval()
 
@@ -70,3 +70,15 @@ def test_operands_on_two_devices_are_not_fused():
             assert not attention.fused_ops(at("cpu"), at("cuda:0"))
         finally:
             attention.torch = real
+
+
+@pytest.mark.parametrize("act,fused", [("silu", True), ("gelu", False), ("relu", False)])
+def test_the_fused_pass_asks_a_layer_for_nothing_of_its_own(monkeypatch, act, fused):
+    """A layer that was saved whole before the fused pass was there holds nothing but its modules."""
+    from msa_b200 import model as M
+    monkeypatch.setattr(M, "fused_ops", lambda *t: True)
+    layer = small_model(hidden_act=act).layers[0]
+    for name in set(vars(layer)) - set(vars(nn.Module())) - {"hidden_size", "layer_idx"}:
+        delattr(layer, name)
+    with torch.no_grad():
+        assert layer.takes_fused(torch.zeros(1, 3, 256, dtype=BF16)) is fused
