@@ -1,8 +1,7 @@
-// Routing on CUDA cores: query-head folding, score-table reset, and the fp32 scoring kernel.
+// Routing on CUDA cores: query-head folding, score-table reset, and the general scoring kernel.
 //
-// The fp32 kernels are the product path for fp32 banks (the reference's CPU-runnable
-// configuration), the general one a cross-check for the tensor-core kernel too; bf16 banks are scored by
-// route_tc.cu.
+// The general kernel scores fp32 banks whose rows the tensor-core kernel of route_fp32_tc.cu cannot fetch, and is a cross-check for
+// both tensor-core kernels; bf16 banks are scored by route_tc.cu.
 #include "common.cuh"
 #include "route.cuh"
 
@@ -174,134 +173,6 @@ route_simt_kernel(const T* __restrict__ qf, const float* __restrict__ row_bias, 
     }
     atomicMax(keys + (long long)sq * table_stride + doc, float_to_key(m * alpha));
   }
-}
-
-// The same for fp32 rows that 16-byte copies can fetch, and sequences of whole 16-row blocks: the path of a question in fp32.
-// Bound by the fp32 units (64 rows x 16,000 chunks x 1024: 29 us of multiply-adds at 128 per clock and SM; the keys at HBM rate: 10).
-// A warp takes 16 rows x 64 chunks, 4 x 8 per lane, as sums over the even and the odd k (fma.rn.f32x2, operands as they lie in shared
-// memory: 12 conflict-free 16-byte loads feed 64 instructions, which the load unit needs half as long again for); with one or two
-// blocks of 16 rows four or two warps share the chunks instead, for there would be too few warps.  Three stages of 32 k ahead by
-// cp.async.  Blocks of rows without a valid token are fetched but not multiplied: their bias is -inf.  16,000 chunks from a cold L2,
-// table reset included, with the kernel above and with this one: 64 rows 136 and 89 us, 32 rows 130 and 60, 16 rows 128 and 54.
-constexpr int kFpChunks = 64, kFpK = 32, kFpStages = 3, kFpPitch = kFpK + 4, kFpMaxWarps = 8;
-
-__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-
-// CI: octets of chunks of a warp; 8 / CI warps share a block of 16 rows.
-template <int CI>
-__global__ void __launch_bounds__(kFpMaxWarps * 32)
-route_fp32_kernel(const float* __restrict__ qf, const float* __restrict__ row_bias, int n_rows, int s_pad, const float* __restrict__ rk,
-                  long long rk_stride, int n_chunks, int kdim, const int32_t* __restrict__ chunk_doc, int n_docs, float alpha,
-                  uint32_t* __restrict__ keys, long long table_stride, int32_t* __restrict__ status) {
-  extern __shared__ __align__(16) float sm[];              // [stage][64 chunks, then the rows][kFpPitch]
-  __shared__ float s_max[kFpMaxWarps][kFpChunks];
-  const int wr = blockDim.x / 32 * CI / 8, rows = 16 * wr, stage = (kFpChunks + rows) * kFpPitch;
-  const int c0 = blockIdx.x * kFpChunks, r0 = blockIdx.y * rows;
-  const int warp = threadIdx.x / 32 % wr, oct0 = threadIdx.x / 32 / wr * CI, lane = threadIdx.x % 32, tx = lane % 8, ty = lane / 8;
-  auto fetch = [&](int step) {
-    const int k0 = step * kFpK;
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sm + (step % kFpStages) * stage);
-    for (int i = threadIdx.x; i < (kFpChunks + rows) * (kFpK / 4); i += blockDim.x) {
-      const int r = i / (kFpK / 4), k = k0 + 4 * (i % (kFpK / 4));
-      const int at = r < kFpChunks ? c0 + r : r0 + r - kFpChunks;
-      const bool on = k < kdim && at < (r < kFpChunks ? n_chunks : n_rows);
-      const float* src = r < kFpChunks ? rk + (on ? at * rk_stride + k : 0) : qf + (on ? (long long)at * kdim + k : 0);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (r * kFpPitch + 4 * (i % (kFpK / 4))) * 4), "l"(src),
-                   "r"(on ? 16u : 0u) : "memory");
-    }
-  };
-  const int steps = (kdim + kFpK - 1) / kFpK;
-#pragma unroll
-  for (int i = 0; i < kFpStages - 1; ++i) {
-    if (i < steps) fetch(i);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  float bias[4];
-  bool live = false;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int r = r0 + warp * 16 + ty + 4 * j;
-    bias[j] = r < n_rows ? row_bias[r] : -INFINITY;
-    live |= bias[j] != -INFINITY;
-  }
-  live = __any_sync(0xffffffffu, live);
-  unsigned long long acc[CI][4];
-#pragma unroll
-  for (int i = 0; i < CI; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-  for (int step = 0; step < steps; ++step) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kFpStages - 2) : "memory");
-    __syncthreads();                                       // this step has landed; the stage before it has been read
-    if (step + kFpStages - 1 < steps) fetch(step + kFpStages - 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    if (!live) continue;
-    const float* a = sm + (step % kFpStages) * stage + (8 * oct0 + tx) * kFpPitch;
-    const float* b = sm + (step % kFpStages) * stage + (kFpChunks + warp * 16 + ty) * kFpPitch;
-#pragma unroll
-    for (int k = 0; k < kFpK; k += 4) {
-      ulonglong2 q[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) q[j] = *reinterpret_cast<const ulonglong2*>(b + 4 * j * kFpPitch + k);
-#pragma unroll
-      for (int i = 0; i < CI; ++i) {
-        const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(a + 8 * i * kFpPitch + k);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { fma2(acc[i][j], c.x, q[j].x); fma2(acc[i][j], c.y, q[j].y); }
-      }
-    }
-  }
-  // the best of the warp's 16 rows (all of one sequence) for every chunk, then of the sequence's warps in this block
-#pragma unroll
-  for (int i = 0; i < CI; ++i) {
-    float m = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      m = fmaxf(m, __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32)) + bias[j]);
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-    if (ty == 0) s_max[warp][8 * (oct0 + i) + tx] = m;
-  }
-  __syncthreads();
-  const int per_seq = s_pad / 16, block0 = r0 / 16, blocks = min(wr, (n_rows - r0) / 16);
-  const int seq0 = block0 / per_seq, n_seq = (block0 + blocks - 1) / per_seq - seq0 + 1;
-  for (int item = threadIdx.x; item < kFpChunks * n_seq; item += blockDim.x) {
-    const int cc = item % kFpChunks, sq = seq0 + item / kFpChunks;
-    if (c0 + cc >= n_chunks) continue;
-    const int w0 = max(sq * per_seq - block0, 0), w1 = min((sq + 1) * per_seq - block0, blocks);
-    float m = -INFINITY;
-    for (int w = w0; w < w1; ++w) m = fmaxf(m, s_max[w][cc]);
-    const int doc = chunk_doc[c0 + cc];
-    if (doc < 1 || doc > n_docs) {                         // an id outside the table: counted, never used as a column
-      atomicAdd(status + 2, 1);
-      continue;
-    }
-    atomicMax(keys + (long long)sq * table_stride + doc, float_to_key(m * alpha));
-  }
-}
-
-template <int CI>
-int launch_route_fp32_t(int wr, int tiles, const float* qf, const float* row_bias, int n_rows, int s_pad, const float* rk, int64_t rk_stride,
-                        int n_chunks, int kdim, const int32_t* chunk_doc, int n_docs, float alpha, uint32_t* keys, int64_t table_stride,
-                        int32_t* status, cudaStream_t stream) {
-  static DeviceSmem state{};
-  const size_t smem = (size_t)kFpStages * (kFpChunks + 16 * wr) * kFpPitch * 4;
-  MSA_OK_OR_RETURN(ensure_dynamic_smem(route_fp32_kernel<CI>, smem, state));
-  route_fp32_kernel<CI><<<dim3((n_chunks + kFpChunks - 1) / kFpChunks, tiles), wr * (8 / CI) * 32, smem, stream>>>(
-      qf, row_bias, n_rows, s_pad, rk, rk_stride, n_chunks, kdim, chunk_doc, n_docs, alpha, keys, table_stride, status);
-  MSA_LAUNCH_OK("route_fp32_kernel");
-  return MSA_OK;
-}
-
-template <typename... Args>
-int launch_route_fp32(const float* qf, const float* row_bias, int n_rows, Args... rest) {
-  const int blocks = n_rows / 16, most = (blocks + kFpMaxWarps - 1) / kFpMaxWarps, wr = (blocks + most - 1) / most, tiles = (blocks + wr - 1) / wr;
-  MSA_REQUIRE(tiles <= 65535, "route (fp32): too many query rows (%d)", n_rows);
-  if (wr == 1) return launch_route_fp32_t<2>(wr, tiles, qf, row_bias, n_rows, rest...);
-  if (wr == 2) return launch_route_fp32_t<4>(wr, tiles, qf, row_bias, n_rows, rest...);
-  return launch_route_fp32_t<8>(wr, tiles, qf, row_bias, n_rows, rest...);
 }
 
 template <typename T>

@@ -1,0 +1,69 @@
+"""fp32 routing as sums of bf16 products: accuracy against chains of fp32 multiply-adds, and numbers that have no exact split."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def route(q, rk, doc, alpha=0.125):
+    from msa_b200 import ops
+    b, _, s, _ = q.shape
+    qf, bias, s_pad = ops.fold_queries(q, torch.ones(b, s, dtype=torch.bool, device=DEV), 1)
+    keys, status = ops.route_scores(qf, bias, b, s_pad, rk, doc, int(doc.max()), alpha)
+    assert status.tolist() == [0, 0, 0, 0]
+    return ops.keys_to_scores(keys)[:, 1:]
+
+
+def want(q, rk, dtype, alpha=0.125):
+    """Every chunk its own document: the best row of the question, rows whose score is not a number left out."""
+    b, h, s, d = q.shape
+    z = q.to(dtype).permute(0, 2, 1, 3).reshape(b, s, -1) @ rk.to(dtype).t()
+    return z.masked_fill(z.isnan(), -torch.inf).amax(1) * alpha
+
+
+@pytest.mark.parametrize("s,h,d,chunks", [(16, 8, 128, 300), (64, 8, 128, 1000), (65, 2, 64, 257), (200, 8, 128, 500), (17, 1, 4, 128), (48, 5, 4, 127)])
+@pytest.mark.parametrize("mean", [0.0, 1.0])
+def test_no_further_off_than_fp32_chains(s, h, d, chunks, mean):
+    g = torch.Generator(device=DEV).manual_seed(s + chunks)
+    q = torch.randn(2, h, s, d, generator=g, device=DEV) + mean           # with a mean every partial sum grows: truncation would add up
+    rk = torch.randn(chunks, h * d, generator=g, device=DEV) + mean
+    doc = torch.arange(1, chunks + 1, device=DEV, dtype=torch.int32)
+    ref = want(q, rk, torch.float64)
+    rows = q.permute(0, 2, 1, 3).reshape(2, s, 1, -1)
+    chain = torch.zeros(2, s, chunks, device=DEV)
+    for k in range(h * d):
+        chain = torch.addcmul(chain, rows[..., k], rk[:, k].view(1, 1, -1))
+    err = lambda x: float((x.double() - ref).norm() / ref.norm())
+    # one chain of fp32 additions over all channels is what the result may be as far off as; 2^-24: its own rounding
+    assert err(route(q, rk, doc)) <= err(chain.amax(1) * 0.125) + 2.0 ** -24
+
+
+@pytest.mark.parametrize("where", ["key", "query"])
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan"), 1e30, -1e36, 2.0 ** 60, 1e-35, 1e-40, 0.0])
+def test_numbers_without_a_split(where, value):
+    g = torch.Generator(device=DEV).manual_seed(5)
+    q = torch.randn(1, 4, 40, 32, generator=g, device=DEV)
+    rk = torch.randn(200, 128, generator=g, device=DEV)
+    if where == "key":
+        rk[131, 77] = value
+    else:
+        q[0, 2, 9, 3] = value
+    doc = torch.arange(1, 201, device=DEV, dtype=torch.int32)
+    ref, got = want(q, rk, torch.float64), route(q, rk, doc).double()
+    ref = torch.where(ref.abs() > torch.finfo(torch.float32).max, ref.sign() * torch.inf, ref).clamp(min=torch.finfo(torch.float32).min)
+    # 128 additions in 32 bits, each off by 2^-24 of a partial sum below the sum of absolute products
+    finite = lambda t: t.abs().nan_to_num(0.0, 0.0, 0.0)
+    size = want(finite(q), finite(rk), torch.float64)
+    assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got[got.isinf()], ref[ref.isinf()])
+    on = ~ref.isinf()
+    assert bool(((got - ref).abs()[on] <= (128 * 2.0 ** -24 * size)[on]).all())
+
+
+def test_all_small_numbers_keep_their_digits():
+    g = torch.Generator(device=DEV).manual_seed(6)
+    q = torch.randn(1, 4, 16, 32, generator=g, device=DEV) * 1e6
+    rk = torch.randn(150, 128, generator=g, device=DEV) * 1e-36
+    doc = torch.arange(1, 151, device=DEV, dtype=torch.int32)
+    ref, got = want(q, rk, torch.float64), route(q, rk, doc).double()
+    assert float((got - ref).norm() / ref.norm()) < 1e-5
