@@ -115,6 +115,23 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The native host side of the memory model's layers (``csrc/host_layer.cpp``)."""
+    global _native
+    if _native is None:
+        lib()
+        try:
+            from . import _native as n
+        except ImportError as e:
+            raise MsaError(f"msa_b200/_native.so cannot be loaded: build it with `python -m msa_b200.build` ({e})") from e
+        n.bind(LIB_PATH)
+        _native = n
+    return _native
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         raise MsaError(f"{what} failed ({rc}): {lib().msa_last_error().decode()}")

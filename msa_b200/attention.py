@@ -116,6 +116,11 @@ class MemorySparseAttention(Qwen3Attention):
             query_states = self.q_norm(query_states.view(hidden_shape)).transpose(1, 2)
             key_states = self.k_norm(key_states.view(hidden_shape)).transpose(1, 2)
             query_states, key_states = apply_rotary_pos_emb(query_states, key_states, cos, sin)
+        return self.o_proj(self.attend(hidden_states, doc_ids, attention_mask, past_key_value, query_states, key_states, value_states)), None
+
+    def attend(self, hidden_states, doc_ids, attention_mask, past_key_value, query_states, key_states, value_states):
+        """The attention of the layer's stage, ``[B, S, heads * head_dim]``: what stands between the input projections (q and k normed
+        and turned; ``[B, heads, S, head_dim]``) and the output product."""
         stage = past_key_value.cache_kwargs[self.layer_idx]["stage"]
         if stage == "prefill_stage1":
             return self._stage1(hidden_states, doc_ids, attention_mask, past_key_value, query_states, key_states,
@@ -248,7 +253,7 @@ class MemorySparseAttention(Qwen3Attention):
             if pooled_rk is not None:
                 cache.update_router_kcache(pooled_rk, self.layer_idx)
         cache.record_kwargs(self.layer_idx, kw)
-        return self.o_proj(attn_output), None
+        return attn_output
 
     def _stage2(self, hidden_states, doc_ids, attention_mask, cache, query_states, key_states, value_states):
         """src/msa/memory_sparse_attention.py:245-359."""
@@ -306,7 +311,7 @@ class MemorySparseAttention(Qwen3Attention):
             "_msa_b200_store": (k_store, v_store, kv_start, kv_len),
         })
         cache.record_kwargs(self.layer_idx, cache_kwargs)
-        return self.o_proj(attn_output), None
+        return attn_output
 
     # ------------------------------------------------------------------------------------ decode
     def _decode(self, attention_mask, cache, query_states, key_states, value_states):
@@ -324,11 +329,16 @@ class MemorySparseAttention(Qwen3Attention):
         # (samples that wait in the interleave loop) says so in meta["step_all_valid"]; those steps, like qa_mode
         # segments, go through the segment path, which stores only the unmasked tokens.
         if q_len == 1 and not cache.meta.get("qa_mode", False) and cache.meta.get("step_all_valid", True):
-            out = ops.sparse_decode_attn(query_states[:, :, 0], k_store, v_store, kv_len, key_states[:, :, 0],
-                                         value_states[:, :, 0], kv_start=kv_start)
-            attn_output = out.view(bsz, 1, n_heads * d)
-            kv_len = kv_len + 1
-            cache_kwargs["kv_lengths"] = cache_kwargs["kv_lengths"] + 1
+            done = A.native().decode(query_states, key_states, value_states, k_store, v_store, kv_start, kv_len, cache_kwargs["kv_lengths"],
+                                     ops.decode_splits(bsz, k_store.shape[1], k_store.shape[2]))
+            if done is not None:
+                attn_output, kv_len, cache_kwargs["kv_lengths"] = done
+            else:
+                out = ops.sparse_decode_attn(query_states[:, :, 0], k_store, v_store, kv_len, key_states[:, :, 0],
+                                             value_states[:, :, 0], kv_start=kv_start)
+                attn_output = out.view(bsz, 1, n_heads * d)
+                kv_len = kv_len + 1
+                cache_kwargs["kv_lengths"] = cache_kwargs["kv_lengths"] + 1
         else:
             # qa_mode segments (:375-380): every token of the segment attends, without a causal mask, to the cache
             # and to the segment's own unmasked tokens.  One kernel appends the unmasked tokens in place (kv_len
@@ -352,7 +362,7 @@ class MemorySparseAttention(Qwen3Attention):
         cache_kwargs["compacked_value_cache"] = v_store[:, :, :cur_len + q_len]
         cache_kwargs["_msa_b200_store"] = (k_store, v_store, kv_start, kv_len)
         cache.record_kwargs(self.layer_idx, cache_kwargs)
-        return self.o_proj(attn_output), None
+        return attn_output
 
     def _adopt_cache(self, cache_kwargs, q_len):
         """Take over a compact cache that was built elsewhere (or has run out of room): copy it once

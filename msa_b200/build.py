@@ -4,7 +4,8 @@
     python -m msa_b200.build --force
 
 Two libraries, each built only when it is asked for or stale: ``libmsa_b200.so`` (memory routing and sparse attention,
-``include/msa_b200.h``) and ``libmsa_b200_lm.so`` (the layered decoder designs, ``include/msa_b200_lm.h``).
+``include/msa_b200.h``) and ``libmsa_b200_lm.so`` (the layered decoder designs, ``include/msa_b200_lm.h``); and with g++ the
+extension ``_native.so`` (host side of the memory model's layers).
 """
 from __future__ import annotations
 
@@ -29,6 +30,11 @@ LIBRARIES = {
 }
 
 
+# The native host side of the memory model's layers: an extension of torch, which binds the first library when it is used.
+LIB_NATIVE, NATIVE_SOURCE = os.path.join(HERE, "_native.so"), "host_layer.cpp"
+LIBRARIES["native"] = (LIB_NATIVE, [NATIVE_SOURCE], [], ["msa_b200.h"])
+
+
 def _nvcc() -> str:
     cand = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
     return cand if os.path.exists(cand) else "nvcc"
@@ -39,12 +45,30 @@ def _stale(name: str) -> bool:
     if not os.path.exists(path):
         return True
     t = os.path.getmtime(path)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh") or f in sources]
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f in sources or (f.endswith(".cuh") and name != "native")]
     deps += [os.path.join(HERE, "..", "include", h) for h in headers]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _build_native() -> None:
+    import sysconfig
+
+    from torch.utils import cpp_extension as ext
+    part = f"{LIB_NATIVE}.{os.getpid()}"
+    paths = [a for p in ext.include_paths() for a in ("-isystem", p)]
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) or "/usr/local/cuda"
+    libs = [f"-L{p}" for p in ext.library_paths()] + ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", *paths, f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include",
+           os.path.join(CSRC, NATIVE_SOURCE), "-o", part, *libs]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {NATIVE_SOURCE}:\n{r.stdout}\n{r.stderr}")
+    os.replace(part, LIB_NATIVE)
+
+
 def _build_one(name: str, verbose: bool) -> None:
+    if name == "native":
+        return _build_native()
     path, sources, extra, _ = LIBRARIES[name]
     tag = f"{name}.{os.getpid()}"          # two processes may build at once: each its own objects, the library by rename
     objdir = os.path.join(HERE, "build")

@@ -20,8 +20,9 @@ import torch.nn.functional as F
 from transformers.activations import ACT2FN
 from transformers.models.qwen3.modeling_qwen3 import Qwen3MLP, Qwen3RMSNorm, Qwen3RotaryEmbedding
 
+from . import _cabi as A
 from . import ops
-from .attention import MemorySparseAttention, fused_ops, plain_module
+from .attention import MemorySparseAttention, fused_ops, nn_module, plain_module
 from .cache import create_cache
 
 SILU = type(ACT2FN["silu"])
@@ -60,6 +61,23 @@ class MSADecoderLayer(nn.Module):
         x, h = add_norm(x, pending, self.input_layernorm)
         attn, _ = self.self_attn(h, doc_ids, attention_mask=attention_mask, position_embeddings=position_embeddings,
                                  past_key_value=past_key_value)
+        return self._behind(x, attn)
+
+    def native(self, parts, x, pending, attention_mask, past_key_value, position_embeddings, doc_ids):
+        """``fused`` with the modules' weights in hand (``parts``): the same launches from native code, where the operands allow it."""
+        n = A.native()
+        at = n.front(parts, x, pending, *position_embeddings)
+        if at is None:
+            if self.takes_fused(x):
+                return self.fused(x, pending, attention_mask, past_key_value, position_embeddings, doc_ids)
+            return self(x if pending is None else x + pending, attention_mask=attention_mask, past_key_value=past_key_value,
+                        position_embeddings=position_embeddings, doc_ids=doc_ids), None
+        x, h, q, k, v = at
+        attn = self.self_attn.attend(h, doc_ids, attention_mask, past_key_value, q, k, v)
+        return n.back(parts, x, attn) or self._behind(x, self.self_attn.o_proj(attn))
+
+    def _behind(self, x, attn):
+        """The stream and the feed-forward's branch behind the attention's."""
         x, h = add_norm(x, attn, self.post_attention_layernorm)
         gate, up = self.mlp.gate_proj(h), self.mlp.up_proj(h)
         if fused_ops(gate, up) and gate.shape == up.shape and gate.shape[-1] % 2 == 0:
@@ -75,6 +93,10 @@ class MSADecoderLayer(nn.Module):
         return hidden_states + self.mlp(self.post_attention_layernorm(hidden_states))
 
 
+# what a layer's native pass steps over, in the order that it asks for
+STEPPED_OVER = (MSADecoderLayer, MemorySparseAttention, Qwen3MLP, SILU, Qwen3RMSNorm, nn.Linear)
+
+
 class MSAModel(nn.Module):
     def __init__(self, config):
         super().__init__()
@@ -84,8 +106,20 @@ class MSAModel(nn.Module):
         self.norm = Qwen3RMSNorm(config.hidden_size, eps=config.rms_norm_eps)
         self.rotary_emb = Qwen3RotaryEmbedding(config=config)
 
+    def _native_layers(self, hidden):
+        """The layers' weights for their native pass, or None where a module of some layer is not what that pass steps over."""
+        if not hidden.is_cuda or torch.is_grad_enabled() or nn_module._has_any_global_hook() or any(
+                c.forward.__module__ != c.__module__ for c in STEPPED_OVER):
+            return None
+        return A.native().layers(tuple(self.layers), STEPPED_OVER)
+
     def _angles(self, hidden, position_ids):
         rot = self.rotary_emb
+        if hidden.is_cuda and hidden.dtype == torch.bfloat16 and plain_module(rot, Qwen3RotaryEmbedding) and rot.rope_type == "default" and (
+                position_ids.get_device() == hidden.get_device()):
+            both = A.native().angles(position_ids, rot.inv_freq, rot.attention_scaling)
+            if both is not None:
+                return both
         if (plain_module(rot, Qwen3RotaryEmbedding) and rot.rope_type == "default" and fused_ops(hidden) and position_ids.is_cuda
                 and position_ids.device == hidden.device == rot.inv_freq.device and position_ids.dtype == torch.int64
                 and position_ids.dim() == 2 and rot.inv_freq.dtype == torch.float32):
@@ -104,6 +138,16 @@ class MSAModel(nn.Module):
         if position_ids is None:
             position_ids = torch.arange(hidden.shape[1], device=hidden.device).unsqueeze(0)
         position_embeddings = self._angles(hidden, position_ids)
+        layers = self._native_layers(hidden)
+        if layers is not None:
+            pending = None
+            for layer, parts in zip(self.layers, layers):
+                hidden, pending = layer.native(parts, hidden, pending, attention_mask, past_key_values, position_embeddings, doc_ids)
+            last = A.native().add_norm(hidden, pending, self.norm, Qwen3RMSNorm)
+            if last is None:
+                last = add_norm(hidden, pending, self.norm) if plain_module(self.norm, Qwen3RMSNorm) else (
+                    None, self.norm(hidden if pending is None else hidden + pending))
+            return SimpleNamespace(last_hidden_state=last[1], past_key_values=past_key_values if use_cache else None)
         if plain_module(self.norm, Qwen3RMSNorm) and fused_ops(hidden, self.norm.weight) and all(
                 plain_module(layer, MSADecoderLayer) and layer.takes_fused(hidden) for layer in self.layers):
             pending = None
