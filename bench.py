@@ -1565,6 +1565,9 @@ def nazerax_kernels(torch, dev, model, z, pk, decode_b):
     leg("ssd_prep", lambda: A.call("msa_lm_ssd_prep", ctypes.byref(sa), p(xbc), p(dt), st), 0, n * d.channels * 4)
     gcum, work = torch.empty((n, d.heads), dtype=torch.float64, device=dev), torch.empty((step.n_chunks, d.heads, d.state, d.vdim), **f32)
     macs = n * d.heads * (2 * d.state * d.vdim + 32 * d.vdim) + n * d.groups * 32 * d.state
+    if A.lib().msa_lm_ssd_walk_supported(d.heads, d.groups, d.state, d.vdim):
+        leg("ssd walk", lambda: A.call("msa_lm_ssd_walk", ctypes.byref(sa), p(xbc), p(dt), p(model.status), st), 2.0 * macs,
+            n * (d.channels * 2 + d.inner * 6 + d.heads * 4) + n_seq * d.heads * d.state * d.vdim * 8)
     leg("ssd chunks (add, carry, read)", lambda: A.call("msa_lm_ssd_chunk", ctypes.byref(sa), p(xbc), p(dt), p(step.chunk_off), step.n_chunks, p(gcum), p(work), st),
         2.0 * macs, n * (d.channels * 2 + d.inner * 6 + d.heads * 4) + n_seq * d.heads * d.state * d.vdim * 8)
     leg("part_norm", lambda: K.part_norm(yd, ssd.norm, d.norm_groups, 1e-5, od), 0, n * d.inner * 6)

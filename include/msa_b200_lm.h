@@ -256,6 +256,10 @@ int msa_lm_ssd_scan(const msa_lm_ssd_args* a, const void* xbc, const float* dt, 
 int msa_lm_ssd_chunk_supported(int32_t n_state, int32_t vdim);
 int msa_lm_ssd_chunk(const msa_lm_ssd_args* a, const void* xbc, const float* dt, const int32_t* chunk_off, int32_t n_chunks, double* gcum,
                      float* work, void* stream);
+/* The same by one block per (portion, two heads of a group) that walks the chunks on tcgen05 with the states in TMEM: no scratch.
+ * n_state 128, vdim 64, an even number of heads per group; status[0]: a code when a bounded wait ran out (the output is not valid then). */
+int msa_lm_ssd_walk_supported(int32_t heads, int32_t groups, int32_t n_state, int32_t vdim);
+int msa_lm_ssd_walk(const msa_lm_ssd_args* a, const void* xbc, const float* dt, int32_t* status, void* stream);
 
 /* out = x / rms(x) * w, every row in `parts` equal parts with a root mean square each. */
 int msa_lm_part_norm(const float* x, int64_t x_stride, const float* w, int32_t n_rows, int32_t width, int32_t parts, float eps, void* out,

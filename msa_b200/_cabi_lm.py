@@ -15,7 +15,7 @@ LIB_PATH = os.path.join(_HERE, "libmsa_b200_lm.so")
 EXPORTS = ["msa_lm_residual_norm", "msa_lm_embed", "msa_lm_silu_mul", "msa_lm_softcap", "msa_lm_tanh_split", "msa_lm_token_shift",
            "msa_lm_group_prep", "msa_lm_conv_store", "msa_lm_group_decode_supported", "msa_lm_group_decode", "msa_lm_wkv_decode",
            "msa_lm_wkv_scan", "msa_lm_wkv_chunk_supported", "msa_lm_wkv_chunk", "msa_lm_ssd_decode", "msa_lm_ssd_prep", "msa_lm_ssd_scan",
-           "msa_lm_ssd_chunk_supported", "msa_lm_ssd_chunk", "msa_lm_part_norm", "msa_lm_latent_prep", "msa_lm_ring_store",
+           "msa_lm_ssd_chunk_supported", "msa_lm_ssd_chunk", "msa_lm_ssd_walk_supported", "msa_lm_ssd_walk", "msa_lm_part_norm", "msa_lm_latent_prep", "msa_lm_ring_store",
            "msa_lm_window_attn", "msa_lm_window_attn_tc_supported", "msa_lm_window_attn_tc", "msa_lm_latent_decode_supported", "msa_lm_latent_decode", "msa_lm_delta_decode", "msa_lm_delta_prep", "msa_lm_delta_prep_split", "msa_lm_delta_chunk_supported", "msa_lm_delta_chunk_workspace", "msa_lm_delta_chunk", "msa_lm_gather_rows", "msa_lm_delta_conv_store", "msa_lm_delta_scan",
            "msa_lm_delta_out", "msa_lm_moe_topk", "msa_lm_moe_sort", "msa_lm_moe_gemm", "msa_lm_moe_gemm_tc",
            "msa_lm_rows_gemm", "msa_lm_argmax"]
@@ -113,6 +113,8 @@ def lib() -> C.CDLL:
             "msa_lm_ssd_scan": [sp, vp, vp, vp],
             "msa_lm_ssd_chunk_supported": [i32, i32],
             "msa_lm_ssd_chunk": [sp, vp, vp, vp, i32, vp, vp, vp],
+            "msa_lm_ssd_walk_supported": [i32, i32, i32, i32],
+            "msa_lm_ssd_walk": [sp, vp, vp, vp, vp],
             "msa_lm_part_norm": [vp, i64, vp, i32, i32, i32, f32, vp, i64, i32, vp],
             "msa_lm_latent_prep": [vp, i64, vp, f32, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32,
                                    i32, vp, i64, vp, i32, vp],

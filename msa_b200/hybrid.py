@@ -267,7 +267,7 @@ class Mamba2(Mixer):
 
     def __init__(self, spec, w: Weights, prefix: str, width: int, eps: float):
         s = self.spec = spec
-        self.eps = eps
+        self.eps, self.status = eps, w.status
         self.w_in = w.stack([(prefix + "in", s.inner + s.channels + s.heads)], width, pad=True)
         self.conv = w.vector(prefix + "conv", s.channels, s.taps).t().contiguous()
         self.conv_b = w.vector(prefix + "conv.b", s.channels)

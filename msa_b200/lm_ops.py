@@ -322,6 +322,13 @@ def wkv_mix(rkvg, decay, spec, w, state, eps, step, out):
     return out
 
 
+def ssd_walks(step, heads: int) -> bool:
+    """Whether walking the chunks of every portion beats all chunks at once: 9 us + 4.5 per chunk of the longest portion against 24 us +
+    0.06 per chunk and head.  64 heads: portions of 2048, 1500, 1911 and 777 tokens 166 and 447 us, one of 1024 80 and 85, of 50 14 and
+    26; 32 heads: the four portions 156 and 232, one of 1024 80 and 52, one of 8192 567 and 316."""
+    return 75 * ((step.max_len + 63) // 64) < step.n_chunks * heads + 250
+
+
 def ssd_mix(proj, spec, w, conv_state, state, eps, step, out):
     """From the projections to the input of the output product; advances the states, fills ``out``."""
     dev, st, f = proj.device, A.stream_ptr(proj.device), dict(dtype=torch.float32, device=proj.device)
@@ -338,7 +345,11 @@ def ssd_mix(proj, spec, w, conv_state, state, eps, step, out):
         xbc, dt = torch.empty((rows, spec.channels), dtype=proj.dtype, device=dev), torch.empty((rows, spec.heads), **f)
         A.call("msa_lm_ssd_prep", C.byref(args), A.ptr(xbc), A.ptr(dt), st)
         conv_store(proj[:, spec.inner:], spec.channels, spec.taps, step, conv_state)
-        if proj.dtype == torch.bfloat16 and A.lib().msa_lm_ssd_chunk_supported(spec.state, spec.vdim):
+        status = getattr(w, "status", None)
+        if (status is not None and proj.dtype == torch.bfloat16 and proj.data_ptr() % 16 == 0 and _rows(proj) % 8 == 0
+                and A.lib().msa_lm_ssd_walk_supported(spec.heads, spec.groups, spec.state, spec.vdim) and ssd_walks(step, spec.heads)):
+            A.call("msa_lm_ssd_walk", C.byref(args), A.ptr(xbc), A.ptr(dt), A.ptr(status), st)
+        elif proj.dtype == torch.bfloat16 and A.lib().msa_lm_ssd_chunk_supported(spec.state, spec.vdim):
             gcum = torch.empty((rows, spec.heads), dtype=torch.float64, device=dev)
             work = torch.empty((step.n_chunks, spec.heads, spec.state, spec.vdim), **f)
             A.call("msa_lm_ssd_chunk", C.byref(args), A.ptr(xbc), A.ptr(dt), A.ptr(step.chunk_off), step.n_chunks, A.ptr(gcum), A.ptr(work), st)

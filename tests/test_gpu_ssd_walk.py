@@ -1,0 +1,90 @@
+"""The state-space recurrence walked chunk by chunk with the states in TMEM, against the recurrence token by token in 64 bits."""
+import ctypes
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+BF16, F32, F64 = torch.bfloat16, torch.float32, torch.float64
+
+
+def case(heads, groups, state, vdim, lens, n_decode, seed=0, dev="cuda:0", step=-1.0):
+    """Packed rows: ``n_decode`` single tokens (not this kernel's), then the portions; odd portions continue, even ones start anew."""
+    g = torch.Generator(device=dev).manual_seed(seed)
+    rnd = lambda *s: torch.randn(s, generator=g, device=dev)
+    n_seq, rows, inner = n_decode + len(lens), sum(lens), heads * vdim
+    cu = torch.tensor([0] + [1] * n_decode + list(lens), device=dev).cumsum(0).int()
+    c = dict(heads=heads, groups=groups, n_state=state, vdim=vdim, n_seq=n_seq, n_decode=n_decode, n_tok=n_decode + rows, cu=cu,
+             slot=torch.randperm(n_seq + 2, generator=g, device=dev)[:n_seq].int(),
+             start=torch.tensor([3] * n_decode + [7 * (i % 2) for i in range(len(lens))], device=dev).int(),
+             xbc=rnd(rows, inner + 2 * groups * state).to(BF16), dt=F.softplus(rnd(rows, heads) + step), a_log=rnd(heads), d_skip=rnd(heads),
+             proj=rnd(n_decode + rows, inner + 8).to(BF16), state=rnd(n_seq + 2, heads, state, vdim))
+    c["y"] = torch.full((n_decode + rows, inner), 7.0, device=dev)
+    return c
+
+
+def walk(c):
+    from msa_b200 import _cabi_lm as A
+    p = A.ptr
+    args = A.SsdArgs(proj=p(c["proj"]), proj_stride=c["proj"].stride(0), conv_w=p(c["d_skip"]), conv_b=p(c["d_skip"]), dt_bias=p(c["d_skip"]),
+                     a_log=p(c["a_log"]), d_skip=p(c["d_skip"]), conv_state=p(c["xbc"]), state=p(c["state"]), tok_seq=p(c["cu"]), slot=p(c["slot"]),
+                     start=p(c["start"]), cu=p(c["cu"]), y=p(c["y"]), taps=4, dtype=A.dtype_code(BF16),
+                     **{k: c[k] for k in ("n_tok", "n_seq", "n_decode", "heads", "vdim", "n_state", "groups")})
+    status = torch.zeros(4, dtype=torch.int32, device=c["y"].device)
+    A.call("msa_lm_ssd_walk", ctypes.byref(args), p(c["xbc"]), p(c["dt"]), p(status), A.stream_ptr(c["y"].device))
+    assert status.tolist() == [0, 0, 0, 0]
+
+
+def recurrence(c, size):
+    """(outputs of the portions' rows, states by portion); ``size``: of absolute values, what rounding errors are relative to."""
+    f = (lambda t: t.to(F64).abs()) if size else (lambda t: t.to(F64))
+    heads, groups, ns, vd, inner = c["heads"], c["groups"], c["n_state"], c["vdim"], c["heads"] * c["vdim"]
+    x, b, k = f(c["xbc"]).split([inner, groups * ns, groups * ns], 1)
+    b, k = (t.view(-1, groups, ns).repeat_interleave(heads // groups, 1) for t in (b, k))
+    x, dt = x.view(-1, heads, vd), c["dt"].to(F64)
+    decay = torch.exp(-torch.exp(c["a_log"].to(F64)) * dt)
+    z = c["proj"][c["n_decode"]:, :inner].to(F64)
+    y, states, cu = torch.empty_like(x), [], c["cu"].tolist()
+    for s in range(c["n_decode"], c["n_seq"]):
+        st = f(c["state"][int(c["slot"][s])]) if int(c["start"][s]) else torch.zeros((heads, ns, vd), dtype=F64, device=x.device)
+        for t in range(cu[s] - c["n_decode"], cu[s + 1] - c["n_decode"]):
+            st = decay[t][:, None, None] * st + dt[t][:, None, None] * b[t][:, :, None] * x[t][:, None]
+            y[t] = (k[t][:, None] @ st)[:, 0] + f(c["d_skip"])[:, None] * x[t]
+        states.append(st)
+    return y.reshape(-1, inner) * f(F.silu(z)), states
+
+
+@pytest.mark.parametrize("heads,groups,lens,n_decode", [
+    (2, 1, [200, 64, 1], 0), (4, 2, [63, 65, 128], 3), (12, 2, [129, 16, 17], 1), (64, 8, [1, 300], 0), (2, 1, [640], 2)])
+@pytest.mark.parametrize("step", [-1.0, 6.0])     # steps of about 0.3, and of 6, which leave nothing of what came before
+def test_walk_is_the_recurrence(heads, groups, lens, n_decode, step):
+    c = case(heads, groups, 128, 64, lens, n_decode, step=step)
+    want, states = recurrence(c, False)
+    size, sizes = recurrence(c, True)
+    untouched = c["state"].clone()
+    walk(c)
+    # operands keep 16 bits or more (2^-17 each of state, scores and weighted values); sums over 64 tokens and 128 channels in 32 bits
+    bound = 2.0 ** -14
+    assert bool(((c["y"][n_decode:].to(F64) - want).abs() <= bound * size + 1e-30).all())
+    assert bool((c["y"][:n_decode] == 7.0).all())
+    mine = c["slot"][n_decode:].long()
+    for i, slot in enumerate(mine.tolist()):
+        assert bool(((c["state"][slot].to(F64) - states[i]).abs() <= bound * sizes[i] + 1e-30).all())
+    other = torch.ones(untouched.shape[0], dtype=torch.bool, device=mine.device)
+    other[mine] = False
+    assert torch.equal(c["state"][other], untouched[other])
+
+
+def test_walk_keeps_portions_apart():
+    """What one portion holds, not-a-numbers too, stays out of the next one's rows and state."""
+    c = case(4, 2, 128, 64, [40, 90], 0, seed=1)
+    want, states = recurrence(c, False)
+    size, sizes = recurrence(c, True)
+    c["xbc"][40:] = float("nan")
+    walk(c)
+    assert bool(((c["y"][:40].to(F64) - want[:40]).abs() <= 2.0 ** -14 * size[:40] + 1e-30).all())
+    slot = int(c["slot"][0])
+    assert bool(((c["state"][slot].to(F64) - states[0]).abs() <= 2.0 ** -14 * sizes[0] + 1e-30).all())
+    assert bool(c["state"][int(c["slot"][1])].isnan().all())
