@@ -236,6 +236,11 @@ int msa_topk_select(const uint32_t* score_keys, int64_t table_stride, int32_t n_
                     int32_t n_cols, int32_t k, const int64_t* doc_ids_table, float* out_scores,
                     int64_t* out_local_ids, int64_t* out_global_ids, void* workspace,
                     int64_t workspace_bytes, void* stream);
+/* The same as the winners of the only rank, what msa_topk_merge makes of one rank's candidates: out_rank 0, out_local_ids -1 where the
+ * score is not above invalid_below.  out_rank null: msa_topk_select. */
+int msa_topk_winners(const uint32_t* score_keys, int64_t table_stride, int32_t n_seq, int32_t n_cols, int32_t k,
+                     const int64_t* doc_ids_table, float* out_scores, int64_t* out_local_ids, int64_t* out_global_ids,
+                     float invalid_below, int32_t* out_rank, void* workspace, int64_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * Routing, steps 2 + 3 in one call for decode-time routing (one query row per sequence).
@@ -257,6 +262,12 @@ int msa_topk_select(const uint32_t* score_keys, int64_t table_stride, int32_t n_
  */
 int64_t msa_route_score_select_workspace_bytes(int32_t n_seq, int32_t k);
 
+int msa_route_score_winners(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
+                            const void* rk, int64_t rk_chunk_stride, int32_t n_chunks, int32_t kdim,
+                            const int32_t* chunk_doc, float alpha, int32_t n_docs, float min_val, int32_t k,
+                            const int64_t* doc_ids_table, float* out_scores, int64_t* out_local_ids,
+                            int64_t* out_global_ids, float invalid_below, int32_t* out_rank, void* workspace,
+                            int64_t workspace_bytes, uint32_t flags, int32_t* status, void* stream);   /* see msa_topk_winners */
 int msa_route_score_select(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
                            const void* rk, int64_t rk_chunk_stride, int32_t n_chunks, int32_t kdim,
                            const int32_t* chunk_doc, float alpha, int32_t n_docs, float min_val, int32_t k,

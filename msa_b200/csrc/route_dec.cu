@@ -483,7 +483,7 @@ using namespace msa;
 
 namespace msa {
 int launch_topk_from_candidates(const unsigned long long* cand, int n_in, int n_seq, int k_eff, const int64_t* doc_ids_table,
-                                float* out_scores, int64_t* out_local, int64_t* out_global, cudaStream_t stream,
+                                float* out_scores, int64_t* out_local, int64_t* out_global, float invalid_below, int32_t* out_rank, cudaStream_t stream,
                                 bool pdl = false);
 }
 
@@ -499,12 +499,12 @@ extern "C" int64_t msa_route_score_select_workspace_bytes(int32_t n_seq, int32_t
   return (int64_t)n_seq * n_sm * (k < kDecMaxKeep ? k : kDecMaxKeep) * (int64_t)sizeof(unsigned long long);
 }
 
-extern "C" int msa_route_score_select(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
+extern "C" int msa_route_score_winners(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
                                       const void* rk, int64_t rk_chunk_stride, int32_t n_chunks, int32_t kdim,
                                       const int32_t* chunk_doc, float alpha, int32_t n_docs, float min_val, int32_t k,
                                       const int64_t* doc_ids_table, float* out_scores, int64_t* out_local_ids,
-                                      int64_t* out_global_ids, void* workspace, int64_t workspace_bytes,
-                                      uint32_t flags, int32_t* status, void* stream) {
+                                      int64_t* out_global_ids, float invalid_below, int32_t* out_rank, void* workspace,
+                                      int64_t workspace_bytes, uint32_t flags, int32_t* status, void* stream) {
   MSA_REQUIRE(q_folded && row_bias && rk && chunk_doc && out_scores && out_local_ids && status && workspace,
               "route_score_select: null pointer");
   MSA_REQUIRE(n_seq >= 1 && n_chunks >= 1 && kdim > 0 && n_docs >= 1 && k >= 1, "route_score_select: bad sizes");
@@ -560,5 +560,16 @@ extern "C" int msa_route_score_select(const void* q_folded, const float* row_bia
   }
   MSA_LAUNCH_OK("route_dec_kernel");
   return launch_topk_from_candidates(p.cand, grid * k_eff, n_seq, k_eff, doc_ids_table, out_scores, out_local_ids,
-                                     out_global_ids, st, pdl);
+                                     out_global_ids, invalid_below, out_rank, st, pdl);
+}
+
+extern "C" int msa_route_score_select(const void* q_folded, const float* row_bias, int32_t dtype, int32_t n_seq,
+                                      const void* rk, int64_t rk_chunk_stride, int32_t n_chunks, int32_t kdim,
+                                      const int32_t* chunk_doc, float alpha, int32_t n_docs, float min_val, int32_t k,
+                                      const int64_t* doc_ids_table, float* out_scores, int64_t* out_local_ids,
+                                      int64_t* out_global_ids, void* workspace, int64_t workspace_bytes,
+                                      uint32_t flags, int32_t* status, void* stream) {
+  return msa_route_score_winners(q_folded, row_bias, dtype, n_seq, rk, rk_chunk_stride, n_chunks, kdim, chunk_doc, alpha, n_docs, min_val, k,
+                                 doc_ids_table, out_scores, out_local_ids, out_global_ids, 0.f, nullptr, workspace, workspace_bytes, flags, status,
+                                 stream);
 }

@@ -31,10 +31,17 @@ __global__ void fold_kernel(const T* __restrict__ q, long long stride_b, long lo
   for (int j = 0; j < V; ++j) acc[j] = 0.f;
 
   auto add_token = [&](int tok) {
+    const T* src = q + (long long)b * stride_b + (long long)h * n_groups * stride_h + (long long)tok * stride_s + d;
+    uint4 raw[4];                  // four heads in flight: one token per sequence is nothing but their latency
     for (int g = 0; g < n_groups; ++g) {
+      if (g % 4 == 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (g + j < n_groups) raw[j] = *reinterpret_cast<const uint4*>(src + (g + j) * stride_h);
+      }
+      const uint4 x = g % 4 == 0 ? raw[0] : g % 4 == 1 ? raw[1] : g % 4 == 2 ? raw[2] : raw[3];
       float v[V];
-      Elem<T>::load(q + (long long)b * stride_b + (long long)(h * n_groups + g) * stride_h +
-                        (long long)tok * stride_s + d, v);
+      Elem<T>::load(reinterpret_cast<const T*>(&x), v);
       if (normalize) {
         float ss = 0.f;
 #pragma unroll

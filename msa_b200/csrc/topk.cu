@@ -21,6 +21,19 @@ constexpr int kMinSlice = 2048;   // items per CTA at level 1 (power of two)
 constexpr int kMaxSlice = 8192;   // 64 KiB of shared memory
 constexpr int kSurvivorCap = 1024;   // items that may pass the threshold of the final level's selection
 
+// Where the final level writes.  With `rank` these are the winners of one rank that holds every document, as topk_merge_kernel would
+// write them: its launch and its results' allocations go (one question in 32 bits 142 -> 128 us).
+struct TopkOut {
+  float* scores; int64_t *local, *global;
+  int32_t* rank; float invalid_below;
+  __device__ __forceinline__ void put(long long o, float score, long long col, const int64_t* doc_ids_table) const {
+    scores[o] = score;
+    local[o] = rank && !(score > invalid_below) ? -1 : col;
+    if (global) global[o] = doc_ids_table ? doc_ids_table[col] : col;
+    if (rank) rank[o] = 0;
+  }
+};
+
 __device__ __forceinline__ void bitonic_sort_desc(unsigned long long* s, int n2) {
   for (int size = 2; size <= n2; size <<= 1)
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -44,7 +57,7 @@ __global__ void __launch_bounds__(kSortThreads)
 sort_topk_kernel(const uint32_t* __restrict__ keys, long long table_stride, int n_cols, int slice,
                  const unsigned long long* __restrict__ cand, int n_in, int n2, int keep,
                  unsigned long long* __restrict__ cand_out, const int64_t* __restrict__ doc_ids_table,
-                 float* __restrict__ out_scores, int64_t* __restrict__ out_local, int64_t* __restrict__ out_global) {
+                 TopkOut out) {
   extern __shared__ unsigned long long s_items[];
   const int row = blockIdx.y, sl = blockIdx.x;
   if (FROM_KEYS) {
@@ -66,11 +79,7 @@ sort_topk_kernel(const uint32_t* __restrict__ keys, long long table_stride, int 
   } else {
     for (int i = threadIdx.x; i < keep; i += kSortThreads) {
       const unsigned long long w = s_items[i];
-      const long long col = 0xffffffffu - (uint32_t)(w & 0xffffffffull);
-      const long long o = (long long)row * keep + i;
-      out_scores[o] = key_to_float((uint32_t)(w >> 32));
-      out_local[o] = col;
-      if (out_global) out_global[o] = doc_ids_table ? doc_ids_table[col] : col;
+      out.put((long long)row * keep + i, key_to_float((uint32_t)(w >> 32)), 0xffffffffu - (uint32_t)(w & 0xffffffffull), doc_ids_table);
     }
   }
 }
@@ -80,8 +89,7 @@ template <bool FROM_KEYS>
 __global__ void __launch_bounds__(kSortThreads)
 select_topk_kernel(const uint32_t* keys, long long table_stride, int n_cols, int slice,
                    const unsigned long long* cand, int n_in, int n2, int keep,
-                   unsigned long long* __restrict__ cand_out, const int64_t* __restrict__ doc_ids_table, float* __restrict__ out_scores,
-                   int64_t* __restrict__ out_local, int64_t* __restrict__ out_global) {
+                   unsigned long long* __restrict__ cand_out, const int64_t* __restrict__ doc_ids_table, TopkOut out) {
   extern __shared__ unsigned long long s_items[];
   __shared__ unsigned long long s_win[(kSortThreads / 32) * kSelectMaxK];
   __shared__ unsigned long long s_final[kSelectMaxK];
@@ -173,17 +181,8 @@ select_topk_kernel(const uint32_t* keys, long long table_stride, int n_cols, int
   }
   for (int i = threadIdx.x; i < keep; i += kSortThreads) {
     const unsigned long long w = s_final[i];
-    const long long o = (long long)row * keep + i;
-    if (w == 0ull) {   // fewer than `keep` real items (producers that dropped entries): an empty slot, not a column
-      out_scores[o] = -INFINITY;
-      out_local[o] = 0;
-      if (out_global) out_global[o] = doc_ids_table ? doc_ids_table[0] : 0;
-      continue;
-    }
-    const long long col = 0xffffffffu - (uint32_t)(w & 0xffffffffull);
-    out_scores[o] = key_to_float((uint32_t)(w >> 32));
-    out_local[o] = col;
-    if (out_global) out_global[o] = doc_ids_table ? doc_ids_table[col] : col;
+    // fewer than `keep` real items (producers that dropped entries): an empty slot, not a column
+    out.put((long long)row * keep + i, w ? key_to_float((uint32_t)(w >> 32)) : -INFINITY, w ? 0xffffffffu - (uint32_t)(w & 0xffffffffull) : 0u, doc_ids_table);
   }
 }
 
@@ -237,7 +236,8 @@ topk_merge_kernel(const float* __restrict__ cand_scores, const int64_t* __restri
 // 0 = empty) gathered from several producers; writes the best k_eff per row.  Used by the fused decode-time
 // routing kernel, whose CTAs are the producers.
 int launch_topk_from_candidates(const unsigned long long* cand, int n_in, int n_seq, int k_eff, const int64_t* doc_ids_table,
-                                float* out_scores, int64_t* out_local, int64_t* out_global, cudaStream_t stream, bool pdl) {
+                                float* out_scores, int64_t* out_local, int64_t* out_global, float invalid_below, int32_t* out_rank,
+                                cudaStream_t stream, bool pdl) {
   MSA_REQUIRE(n_in >= 1 && n_in <= kMaxSlice && k_eff >= 1 && k_eff <= kSelectMaxK && n_seq >= 1 && n_seq <= 65535,
               "topk (candidates): bad sizes");
   const int n2 = pow2_ceil(n_in);
@@ -245,7 +245,7 @@ int launch_topk_from_candidates(const unsigned long long* cand, int n_in, int n_
   MSA_OK_OR_RETURN(ensure_dynamic_smem(select_topk_kernel<false>, kMaxSlice * 8, configured));
   MSA_CUDA_OK(launch_kernel_pdl(select_topk_kernel<false>, dim3(1, n_seq), dim3(kSortThreads), (size_t)n2 * 8, stream, pdl,
                                 (const uint32_t*)nullptr, 0ll, 0, 0, cand, n_in, n2, k_eff, (unsigned long long*)nullptr,
-                                doc_ids_table, out_scores, out_local, out_global));
+                                doc_ids_table, TopkOut{out_scores, out_local, out_global, out_rank, invalid_below}));
   return MSA_OK;
 }
 
@@ -261,15 +261,17 @@ extern "C" int64_t msa_topk_workspace_bytes(int32_t n_seq, int32_t n_cols, int32
   return (int64_t)n_seq * n_slices * (k < n_cols ? k : n_cols) * (int64_t)sizeof(unsigned long long);
 }
 
-extern "C" int msa_topk_select(const uint32_t* score_keys, int64_t table_stride, int32_t n_seq, int32_t n_cols,
-                               int32_t k, const int64_t* doc_ids_table, float* out_scores, int64_t* out_local_ids,
-                               int64_t* out_global_ids, void* workspace, int64_t workspace_bytes, void* stream) {
+extern "C" int msa_topk_winners(const uint32_t* score_keys, int64_t table_stride, int32_t n_seq, int32_t n_cols,
+                                int32_t k, const int64_t* doc_ids_table, float* out_scores, int64_t* out_local_ids,
+                                int64_t* out_global_ids, float invalid_below, int32_t* out_rank, void* workspace, int64_t workspace_bytes,
+                                void* stream) {
   MSA_REQUIRE(score_keys && out_scores && out_local_ids, "topk_select: null pointer");
   MSA_REQUIRE(n_seq >= 0 && n_cols >= 1 && k >= 1, "topk_select: bad sizes (n_cols=%d k=%d)", n_cols, k);
   MSA_REQUIRE(k <= kMaxK, "topk_select: k=%d exceeds the supported maximum %d", k, kMaxK);
   MSA_REQUIRE(table_stride >= n_cols, "topk_select: table_stride < n_cols");
   MSA_REQUIRE(n_seq <= 65535, "topk_select: at most 65535 rows per call");
   if (n_seq == 0) return MSA_OK;
+  const TopkOut out{out_scores, out_local_ids, out_global_ids, out_rank, invalid_below};
   const int k_eff = k < n_cols ? k : n_cols;
   int slice, n_slices;
   topk_plan(n_cols, k, &slice, &n_slices);
@@ -286,12 +288,10 @@ extern "C" int msa_topk_select(const uint32_t* score_keys, int64_t table_stride,
     const int n2 = pow2_ceil(n_cols);
     if (small_k)
       select_topk_kernel<true><<<dim3(1, n_seq), kSortThreads, (size_t)n2 * 8, st>>>(
-          score_keys, table_stride, n_cols, n2, nullptr, 0, n2, k_eff, nullptr, doc_ids_table, out_scores,
-          out_local_ids, out_global_ids);
+          score_keys, table_stride, n_cols, n2, nullptr, 0, n2, k_eff, nullptr, doc_ids_table, out);
     else
       sort_topk_kernel<true><<<dim3(1, n_seq), kSortThreads, (size_t)n2 * 8, st>>>(
-          score_keys, table_stride, n_cols, n2, nullptr, 0, n2, k_eff, nullptr, doc_ids_table, out_scores,
-          out_local_ids, out_global_ids);
+          score_keys, table_stride, n_cols, n2, nullptr, 0, n2, k_eff, nullptr, doc_ids_table, out);
     MSA_LAUNCH_OK("topk kernel");
     return MSA_OK;
   }
@@ -301,20 +301,26 @@ extern "C" int msa_topk_select(const uint32_t* score_keys, int64_t table_stride,
   const int n_in = n_slices * k_eff, n2 = pow2_ceil(n_in);
   if (small_k) {
     select_topk_kernel<true><<<dim3(n_slices, n_seq), kSortThreads, (size_t)slice * 8, st>>>(
-        score_keys, table_stride, n_cols, slice, nullptr, 0, slice, k_eff, cand, nullptr, nullptr, nullptr, nullptr);
+        score_keys, table_stride, n_cols, slice, nullptr, 0, slice, k_eff, cand, nullptr, TopkOut{});
     MSA_LAUNCH_OK("select_topk_kernel (slices)");
     select_topk_kernel<false><<<dim3(1, n_seq), kSortThreads, (size_t)n2 * 8, st>>>(
-        nullptr, 0, 0, 0, cand, n_in, n2, k_eff, nullptr, doc_ids_table, out_scores, out_local_ids,
-        out_global_ids);
+        nullptr, 0, 0, 0, cand, n_in, n2, k_eff, nullptr, doc_ids_table, out);
   } else {
     sort_topk_kernel<true><<<dim3(n_slices, n_seq), kSortThreads, (size_t)slice * 8, st>>>(
-        score_keys, table_stride, n_cols, slice, nullptr, 0, slice, k_eff, cand, nullptr, nullptr, nullptr, nullptr);
+        score_keys, table_stride, n_cols, slice, nullptr, 0, slice, k_eff, cand, nullptr, TopkOut{});
     MSA_LAUNCH_OK("sort_topk_kernel (slices)");
     sort_topk_kernel<false><<<dim3(1, n_seq), kSortThreads, (size_t)n2 * 8, st>>>(
-        nullptr, 0, 0, 0, cand, n_in, n2, k_eff, nullptr, doc_ids_table, out_scores, out_local_ids, out_global_ids);
+        nullptr, 0, 0, 0, cand, n_in, n2, k_eff, nullptr, doc_ids_table, out);
   }
   MSA_LAUNCH_OK("sort_topk_kernel (final)");
   return MSA_OK;
+}
+
+extern "C" int msa_topk_select(const uint32_t* score_keys, int64_t table_stride, int32_t n_seq, int32_t n_cols,
+                               int32_t k, const int64_t* doc_ids_table, float* out_scores, int64_t* out_local_ids,
+                               int64_t* out_global_ids, void* workspace, int64_t workspace_bytes, void* stream) {
+  return msa_topk_winners(score_keys, table_stride, n_seq, n_cols, k, doc_ids_table, out_scores, out_local_ids, out_global_ids, 0.f, nullptr,
+                          workspace, workspace_bytes, stream);
 }
 
 extern "C" int msa_topk_merge(const float* cand_scores, const int64_t* cand_local, const int64_t* cand_global,

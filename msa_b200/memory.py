@@ -531,18 +531,27 @@ class Memory:
         torch.cuda.current_stream(self.device).wait_event(ready[1])      # join, whatever happens next
         return self._table if ready[0] == n_seq else None
 
-    def score_folded(self, layer_idx: int, q_folded, row_bias, n_seq: int, s_pad: int, n_heads: int, top_k: int,
-                     scale: float = 1.0, out=None):
-        """Score ``n_seq`` folded sequences (head_reduce "mean") against this shard and select ``top_k``
-        documents each (``out``: see ``ops.topk_select``).  chunk_reduce "max" is one fused kernel; "mean"
-        fills a per-chunk table with the same kernel (every chunk its own document) and reduces it."""
-        desc = self.block_desc
+    def _router_keys(self, layer_idx: int, s_pad: int):
+        """The layer's router keys for rows of ``s_pad`` tokens, and whether they are the tile-blocked ones."""
         blk = self.blocks[layer_idx]
         use_blocked = blk.rk_blocked is not None and (blk.rk is None or s_pad == 1)   # bandwidth-bound shapes, or no rows left
-        keys_src = blk.rk_blocked if use_blocked else blk.rk
+        return (blk.rk_blocked if use_blocked else blk.rk), use_blocked
+
+    def _selects_in_routing(self, layer_idx: int, n_seq: int, s_pad: int, top_k: int) -> bool:
+        """Whether ``score_folded`` takes the kernel that keeps no score table."""
+        keys_src, use_blocked = self._router_keys(layer_idx, s_pad)
+        return (self.chunk_reduce_method == "max" and self.fused_decode_routing
+                and ops.route_score_select_supported(keys_src, n_seq, s_pad, top_k, use_blocked))
+
+    def score_folded(self, layer_idx: int, q_folded, row_bias, n_seq: int, s_pad: int, n_heads: int, top_k: int,
+                     scale: float = 1.0, out=None, winners: bool = False):
+        """Score ``n_seq`` folded sequences (head_reduce "mean") against this shard and select ``top_k``
+        documents each (``out``, ``winners``: see ``ops.topk_select``).  chunk_reduce "max" is one fused kernel; "mean"
+        fills a per-chunk table with the same kernel (every chunk its own document) and reduces it."""
+        desc = self.block_desc
+        keys_src, use_blocked = self._router_keys(layer_idx, s_pad)
         min_val = torch.finfo(keys_src.dtype).min
-        if self.chunk_reduce_method == "max" and self.fused_decode_routing and \
-                ops.route_score_select_supported(keys_src, n_seq, s_pad, top_k, use_blocked):
+        if self._selects_in_routing(layer_idx, n_seq, s_pad, top_k):
             # one token per sequence: scoring and per-CTA selection in one launch, no score table
             need = (n_seq, top_k)
             ws = self.__dict__.get("_select_ws")
@@ -551,7 +560,7 @@ class Memory:
                 ws = self._select_ws = (need, torch.empty((max(n_bytes, 8) + 7) // 8, dtype=torch.int64, device=self.device))
             self._take_prepared_table(n_seq)      # joins a table reset that a caller may have started
             return ops.route_score_select(q_folded, row_bias, n_seq, keys_src, desc.chunk_doc, desc.nr_docs, scale / n_heads,
-                                          top_k, desc.doc_ids, min_val, self._status, ws[1], out, blocked=use_blocked)
+                                          top_k, desc.doc_ids, min_val, self._status, ws[1], out, blocked=use_blocked, winners=winners)
         prepared = self._take_prepared_table(n_seq)
         if self.chunk_reduce_method == "max":
             keys, _ = ops.route_scores(q_folded, row_bias, n_seq, s_pad, keys_src, desc.chunk_doc, desc.nr_docs,
@@ -565,7 +574,7 @@ class Memory:
             chunk_keys, _ = ops.route_scores(q_folded, row_bias, n_seq, s_pad, keys_src, ident, c, alpha=scale / n_heads,
                                              min_val=min_val, status=self._status, blocked=use_blocked)
             keys = ops.route_reduce_chunks(chunk_keys, desc.chunk_doc, desc.nr_docs, "mean", min_val, status=self._status)
-        return self._select(keys, n_seq, top_k, out)
+        return self._select(keys, n_seq, top_k, out, winners)
 
     def score_unfolded(self, layer_idx: int, query_states, query_mask, top_k: int, scale: float = 1.0, out=None):
         """head_reduce "max": the heads cannot be folded, so the unfolded queries ``[B, Hq, S, D]`` are scored per
@@ -581,13 +590,13 @@ class Memory:
                                        status=self._status)
         return self._select(keys, query_states.shape[0], top_k, out)
 
-    def _select(self, keys, n_seq: int, top_k: int, out=None):
+    def _select(self, keys, n_seq: int, top_k: int, out=None, winners: bool = False):
         desc = self.block_desc
         need = ops.topk_workspace_bytes(n_seq, desc.nr_docs + 1, top_k)
         ws = getattr(self, "_topk_ws", None)
         if need and (ws is None or ws.numel() * 8 < need):
             ws = self._topk_ws = torch.empty((need + 7) // 8, dtype=torch.int64, device=self.device)
-        return ops.topk_select(keys, top_k, desc.doc_ids, workspace=ws if need else None, out=out)
+        return ops.topk_select(keys, top_k, desc.doc_ids, workspace=ws if need else None, out=out, winners=winners)
 
     def prefill_stage2(self, layer_idx: int, query_states: torch.Tensor, query_mask: torch.Tensor):
         """src/msa_service.py:703-828.  query_states ``[B, Hkv, G, S, D]``, query_mask

@@ -261,11 +261,11 @@ def route_score_select(q_folded: torch.Tensor, row_bias: torch.Tensor, n_seq: in
                        chunk_doc: torch.Tensor, n_docs: int, alpha: float, top_k: int,
                        doc_ids_table: Optional[torch.Tensor] = None, min_val: Optional[float] = None,
                        status: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None, out=None,
-                       blocked: bool = False):
+                       blocked: bool = False, winners: bool = False, invalid_below: float = -1e9):
     """Decode-time routing in one call: scores ``n_seq`` single-row queries against the shard and selects the best
     ``top_k`` documents of each, without a score table (see ``msa_route_score_select``).  Same results, ties included,
     as ``route_scores`` + ``topk_select``.  ``rk`` as in ``route_scores`` (row major, or tile-blocked with ``blocked``).
-    Returns ``(scores f32, local_ids i64, global_ids i64)``, ``[n_seq, k_eff]``."""
+    Returns ``(scores f32, local_ids i64, global_ids i64)``, ``[n_seq, k_eff]``; ``winners``: as ``topk_select``."""
     A.need_cuda(q_folded, row_bias, rk, chunk_doc, doc_ids_table, status, workspace)
     dev = rk.device
     if chunk_doc.dtype != torch.int32:
@@ -298,13 +298,15 @@ def route_score_select(q_folded: torch.Tensor, row_bias: torch.Tensor, n_seq: in
         raise A.MsaError("route_score_select: no CUDA device is current")
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         workspace = torch.empty((need + 7) // 8, dtype=torch.int64, device=dev)
-    A.check(A.lib().msa_route_score_select(A.ptr(q_folded), A.ptr(row_bias), A.dtype_code(rk.dtype), n_seq, A.ptr(rk2),
-                                           stride, c, kdim, A.ptr(chunk_doc), float(alpha), n_docs,
-                                           float(min_val), top_k, A.ptr(doc_ids_table), A.ptr(scores), A.ptr(local),
-                                           A.ptr(glob), A.ptr(workspace), workspace.numel() * workspace.element_size(),
-                                           A.ROUTE_KEYS_BLOCKED if blocked else 0, A.ptr(status), A.stream_ptr(dev)),
+    rank = torch.empty((n_seq, k_eff), dtype=torch.int32, device=dev) if winners else None
+    A.check(A.lib().msa_route_score_winners(A.ptr(q_folded), A.ptr(row_bias), A.dtype_code(rk.dtype), n_seq, A.ptr(rk2),
+                                            stride, c, kdim, A.ptr(chunk_doc), float(alpha), n_docs,
+                                            float(min_val), top_k, A.ptr(doc_ids_table), A.ptr(scores), A.ptr(local),
+                                            A.ptr(glob), float(invalid_below), A.ptr(rank), A.ptr(workspace),
+                                            workspace.numel() * workspace.element_size(),
+                                            A.ROUTE_KEYS_BLOCKED if blocked else 0, A.ptr(status), A.stream_ptr(dev)),
             "msa_route_score_select")
-    return scores, local, glob
+    return (scores, local, glob, rank) if winners else (scores, local, glob)
 
 
 def route_table_reset(keys: torch.Tensor, n_docs: int, min_val: float, status: Optional[torch.Tensor] = None):
@@ -318,10 +320,11 @@ def topk_workspace_bytes(n_seq: int, n_cols: int, k: int) -> int:
 
 
 def topk_select(keys: torch.Tensor, k: int, doc_ids_table: Optional[torch.Tensor] = None, n_cols: Optional[int] = None,
-                workspace: Optional[torch.Tensor] = None, out=None):
+                workspace: Optional[torch.Tensor] = None, out=None, winners: bool = False, invalid_below: float = -1e9):
     """Exact top-k of every row of a key table.  Returns ``(scores f32, local_ids i64, global_ids i64)``,
     each ``[n_seq, min(k, n_cols)]``, sorted by descending score (ties: ascending column).
-    ``out``: three contiguous tensors of those shapes to write into (e.g. the planes of ``candidate_buffer``)."""
+    ``out``: three contiguous tensors of those shapes to write into (e.g. the planes of ``candidate_buffer``).
+    ``winners``: what ``topk_merge`` makes of one rank's candidates, ``(scores, local_ids (-1 = invalid), global_ids, rank i32)``."""
     A.need_cuda(keys, doc_ids_table)
     n_seq = keys.shape[0]
     n_cols = keys.shape[1] if n_cols is None else n_cols
@@ -339,11 +342,12 @@ def topk_select(keys: torch.Tensor, k: int, doc_ids_table: Optional[torch.Tensor
     need = int(A.lib().msa_topk_workspace_bytes(n_seq, n_cols, k))
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         workspace = torch.empty((need + 7) // 8, dtype=torch.int64, device=dev)
-    A.check(A.lib().msa_topk_select(A.ptr(keys), keys.stride(0), n_seq, n_cols, k, A.ptr(doc_ids_table),
-                                    A.ptr(scores), A.ptr(local), A.ptr(glob), A.ptr(workspace),
-                                    workspace.numel() * workspace.element_size() if workspace is not None else 0,
-                                    A.stream_ptr(dev)), "msa_topk_select")
-    return scores, local, glob
+    rank = torch.empty((n_seq, k_eff), dtype=torch.int32, device=dev) if winners else None
+    A.check(A.lib().msa_topk_winners(A.ptr(keys), keys.stride(0), n_seq, n_cols, k, A.ptr(doc_ids_table),
+                                     A.ptr(scores), A.ptr(local), A.ptr(glob), float(invalid_below), A.ptr(rank), A.ptr(workspace),
+                                     workspace.numel() * workspace.element_size() if workspace is not None else 0,
+                                     A.stream_ptr(dev)), "msa_topk_select")
+    return (scores, local, glob, rank) if winners else (scores, local, glob)
 
 
 def candidate_buffer(n_seq: int, k: int, device):
