@@ -385,6 +385,13 @@ int msa_gather_run(const int64_t* plan, int32_t n_items, int32_t dtype, int32_t 
 int64_t msa_decode_workspace_bytes(int32_t n_seq, int32_t n_q_heads, int32_t head_dim,
                                    int32_t n_splits);
 
+/* ... and the lengths behind the appended token: next_len = kv_len + 1, next_lengths = lengths + 1 (null: not wanted). */
+int msa_sparse_decode_attn_next(const void* q, int32_t dtype, void* k_cache, void* v_cache,
+                                int64_t stride_b, int64_t stride_h, const int32_t* kv_start,
+                                const int32_t* kv_len, const void* new_k, const void* new_v,
+                                int32_t n_seq, int32_t n_q_heads, int32_t n_kv_heads, int32_t head_dim,
+                                float scale, void* out, void* workspace, int64_t workspace_bytes,
+                                int32_t n_splits, const int64_t* lengths, int32_t* next_len, int64_t* next_lengths, void* stream);
 int msa_sparse_decode_attn(const void* q, int32_t dtype, void* k_cache, void* v_cache,
                            int64_t stride_b, int64_t stride_h, const int32_t* kv_start,
                            const int32_t* kv_len, const void* new_k, const void* new_v,

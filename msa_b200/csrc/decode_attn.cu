@@ -18,15 +18,22 @@ constexpr int kMaxAcc = 4;  // float4 accumulators per thread: G*D <= 2048
 template <typename T> struct DecTile { static constexpr int kKeys = 64; };
 template <> struct DecTile<float> { static constexpr int kKeys = 32; };
 
+// With `len`, the launch that appends also writes the lengths behind it: [n_seq] each, `old` and `lengths` as the caller counts.
+struct DecodeNext { const int64_t* old; int32_t* len; int64_t* lengths; };
+
 template <typename T>
 __global__ void append_kv_kernel(T* __restrict__ k_cache, T* __restrict__ v_cache, long long stride_b,
                                  long long stride_h, const int32_t* __restrict__ kv_start,
                                  const int32_t* __restrict__ kv_len, const T* __restrict__ new_k,
-                                 const T* __restrict__ new_v, int n_kv_heads, int head_dim) {
+                                 const T* __restrict__ new_v, int n_kv_heads, int head_dim, const DecodeNext next) {
   const int b = blockIdx.y, h = blockIdx.x;
   const long long pos = (kv_start ? kv_start[b] : 0) + (long long)kv_len[b];
   const long long dst = (long long)b * stride_b + (long long)h * stride_h + pos * head_dim;
   const long long src = ((long long)b * n_kv_heads + h) * head_dim;
+  if (next.len && h == 0 && threadIdx.x == 0) {
+    next.len[b] = kv_len[b] + 1;
+    next.lengths[b] = next.old[b] + 1;
+  }
   for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
     k_cache[dst + d] = new_k[src + d];
     v_cache[dst + d] = new_v[src + d];
@@ -200,14 +207,14 @@ template <typename T>
 int launch_decode(const void* q, void* k_cache, void* v_cache, int64_t stride_b, int64_t stride_h,
                   const int32_t* kv_start, const int32_t* kv_len, const void* new_k, const void* new_v, int n_seq,
                   int n_q_heads, int n_kv_heads, int head_dim, float scale, void* out, void* workspace,
-                  int n_splits, cudaStream_t stream) {
+                  int n_splits, DecodeNext next, cudaStream_t stream) {
   constexpr int KT = DecTile<T>::kKeys;
   constexpr int V = Elem<T>::kVec;
   const int G = n_q_heads / n_kv_heads;
   if (new_k) {
     append_kv_kernel<T><<<dim3(n_kv_heads, n_seq), 128, 0, stream>>>(
         (T*)k_cache, (T*)v_cache, stride_b, stride_h, kv_start, kv_len, (const T*)new_k, (const T*)new_v,
-        n_kv_heads, head_dim);
+        n_kv_heads, head_dim, next);
     MSA_LAUNCH_OK("append_kv_kernel");
   }
   const size_t smem = (size_t)KT * (head_dim + V) * sizeof(T) + (size_t)KT * head_dim * sizeof(T) +
@@ -232,12 +239,12 @@ int launch_decode(const void* q, void* k_cache, void* v_cache, int64_t stride_b,
 int launch_decode_mma(const void* q, void* k_cache, void* v_cache, int64_t stride_b, int64_t stride_h,
                       const int32_t* kv_start, const int32_t* kv_len, const void* new_k, const void* new_v, int n_seq,
                       int n_q_heads, int n_kv_heads, float scale, void* out, void* workspace, int n_splits,
-                      cudaStream_t stream) {
+                      DecodeNext next, cudaStream_t stream) {
   using T = __nv_bfloat16;
   if (new_k) {
     append_kv_kernel<T><<<dim3(n_kv_heads, n_seq), 128, 0, stream>>>(
         (T*)k_cache, (T*)v_cache, stride_b, stride_h, kv_start, kv_len, (const T*)new_k, (const T*)new_v,
-        n_kv_heads, kMmaD);
+        n_kv_heads, kMmaD, next);
     MSA_LAUNCH_OK("append_kv_kernel");
   }
   static DeviceSmem configured{};
@@ -263,11 +270,14 @@ extern "C" int64_t msa_decode_workspace_bytes(int32_t n_seq, int32_t n_q_heads, 
   return (int64_t)n_seq * n_q_heads * n_splits * (head_dim + 2) * (int64_t)sizeof(float);
 }
 
-extern "C" int msa_sparse_decode_attn(const void* q, int32_t dtype, void* k_cache, void* v_cache, int64_t stride_b,
+extern "C" int msa_sparse_decode_attn_next(const void* q, int32_t dtype, void* k_cache, void* v_cache, int64_t stride_b,
                                       int64_t stride_h, const int32_t* kv_start, const int32_t* kv_len,
                                       const void* new_k, const void* new_v, int32_t n_seq, int32_t n_q_heads,
                                       int32_t n_kv_heads, int32_t head_dim, float scale, void* out, void* workspace,
-                                      int64_t workspace_bytes, int32_t n_splits, void* stream) {
+                                      int64_t workspace_bytes, int32_t n_splits, const int64_t* lengths, int32_t* next_len,
+                                      int64_t* next_lengths, void* stream) {
+  MSA_REQUIRE(!next_len || (new_k && lengths && next_lengths), "decode: the next lengths need a token to append and the lengths before");
+  const DecodeNext next{lengths, next_len, next_lengths};
   MSA_REQUIRE(dtype_ok(dtype), "decode: unknown dtype %d", dtype);
   MSA_REQUIRE(q && k_cache && v_cache && kv_len && out, "decode: null pointer");
   MSA_REQUIRE((new_k == nullptr) == (new_v == nullptr), "decode: new_k and new_v must be given together");
@@ -288,12 +298,21 @@ extern "C" int msa_sparse_decode_attn(const void* q, int32_t dtype, void* k_cach
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == MSA_BF16 && head_dim == kMmaD && n_q_heads / n_kv_heads <= 8)
     return launch_decode_mma(q, k_cache, v_cache, stride_b, stride_h, kv_start, kv_len, new_k, new_v, n_seq, n_q_heads,
-                             n_kv_heads, scale, out, workspace, n_splits, st);
+                             n_kv_heads, scale, out, workspace, n_splits, next, st);
   return dtype == MSA_BF16
              ? launch_decode<__nv_bfloat16>(q, k_cache, v_cache, stride_b, stride_h, kv_start, kv_len, new_k, new_v,
-                                            n_seq, n_q_heads, n_kv_heads, head_dim, scale, out, workspace, n_splits, st)
+                                            n_seq, n_q_heads, n_kv_heads, head_dim, scale, out, workspace, n_splits, next, st)
              : launch_decode<float>(q, k_cache, v_cache, stride_b, stride_h, kv_start, kv_len, new_k, new_v, n_seq,
-                                    n_q_heads, n_kv_heads, head_dim, scale, out, workspace, n_splits, st);
+                                    n_q_heads, n_kv_heads, head_dim, scale, out, workspace, n_splits, next, st);
+}
+
+extern "C" int msa_sparse_decode_attn(const void* q, int32_t dtype, void* k_cache, void* v_cache, int64_t stride_b,
+                                      int64_t stride_h, const int32_t* kv_start, const int32_t* kv_len,
+                                      const void* new_k, const void* new_v, int32_t n_seq, int32_t n_q_heads,
+                                      int32_t n_kv_heads, int32_t head_dim, float scale, void* out, void* workspace,
+                                      int64_t workspace_bytes, int32_t n_splits, void* stream) {
+  return msa_sparse_decode_attn_next(q, dtype, k_cache, v_cache, stride_b, stride_h, kv_start, kv_len, new_k, new_v, n_seq, n_q_heads, n_kv_heads,
+                                     head_dim, scale, out, workspace, workspace_bytes, n_splits, nullptr, nullptr, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------------------

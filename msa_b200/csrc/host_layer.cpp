@@ -4,7 +4,8 @@
 // them (module calls, attribute look-ups through nn.Module.__getattr__, ctypes); 371 us now, and 16 questions of 96 tokens 1361 us
 // instead of 1566.  Here a layer is two calls around the attention of its stage:
 // `front` (residual add and norm, q / k / v, head norm and rotation) and `back` (output product, residual add and norm, gated
-// feed-forward), and a third for the attention of a single token.  Products are the same at::linear calls that nn.Linear makes.
+// feed-forward), and a third for the attention of a single token.  Products are the library calls
+// that nn.Linear comes to.
 //
 // Nothing is kept between calls.  `layers` reads the modules anew each time and answers None where anything is not what it steps
 // over: another class, a hook, a forward of its own, a bias, a subclass of Tensor, another device or type; every other function
@@ -26,7 +27,7 @@ using at::Tensor;
 namespace py = pybind11;
 
 #define MSA_FUNCTIONS(F) \
-  F(msa_last_error) F(msa_add_rmsnorm) F(msa_heads_norm_rope) F(msa_silu_mul_parts) F(msa_rope_table) F(msa_decode_workspace_bytes) F(msa_sparse_decode_attn)
+  F(msa_last_error) F(msa_add_rmsnorm) F(msa_heads_norm_rope) F(msa_silu_mul_parts) F(msa_rope_table) F(msa_decode_workspace_bytes) F(msa_sparse_decode_attn_next)
 struct Library {
 #define MSA_MEMBER(name) decltype(&::name) name = nullptr;
   MSA_FUNCTIONS(MSA_MEMBER)
@@ -171,6 +172,12 @@ py::object layers(const py::tuple& modules, const py::tuple& classes) {
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 bool rows_fit(const Tensor& x) { return x.dim() == 3 && x.numel() > 0 && x.size(0) * x.size(1) < (1ll << 31); }
 
+// x w^T for rows [batch, tokens, features]: the product that at::linear comes to, without its detour over shapes (6.5 -> 4 us a call)
+Tensor product(const Tensor& x, const Tensor& w) {
+  const int64_t b = x.size(0), s = x.size(1);
+  return at::mm(x.view({b * s, x.size(2)}), w.t()).view({b, s, w.size(0)});
+}
+
 // (x + branch, norm(x + branch))
 std::pair<Tensor, Tensor> add_norm_of(const Tensor& x, const Tensor& branch, const Norm& n) {
   const int64_t hidden = x.size(-1);
@@ -209,7 +216,7 @@ py::object front(const Layer& l, const py::object& x_, const py::object& branch_
     return py::none();
   const c10::cuda::CUDAGuard guard(dev);
   auto [x_new, h] = add_norm_of(x, branch, l.in);
-  const Tensor q0 = at::linear(h, l.q), k0 = at::linear(h, l.k), v = at::linear(h, l.v);
+  const Tensor q0 = product(h, l.q), k0 = product(h, l.k), v = product(h, l.v);
   Tensor q = at::empty_like(q0), k = at::empty_like(k0);
   const int64_t heads = l.q.size(0), kv = l.k.size(0);
   check(lib.msa_heads_norm_rope(q0.const_data_ptr(), heads, k0.const_data_ptr(), kv, (int32_t)(x.size(0) * x.size(1)), (int32_t)(heads / kHead),
@@ -228,14 +235,14 @@ py::object back(const Layer& l, const py::object& x_, const py::object& attn_) {
       attn.size(1) != x.size(1) || attn.size(2) != l.o.size(1))
     return py::none();
   const c10::cuda::CUDAGuard guard(dev);
-  auto [x_new, h] = add_norm_of(x, at::linear(attn, l.o), l.post);
-  const Tensor gate = at::linear(h, l.gate), up = at::linear(h, l.up);
+  auto [x_new, h] = add_norm_of(x, product(attn, l.o), l.post);
+  const Tensor gate = product(h, l.gate), up = product(h, l.up);
   Tensor act = at::empty_like(gate);
   const int64_t ffn = l.gate.size(0);
   check(lib.msa_silu_mul_parts(gate.const_data_ptr(), ffn, up.const_data_ptr(), ffn, (int32_t)(x.size(0) * x.size(1)), (int32_t)ffn, act.data_ptr(),
                                stream_of(x)),
         "msa_silu_mul_parts");
-  return py::make_tuple(x_new, at::linear(act, l.down));
+  return py::make_tuple(x_new, product(act, l.down));
 }
 
 // cos and sin of positions [batch, tokens] (int64): bf16 [batch, tokens, 2 * frequencies]
@@ -273,12 +280,17 @@ py::object decode(const py::object& q_, const py::object& k_, const py::object& 
   Tensor out = at::empty({b, 1, hq * d}, q.options()), space;
   const int64_t need = lib.msa_decode_workspace_bytes((int32_t)b, (int32_t)hq, (int32_t)d, (int32_t)n_splits);
   if (need > 0) space = at::empty({need / 4}, q.options().dtype(at::kFloat));
-  check(lib.msa_sparse_decode_attn(q.const_data_ptr(), MSA_BF16, ks.data_ptr(), vs.data_ptr(), ks.stride(0), ks.stride(1),
+  const bool counts = takes(lengths, at::kLong, dev) && lengths.numel() == b && lengths.dim() == 1 && len.dim() == 1;
+  const Tensor next_len = counts ? at::empty_like(len) : Tensor(), next_lengths = counts ? at::empty_like(lengths) : Tensor();
+  check(lib.msa_sparse_decode_attn_next(q.const_data_ptr(), MSA_BF16, ks.data_ptr(), vs.data_ptr(), ks.stride(0), ks.stride(1),
                                    static_cast<const int32_t*>(start.const_data_ptr()), static_cast<const int32_t*>(len.const_data_ptr()),
                                    k.const_data_ptr(), v.const_data_ptr(), (int32_t)b, (int32_t)hq, (int32_t)hkv, (int32_t)d,
                                    (float)(1.0 / std::sqrt((double)d)), out.data_ptr(), need > 0 ? space.data_ptr() : nullptr, need > 0 ? need : 0,
-                                   (int32_t)n_splits, stream_of(q)),
+                                   (int32_t)n_splits, counts ? static_cast<const int64_t*>(lengths.const_data_ptr()) : nullptr,
+                                   counts ? static_cast<int32_t*>(next_len.data_ptr()) : nullptr,
+                                   counts ? static_cast<int64_t*>(next_lengths.data_ptr()) : nullptr, stream_of(q)),
         "msa_sparse_decode_attn");
+  if (counts) return py::make_tuple(out, next_len, next_lengths);
   return py::make_tuple(out, len.add(1), lengths.add(1));
 }
 
