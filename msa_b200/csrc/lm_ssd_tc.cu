@@ -13,9 +13,9 @@
 // Warps by role: 0-7 scores -> P, 8-11 states and the values (weighted as TMEM planes, transposed in shared memory), 12-19 outputs,
 // 20-22 fetch (two chunks' buffers) and sum up the decays, 23 issues the products.
 // What bounds it: instructions of the conversions (3,700 per scheduler and chunk, issued at 0.43 a cycle: their latencies, with five
-// or six warps per scheduler) and the order scores -> P -> outputs -> next scores, which share TMEM.  Portions of 2048, 1500, 1911 and
-// 777 tokens, 64 heads, from a cold L2: 166 us, where the three kernels over all chunks at once take 447 (chunk states through HBM
-// four times, products on mma.sync).
+// or six warps per scheduler), 56 products of some 70 cycles each, whatever their columns, and the order scores -> P -> outputs -> next
+// scores, which share TMEM.  Portions of 2048, 1500, 1911 and 777 tokens, 64 heads, from a cold L2: 173 us, where the three kernels
+// over all chunks at once take 447 (chunk states through HBM four times, products on mma.sync).
 #include "lm_linear.cuh"
 #include "mma_helpers.cuh"
 #include "tc_attn_common.cuh"
@@ -37,7 +37,7 @@ struct SsdTcParams {
   const float* dt;               // [rows, heads]
   int32_t* status;
 };
-struct SsdTcBars { uint64_t full[2], free[2], g_full, z_done, p_ready, s_ready, x_ready, s_done, o_done, o_free, drain; };
+struct SsdTcBars { uint64_t full[2], free[2], g_full[2], z_done, p_ready, s_ready, x_ready, s_done, o_done, o_free, drain; };
 struct SsdTcDecay {              // of a chunk, per head
   float gh[2][kStRows], gl[2][kStRows], eg[2][kStRows], dt[2][kStRows], w[2][kStRows], all[2];      // G as a pair of floats
 };
@@ -63,8 +63,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
   const int len = a.cu[sq + 1] - a.cu[sq], n_chunks = (len + kStRows - 1) / kStRows;
   const long long n0 = a.cu[sq], row0 = n0 - a.n_decode;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars.full[i], 3); mbar_init(&bars.free[i], 9); }
-    mbar_init(&bars.g_full, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars.full[i], 3); mbar_init(&bars.free[i], 9); mbar_init(&bars.g_full[i], 1); }
     mbar_init(&bars.z_done, 1); mbar_init(&bars.s_done, 1); mbar_init(&bars.o_done, 1); mbar_init(&bars.drain, 1);
     mbar_init(&bars.p_ready, 8); mbar_init(&bars.s_ready, 4); mbar_init(&bars.x_ready, 4); mbar_init(&bars.o_free, 8);
     s_abort = 0;
@@ -195,10 +194,10 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
       if (warp > 8) continue;
       if (!(ok = wait(&bars.x_ready, ch, 64))) break;      // the four warps have read the values: the gates take their place
       if (lane == 0) {
-        mbar_expect_tx(&bars.g_full, 2 * kStPlane);
+        mbar_expect_tx(&bars.g_full[b], 2 * kStPlane);
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk)
-          tma_load_2d(sm + b * kStBuf + kStX + blk * kStPlane, &map_g, h0 * kStV + blk * 64, (int)n0 + ch * kStRows, &bars.g_full);
+          tma_load_2d(sm + b * kStBuf + kStX + blk * kStPlane, &map_g, h0 * kStV + blk * 64, (int)n0 + ch * kStRows, &bars.g_full[b]);
       }
     }
     if (ok && n_chunks > 0 && wait(&bars.s_done, n_chunks + 1, 54)) {
@@ -233,7 +232,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
       }
       tc_fence_before();
       arrive(&bars.o_free);
-      if (!wait(&bars.g_full, ch, 63)) break;
+      if (!wait(&bars.g_full[b], ch >> 1, 63)) break;      // a barrier per buffer: the next chunk's gates may come before these are asked for
       const unsigned char *row = sm + kStXt + b * 2 * kStPlane, *gate = sm + b * kStBuf + kStX + hd * kStPlane + col % 8 * 2;
       float* dst = out + (long long)(ch * kStRows + part) * inner;
 #pragma unroll
@@ -364,16 +363,18 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
       if (!(ok = one(&bars.p_ready, ch, 61))) break;
       tc_fence_after();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {                                     // tokens k*16 .. reach the columns from there on
+      for (int k = 0; k < 4; ++k) {
+        // Tokens from 32 on reach the columns from there on (P has nothing before).  Halves of 32 columns throughout: products into the
+        // same columns keep their order only if they have the same shape.
         const uint64_t x = make_smem_desc(smem_u32(sm + kStXt + b * 2 * kStPlane)) + 2 * k;
-        const uint32_t id = idesc | n_of(kStRows - 16 * k);
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const uint64_t hi = make_smem_desc(planes + hh * 2 * kStPlane + k * 2048) + 2 * k, lo = hi + kStPlane / 16;
-          const uint32_t d = tmem + (hh ? kStO2 : kStZ) + 16 * k;
-          tc_mma_bf16(d, x, lo, id, k > 0);
-          tc_mma_bf16(d, x, hi, id, 1u);
-        }
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+            for (int j = k / 2; j < 2; ++j)
+              tc_mma_bf16(tmem + (hh ? kStO2 : kStZ) + 32 * j, x,
+                          make_smem_desc(planes + (hh * 2 + 1 - e) * kStPlane + j * 4096) + 2 * k, idesc | n_of(32), k > 0 || e > 0);
       }
       tc_commit(&bars.o_done);
       tc_commit(&bars.free[b]);

@@ -323,10 +323,10 @@ def wkv_mix(rkvg, decay, spec, w, state, eps, step, out):
 
 
 def ssd_walks(step, heads: int) -> bool:
-    """Whether walking the chunks of every portion beats all chunks at once: 9 us + 4.5 per chunk of the longest portion against 24 us +
-    0.06 per chunk and head.  64 heads: portions of 2048, 1500, 1911 and 777 tokens 166 and 447 us, one of 1024 80 and 85, of 50 14 and
-    26; 32 heads: the four portions 156 and 232, one of 1024 80 and 52, one of 8192 567 and 316."""
-    return 75 * ((step.max_len + 63) // 64) < step.n_chunks * heads + 250
+    """Whether walking the chunks of every portion beats all chunks at once: 10 us + 4.7 per chunk of the longest portion against 24 us +
+    0.06 per chunk and head.  64 heads: portions of 2048, 1500, 1911 and 777 tokens 173 and 447 us, one of 1024 85 and 85, of 50 15 and
+    26; 32 heads: the four portions 163 and 232, one of 1024 84 and 54, one of 8192 599 and 316."""
+    return 78 * ((step.max_len + 63) // 64) < step.n_chunks * heads + 250
 
 
 def ssd_mix(proj, spec, w, conv_state, state, eps, step, out):

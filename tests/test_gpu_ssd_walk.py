@@ -77,6 +77,17 @@ def test_walk_is_the_recurrence(heads, groups, lens, n_decode, step):
     assert torch.equal(c["state"][other], untouched[other])
 
 
+def test_walk_repeats_itself():
+    """Many blocks and whole chunks, so that every role runs ahead of the others as far as it may: the same bits each time."""
+    first = None
+    for _ in range(5):
+        c = case(32, 4, 128, 64, [700, 512, 333, 640], 0, seed=2)
+        walk(c)
+        if first is None:
+            first = c["y"].clone(), c["state"].clone()
+        assert torch.equal(c["y"], first[0]) and torch.equal(c["state"], first[1])
+
+
 def test_walk_keeps_portions_apart():
     """What one portion holds, not-a-numbers too, stays out of the next one's rows and state."""
     c = case(4, 2, 128, 64, [40, 90], 0, seed=1)
