@@ -4,7 +4,8 @@
 //     q.k = qh.kh + (qh.km + qm.kh) + (qh.kl + qm.km + ql.kh)  + terms below 2^-25 of |q||k|,
 // six bf16 products with fp32 accumulation.  The tensor core cuts off what it aligns away while it accumulates; the leading
 // product is therefore summed over 64 channels at a time and the parts are added in registers, rounded to nearest; the five small
-// ones share an accumulator.  Against 64 bits (16,000 chunks x 64 rows x 1024) that is no further off than chains of fp32
+// ones go over all channels, two rows' planes side by side where the key's plane is the same (a product costs some 70 cycles,
+// whatever its columns: four per 16 channels, not six).  Against 64 bits (16,000 chunks x 64 rows x 1024) that is no further off than chains of fp32
 // multiply-adds.  Numbers for which the split is not exact or a part could overflow (not finite, 2^60 and more, below 2^-100 but
 // not zero) send the block's scores to such chains (slow; not met by keys and queries that stand for anything).
 //
@@ -13,7 +14,7 @@
 // memory (B); 11 fetches boxes and issues the products; 12-15 add up the parts and publish.
 //
 // Bound by the conversions (6.5 instructions per element of 128 x 1024 keys and 64 x 1024 rows per block) and the latency of the chain
-// box -> planes -> products, with one block per SM; the keys at HBM rate would take 10 us.  64 rows x 16,000 chunks x 1024: 33.6 us,
+// box -> planes -> products, with one block per SM; the keys at HBM rate would take 10 us.  64 rows x 16,000 chunks x 1024: 29.6 us,
 // 76.4 with fp32 multiply-adds on the CUDA cores (whose floor is 29); the error against 64 bits 1.0e-7 where that had 3.0e-7.
 #include <cuda.h>
 
@@ -25,7 +26,7 @@ namespace msa {
 
 constexpr int kRfChunks = 128, kRfRows = 64, kRfStages = 8, kRfBox = kRfChunks * 128;       // a box: 32 channels of 128 chunks
 constexpr int kRfThreads = 16 * 32, kRfQThreads = 3 * 32, kRfSmem = kRfStages * kRfBox + 2 * 3 * kRfRows * 128 + 1024;
-constexpr uint32_t kRfLead = 0, kRfSmall = 2 * kRfRows, kRfPlanes = 3 * kRfRows;              // TMEM columns
+constexpr uint32_t kRfLead = 0, kRfSmall = 2 * kRfRows, kRfLast = 4 * kRfRows, kRfPlanes = 5 * kRfRows;      // TMEM columns
 constexpr float kRfTop = 0x1p60f, kRfLow = 0x1p-100f;
 
 struct RouteFp32Params {
@@ -193,10 +194,11 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
       };
       for (int box = 0; box < min(n_box, kRfStages); ++box) fetch(box);
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(kRfChunks >> 4) << 24);
+      const uint32_t idesc2 = idesc + ((uint32_t)(p.bn >> 3) << 17);          // two planes of the rows at once
       bool ok = true;
       for (int kb = 0; kb < n_kb && ok; ++kb) {
         const int b = kb & 1;
-        const uint32_t ph = (kb >> 1) & 1u, lead = tmem + kRfLead + b * kRfRows, small = tmem + kRfSmall;
+        const uint32_t ph = (kb >> 1) & 1u, lead = tmem + kRfLead + b * kRfRows, small = tmem + kRfSmall, last = tmem + kRfLast;
         if (!(ok = mbar_wait(&s_b_full[b], ph, abort_flag, p.status, 26))) break;
         if (!(ok = mbar_wait(&s_d_empty[b], ph ^ 1u, abort_flag, p.status, 27))) break;
         const uint64_t q = make_smem_desc(smem_u32(planes) + b * b_bytes);
@@ -208,13 +210,11 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             const uint32_t a = tmem + kRfPlanes + half * 48 + k * 8;
-            const uint64_t qh = q + (uint64_t)(2 * (2 * half + k)), qm = qh + plane, ql = qm + plane;
+            const uint64_t qh = q + (uint64_t)(2 * (2 * half + k)), qm = qh + plane;
             tc_mma_bf16_ts(lead, a, qh, idesc, (half | k) ? 1u : 0u);
-            tc_mma_bf16_ts(small, a + 32, qh, idesc, (kb | half | k) ? 1u : 0u);
-            tc_mma_bf16_ts(small, a + 16, qm, idesc, 1u);
-            tc_mma_bf16_ts(small, a, ql, idesc, 1u);
-            tc_mma_bf16_ts(small, a + 16, qh, idesc, 1u);
-            tc_mma_bf16_ts(small, a, qm, idesc, 1u);
+            tc_mma_bf16_ts(small, a, qm, idesc2, (kb | half | k) ? 1u : 0u);          // kh qm | kh ql
+            tc_mma_bf16_ts(small, a + 16, qh, idesc2, 1u);                            // km qh | km qm
+            tc_mma_bf16_ts(last, a + 32, qh, idesc, (kb | half | k) ? 1u : 0u);       // kl qh
           }
           tc_commit(&s_t_empty[half]);
         }
@@ -254,7 +254,7 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
       if (!ok) break;
       tc_fence_after();
       add(kRfLead + (kb & 1) * kRfRows);
-      if (kb + 1 == n_kb) add(kRfSmall);
+      if (kb + 1 == n_kb) { add(kRfSmall); add(kRfSmall + p.bn); add(kRfLast); }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_d_empty[kb & 1]);
