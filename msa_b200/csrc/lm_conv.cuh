@@ -61,6 +61,12 @@ struct ConvWindow {
     }
     x[TAPS - 1] = *reinterpret_cast<const Raw*>(src.proj + n * src.proj_stride + c);
   }
+  // Moves on by one row whose input is in hand.
+  __device__ __forceinline__ void push(Raw next) {
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; ++j) x[j] = x[j + 1];
+    x[TAPS - 1] = next;
+  }
   __device__ __forceinline__ float4 value(const float4 (&w)[TAPS]) const {
     float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll

@@ -189,6 +189,24 @@ __global__ void __launch_bounds__(256) ssd_prep_vec_kernel(const msa_lm_ssd_args
 #pragma unroll
   for (int j = 0; j < TAPS; ++j) w[j] = load4(a.conv_w + (long long)j * L.chan + c);
   const float4 bias = load4(a.conv_b + c);
+  const long long first = (long long)a.n_decode + row0;
+  const int s0 = a.tok_seq[first];
+  if (n_here == kSpRows && a.tok_seq[first + kSpRows - 1] == s0) {
+    // rows of one sequence: every input in flight at once (row by row, each waits for the one before: 63 us for 6236 rows x 6144
+    // channels, 55 now; at HBM rate 24)
+    typename Raw4<T>::type x[kSpRows];
+#pragma unroll
+    for (int r = 0; r < kSpRows; ++r) x[r] = *reinterpret_cast<const typename Raw4<T>::type*>(src.proj + (first + r) * src.proj_stride + c);
+    win.move(src, first, (int)first - a.cu[s0], a.start[s0], a.slot[s0], c, true);
+#pragma unroll
+    for (int r = 0; r < kSpRows; ++r) {
+      if (r > 0) win.push(x[r]);
+      const float4 y = win.value(w);
+      store4(xbc + (long long)(row0 + r) * L.chan + c,
+             make_float4(silu_act<T>(y.x + bias.x), silu_act<T>(y.y + bias.y), silu_act<T>(y.z + bias.z), silu_act<T>(y.w + bias.w)));
+    }
+    return;
+  }
 #pragma unroll
   for (int r = 0; r < kSpRows; ++r) {
     if (r >= n_here) break;
@@ -388,6 +406,39 @@ __global__ void __launch_bounds__(256) wkv_out_kernel(const msa_lm_wkv_args a, c
     out[row * out_stride + h * a.dim + i] = from_f<T>(src[i] * inv * a.norm[h * a.dim + i] * silu_act<T>(to_f(g[i])));
 }
 
+// Parts of up to 1024 elements in fours: a warp per part, read once, no barrier (a block per part reads twice around two barriers:
+// 6236 rows x 8 parts of 512 elements took 39 us, 30 now; at HBM rate 24).  Below two blocks per SM the launch is nothing but latency, and a block
+// per part is the shorter one (64 parts: 2.0 and 3.8 us).
+template <typename T, int N>
+__global__ void __launch_bounds__(256) part_norm_warp_kernel(const float* __restrict__ x, long long x_stride, const float* __restrict__ w, int size,
+                                                             int parts, long long n_items, int n_rows, float eps, T* __restrict__ out,
+                                                             long long out_stride) {
+  let_product_start(n_rows);
+  const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (item >= n_items) return;
+  const long long row = item / parts;
+  const int c0 = (int)(item - row * parts) * size, lane = threadIdx.x & 31;
+  const float* src = x + row * x_stride + c0;
+  T* dst = out + row * out_stride + c0;
+  float4 v[N], g[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int i = (k * 32 + lane) * 4;
+    const bool on = i < size;
+    v[k] = on ? load4(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    g[k] = on ? load4(w + c0 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < N; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+  const float inv = 1.f / sqrtf(warp_sum_f(ss) / (float)size + eps);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int i = (k * 32 + lane) * 4;
+    if (i < size) store4(dst + i, make_float4(v[k].x * inv * g[k].x, v[k].y * inv * g[k].y, v[k].z * inv * g[k].z, v[k].w * inv * g[k].w));
+  }
+}
+
 // One block per (row, part).
 template <typename T, int V>
 __global__ void __launch_bounds__(256) part_norm_kernel(const float* __restrict__ x, long long x_stride, const float* __restrict__ w,
@@ -530,6 +581,19 @@ extern "C" int msa_lm_part_norm(const float* x, int64_t x_stride, const float* w
                   reinterpret_cast<uintptr_t>(out) % (4 * dtype_size(dtype)) == 0;
   const int per = v4 ? size / 4 : size, threads = per >= 256 ? 256 : (per + 31) / 32 * 32;
   const dim3 grid((unsigned)n_rows, (unsigned)parts);
+  int n_sm = 0;
+  MSA_OK_OR_RETURN(device_sm_count(&n_sm));
+  if (v4 && size <= 1024 && (long long)n_rows * parts >= 16 * n_sm) {
+    const long long items = (long long)n_rows * parts, blocks = (items + 7) / 8;
+    MSA_REQUIRE(blocks < (1ll << 31), "part_norm: too many rows");
+    const int n = (size + 127) / 128;
+    MSA_LM_DISPATCH(dtype, {
+      auto kernel = n <= 1 ? part_norm_warp_kernel<T, 1> : n <= 2 ? part_norm_warp_kernel<T, 2> : n <= 4 ? part_norm_warp_kernel<T, 4> : part_norm_warp_kernel<T, 8>;
+      kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(x, x_stride, w, size, parts, items, n_rows, eps, (T*)out, out_stride);
+    });
+    MSA_LAUNCH_OK("part_norm_warp_kernel");
+    return MSA_OK;
+  }
   MSA_LM_DISPATCH(dtype, {
     if (v4) part_norm_kernel<T, 4><<<grid, threads, 0, (cudaStream_t)stream>>>(x, x_stride, w, size, eps, (T*)out, out_stride);
     else part_norm_kernel<T, 1><<<grid, threads, 0, (cudaStream_t)stream>>>(x, x_stride, w, size, eps, (T*)out, out_stride);

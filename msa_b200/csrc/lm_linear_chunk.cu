@@ -572,8 +572,9 @@ __global__ void __launch_bounds__(256, 2) ssd_read_kernel(const SsdChunkParams p
       for (int e = 0; e < 2; ++e) {
         const int t = r0 + 8 * e;
         const double gt = e ? g1 : g0;
-        const float p0 = i <= t ? s[2 * m + x][2 * e] * exp2f((float)(gt - gx)) * di.x : 0.f;
-        const float p1 = i + 1 <= t ? s[2 * m + x][2 * e + 1] * exp2f((float)(gt - gy)) * di.y : 0.f;
+        // masked as bits: a branch around every element would expose its whole latency
+        const float p0 = __uint_as_float(__float_as_uint(s[2 * m + x][2 * e] * exp2f((float)(gt - gx)) * di.x) & (i <= t ? 0xffffffffu : 0u));
+        const float p1 = __uint_as_float(__float_as_uint(s[2 * m + x][2 * e + 1] * exp2f((float)(gt - gy)) * di.y) & (i + 1 <= t ? 0xffffffffu : 0u));
         lc_split2(p0, p1, ah[2 * x + e], al[2 * x + e]);
       }
     }
