@@ -366,6 +366,10 @@ int msa_gather_plan_resident(const int64_t* sel_local, const int32_t* sel_rank, 
 int msa_gather_run(const int64_t* plan, int32_t n_items, int32_t dtype, int32_t n_kv_heads,
                    int32_t head_dim, void* out_k, void* out_v, int64_t out_head_stride,
                    int64_t out_entries, int64_t out_sample_stride, int32_t max_ctas, void* stream);
+/* The same packed result [n_kv_heads, *total, head_dim] with the plan's own total, read on the device: it may be launched before the host
+ * knows it.  out_k and out_v have room for `capacity` entries, at least as many as the plan can list. */
+int msa_gather_run_total(const int64_t* plan, int32_t n_items, int32_t dtype, int32_t n_kv_heads, int32_t head_dim, void* out_k,
+                         void* out_v, int64_t capacity, const int64_t* total, int32_t max_ctas, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * Decode attention over the sparse context (split-KV flash-decode, GQA).

@@ -191,7 +191,12 @@ constexpr int kGatherThreads = 256;
 template <typename T>
 __global__ void __launch_bounds__(kGatherThreads)
 gather_kernel(const int64_t* __restrict__ plan, int n_items, int n_kv_heads, int head_dim, T* __restrict__ out_k,
-              T* __restrict__ out_v, long long out_head_stride, long long out_entries, long long out_sample_stride) {
+              T* __restrict__ out_v, long long out_head_stride, long long out_entries, long long out_sample_stride,
+              const int64_t* __restrict__ total) {
+  if (total) {                                     // packed by what the plan found: [heads, total, head_dim], in room for out_entries
+    out_entries = min(out_entries, (long long)*total);
+    out_head_stride = out_entries * head_dim;
+  }
   constexpr int V = Elem<T>::kVec;
   const int vec_half = n_kv_heads * head_dim / V;  // 16-byte vectors in one chunk's K (or V)
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -313,9 +318,9 @@ extern "C" int msa_gather_plan_resident(const int64_t* sel_local, const int32_t*
                             resident, slot_len, stream);
 }
 
-extern "C" int msa_gather_run(const int64_t* plan, int32_t n_items, int32_t dtype, int32_t n_kv_heads,
-                              int32_t head_dim, void* out_k, void* out_v, int64_t out_head_stride,
-                              int64_t out_entries, int64_t out_sample_stride, int32_t max_ctas, void* stream) {
+static int gather_launch(const int64_t* plan, int32_t n_items, int32_t dtype, int32_t n_kv_heads,
+                         int32_t head_dim, void* out_k, void* out_v, int64_t out_head_stride,
+                         int64_t out_entries, int64_t out_sample_stride, const int64_t* total, int32_t max_ctas, void* stream) {
   MSA_REQUIRE(dtype_ok(dtype), "gather_run: unknown dtype %d", dtype);
   MSA_REQUIRE(plan && n_items >= 0 && n_kv_heads > 0 && head_dim > 0 && max_ctas >= 0 && out_sample_stride >= 0,
               "gather_run: bad arguments");
@@ -333,11 +338,24 @@ extern "C" int msa_gather_run(const int64_t* plan, int32_t n_items, int32_t dtyp
   if (dtype == MSA_BF16)
     gather_kernel<__nv_bfloat16><<<grid, kGatherThreads, 0, (cudaStream_t)stream>>>(
         plan, n_items, n_kv_heads, head_dim, (__nv_bfloat16*)out_k, (__nv_bfloat16*)out_v, out_head_stride, out_entries,
-        out_sample_stride);
+        out_sample_stride, total);
   else
     gather_kernel<float><<<grid, kGatherThreads, 0, (cudaStream_t)stream>>>(
         plan, n_items, n_kv_heads, head_dim, (float*)out_k, (float*)out_v, out_head_stride, out_entries,
-        out_sample_stride);
+        out_sample_stride, total);
   MSA_LAUNCH_OK("gather_kernel");
   return MSA_OK;
+}
+
+extern "C" int msa_gather_run(const int64_t* plan, int32_t n_items, int32_t dtype, int32_t n_kv_heads,
+                              int32_t head_dim, void* out_k, void* out_v, int64_t out_head_stride,
+                              int64_t out_entries, int64_t out_sample_stride, int32_t max_ctas, void* stream) {
+  return gather_launch(plan, n_items, dtype, n_kv_heads, head_dim, out_k, out_v, out_head_stride, out_entries, out_sample_stride, nullptr, max_ctas,
+                       stream);
+}
+
+extern "C" int msa_gather_run_total(const int64_t* plan, int32_t n_items, int32_t dtype, int32_t n_kv_heads, int32_t head_dim, void* out_k,
+                                    void* out_v, int64_t capacity, const int64_t* total, int32_t max_ctas, void* stream) {
+  MSA_REQUIRE(total && capacity >= 0, "gather_run_total: null total or negative capacity");
+  return gather_launch(plan, n_items, dtype, n_kv_heads, head_dim, out_k, out_v, 0, capacity, 0, total, max_ctas, stream);
 }

@@ -469,6 +469,21 @@ def gather_run(plan: torch.Tensor, dtype: torch.dtype, n_kv_heads: int, head_dim
     return out_k, out_v
 
 
+def gather_run_total(plan: torch.Tensor, dtype: torch.dtype, n_kv_heads: int, head_dim: int, capacity: int, total: torch.Tensor,
+                     max_ctas: int = 0):
+    """Run a packed plan before the host knows its ``total``: flat storage for ``capacity`` entries each of K and V, of which the first
+    ``total`` make ``[Hkv, total, D]`` (see ``packed_entries``)."""
+    A.need_cuda(plan, total)
+    out = [torch.empty(n_kv_heads * capacity * head_dim, dtype=dtype, device=plan.device) for _ in range(2)]
+    A.check(A.lib().msa_gather_run_total(A.ptr(plan), plan.shape[0], A.dtype_code(dtype), n_kv_heads, head_dim, A.ptr(out[0]), A.ptr(out[1]),
+                                         capacity, A.ptr(total), int(max_ctas), A.stream_ptr(plan.device)), "msa_gather_run_total")
+    return out
+
+
+def packed_entries(store: torch.Tensor, n_kv_heads: int, head_dim: int, total: int) -> torch.Tensor:
+    return store[:n_kv_heads * total * head_dim].view(n_kv_heads, total, head_dim)
+
+
 # ---------------------------------------------------------------------------------------
 # Decode attention
 # ---------------------------------------------------------------------------------------
