@@ -175,7 +175,6 @@ __device__ __forceinline__ void group_mma(float (&c)[4], const uint32_t (&a)[4],
 
 template <int D, int DV, bool FULL>
 __global__ void __launch_bounds__(kMmaWarps * 32, 2) group_decode_kernel(const GroupDecodeParams p) {
-  grid_launch_dependents();
   constexpr int kRows = FULL ? 16 : 8, NE = FULL ? 2 : 1;
   constexpr int kPk = D * 2 + 16, kPv = DV * 2 + 16, kStage = kMmaKeys * (kPk + kPv);
   constexpr int kVk = D / 8, kVv = DV / 8;               // 16-byte pieces of a key, of a value

@@ -41,7 +41,6 @@ __device__ __forceinline__ void bulk_row(uint32_t dst, const void* src, uint32_t
 
 template <int MT, int NT, int KS>
 __global__ void __launch_bounds__(kLdThreads, 1) latent_decode_kernel(const LatentDecodeParams p) {
-  grid_launch_dependents();
   constexpr int KQ = 8 / MT, kRows = MT * 16, kPart = 72;            // slices of the reduction; floats per partial row
   constexpr int TPR = kLdThreads / kRows, KPT = kLdKeys / TPR;       // softmax: threads per row, keys per thread
   extern __shared__ __align__(16) unsigned char sm[];
