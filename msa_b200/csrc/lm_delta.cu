@@ -316,9 +316,12 @@ delta_out_kernel(const msa_lm_delta_args a, const float* __restrict__ o, T* __re
 // (twice, the second time from L1 / L2) and written once.
 constexpr int kDdThreads = 256;
 
-// STAGE: the state is copied to shared memory before anything else (cp.async) and read from there both times.
+// STAGE: the state is fetched before anything else, each thread's first kDdRegRows rows into registers and the others to shared memory
+// (cp.async), and read from there both times; a thread's elements are its own.  A 128 x 128 state in shared memory alone lets three
+// blocks share an SM, and the 512 blocks of 32 sequences x 16 heads then come in a wave and a sixth: 22.5 us, 19.5 with four blocks.
+constexpr int kDdRegRows = 5;
 template <typename T, int V, bool STAGE>
-__global__ void __launch_bounds__(kDdThreads)
+__global__ void __launch_bounds__(kDdThreads, STAGE ? 4 : 1)
 delta_decode_kernel(const msa_lm_delta_args a, T* __restrict__ out, long long out_stride, int groups) {
   let_product_start(gridDim.y);
   extern __shared__ float sm[];
@@ -333,14 +336,25 @@ delta_decode_kernel(const msa_lm_delta_args a, T* __restrict__ out, long long ou
   float* s_r = s_c + groups * dv;         // [groups][dv]
   const int slot = a.slot[b], p = a.pos[b];
   float* S = a.state + (((long long)slot * a.heads + h) * dk) * dv;
-  float* s_state = sm + (2 * dk + dv + 3) / 4 * 4 + 2 * groups * dv;   // [dk][dv]
+  const bool zero = p == 0;
+  const int cols = dv / V, rg = threadIdx.x / cols, cv = (threadIdx.x % cols) * V;   // groups * cols <= blockDim
+  const bool active = rg < groups;
+  float* s_state = sm + (2 * dk + dv + 3) / 4 * 4 + 2 * groups * dv;   // [dk - d_smem][dv]
+  const int d_smem = kDdRegRows * groups;                              // rows from here on are in shared memory
+  float4 held[STAGE ? kDdRegRows : 1];
   if constexpr (STAGE) {
-    if (p != 0) {
+#pragma unroll
+    for (int k = 0; k < kDdRegRows; ++k) {
+      const int d = rg + k * groups;
+      held[k] = !zero && active && d < dk ? load4(S + (long long)d * dv + cv) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const int rest = (dk - d_smem) * dv / 4;
+    if (!zero) {
       const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_state);
-      for (int i = threadIdx.x; i < dk * dv / 4; i += kDdThreads)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 16), "l"(S + (long long)i * 4) : "memory");
+      for (int i = threadIdx.x; i < rest; i += kDdThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 16), "l"(S + (long long)d_smem * dv + (long long)i * 4) : "memory");
     } else {
-      for (int i = threadIdx.x; i < dk * dv / 4; i += kDdThreads) store4(s_state + i * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+      for (int i = threadIdx.x; i < rest; i += kDdThreads) store4(s_state + i * 4, make_float4(0.f, 0.f, 0.f, 0.f));
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -351,8 +365,25 @@ delta_decode_kernel(const msa_lm_delta_args a, T* __restrict__ out, long long ou
   const float gate0 = threadIdx.x < dv ? to_f(gate[threadIdx.x]) : 0.f, norm0 = threadIdx.x < dv ? a.w_norm[threadIdx.x] : 0.f;
   const T* old = conv_half<T>(a, L.chan, slot, p);
   T* fresh = reinterpret_cast<T*>(a.conv_state) + ((long long)slot * 2 + ((p + 1) & 1)) * keep * L.chan;
-  for (int i = threadIdx.x; i < 2 * dk + dv; i += kDdThreads) {
-    const int c = i < dk ? hk * dk + i : (i < 2 * dk ? L.nqk + hk * dk + (i - dk) : 2 * L.nqk + h * dv + (i - 2 * dk));
+  const int n_conv = 2 * dk + dv;
+  auto channel = [&](int i) { return i < dk ? hk * dk + i : (i < 2 * dk ? L.nqk + hk * dk + (i - dk) : 2 * L.nqk + h * dv + (i - 2 * dk)); };
+  if (a.taps <= kConvHeld) {
+    for (int i0 = threadIdx.x; i0 < n_conv; i0 += 2 * kDdThreads) {
+      ConvToken<T> in[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (i0 + u * kDdThreads < n_conv) in[u].fetch(proj, old, a.conv_w, p, a.taps, L.chan, channel(i0 + u * kDdThreads));
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = i0 + u * kDdThreads;
+        if (i >= n_conv) break;
+        sm[i] = silu_f(in[u].template value<false>(p, a.taps));
+        if (i >= 2 * dk || h % group == 0) in[u].leave(fresh, a.taps, L.chan, channel(i));
+      }
+    }
+  } else
+  for (int i = threadIdx.x; i < n_conv; i += kDdThreads) {
+    const int c = channel(i);
     const bool writer = i >= 2 * dk || h % group == 0;
     const float* w = a.conv_w + c;
     float acc = 0.f;
@@ -389,19 +420,19 @@ delta_decode_kernel(const msa_lm_delta_args a, T* __restrict__ out, long long ou
   qk *= sq * sk;
   const float beta = sigmoid_f(raw_beta);
   const float g = expf(-expf(a_log) * softplus_f(raw_decay + dt_bias));
-  const bool zero = p == 0;
-  const int cols = dv / V, rg = threadIdx.x / cols, cv = (threadIdx.x % cols) * V;   // groups * cols <= blockDim
-  const bool active = rg < groups;
   if constexpr (STAGE) {
     if (active) {
       float4 ac = make_float4(0.f, 0.f, 0.f, 0.f), ar = ac;
-#pragma unroll 4
-      for (int d = rg; d < dk; d += groups) {
-        const float4 x = load4(s_state + d * dv + cv);
+      auto add = [&](int d, const float4& x) {
         const float kd = s_k[d], qd = s_q[d];
         ac.x = fmaf(x.x, kd, ac.x); ac.y = fmaf(x.y, kd, ac.y); ac.z = fmaf(x.z, kd, ac.z); ac.w = fmaf(x.w, kd, ac.w);
         ar.x = fmaf(x.x, qd, ar.x); ar.y = fmaf(x.y, qd, ar.y); ar.z = fmaf(x.z, qd, ar.z); ar.w = fmaf(x.w, qd, ar.w);
-      }
+      };
+#pragma unroll
+      for (int k = 0; k < kDdRegRows; ++k)
+        if (rg + k * groups < dk) add(rg + k * groups, held[k]);
+#pragma unroll 2
+      for (int d = rg + d_smem; d < dk; d += groups) add(d, load4(s_state + (d - d_smem) * dv + cv));
       store4(s_c + rg * dv + cv, ac);
       store4(s_r + rg * dv + cv, ar);
     }
@@ -444,12 +475,15 @@ delta_decode_kernel(const msa_lm_delta_args a, T* __restrict__ out, long long ou
   if constexpr (STAGE) {
     if (active) {
       const float4 u = load4(s_c + cv);
-#pragma unroll 4
-      for (int d = rg; d < dk; d += groups) {
-        const float4 x = load4(s_state + d * dv + cv);
+      auto put = [&](int d, const float4& x) {
         const float kd = s_k[d];
         store4(S + (long long)d * dv + cv, make_float4(fmaf(kd, u.x, g * x.x), fmaf(kd, u.y, g * x.y), fmaf(kd, u.z, g * x.z), fmaf(kd, u.w, g * x.w)));
-      }
+      };
+#pragma unroll
+      for (int k = 0; k < kDdRegRows; ++k)
+        if (rg + k * groups < dk) put(rg + k * groups, held[k]);
+#pragma unroll 4
+      for (int d = rg + d_smem; d < dk; d += groups) put(d, load4(s_state + (d - d_smem) * dv + cv));
     }
   } else
   for (int cs = 0; cs < cols; cs += kDdThreads) {
@@ -503,6 +537,7 @@ extern "C" int msa_lm_delta_decode(const msa_lm_delta_args* a, void* out, int64_
   const int cols = a->vdim / v;
   const int groups = cols >= kDdThreads ? 1 : kDdThreads / cols;
   const size_t smem = (size_t)4 * ((2 * a->dim + a->vdim + 3) / 4 * 4 + 2 * groups * a->vdim);
+  const size_t rest = (size_t)(a->dim > kDdRegRows * groups ? a->dim - kDdRegRows * groups : 0) * a->vdim * 4;
   const bool stage = v == 4 && cols <= kDdThreads && (size_t)a->dim * a->vdim * 4 + smem <= 110 * 1024;
   const dim3 grid((unsigned)a->heads, (unsigned)a->n_decode);
   MSA_LM_DISPATCH(a->dtype, {
@@ -512,7 +547,7 @@ extern "C" int msa_lm_delta_decode(const msa_lm_delta_args* a, void* out, int64_
       return MSA_OK;
     };
     static DeviceSmem staged, st4, st1;
-    if (stage) MSA_OK_OR_RETURN(launch(delta_decode_kernel<T, 4, true>, staged, smem + (size_t)a->dim * a->vdim * 4));
+    if (stage) MSA_OK_OR_RETURN(launch(delta_decode_kernel<T, 4, true>, staged, smem + rest));
     else if (v == 4) MSA_OK_OR_RETURN(launch(delta_decode_kernel<T, 4, false>, st4, smem));
     else MSA_OK_OR_RETURN(launch(delta_decode_kernel<T, 1, false>, st1, smem));
   });

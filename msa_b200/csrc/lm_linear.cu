@@ -133,17 +133,50 @@ __global__ void __launch_bounds__(kLinThreads, 4) ssd_decode_kernel(const msa_lm
   StatePass<V> pass(a.state + ((long long)slot * a.heads + h) * ns * vd, ns, vd, pos == 0);
   pass.fetch();
   const T* proj = reinterpret_cast<const T*>(a.proj) + (long long)b * a.proj_stride;
-  const float dt = softplus_f(to_f(proj[L.inner + L.chan + h]) + a.dt_bias[h]);
-  const float decay = expf(-expf(a.a_log[h]) * dt);
+  const float raw_dt = to_f(proj[L.inner + L.chan + h]), dt_bias = a.dt_bias[h], a_log = a.a_log[h], d_skip = a.d_skip[h];
+  const T gate0 = (int)threadIdx.x < vd ? proj[h * vd + threadIdx.x] : from_f<T>(0.f);
   const ConvSource<T> src{reinterpret_cast<const T*>(a.proj) + L.inner, a.proj_stride, reinterpret_cast<T*>(a.conv_state), L.chan, a.taps};
   const bool lead = h % per == 0;                          // the group's first head hands B and C on
-  for (int i = threadIdx.x; i < vd + 2 * ns; i += kLinThreads) {
-    const int c = i < vd ? h * vd + i : (i < vd + ns ? L.inner + gr * ns + (i - vd) : L.inner + L.bc + gr * ns + (i - vd - ns));
-    const float y = silu_act<T>(src.value(a.conv_w, b, 0, pos, slot, c) + a.conv_b[c]);
-    const float z = to_f(from_f<T>(y));                    // as the portions see it
+  const int n_conv = vd + 2 * ns;
+  auto channel = [&](int i) { return i < vd ? h * vd + i : (i < vd + ns ? L.inner + gr * ns + (i - vd) : L.inner + L.bc + gr * ns + (i - vd - ns)); };
+  float dt = 0.f, decay = 0.f;
+  auto gates = [&] {
+    dt = softplus_f(raw_dt + dt_bias);
+    decay = expf(-expf(a_log) * dt);
+  };
+  auto keep = [&](int i, float conv) {
+    const float z = to_f(from_f<T>(silu_act<T>(conv)));    // as the portions see it
     if (i < vd) { s_x[i] = z; s_v[i] = dt * z; }
     else if (i < vd + ns) s_b[i - vd] = z;
     else s_c[i - vd - ns] = z;
+  };
+  if (a.taps <= kConvHeld) {
+    for (int i0 = threadIdx.x; i0 < n_conv; i0 += 2 * kLinThreads) {
+      ConvToken<T> in[2];
+      float bias[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (i0 + u * kLinThreads < n_conv) {
+          const int c = channel(i0 + u * kLinThreads);
+          in[u].fetch(proj + L.inner, src.half(slot, pos), a.conv_w, pos, a.taps, L.chan, c);
+          bias[u] = a.conv_b[c];
+        }
+      if (i0 == (int)threadIdx.x) gates();
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = i0 + u * kLinThreads;
+        if (i >= n_conv) break;
+        keep(i, in[u].template value<true>(pos, a.taps) + bias[u]);
+        if (i < vd || lead) in[u].leave(src.half(slot, pos + 1), a.taps, L.chan, channel(i));
+      }
+    }
+    if ((int)threadIdx.x >= n_conv) gates();
+  } else
+  for (int i = threadIdx.x; i < n_conv || i == (int)threadIdx.x; i += kLinThreads) {
+    if (i == (int)threadIdx.x) gates();
+    if (i >= n_conv) break;
+    const int c = channel(i);
+    keep(i, src.value(a.conv_w, b, 0, pos, slot, c) + a.conv_b[c]);
     if ((i < vd || lead) && a.taps > 1) {
       T* dst = src.half(slot, pos + 1) + c;
       for (int j = 0; j < a.taps - 1; ++j) {
@@ -159,8 +192,8 @@ __global__ void __launch_bounds__(kLinThreads, 4) ssd_decode_kernel(const msa_lm
   pass.template run<true>(s_c, s_b, nullptr, decay, s_v, part);
   __syncthreads();
   for (int i = threadIdx.x; i < vd; i += kLinThreads) {
-    const float y = fmaf(decay, pass.total(part, i), fmaf(cb, s_v[i], a.d_skip[h] * s_x[i]));
-    a.y[(long long)b * L.inner + h * vd + i] = y * silu_act<T>(to_f(proj[h * vd + i]));
+    const float y = fmaf(decay, pass.total(part, i), fmaf(cb, s_v[i], d_skip * s_x[i]));
+    a.y[(long long)b * L.inner + h * vd + i] = y * silu_act<T>(to_f(i == (int)threadIdx.x ? gate0 : proj[h * vd + i]));
   }
 }
 
