@@ -313,7 +313,8 @@ delta_out_kernel(const msa_lm_delta_args a, const float* __restrict__ o, T* __re
 
 // ---- decode: everything between the projections and the output product -----------------------------------------------
 // One block per (sequence, head).  Threads form a grid of row groups x column vectors over the state; the state is read
-// (twice, the second time from L1 / L2) and written once.
+// (twice, the second time from L1 / L2) and written once.  Neither launched early nor letting the product behind it start early: see
+// kEarlyRows.
 constexpr int kDdThreads = 256;
 
 // STAGE: the state is fetched before anything else, each thread's first kDdRegRows rows into registers and the others to shared memory
@@ -323,7 +324,6 @@ constexpr int kDdRegRows = 5;
 template <typename T, int V, bool STAGE>
 __global__ void __launch_bounds__(kDdThreads, STAGE ? 4 : 1)
 delta_decode_kernel(const msa_lm_delta_args a, T* __restrict__ out, long long out_stride, int groups) {
-  let_product_start(gridDim.y);
   extern __shared__ float sm[];
   __shared__ float s_part[32];
   const DeltaLayout L(a);

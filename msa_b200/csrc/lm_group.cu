@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(256) group_prep_kernel(const msa_lm_group_args
 // Four channels per thread, up to eight packed rows per block: every input is loaded once.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(256) group_prep_vec_kernel(const msa_lm_group_args a, int row_blocks, int rows) {
+  grid_dependency_wait();
   extern __shared__ float2 s_turn[];            // [rows][rot / 2]
   const GroupLayout L(a);
   if ((int)blockIdx.x >= row_blocks) {
@@ -383,12 +384,14 @@ extern "C" int msa_lm_group_prep(const msa_lm_group_args* args, void* stream) {
     const int rows = a.n_tok <= 256 ? 1 : kGpRows, row_blocks = (a.n_tok + rows - 1) / rows;
     const dim3 grid((unsigned)(row_blocks + a.n_old), (unsigned)((L.chan + 1023) / 1024));
     MSA_LM_DISPATCH(a.dtype, {
+      void (*kernel)(msa_lm_group_args, int, int);
       switch (a.taps) {
-        case 1: group_prep_vec_kernel<T, 1><<<grid, 256, rows * turn, st>>>(a, row_blocks, rows); break;
-        case 2: group_prep_vec_kernel<T, 2><<<grid, 256, rows * turn, st>>>(a, row_blocks, rows); break;
-        case 3: group_prep_vec_kernel<T, 3><<<grid, 256, rows * turn, st>>>(a, row_blocks, rows); break;
-        default: group_prep_vec_kernel<T, 4><<<grid, 256, rows * turn, st>>>(a, row_blocks, rows);
+        case 1: kernel = group_prep_vec_kernel<T, 1>; break;
+        case 2: kernel = group_prep_vec_kernel<T, 2>; break;
+        case 3: kernel = group_prep_vec_kernel<T, 3>; break;
+        default: kernel = group_prep_vec_kernel<T, 4>;
       }
+      MSA_CUDA_OK(launch_kernel_pdl(kernel, grid, dim3(256), rows * turn, st, a.n_tok <= kEarlyRows, a, row_blocks, rows));
     });
     MSA_LAUNCH_OK("group_prep_vec_kernel");
     return MSA_OK;

@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(128) latent_prep_kernel(const LatentPrepParams
 // registers before the token's angles are computed, and the heads' rotated parts are turned two pairs at a time.
 template <typename T>
 __global__ void __launch_bounds__(128) latent_prep_vec_kernel(const LatentPrepParams p) {
+  grid_dependency_wait();
   __shared__ float s_part[32];
   extern __shared__ float2 s_turn[];
   const int width = p.rank + p.rot, tid = threadIdx.x;
@@ -264,7 +265,9 @@ extern "C" int msa_lm_latent_prep(void* proj, int64_t proj_stride, const float* 
   auto ok4 = [&](const void* q) { return q == nullptr || reinterpret_cast<uintptr_t>(q) % e4 == 0; };
   if (dim % 4 == 0 && rot % 4 == 0 && rank % 4 == 0 && rank <= 512 && proj_stride % 4 == 0 && ok4(proj) && ok4(ring) && ok4(ctx) &&
       aligned16(w_norm) && ring_rows < (1ll << 31)) {
-    MSA_LM_DISPATCH(dtype, { latent_prep_vec_kernel<T><<<n_tok + n_old, 128, (size_t)rot * 4, (cudaStream_t)stream>>>(p); });
+    MSA_LM_DISPATCH(dtype, {
+      MSA_CUDA_OK(launch_kernel_pdl(latent_prep_vec_kernel<T>, dim3(n_tok + n_old), dim3(128), (size_t)rot * 4, (cudaStream_t)stream, n_tok <= kEarlyRows, p));
+    });
     MSA_LAUNCH_OK("latent_prep_vec_kernel");
     return MSA_OK;
   }

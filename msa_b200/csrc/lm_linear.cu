@@ -83,6 +83,7 @@ inline int pass_groups(int dv, int v) { return dv / v >= kLinThreads ? 1 : kLinT
 template <typename T, int V>
 __global__ void __launch_bounds__(kLinThreads, 4) wkv_decode_kernel(const msa_lm_wkv_args a, T* __restrict__ out, long long out_stride) {
   let_product_start(gridDim.y);
+  grid_dependency_wait();
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_part[32];
   const int h = blockIdx.x, b = blockIdx.y, dim = a.dim, pad = (dim + 3) / 4 * 4;
@@ -123,6 +124,7 @@ struct SsdLayout {
 template <typename T, int V>
 __global__ void __launch_bounds__(kLinThreads, 4) ssd_decode_kernel(const msa_lm_ssd_args a) {
   let_product_start(gridDim.y);
+  grid_dependency_wait();
   extern __shared__ __align__(16) float sm[];
   __shared__ float s_part[32];
   const SsdLayout L(a);
@@ -529,8 +531,8 @@ extern "C" int msa_lm_wkv_decode(const msa_lm_wkv_args* a, void* out, int64_t ou
   MSA_REQUIRE(smem <= 48 * 1024, "wkv_decode: head size %d is too large", a->dim);
   const dim3 grid((unsigned)a->heads, (unsigned)a->n_decode);
   MSA_LM_DISPATCH(a->dtype, {
-    if (v == 4) wkv_decode_kernel<T, 4><<<grid, kLinThreads, smem, (cudaStream_t)stream>>>(*a, (T*)out, out_stride);
-    else wkv_decode_kernel<T, 1><<<grid, kLinThreads, smem, (cudaStream_t)stream>>>(*a, (T*)out, out_stride);
+    auto kernel = v == 4 ? wkv_decode_kernel<T, 4> : wkv_decode_kernel<T, 1>;
+    MSA_CUDA_OK(launch_kernel_pdl(kernel, grid, dim3(kLinThreads), smem, (cudaStream_t)stream, a->n_decode <= kEarlyRows, *a, (T*)out, (long long)out_stride));
   });
   MSA_LAUNCH_OK("wkv_decode_kernel");
   return MSA_OK;
@@ -559,8 +561,8 @@ extern "C" int msa_lm_ssd_decode(const msa_lm_ssd_args* a, void* stream) {
   MSA_REQUIRE(smem <= 48 * 1024, "ssd_decode: sizes (%d, %d) are too large", a->n_state, a->vdim);
   const dim3 grid((unsigned)a->heads, (unsigned)a->n_decode);
   MSA_LM_DISPATCH(a->dtype, {
-    if (v == 4) ssd_decode_kernel<T, 4><<<grid, kLinThreads, smem, (cudaStream_t)stream>>>(*a);
-    else ssd_decode_kernel<T, 1><<<grid, kLinThreads, smem, (cudaStream_t)stream>>>(*a);
+    auto kernel = v == 4 ? ssd_decode_kernel<T, 4> : ssd_decode_kernel<T, 1>;
+    MSA_CUDA_OK(launch_kernel_pdl(kernel, grid, dim3(kLinThreads), smem, (cudaStream_t)stream, a->n_decode <= kEarlyRows, *a));
   });
   MSA_LAUNCH_OK("ssd_decode_kernel");
   return MSA_OK;

@@ -21,7 +21,6 @@ static __global__ void __launch_bounds__(128) merge_partials_kernel(const MergeP
   const long long row = blockIdx.x;
   const int b = (int)(row / p.heads), h = (int)(row % p.heads);
   const int c = threadIdx.x * 4, splits = p.splits, cols = p.cols;
-  grid_dependency_wait();
   const float g = p.gate ? sigmoid_f(__bfloat162float(p.gate[b * p.gate_row + h])) : 1.f;
   float m = p.sink ? 0.f : -INFINITY, l = p.sink ? 1.f : 0.f;
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);

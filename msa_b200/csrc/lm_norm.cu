@@ -120,6 +120,7 @@ __global__ void residual_norm_kernel(const ResNormParams p) {
 template <typename T, typename TY>
 __global__ void __launch_bounds__(1024) residual_norm_once_kernel(const ResNormParams p) {
   let_product_start(gridDim.x);
+  grid_dependency_wait();
   __shared__ float s_part[32];
   const long long r = blockIdx.x;
   const long long rb = p.rows ? p.rows[r] : r;
@@ -313,6 +314,7 @@ __global__ void embed_kernel(const msa_lm_embed_args a) {
 
 // x = cap * tanh(x / cap), in place.
 __global__ void __launch_bounds__(256) softcap_kernel(float* x, long long n, float cap) {
+  grid_dependency_wait();
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) x[i] = cap * tanhf(x[i] / cap);
 }
 
@@ -373,8 +375,9 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ 
 // out[r, part * cols + c] = part-th share of tanh(x[r, c]): with two parts the bf16 rounding and what it leaves behind,
 // so that a product over both keeps 16 significant bits.
 template <typename T>
-__global__ void __launch_bounds__(256) tanh_split_kernel(const float* __restrict__ x, int cols, int parts, long long n, T* __restrict__ out) {
+__global__ void __launch_bounds__(256) tanh_split_kernel(const float* x, int cols, int parts, long long n, T* __restrict__ out) {
   if (n <= (long long)kEarlyRows * cols) grid_launch_dependents();
+  grid_dependency_wait();
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
     const long long r = i / cols;
     const int c = (int)(i - r * cols);
@@ -479,8 +482,8 @@ extern "C" int msa_lm_residual_norm(const float* base, int64_t base_stride, cons
   if (v4 && width <= 4096 && n_rows <= 512) {
     const int once = (width / 4 + 31) / 32 * 32;
     MSA_LM_DISPATCH(dtype, {
-      if (y && y_dtype == MSA_BF16) residual_norm_once_kernel<T, __nv_bfloat16><<<n_rows, once, 0, st>>>(p);
-      else residual_norm_once_kernel<T, float><<<n_rows, once, 0, st>>>(p);
+      auto kernel = y && y_dtype == MSA_BF16 ? residual_norm_once_kernel<T, __nv_bfloat16> : residual_norm_once_kernel<T, float>;
+      MSA_CUDA_OK(launch_kernel_pdl(kernel, dim3(n_rows), dim3(once), 0, st, n_rows <= kEarlyRows && !inv, p));   // inv: behind the experts
     });
     MSA_LAUNCH_OK("residual_norm_once_kernel");
     return MSA_OK;
@@ -539,7 +542,7 @@ inline int flat_grid(long long n) { return (int)((n + 255) / 256 < 148 * 16 ? (n
 extern "C" int msa_lm_softcap(float* x, int64_t n, float cap, void* stream) {
   MSA_REQUIRE(x && n >= 0 && cap > 0.f, "softcap: bad arguments");
   if (n == 0) return MSA_OK;
-  softcap_kernel<<<flat_grid(n), 256, 0, (cudaStream_t)stream>>>(x, n, cap);
+  MSA_CUDA_OK(launch_kernel_pdl(softcap_kernel, dim3(flat_grid(n)), dim3(256), 0, (cudaStream_t)stream, true, x, (long long)n, cap));
   MSA_LAUNCH_OK("softcap_kernel");
   return MSA_OK;
 }
@@ -556,7 +559,10 @@ extern "C" int msa_lm_tanh_split(const float* x, int32_t n_rows, int32_t cols, i
   MSA_REQUIRE(dtype_ok(dtype) && x && out && n_rows >= 0 && cols > 0 && parts >= 1, "tanh_split: bad arguments");
   const long long n = (long long)n_rows * cols;
   if (n == 0) return MSA_OK;
-  MSA_LM_DISPATCH(dtype, { tanh_split_kernel<T><<<flat_grid(n), 256, 0, (cudaStream_t)stream>>>(x, cols, parts, n, (T*)out); });
+  MSA_LM_DISPATCH(dtype, {
+    MSA_CUDA_OK(launch_kernel_pdl(tanh_split_kernel<T>, dim3(flat_grid(n)), dim3(256), 0, (cudaStream_t)stream, n <= (long long)kEarlyRows * cols,
+                                  x, cols, parts, (long long)n, (T*)out));
+  });
   MSA_LAUNCH_OK("tanh_split_kernel");
   return MSA_OK;
 }

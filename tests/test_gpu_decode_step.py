@@ -1,9 +1,9 @@
-"""Kernels of a decode step: states held in registers and shared memory, convolutions of one token."""
+"""Kernels of a decode step: states held in registers and shared memory, convolutions of one token, launches of few rows."""
 import pytest
 import torch
 
 from tests import hybrid_util as U
-from tests.test_gpu_hybrid import OneMixer, bf16_rows, exact_products, mixer_case, mixer_close  # noqa: F401
+from tests.test_gpu_hybrid import OneMixer, bf16_rows, exact_products, mixer_case, mixer_close, model  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -29,3 +29,25 @@ def test_token_by_token(kind, spec, dtype):
         at += n
     assert at == h.shape[0]
     mixer_close(torch.cat(out), oracle(h), dtype)
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8, 9])
+@pytest.mark.parametrize("name", ["wide", "par-wide", "mixed", "par-mixed"])
+def test_queued_steps_are_as_steps_that_wait(name, rows):
+    """Up to 8 rows, kernels start while the one before them runs: the bits are those of steps with the device idle in between,
+    and of a second run."""
+    m = model(name, torch.bfloat16)
+    g = torch.Generator().manual_seed(rows)
+    toks = torch.randint(0, m.config.vocab, (6, rows), generator=g).tolist()
+    seen = []
+    for wait in (True, False, False):
+        cache = m.new_cache(rows, 16)
+        for i in range(rows):
+            cache.acquire(i)
+        out = []
+        for t in toks:
+            out.append(m.run([(i, [t[i]], [0]) for i in range(rows)], cache))
+            if wait:
+                torch.cuda.synchronize()
+        seen.append(torch.stack(out))
+    assert torch.isfinite(seen[0]).all() and torch.equal(seen[0], seen[1]) and torch.equal(seen[0], seen[2])
