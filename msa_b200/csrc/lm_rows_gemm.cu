@@ -16,7 +16,7 @@
 
 namespace msa {
 
-constexpr int kRgMaxRows = 8, kRgMaxWarps = 16, kRgBlock = 32;    // kRgBlock: K of a 16-byte load per lane
+constexpr int kRgMaxRows = 8, kRgMaxWarps = 16, kRgBlock = 32, kRgTurn = 4;   // kRgBlock: K of a 16-byte load per lane
 
 struct RowsGemmParams {
   const __nv_bfloat16* x; long long x_stride, x_batch;
@@ -36,6 +36,10 @@ __device__ __forceinline__ uint4 ld_fresh(const __nv_bfloat16* p) {
   asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+// The same, into shared memory.  Without `in`: zeros.
+__device__ __forceinline__ void send_fresh(uint32_t dst, const __nv_bfloat16* p, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p), "r"(in ? 16 : 0) : "memory");
+}
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -43,13 +47,20 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 
 // MT: 16-row tiles of w per warp (with the activation 2: gate rows and the up rows that belong to them).  A block's rows of w:
 // 16 * MT; blockDim / 32 slices of K.
-template <int MT, bool ACT>
+// AHEAD: x comes through shared memory, two turns ahead.  Loaded when its turn is there, it costs each turn its way from L2: 2048 x 10240
+// took 10.4 us so and 9.2 ahead, 2048 x 6144 6.9 and 6.5, 10304 x 2048 10.6 and 9.2, 32768 x 2048 26.1 and 23.7 (8 rows).  With two turns or
+// fewer there is nothing to be ahead of (2048 x 2048 3.5 and 4.0), and with the activation it was slower (12288 x 2048 10.9 and 11.5, 6144 x
+// 1024 3.6 and 5.2: fewer registers, more blocks on the SMs that are free first).
+template <int MT, bool ACT, bool AHEAD>
 __global__ void __launch_bounds__(kRgMaxWarps * 32) rows_gemm_kernel(const RowsGemmParams p) {
-  extern __shared__ float s_part[];                                // [warp][row of x][16 * MT + 4]
-  constexpr int kRows = 16 * MT, kPitch = kRows + 4, KB = 4 / MT;   // KB: blocks of K fetched at once
+  extern __shared__ __align__(16) unsigned char smem[];
+  constexpr int kRows = 16 * MT, kPitch = kRows + 4, KB = kRgTurn / MT;   // KB: blocks of K fetched at once
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, warps = blockDim.x / 32, g = lane / 4, t = lane % 4;
   const int cols = ACT ? 16 : kRows, f0 = blockIdx.x * cols;       // output columns of this block
   grid_launch_dependents();
+  // x of two turns: a lane's own pieces, which no other lane reads.  Then the sums, [warp][row of x][kPitch].
+  uint4* s_x = reinterpret_cast<uint4*>(smem) + warp * 2 * KB * 32 + lane;
+  float* s_part = reinterpret_cast<float*>(smem + (AHEAD ? (size_t)warps * 2 * KB * 512 : 0));
   const __nv_bfloat16* w = p.w + blockIdx.y * p.w_batch + 8 * t;
   const __nv_bfloat16* wr[MT][2];
 #pragma unroll
@@ -82,10 +93,22 @@ __global__ void __launch_bounds__(kRgMaxWarps * 32) rows_gemm_kernel(const RowsG
         for (int h = 0; h < 2; ++h) a[i][m][h] = k < k_end ? ld_stream(wr[m][h] + k) : zero;
     }
   };
-  auto multiply = [&](const uint4 (&a)[KB][MT][2], int b) {
-    uint4 v[KB];
+  auto send = [&](int turn, int b) {
 #pragma unroll
-    for (int i = 0; i < KB; ++i) v[i] = (b + i) * kRgBlock < k_end ? ld_fresh(x + (b + i) * kRgBlock) : zero;
+    for (int i = 0; i < KB; ++i) {
+      const bool in = g < p.n && (b + i) * kRgBlock < k_end;          // rows past the last one: zeros, nobody reads their sums
+      send_fresh((uint32_t)__cvta_generic_to_shared(s_x + (turn * KB + i) * 32), in ? x + (b + i) * kRgBlock : x, in);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto multiply = [&](const uint4 (&a)[KB][MT][2], int turn, int b) {
+    uint4 v[KB];
+    if constexpr (AHEAD) asm volatile("cp.async.wait_group 1;" ::: "memory");   // the turn's pieces; the next turn's may be on their way
+#pragma unroll
+    for (int i = 0; i < KB; ++i) {
+      if constexpr (!AHEAD) v[i] = (b + i) * kRgBlock < k_end ? ld_fresh(x + (b + i) * kRgBlock) : zero;
+      else v[i] = s_x[(turn * KB + i) * 32];
+    }
 #pragma unroll
     for (int i = 0; i < KB; ++i)
 #pragma unroll
@@ -94,15 +117,21 @@ __global__ void __launch_bounds__(kRgMaxWarps * 32) rows_gemm_kernel(const RowsG
         mma16816(acc[m], lo.x, hi.x, lo.y, hi.y, v[i].x, v[i].y);
         mma16816(acc[m], lo.z, hi.z, lo.w, hi.w, v[i].z, v[i].w);
       }
+    if constexpr (AHEAD) __syncwarp();                              // read before the next pieces land there
   };
   if (!p.early) grid_dependency_wait();
   fetch(a[0], b0);
   fetch(a[1], b0 + KB);
   if (p.early) grid_dependency_wait();
+  if constexpr (AHEAD) {
+    send(0, b0);
+    send(1, b0 + KB);
+  }
   for (int b = b0; b < b1; b += 2 * KB) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      multiply(a[i], b + i * KB);
+      multiply(a[i], i, b + i * KB);
+      if constexpr (AHEAD) send(i, b + (2 + i) * KB);
       fetch(a[i], b + (2 + i) * KB);
     }
   }
@@ -126,21 +155,28 @@ __global__ void __launch_bounds__(kRgMaxWarps * 32) rows_gemm_kernel(const RowsG
   }
 }
 
+template <int MT, bool ACT, bool AHEAD>
+int launch_rows_gemm(const RowsGemmParams& p, int batch, int cols, int warps, cudaStream_t stream) {
+  static DeviceSmem state{};
+  const size_t smem = (size_t)warps * ((AHEAD ? 2 * (kRgTurn / MT) * 512 : 0) + kRgMaxRows * (16 * MT + 4) * 4);
+  auto kernel = rows_gemm_kernel<MT, ACT, AHEAD>;
+  MSA_OK_OR_RETURN(ensure_dynamic_smem(kernel, smem, state));
+  MSA_CUDA_OK(launch_kernel_pdl(kernel, dim3((unsigned)((p.features + cols - 1) / cols), (unsigned)batch), dim3(warps * 32), smem, stream,
+                                p.early != 0, p));
+  return MSA_OK;
+}
+
 template <int MT, bool ACT>
 int launch_rows_gemm(const RowsGemmParams& p, int batch, cudaStream_t stream) {
-  static DeviceSmem state{};
   const int cols = ACT ? 16 : 16 * MT, blocks = (p.k + kRgBlock - 1) / kRgBlock;
   const long long ctas = (long long)((p.features + cols - 1) / cols) * batch;
   int n_sm = 0;
   MSA_OK_OR_RETURN(device_sm_count(&n_sm));
   int warps = ctas <= n_sm ? 16 : (ctas <= 2 * n_sm ? 8 : 4);      // 16 warps fit an SM: one block of them, two or four
   while (warps > 1 && blocks < 2 * warps) warps /= 2;              // at least 64 of K per warp
-  const size_t smem = (size_t)warps * kRgMaxRows * (16 * MT + 4) * 4;
-  auto kernel = rows_gemm_kernel<MT, ACT>;
-  MSA_OK_OR_RETURN(ensure_dynamic_smem(kernel, smem, state));
-  MSA_CUDA_OK(launch_kernel_pdl(kernel, dim3((unsigned)((p.features + cols - 1) / cols), (unsigned)batch), dim3(warps * 32), smem, stream,
-                                p.early != 0, p));
-  return MSA_OK;
+  if constexpr (!ACT)
+    if (blocks > 2 * (kRgTurn / MT) * warps) return launch_rows_gemm<MT, ACT, true>(p, batch, cols, warps, stream);
+  return launch_rows_gemm<MT, ACT, false>(p, batch, cols, warps, stream);
 }
 
 }  // namespace msa
