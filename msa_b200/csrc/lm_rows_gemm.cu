@@ -7,8 +7,8 @@
 // 16-byte load, and feeds them to two products.  The kernel is launched early (programmatic dependent launch): the first pieces of the
 // weights, which no kernel of a step writes, are fetched while the kernel before it still runs; all else waits for that kernel.
 //
-// Measured (bf16 out, 8 rows, a chain of products with fresh weights in a CUDA graph; torch.mm beside it): 2048 x 2048 3.6 us
-// (6.7), 2048 x 6144 7.0 (14.9), 2048 x 10240 10.5 (23.1), 12288 x 2048 11.0 (9.9 and 1.8 for the gate, which is part of this one).
+// Measured (bf16 out, 8 rows, a chain of products with fresh weights in a CUDA graph; torch.mm beside it): 2048 x 2048 3.5 us
+// (6.7), 2048 x 6144 6.5 (14.9), 2048 x 10240 9.2 (23.1), 12288 x 2048 10.9 (9.9 and 1.8 for the gate, which is part of this one).
 // Weights through a TMA ring into tcgen05.mma with 16 columns took 12.9 us for 12288 x 2048 and 12.4 for 2048 x 10240: four
 // products per 16 KB cost about as much as fetching them, and start and end of a tile another 3 us.  With 16 rows this kernel's x takes as
 // much from L2 as w from HBM, and a whole decode step was no faster than with the library's products (459 us both).
@@ -198,9 +198,9 @@ extern "C" int msa_lm_rows_gemm(const msa_lm_rows_gemm_args* args, void* stream)
   if (a.act) return launch_rows_gemm<2, true>(p, a.batch, st);
   int n_sm = 0;
   MSA_OK_OR_RETURN(device_sm_count(&n_sm));
-  // Taller tiles halve what the rows of x take from L2.  Tiles of 16 and of 32 rows, 8 rows of x in a chain of products: 9472 x 2048 10.7 and 9.6 us,
-  // 12288 x 2048 16.4 and 12.9, 16384 x 4096 32.8 and 27.1, a vocabulary of 32768 x 2048 33.3 and 28.2, of 151936 x 2048 122.4 and 104.5.
-  // Below the line both read about the same (4736 x 2048 5.3 and 5.3, 6144 x 2048 7.9 and 7.5, 4096 x 4096 9.3 and 8.9), but for the
-  // smallest, where 32 rows were faster (2048 x 2048 3.9 and 3.0) and are not taken yet: they split K over other warps, which moves last bits.
+  // Taller tiles halve what the rows of x take from L2.  Tiles of 16 and of 32 rows, 8 rows of x in a chain of products: 9472 x 2048 8.7 and 7.4 us,
+  // 12288 x 2048 12.5 and 10.2, 16384 x 4096 26.6 and 25.1, a vocabulary of 32768 x 2048 27.2 and 24.1, of 151936 x 2048 102.5 and 94.9.
+  // Below the line 32 rows are faster too (4736 x 2048 5.1 and 4.8, 8192 x 2048 7.7 and 6.6, 4096 x 4096 7.3 and 7.2) and are not taken:
+  // they split K over other warps, which moves last bits.
   return (long long)a.w_rows * a.batch >= 64ll * n_sm ? launch_rows_gemm<2, false>(p, a.batch, st) : launch_rows_gemm<1, false>(p, a.batch, st);
 }
