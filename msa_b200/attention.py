@@ -330,7 +330,7 @@ class MemorySparseAttention(Qwen3Attention):
         # segments, go through the segment path, which stores only the unmasked tokens.
         if q_len == 1 and not cache.meta.get("qa_mode", False) and cache.meta.get("step_all_valid", True):
             done = A.native().decode(query_states, key_states, value_states, k_store, v_store, kv_start, kv_len, cache_kwargs["kv_lengths"],
-                                     ops.decode_splits(bsz, k_store.shape[1], k_store.shape[2]))
+                                     ops.decode_splits(bsz, k_store.shape[1], k_store.shape[2])) if ops.own("sparse_decode_attn") else None
             if done is not None:
                 attn_output, kv_len, cache_kwargs["kv_lengths"] = done
             else:

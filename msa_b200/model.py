@@ -109,14 +109,14 @@ class MSAModel(nn.Module):
     def _native_layers(self, hidden):
         """The layers' weights for their native pass, or None where a module of some layer is not what that pass steps over."""
         if not hidden.is_cuda or torch.is_grad_enabled() or nn_module._has_any_global_hook() or any(
-                c.forward.__module__ != c.__module__ for c in STEPPED_OVER):
+                c.forward.__module__ != c.__module__ for c in STEPPED_OVER) or not ops.own():
             return None
         return A.native().layers(tuple(self.layers), STEPPED_OVER)
 
     def _angles(self, hidden, position_ids):
         rot = self.rotary_emb
         if hidden.is_cuda and hidden.dtype == torch.bfloat16 and plain_module(rot, Qwen3RotaryEmbedding) and rot.rope_type == "default" and (
-                position_ids.get_device() == hidden.get_device()):
+                position_ids.get_device() == hidden.get_device()) and ops.own("rope_table"):
             both = A.native().angles(position_ids, rot.inv_freq, rot.attention_scaling)
             if both is not None:
                 return both

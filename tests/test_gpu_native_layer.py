@@ -141,3 +141,15 @@ def test_what_else_goes_through_the_modules(monkeypatch):
         own = net.layers[0].self_attn.q_proj
         own.weight = nn.Parameter(own.weight.float())
         assert layers() is None
+
+
+@pytest.mark.parametrize("name,run", [("add_rmsnorm", block), ("silu_mul_parts", block), ("heads_norm_rope", block), ("rope_table", token),
+                                      ("sparse_decode_attn", token)])
+def test_a_function_put_in_the_place_of_an_op_is_called(monkeypatch, name, run):
+    from msa_b200 import ops
+    net, calls, real = model(), [], getattr(ops, name)
+    with torch.no_grad():
+        want = run(net)
+        monkeypatch.setattr(ops, name, lambda *a, **k: calls.append(1) or real(*a, **k))
+        got = run(net)
+    assert calls and all(torch.equal(a, b) for a, b in zip(got, want))
