@@ -73,7 +73,7 @@ template <> __device__ __forceinline__ float silu_act<__nv_bfloat16>(float z) { 
 // Rows up to which the product behind a kernel may be rows_gemm_kernel, which fetches its weights early.  The library's products gain
 // nothing by it: behind a part_norm of 6236 rows they crowded it out (39 -> 53 us).
 // The small kernels behind such a product (norms, rotations, decode states) are launched early too and wait at their top: their blocks
-// are in place when the product's last one ends, 0.5 to 1 us each, 260 us instead of 274 for a token of 8 sequences in 40 launches.  Not so
+// are in place when the product's last one ends, 0.5 to 1 us each, 271 us instead of 280 for a token of 8 sequences in 40 launches.  Not so
 // kernels that need another split of shared memory and L1, which an SM takes on when it is empty (delta_decode_kernel took 16.4 us instead of
 // 8.3, and the products after it kept its small L1: 20 us instead of 10), nor what follows one; those end the chain on purpose.
 constexpr int kEarlyRows = 8;
