@@ -432,17 +432,11 @@ __global__ void __launch_bounds__(2 * N) ssd_add_kernel(const SsdChunkParams p) 
     const int lane = threadIdx.x, r = 2 * lane;
     const double rate = -1.4426950408889634 * expf(a.a_log[h]);
     const float d0 = r < ch.len ? p.dt[(row0 + r) * a.heads + h] : 0.f, d1 = r + 1 < ch.len ? p.dt[(row0 + r + 1) * a.heads + h] : 0.f;
-    double sum = rate * d0 + rate * d1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double x = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= o) sum += x;
-    }
-    const double total = __shfl_sync(0xffffffffu, sum, 31), g0 = sum - rate * d1;
-    if (r < ch.len) p.gcum[(row0 + r) * a.heads + h] = g0;
-    if (r + 1 < ch.len) p.gcum[(row0 + r + 1) * a.heads + h] = sum;
-    s_w[r] = d0 * exp2f((float)(total - g0));
-    s_w[r + 1] = d1 * exp2f((float)(total - sum));
+    const SsdDecays g = ssd_decays(rate, d0, d1);
+    if (r < ch.len) p.gcum[(row0 + r) * a.heads + h] = g.first;
+    if (r + 1 < ch.len) p.gcum[(row0 + r + 1) * a.heads + h] = g.second;
+    s_w[r] = d0 * exp2f((float)(g.total - g.first));
+    s_w[r + 1] = d1 * exp2f((float)(g.total - g.second));
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kLcRows * (V / 4); i += kThreads) {

@@ -4,18 +4,22 @@
 // Transposed, a thread's TMEM lane is a value column; two heads of 64 make the 128 lanes.  With the chunk's keys B and queries C (one
 // set per group), its values X, steps dt and running log2 decays G (per head):
 //     scores = C B^T                          P_h = scores * 2^(G_t - G_i) dt_i below the diagonal, hi / lo planes in shared memory
-//     O1^T = S^T C^T                          O2_h^T = X^T P_h^T  (for both heads' lanes; each reads its own)
-//     S^T = 2^(G_C) S^T + (w X)^T B           w_i = dt_i 2^(G_C - G_i)
-//     y = (2^G O1 + O2 + skip x) silu(gate)
-// 32-bit operands (state, scores with their decays, weighted values) enter as hi / lo pairs of bf16; sums are fp32.  The scores come
-// twice, in the lower and the upper 64 lanes (C lies in shared memory twice), so that 128 threads make the two heads' P.
+//     R^T = S^T C^T                           O_h^T = 2^G R^T + X^T P_h^T  (for both heads' lanes; each reads its own)
+//     dS^T = (w X)^T B, w_i = dt_i 2^(G_C - G_i)     S' = fma(2^(G_C), S, dS)
+//     y = (O + skip x) silu(gate)
+// 32-bit operands (state, scores with their decays, weighted values) enter as hi / lo pairs of bf16; sums are fp32.  Every sum runs as in the
+// kernels over all chunks at once (running decays in 64 bits, the same products in the same order) and the bits are theirs, so that a
+// sequence does not depend on what else is in a step.  In particular no sum on the tensor core, which cuts off what it aligns away, goes
+// on over chunks: the state is rounded to nearest once a chunk.
+//
+// The scores come twice, in the lower and the upper 64 lanes (C lies in shared memory twice), so that 128 threads make the two heads' P.
 //
 // Warps by role: 0-7 scores -> P, 8-11 states and the values (weighted as TMEM planes, transposed in shared memory), 12-19 outputs,
 // 20-22 fetch (two chunks' buffers) and sum up the decays, 23 issues the products.
-// What bounds it: instructions of the conversions (3,700 per scheduler and chunk, issued at 0.43 a cycle: their latencies, with five
-// or six warps per scheduler), 56 products of some 70 cycles each, whatever their columns, and the order scores -> P -> outputs -> next
-// scores, which share TMEM.  Portions of 2048, 1500, 1911 and 777 tokens, 64 heads, from a cold L2: 173 us, where the three kernels
-// over all chunks at once take 447 (chunk states through HBM four times, products on mma.sync).
+// What bounds it: instructions of the conversions (their latencies, with five or six warps per scheduler), 56 products of some 70 cycles
+// each, whatever their columns, and the chains scores -> P -> outputs and state -> read-out -> outputs.  Portions of 2048, 1500, 1911 and 777
+// tokens, 64 heads, from a cold L2: 187 us, where the three kernels over all chunks at once take 425 (chunk states through HBM four
+// times, products on mma.sync).  With the state as the tensor core's accumulator and its read-out added to the outputs at the end it took 172.
 #include "lm_linear.cuh"
 #include "mma_helpers.cuh"
 #include "tc_attn_common.cuh"
@@ -28,8 +32,9 @@ constexpr int kStC = 0, kStB = 4 * kStPlane, kStX = kStB + 2 * kStPlane, kStBuf 
 // per head hi, lo; values transposed (two chunks').  The gates come where the values were, once those are transposed.
 constexpr int kStP = 2 * kStBuf, kStXt = kStP + 4 * kStPlane;
 constexpr size_t kStSmem = kStXt + 4 * kStPlane + 1024;
-// TMEM columns: states, their planes, scores and then head 0's O2, planes of the weighted values, O1, head 1's O2
-constexpr uint32_t kStS = 0, kStSh = 128, kStSl = 192, kStZ = 256, kStWh = 320, kStWl = 352, kStO1 = 384, kStO2 = 448;
+// TMEM columns: states; what the chunk adds to them, 16 columns at a time replaced by the new state's planes (8 hi, 8 lo); scores; planes of the
+// weighted values; outputs of head 0 and of head 1
+constexpr uint32_t kStS = 0, kStD = 128, kStZ = 256, kStWh = 320, kStWl = 352, kStO1 = 384, kStO2 = 448;
 
 struct SsdTcParams {
   msa_lm_ssd_args a;
@@ -37,10 +42,12 @@ struct SsdTcParams {
   const float* dt;               // [rows, heads]
   int32_t* status;
 };
-struct SsdTcBars { uint64_t full[2], free[2], g_full[2], z_done, p_ready, s_ready, x_ready, s_done, o_done, o_free, drain; };
-struct SsdTcDecay {              // of a chunk, per head
-  float gh[2][kStRows], gl[2][kStRows], eg[2][kStRows], dt[2][kStRows], w[2][kStRows], all[2];      // G as a pair of floats
+struct SsdTcBars { uint64_t full[2], free[2], g_full[2], z_done, p_ready, s_ready, x_ready, s_done, r_done, r_ready, h_done, o_done, o_free, drain; };
+struct __align__(16) SsdTcDecay {              // of a chunk, per head; g is read two at a time
+  double g[2][kStRows];
+  float eg[2][kStRows], dt[2][kStRows], w[2][kStRows], all[2];
 };
+static_assert(sizeof(SsdTcDecay) % 16 == 0, "the second chunk's pairs of doubles");
 
 __device__ __forceinline__ void st_split2(float x, float y, uint32_t& hi, uint32_t& lo) {
   hi = pack2_bf16(x, y);
@@ -51,7 +58,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
                                                                 const __grid_constant__ CUtensorMap map_g, const SsdTcParams p) {
   extern __shared__ unsigned char dyn[];
   __shared__ SsdTcBars bars;
-  __shared__ __align__(16) SsdTcDecay s_d[2];
+  __shared__ SsdTcDecay s_d[2];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
   const msa_lm_ssd_args& a = p.a;
@@ -65,7 +72,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&bars.full[i], 3); mbar_init(&bars.free[i], 9); mbar_init(&bars.g_full[i], 1); }
     mbar_init(&bars.z_done, 1); mbar_init(&bars.s_done, 1); mbar_init(&bars.o_done, 1); mbar_init(&bars.drain, 1);
-    mbar_init(&bars.p_ready, 8); mbar_init(&bars.s_ready, 4); mbar_init(&bars.x_ready, 4); mbar_init(&bars.o_free, 8);
+    mbar_init(&bars.r_done, 1); mbar_init(&bars.h_done, 1); mbar_init(&bars.r_ready, 8); mbar_init(&bars.p_ready, 8); mbar_init(&bars.s_ready, 4); mbar_init(&bars.x_ready, 4); mbar_init(&bars.o_free, 8);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -96,7 +103,7 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
       const SsdTcDecay& d = s_d[ch & 1];
       if (!wait(&bars.full[ch & 1], ch >> 1, 50) || !wait(&bars.z_done, ch, 51)) break;      // the products before have left P, too
       tc_fence_after();
-      const float gth = d.gh[hd][t], gtl = d.gl[hd][t];
+      const double gt = d.g[hd][t];
       unsigned char* row = sm + kStP + hd * 2 * kStPlane;
       if (on) {
 #pragma unroll
@@ -107,10 +114,10 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 16; i += 2) {
-            const float2 gh = *reinterpret_cast<const float2*>(&d.gh[hd][c0 + i]), gl = *reinterpret_cast<const float2*>(&d.gl[hd][c0 + i]);
+            const double2 g = *reinterpret_cast<const double2*>(&d.g[hd][c0 + i]);
             const float2 dt = *reinterpret_cast<const float2*>(&d.dt[hd][c0 + i]);
-            const float x = __uint_as_float(z[i]) * ex2_approx((gth - gh.x) + (gtl - gl.x)) * dt.x;
-            const float y = __uint_as_float(z[i + 1]) * ex2_approx((gth - gh.y) + (gtl - gl.y)) * dt.y;
+            const float x = __uint_as_float(z[i]) * exp2f((float)(gt - g.x)) * dt.x;
+            const float y = __uint_as_float(z[i + 1]) * exp2f((float)(gt - g.y)) * dt.y;
             // masked as bits: a branch around every element would expose its whole latency
             st_split2(__uint_as_float(__float_as_uint(x) & (c0 + i <= t ? 0xffffffffu : 0u)),
                       __uint_as_float(__float_as_uint(y) & (c0 + i + 1 <= t ? 0xffffffffu : 0u)), hi[i / 2], lo[i / 2]);
@@ -131,19 +138,21 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
     // ---- states, and the chunk's values: weighted and transposed
     float* state = a.state + ((long long)a.slot[sq] * a.heads + h0 + hd) * kStN * kStV + col % kStV;
     const bool fresh = a.start[sq] == 0;
-    auto put_state = [&](int n, const uint32_t (&x)[32], float all) {   // 32 of the state's rows: planes, and decayed by the chunk
-      uint32_t hi[16], lo[16];
+    auto put_state = [&](int n, const uint32_t (&x)[16]) {              // 16 of the state's rows and their planes
+      uint32_t planes[16];
 #pragma unroll
-      for (int j = 0; j < 32; j += 16) {
-        uint32_t s[16];
+      for (int i = 0; i < 8; ++i) st_split2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]), planes[i], planes[8 + i]);
+      tmem_st16(lanes + kStS + n, x);
+      tmem_st16(lanes + kStD + n, planes);
+    };
+    float all = 1.f;
+    auto next_state = [&](int n, uint32_t (&x)[16]) {                   // the state behind a chunk: decayed, and what the chunk adds
+      uint32_t add[16];
+      tmem_ld16(lanes + kStS + n, x);
+      tmem_ld16(lanes + kStD + n, add);
+      tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) s[i] = __float_as_uint(__uint_as_float(x[j + i]) * all);
-        tmem_st16(lanes + kStS + n + j, s);
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) st_split2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]), hi[i], lo[i]);
-      tmem_st16(lanes + kStSh + n / 2, hi);
-      tmem_st16(lanes + kStSl + n / 2, lo);
+      for (int i = 0; i < 16; ++i) x[i] = __float_as_uint(fmaf(all, __uint_as_float(x[i]), __uint_as_float(add[i])));
     };
     if (n_chunks == 0 && fresh)
       for (int n = 0; n < kStN; ++n) state[n * kStV] = 0.f;
@@ -153,18 +162,17 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
       if (!(ok = wait(&bars.full[b], ch >> 1, 52))) break;
       if (ch > 0 && !(ok = wait(&bars.s_done, ch + 1, 53))) break;
       tc_fence_after();
-      const float all = s_d[b].all[hd];
-      for (int n = 0; n < kStN; n += 32) {
-        uint32_t x[32];
+      for (int n = 0; n < kStN; n += 16) {
+        uint32_t x[16];
         if (ch == 0) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) x[i] = fresh ? 0u : __float_as_uint(state[(n + i) * kStV]);
+          for (int i = 0; i < 16; ++i) x[i] = fresh ? 0u : __float_as_uint(state[(n + i) * kStV]);
         } else {
-          tmem_ld32(lanes + kStS + n, x);
-          tmem_ld_wait();
+          next_state(n, x);
         }
-        put_state(n, x, all);
+        put_state(n, x);
       }
+      all = s_d[b].all[hd];
       tmem_st_wait();
       tc_fence_before();
       arrive(&bars.s_ready);
@@ -202,33 +210,45 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
     }
     if (ok && n_chunks > 0 && wait(&bars.s_done, n_chunks + 1, 54)) {
       tc_fence_after();
-      for (int n = 0; n < kStN; n += 32) {
-        uint32_t x[32];
-        tmem_ld32(lanes + kStS + n, x);
-        tmem_ld_wait();
+      for (int n = 0; n < kStN; n += 16) {
+        uint32_t x[16];
+        next_state(n, x);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) state[(n + i) * kStV] = __uint_as_float(x[i]);
+        for (int i = 0; i < 16; ++i) state[(n + i) * kStV] = __uint_as_float(x[i]);
       }
     }
   } else if (warp < 20) {
-    // ---- outputs: half of the tokens to four warps each
+    // ---- outputs: half of the tokens to four warps each.  The read-out of the state is decayed where it stands; the chunk's own tokens add to it.
     const int part = (warp - 12) / 4 * (kStRows / 2);
     const float skip = a.d_skip[h0 + hd];
     float* out = a.y + n0 * inner + h0 * kStV + col;
-    const uint32_t o2 = lanes + (hd ? kStO2 : kStZ) + part;
+    const uint32_t own = lanes + (hd ? kStO2 : kStO1) + part;
     for (int ch = 0; ch < n_chunks; ++ch) {
       const int b = ch & 1, rows = min(kStRows, len - ch * kStRows);
       float o[kStRows / 2];
-      if (!wait(&bars.full[b], ch >> 1, 62) || !wait(&bars.o_done, ch, 55)) break;
+      if (!wait(&bars.full[b], ch >> 1, 62) || !wait(&bars.r_done, ch, 65)) break;
       tc_fence_after();
 #pragma unroll
       for (int t = 0; t < kStRows / 2; t += 16) {
-        uint32_t x[16], y[16];
+        uint32_t x[16];
         tmem_ld16(lanes + kStO1 + part + t, x);
-        tmem_ld16(o2 + t, y);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) o[t + i] = fmaf(s_d[b].eg[hd][part + t + i], __uint_as_float(x[i]), __uint_as_float(y[i]));
+        for (int i = 0; i < 16; ++i) x[i] = __float_as_uint(s_d[b].eg[hd][part + t + i] * __uint_as_float(x[i]));
+        tmem_st16(own + t, x);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      arrive(&bars.r_ready);
+      if (!wait(&bars.o_done, ch, 55)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int t = 0; t < kStRows / 2; t += 16) {
+        uint32_t x[16];
+        tmem_ld16(own + t, x);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[t + i] = __uint_as_float(x[i]);
       }
       tc_fence_before();
       arrive(&bars.o_free);
@@ -298,24 +318,18 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
         const int r = 2 * lane;
         const float* dt = p.dt + (row0 + ch * kStRows) * a.heads + h0 + k;
         const float d0 = r < rows ? dt[(long long)r * a.heads] : 0.f, d1 = r + 1 < rows ? dt[(long long)(r + 1) * a.heads] : 0.f;
-        double sum = rate * d0 + rate * d1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const double x = __shfl_up_sync(0xffffffffu, sum, o);
-          if (lane >= o) sum += x;
-        }
-        const double total = __shfl_sync(0xffffffffu, sum, 31), g[2] = {sum - rate * d1, sum};
+        const SsdDecays g = ssd_decays(rate, d0, d1);
+        const double row[2] = {g.first, g.second};
         const float step[2] = {d0, d1};
         SsdTcDecay& d = s_d[b];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          d.gh[k][r + e] = (float)g[e];
-          d.gl[k][r + e] = (float)(g[e] - (double)(float)g[e]);
-          d.eg[k][r + e] = exp2f((float)g[e]);
+          d.g[k][r + e] = row[e];
+          d.eg[k][r + e] = exp2f((float)row[e]);
           d.dt[k][r + e] = step[e];
-          d.w[k][r + e] = step[e] * exp2f((float)(total - g[e]));
+          d.w[k][r + e] = step[e] * exp2f((float)(g.total - row[e]));
         }
-        if (lane == 0) d.all[k] = exp2f((float)total);
+        if (lane == (rows - 1) / 2) d.all[k] = exp2f((float)((rows & 1) ? g.first : g.second));
       }
       if (rows < kStRows) {
         cp_async_wait<0>();
@@ -336,46 +350,54 @@ __global__ void __launch_bounds__(kStThreads, 1) ssd_tc_kernel(const __grid_cons
     for (int ch = 0; ch < n_chunks && ok; ++ch) {
       const int b = ch & 1;
       const uint32_t base = smem_u32(sm + b * kStBuf), planes = smem_u32(sm + kStP);
-      if (!(ok = one(&bars.full[b], ch >> 1, 57) && one(&bars.o_free, ch + 1, 58))) break;
+      if (!(ok = one(&bars.full[b], ch >> 1, 57))) break;
       tc_fence_after();
 #pragma unroll
       for (int k = 0; k < 8; ++k)
         tc_mma_bf16(tmem + kStZ, make_smem_desc(base + kStC + k / 4 * 2 * kStPlane) + 2 * (k % 4), make_smem_desc(base + kStB + k / 4 * kStPlane) + 2 * (k % 4),
                     idesc | n_of(kStRows), k > 0);
       tc_commit(&bars.z_done);
-      if (!(ok = one(&bars.s_ready, ch, 59))) break;
+      if (!(ok = one(&bars.s_ready, ch, 59) && one(&bars.o_free, ch + 1, 58))) break;
       tc_fence_after();
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const uint64_t c = make_smem_desc(base + kStC + k / 4 * 2 * kStPlane) + 2 * (k % 4);
-        tc_mma_bf16_ts(tmem + kStO1, tmem + kStSl + 8 * k, c, idesc | n_of(kStRows), k > 0);
-        tc_mma_bf16_ts(tmem + kStO1, tmem + kStSh + 8 * k, c, idesc | n_of(kStRows), 1u);
+        const uint32_t s = tmem + kStD + 16 * k;
+        tc_mma_bf16_ts(tmem + kStO1, s + 8, c, idesc | n_of(kStRows), k > 0);
+        tc_mma_bf16_ts(tmem + kStO1, s, c, idesc | n_of(kStRows), 1u);
       }
-      if (!(ok = one(&bars.x_ready, ch, 60))) break;
+      tc_commit(&bars.r_done);
+      if (!(ok = one(&bars.x_ready, ch, 60) && one(&bars.r_done, ch, 66))) break;          // the planes have been read: their place is taken
       tc_fence_after();
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const uint64_t key = make_smem_desc_mn(base + kStB + k * 2048, kStPlane);
-        tc_mma_bf16_ts(tmem + kStS, tmem + kStWl + 8 * k, key, idesc | (1u << 16) | n_of(kStN), 1u);
-        tc_mma_bf16_ts(tmem + kStS, tmem + kStWh + 8 * k, key, idesc | (1u << 16) | n_of(kStN), 1u);
+        tc_mma_bf16_ts(tmem + kStD, tmem + kStWl + 8 * k, key, idesc | (1u << 16) | n_of(kStN), k > 0);
+        tc_mma_bf16_ts(tmem + kStD, tmem + kStWh + 8 * k, key, idesc | (1u << 16) | n_of(kStN), 1u);
       }
       tc_commit(&bars.s_done);
-      if (!(ok = one(&bars.p_ready, ch, 61))) break;
+      if (!(ok = one(&bars.p_ready, ch, 61) && one(&bars.r_ready, ch, 67))) break;
       tc_fence_after();
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        // Tokens from 32 on reach the columns from there on (P has nothing before).  Halves of 32 columns throughout: products into the
-        // same columns keep their order only if they have the same shape.
+      // 16 tokens reach the columns from theirs on.  First 32 columns at a time, then the 16 left; products into the same columns keep their
+      // order only if they have the same shape, hence the wait between.
+      auto add = [&](int k, int c0, int n) {
         const uint64_t x = make_smem_desc(smem_u32(sm + kStXt + b * 2 * kStPlane)) + 2 * k;
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh)
+            tc_mma_bf16(tmem + (hh ? kStO2 : kStO1) + c0, x, make_smem_desc(planes + (hh * 2 + 1 - e) * kStPlane + c0 * 128) + 2 * k, idesc | n_of(n), 1u);
+      };
 #pragma unroll
-            for (int j = k / 2; j < 2; ++j)
-              tc_mma_bf16(tmem + (hh ? kStO2 : kStZ) + 32 * j, x,
-                          make_smem_desc(planes + (hh * 2 + 1 - e) * kStPlane + j * 4096) + 2 * k, idesc | n_of(32), k > 0 || e > 0);
+      for (int k = 0; k < 3; ++k) {
+        if (k == 0) add(k, 0, 32);
+        add(k, 32, 32);
       }
+      tc_commit(&bars.h_done);
+      if (!(ok = one(&bars.h_done, ch, 68))) break;
+      tc_fence_after();
+      add(1, 16, 16);
+      add(3, 48, 16);
       tc_commit(&bars.o_done);
       tc_commit(&bars.free[b]);
     }

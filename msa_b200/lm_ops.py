@@ -323,10 +323,10 @@ def wkv_mix(rkvg, decay, spec, w, state, eps, step, out):
 
 
 def ssd_walks(step, heads: int) -> bool:
-    """Whether walking the chunks of every portion beats all chunks at once: 10 us + 4.7 per chunk of the longest portion against 24 us +
-    0.06 per chunk and head.  64 heads: portions of 2048, 1500, 1911 and 777 tokens 173 and 447 us, one of 1024 85 and 85, of 50 15 and
-    26; 32 heads: the four portions 163 and 232, one of 1024 84 and 54, one of 8192 599 and 316."""
-    return 78 * ((step.max_len + 63) // 64) < step.n_chunks * heads + 250
+    """Whether walking the chunks of every portion beats all chunks at once, which come to the same bits: 10 us + 5.1 per chunk of the longest
+    portion against 20 us + 0.064 per chunk and head.  64 heads: portions of 2048, 1500, 1911 and 777 tokens 187 and 425 us, one of 1024 88
+    and 81, of 50 16 and 26; 32 heads: the four portions 171 and 220, one of 1024 88 and 50, one of 8192 623 and 302."""
+    return 80 * ((step.max_len + 63) // 64) < step.n_chunks * heads + 150
 
 
 def ssd_mix(proj, spec, w, conv_state, state, eps, step, out):

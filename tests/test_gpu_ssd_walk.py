@@ -25,16 +25,35 @@ def case(heads, groups, state, vdim, lens, n_decode, seed=0, dev="cuda:0", step=
     return c
 
 
-def walk(c):
+def args_of(c):
     from msa_b200 import _cabi_lm as A
     p = A.ptr
-    args = A.SsdArgs(proj=p(c["proj"]), proj_stride=c["proj"].stride(0), conv_w=p(c["d_skip"]), conv_b=p(c["d_skip"]), dt_bias=p(c["d_skip"]),
+    return A.SsdArgs(proj=p(c["proj"]), proj_stride=c["proj"].stride(0), conv_w=p(c["d_skip"]), conv_b=p(c["d_skip"]), dt_bias=p(c["d_skip"]),
                      a_log=p(c["a_log"]), d_skip=p(c["d_skip"]), conv_state=p(c["xbc"]), state=p(c["state"]), tok_seq=p(c["cu"]), slot=p(c["slot"]),
                      start=p(c["start"]), cu=p(c["cu"]), y=p(c["y"]), taps=4, dtype=A.dtype_code(BF16),
                      **{k: c[k] for k in ("n_tok", "n_seq", "n_decode", "heads", "vdim", "n_state", "groups")})
+
+
+def walk(c):
+    from msa_b200 import _cabi_lm as A
+    p, args = A.ptr, args_of(c)
     status = torch.zeros(4, dtype=torch.int32, device=c["y"].device)
     A.call("msa_lm_ssd_walk", ctypes.byref(args), p(c["xbc"]), p(c["dt"]), p(status), A.stream_ptr(c["y"].device))
     assert status.tolist() == [0, 0, 0, 0]
+
+
+def all_at_once(c):
+    """The kernels over all chunks at once: (outputs, states), ``c`` as it was."""
+    from msa_b200 import _cabi_lm as A
+    p, dev = A.ptr, c["y"].device
+    mine = dict(c, y=c["y"].clone(), state=c["state"].clone())
+    lens = c["cu"].diff()[c["n_decode"]:]
+    off = torch.cat([torch.zeros(1, device=dev), ((lens + 63) // 64).cumsum(0)]).int()
+    n = int(off[-1])
+    gcum = torch.empty((c["xbc"].shape[0], c["heads"]), dtype=F64, device=dev)
+    work = torch.empty((n, c["heads"], c["n_state"], c["vdim"]), device=dev)
+    A.call("msa_lm_ssd_chunk", ctypes.byref(args_of(mine)), p(c["xbc"]), p(c["dt"]), p(off), n, p(gcum), p(work), A.stream_ptr(dev))
+    return mine["y"], mine["state"]
 
 
 def recurrence(c, size):
@@ -99,3 +118,51 @@ def test_walk_keeps_portions_apart():
     slot = int(c["slot"][0])
     assert bool(((c["state"][slot].to(F64) - states[0]).abs() <= 2.0 ** -14 * sizes[0] + 1e-30).all())
     assert bool(c["state"][int(c["slot"][1])].isnan().all())
+
+
+def same(x, y):
+    """Equal numbers; not-a-numbers in the same places."""
+    return torch.equal(x.nan_to_num(12345.0), y.nan_to_num(12345.0))
+
+
+@pytest.mark.parametrize("heads,groups,lens,n_decode", [
+    (2, 1, [1, 2, 15, 16, 17, 31, 33], 0), (4, 2, [47, 48, 49, 63, 64, 65], 3), (12, 2, [129, 190, 191, 192], 1), (64, 8, [1, 300, 4096], 0),
+    (32, 4, [2048, 1500, 1911, 777], 2)])
+@pytest.mark.parametrize("step,a_log", [(-1.0, 0.0), (6.0, 0.0), (-4.0, -9.0)])
+def test_walk_gives_the_bits_of_all_chunks_at_once(heads, groups, lens, n_decode, step, a_log):
+    """What else is in a step decides between the two, so a sequence's numbers may not depend on it."""
+    c = case(heads, groups, 128, 64, lens, n_decode, seed=4, step=step)
+    c["a_log"] += a_log
+    y, state = all_at_once(c)
+    walk(c)
+    assert torch.equal(c["y"], y) and torch.equal(c["state"], state)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("at", [5, 16, 40, 63, 64, 100, 127])
+def test_walk_spreads_non_finite_values_no_further(at, value):
+    """Neither to earlier tokens than those of its 16 rows, where masked weights multiply it, nor to other heads."""
+    c = case(4, 2, 128, 64, [130], 0, seed=6)
+    c["xbc"][at, 64:128] = value                  # values of head 1
+    y, state = all_at_once(c)
+    walk(c)
+    assert same(c["y"], y) and same(c["state"], state)
+    assert bool(c["y"][:at // 16 * 16].isfinite().all()) and not bool(c["y"][at, 64:128].isfinite().any())
+    assert bool(c["y"][:, :64].isfinite().all()) and bool(c["y"][:, 128:].isfinite().all())
+
+
+def test_walk_keeps_what_decays_slowly():
+    """Steps that nothing is forgotten over, all writes of one sign, two portions in a row: the state against 64 bits.  Its operands keep
+    2^-17; a chunk's sum of eight products loses up to 2^-23 each; the state is rounded to nearest once a chunk, its decay likewise."""
+    c = case(4, 1, 128, 64, [4096, 1000], 0, seed=7, step=-4.0)
+    c["a_log"].fill_(-9.0)
+    c["xbc"] = c["xbc"].abs() + 0.5
+    exact, chunks, slots = c["state"].to(F64), 0, c["slot"].tolist()
+    for start in (0, 1):
+        c["start"].fill_(start)
+        for slot, want in zip(slots, recurrence(dict(c, state=exact), False)[1]):
+            exact[slot] = want
+        walk(c)
+        chunks += 64
+        off = ((c["state"].to(F64) - exact).abs() / exact.abs())[slots]
+        assert float(off.max()) <= 2.0 ** -17 + 2.0 ** -20 + 2 * chunks * 2.0 ** -24 and float(off.mean()) <= 2.0 ** -19
