@@ -442,8 +442,11 @@ __global__ void __launch_bounds__(256) wkv_out_kernel(const msa_lm_wkv_args a, c
 }
 
 // Parts of up to 1024 elements in fours: a warp per part, read once, no barrier (a block per part reads twice around two barriers:
-// 6236 rows x 8 parts of 512 elements took 39 us, 30 now; at HBM rate 24).  Below two blocks per SM the launch is nothing but latency, and a block
-// per part is the shorter one (64 parts: 2.0 and 3.8 us).
+// 6236 rows x 8 parts of 512 elements from a cold L2, events around the launch, 45 us by blocks and 33 by warps; at HBM rate 24).  Below two
+// blocks per SM the launch is nothing but latency, and a block per part is the shorter one (64 parts: 2.0 and 3.8 us).  The sums are the
+// block's, 128 elements after 128, so that a row's bits do not depend on how many rows there are; one text for its squares, with the
+// multiply-adds named, since two loops around the same text came to different ones.
+__device__ __forceinline__ float squares(const float4& v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.x, v.x, __fmul_rn(v.y, v.y)))); }
 template <typename T, int N>
 __global__ void __launch_bounds__(256) part_norm_warp_kernel(const float* __restrict__ x, long long x_stride, const float* __restrict__ w, int size,
                                                              int parts, long long n_items, int n_rows, float eps, T* __restrict__ out,
@@ -463,10 +466,16 @@ __global__ void __launch_bounds__(256) part_norm_warp_kernel(const float* __rest
     v[k] = on ? load4(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     g[k] = on ? load4(w + c0 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  float ss = 0.f;
+  float ss[N], sum = 0.f;
 #pragma unroll
-  for (int k = 0; k < N; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
-  const float inv = 1.f / sqrtf(warp_sum_f(ss) / (float)size + eps);
+  for (int k = 0; k < N; ++k) ss[k] = squares(v[k]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) ss[k] += __shfl_xor_sync(0xffffffffu, ss[k], o);
+#pragma unroll
+  for (int k = 0; k < N; ++k) sum += ss[k];
+  const float inv = 1.f / sqrtf(sum / (float)size + eps);
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const int i = (k * 32 + lane) * 4;
@@ -486,7 +495,7 @@ __global__ void __launch_bounds__(256) part_norm_kernel(const float* __restrict_
   T* dst = out + row * out_stride + c0;
   float ss = 0.f;
   for (int i = threadIdx.x * V; i < size; i += blockDim.x * V) {
-    if constexpr (V == 4) { const float4 v = load4(src + i); ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
+    if constexpr (V == 4) ss += squares(load4(src + i));
     else ss += src[i] * src[i];
   }
   const float inv = 1.f / sqrtf(block_sum(ss, s_part) / (float)size + eps);
