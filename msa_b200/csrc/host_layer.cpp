@@ -19,6 +19,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <array>
+
 #include "../../include/msa_b200.h"
 
 namespace {
@@ -61,6 +63,11 @@ bool bf16(const Tensor& t, c10::Device device) { return takes(t, at::kBFloat16, 
 bool quiet() {                                     // no gradient to keep, nobody who watches or changes calls
   return !at::GradMode::is_enabled() && !at::autocast::is_autocast_enabled(at::kCUDA) && !c10::impl::dispatch_mode_enabled() &&
          !at::impl::torch_function_mode_enabled() && lib.msa_last_error;
+}
+// Allocations, products and launches, which may block (a full launch queue, a device that is asked for memory): Python's other threads go on.
+template <typename F> auto unlocked(const F& work) {
+  const py::gil_scoped_release release;
+  return work();
 }
 PyTypeObject *tensor_type = nullptr, *parameter_type = nullptr;
 bool exact(PyObject* o) { return o && (Py_TYPE(o) == tensor_type || Py_TYPE(o) == parameter_type); }
@@ -201,8 +208,10 @@ py::object add_norm(const py::object& x_, const py::object& branch_, const py::o
   if (!quiet() || !x.defined() || !x.is_cuda() || !bf16(x, x.device()) || !rows_fit(x) || x.size(2) % 2 || x.size(2) > kMaxHidden ||
       !operand(branch_, x.device(), x, true, branch) || !vector(n, x.size(2), x.device()))
     return py::none();
-  const c10::cuda::CUDAGuard guard(x.device());
-  auto r = add_norm_of(x, branch, n);
+  const auto r = unlocked([&] {
+    const c10::cuda::CUDAGuard guard(x.device());
+    return add_norm_of(x, branch, n);
+  });
   return py::make_tuple(r.first, r.second);
 }
 
@@ -214,17 +223,20 @@ py::object front(const Layer& l, const py::object& x_, const py::object& branch_
   if (!quiet() || !bf16(x, dev) || !rows_fit(x) || x.size(2) != l.hidden || !operand(branch_, dev, x, true, branch) || !bf16(cos, dev) || !bf16(sin, dev) ||
       cos.sizes() != sin.sizes() || cos.dim() != 3 || cos.size(2) != kHead || cos.size(1) != x.size(1) || (cos.size(0) != x.size(0) && cos.size(0) != 1))
     return py::none();
-  const c10::cuda::CUDAGuard guard(dev);
-  auto [x_new, h] = add_norm_of(x, branch, l.in);
-  const Tensor q0 = product(h, l.q), k0 = product(h, l.k), v = product(h, l.v);
-  Tensor q = at::empty_like(q0), k = at::empty_like(k0);
-  const int64_t heads = l.q.size(0), kv = l.k.size(0);
-  check(lib.msa_heads_norm_rope(q0.const_data_ptr(), heads, k0.const_data_ptr(), kv, (int32_t)(x.size(0) * x.size(1)), (int32_t)(heads / kHead),
-                                (int32_t)(kv / kHead), (int32_t)kHead, l.q_norm.w.const_data_ptr(), l.k_norm.w.const_data_ptr(), (float)l.q_norm.eps,
-                                cos.const_data_ptr(), sin.const_data_ptr(), (int32_t)(cos.size(0) * cos.size(1)), q.data_ptr(), k.data_ptr(), stream_of(x)),
-        "msa_heads_norm_rope");
-  auto heads_of = [&](const Tensor& t) { return t.view({x.size(0), x.size(1), -1, kHead}).transpose(1, 2); };
-  return py::make_tuple(x_new, h, heads_of(q), heads_of(k), heads_of(v));
+  const auto r = unlocked([&] {
+    const c10::cuda::CUDAGuard guard(dev);
+    auto [x_new, h] = add_norm_of(x, branch, l.in);
+    const Tensor q0 = product(h, l.q), k0 = product(h, l.k), v = product(h, l.v);
+    Tensor q = at::empty_like(q0), k = at::empty_like(k0);
+    const int64_t heads = l.q.size(0), kv = l.k.size(0);
+    check(lib.msa_heads_norm_rope(q0.const_data_ptr(), heads, k0.const_data_ptr(), kv, (int32_t)(x.size(0) * x.size(1)), (int32_t)(heads / kHead),
+                                  (int32_t)(kv / kHead), (int32_t)kHead, l.q_norm.w.const_data_ptr(), l.k_norm.w.const_data_ptr(), (float)l.q_norm.eps,
+                                  cos.const_data_ptr(), sin.const_data_ptr(), (int32_t)(cos.size(0) * cos.size(1)), q.data_ptr(), k.data_ptr(), stream_of(x)),
+          "msa_heads_norm_rope");
+    auto heads_of = [&](const Tensor& t) { return t.view({x.size(0), x.size(1), -1, kHead}).transpose(1, 2); };
+    return std::array<Tensor, 5>{x_new, h, heads_of(q), heads_of(k), heads_of(v)};
+  });
+  return py::make_tuple(r[0], r[1], r[2], r[3], r[4]);
 }
 
 // (stream with the attention's branch, the feed-forward's branch)
@@ -234,15 +246,18 @@ py::object back(const Layer& l, const py::object& x_, const py::object& attn_) {
   if (!quiet() || !bf16(x, dev) || !rows_fit(x) || x.size(2) != l.hidden || !bf16(attn, dev) || attn.dim() != 3 || attn.size(0) != x.size(0) ||
       attn.size(1) != x.size(1) || attn.size(2) != l.o.size(1))
     return py::none();
-  const c10::cuda::CUDAGuard guard(dev);
-  auto [x_new, h] = add_norm_of(x, product(attn, l.o), l.post);
-  const Tensor gate = product(h, l.gate), up = product(h, l.up);
-  Tensor act = at::empty_like(gate);
-  const int64_t ffn = l.gate.size(0);
-  check(lib.msa_silu_mul_parts(gate.const_data_ptr(), ffn, up.const_data_ptr(), ffn, (int32_t)(x.size(0) * x.size(1)), (int32_t)ffn, act.data_ptr(),
-                               stream_of(x)),
-        "msa_silu_mul_parts");
-  return py::make_tuple(x_new, product(act, l.down));
+  const auto r = unlocked([&] {
+    const c10::cuda::CUDAGuard guard(dev);
+    auto [x_new, h] = add_norm_of(x, product(attn, l.o), l.post);
+    const Tensor gate = product(h, l.gate), up = product(h, l.up);
+    Tensor act = at::empty_like(gate);
+    const int64_t ffn = l.gate.size(0);
+    check(lib.msa_silu_mul_parts(gate.const_data_ptr(), ffn, up.const_data_ptr(), ffn, (int32_t)(x.size(0) * x.size(1)), (int32_t)ffn, act.data_ptr(),
+                                 stream_of(x)),
+          "msa_silu_mul_parts");
+    return std::pair<Tensor, Tensor>{x_new, product(act, l.down)};
+  });
+  return py::make_tuple(r.first, r.second);
 }
 
 // cos and sin of positions [batch, tokens] (int64): bf16 [batch, tokens, 2 * frequencies]
@@ -251,13 +266,16 @@ py::object angles(const py::object& positions_, const py::object& inv_freq_, dou
   if (!quiet() || !pos.defined() || !pos.is_cuda() || !takes(pos, at::kLong, pos.device()) || !takes(freq, at::kFloat, pos.device()) || pos.dim() != 2 ||
       freq.dim() != 1 || pos.numel() == 0 || pos.numel() >= (1ll << 31))
     return py::none();
-  const c10::cuda::CUDAGuard guard(pos.device());
-  const Tensor both = at::empty({2, pos.size(0), pos.size(1), 2 * freq.size(0)}, pos.options().dtype(at::kBFloat16));
-  Tensor cos = both.select(0, 0), sin = both.select(0, 1);
-  check(lib.msa_rope_table(static_cast<const int64_t*>(pos.const_data_ptr()), static_cast<const float*>(freq.const_data_ptr()), (int32_t)pos.numel(),
-                           (int32_t)freq.size(0), (float)scaling, cos.data_ptr(), sin.data_ptr(), stream_of(pos)),
-        "msa_rope_table");
-  return py::make_tuple(cos, sin);
+  const auto r = unlocked([&] {
+    const c10::cuda::CUDAGuard guard(pos.device());
+    const Tensor both = at::empty({2, pos.size(0), pos.size(1), 2 * freq.size(0)}, pos.options().dtype(at::kBFloat16));
+    Tensor cos = both.select(0, 0), sin = both.select(0, 1);
+    check(lib.msa_rope_table(static_cast<const int64_t*>(pos.const_data_ptr()), static_cast<const float*>(freq.const_data_ptr()), (int32_t)pos.numel(),
+                             (int32_t)freq.size(0), (float)scaling, cos.data_ptr(), sin.data_ptr(), stream_of(pos)),
+          "msa_rope_table");
+    return std::pair<Tensor, Tensor>{cos, sin};
+  });
+  return py::make_tuple(r.first, r.second);
 }
 
 // The attention of one token per sequence over its compact cache, which takes the token in: q, k, v [batch, heads, 1, 128].
@@ -269,7 +287,6 @@ py::object decode(const py::object& q_, const py::object& k_, const py::object& 
   if (!quiet() || !q4.defined() || !q4.is_cuda() || q4.dim() != 4 || q4.size(2) != 1 || !k4.defined() || !v4.defined() || k4.dim() != 4 || v4.dim() != 4)
     return py::none();
   const c10::Device dev = q4.device();
-  const c10::cuda::CUDAGuard guard(dev);
   const Tensor q = q4.select(2, 0), k = k4.select(2, 0), v = v4.select(2, 0);
   const int64_t b = q.size(0), hq = q.size(1), d = q.size(2), hkv = k.size(1);
   if (!bf16(q, dev) || !bf16(k, dev) || !bf16(v, dev) || !bf16(ks, dev) || !bf16(vs, dev) || d != kHead || b == 0 || hkv == 0 || hq % hkv ||
@@ -277,21 +294,24 @@ py::object decode(const py::object& q_, const py::object& k_, const py::object& 
       ks.size(1) != hkv || ks.size(3) != d || !takes(start, at::kInt, dev) || !takes(len, at::kInt, dev) || start.numel() != b || len.numel() != b ||
       !lengths.defined() || !plain_key_set(lengths) || lengths.device() != dev || n_splits < 1)
     return py::none();
-  Tensor out = at::empty({b, 1, hq * d}, q.options()), space;
-  const int64_t need = lib.msa_decode_workspace_bytes((int32_t)b, (int32_t)hq, (int32_t)d, (int32_t)n_splits);
-  if (need > 0) space = at::empty({need / 4}, q.options().dtype(at::kFloat));
-  const bool counts = takes(lengths, at::kLong, dev) && lengths.numel() == b && lengths.dim() == 1 && len.dim() == 1;
-  const Tensor next_len = counts ? at::empty_like(len) : Tensor(), next_lengths = counts ? at::empty_like(lengths) : Tensor();
-  check(lib.msa_sparse_decode_attn_next(q.const_data_ptr(), MSA_BF16, ks.data_ptr(), vs.data_ptr(), ks.stride(0), ks.stride(1),
-                                   static_cast<const int32_t*>(start.const_data_ptr()), static_cast<const int32_t*>(len.const_data_ptr()),
-                                   k.const_data_ptr(), v.const_data_ptr(), (int32_t)b, (int32_t)hq, (int32_t)hkv, (int32_t)d,
-                                   (float)(1.0 / std::sqrt((double)d)), out.data_ptr(), need > 0 ? space.data_ptr() : nullptr, need > 0 ? need : 0,
-                                   (int32_t)n_splits, counts ? static_cast<const int64_t*>(lengths.const_data_ptr()) : nullptr,
-                                   counts ? static_cast<int32_t*>(next_len.data_ptr()) : nullptr,
-                                   counts ? static_cast<int64_t*>(next_lengths.data_ptr()) : nullptr, stream_of(q)),
-        "msa_sparse_decode_attn");
-  if (counts) return py::make_tuple(out, next_len, next_lengths);
-  return py::make_tuple(out, len.add(1), lengths.add(1));
+  const auto r = unlocked([&] {
+    const c10::cuda::CUDAGuard guard(dev);
+    Tensor out = at::empty({b, 1, hq * d}, q.options()), space;
+    const int64_t need = lib.msa_decode_workspace_bytes((int32_t)b, (int32_t)hq, (int32_t)d, (int32_t)n_splits);
+    if (need > 0) space = at::empty({need / 4}, q.options().dtype(at::kFloat));
+    const bool counts = takes(lengths, at::kLong, dev) && lengths.numel() == b && lengths.dim() == 1 && len.dim() == 1;
+    const Tensor next_len = counts ? at::empty_like(len) : Tensor(), next_lengths = counts ? at::empty_like(lengths) : Tensor();
+    check(lib.msa_sparse_decode_attn_next(q.const_data_ptr(), MSA_BF16, ks.data_ptr(), vs.data_ptr(), ks.stride(0), ks.stride(1),
+                                     static_cast<const int32_t*>(start.const_data_ptr()), static_cast<const int32_t*>(len.const_data_ptr()),
+                                     k.const_data_ptr(), v.const_data_ptr(), (int32_t)b, (int32_t)hq, (int32_t)hkv, (int32_t)d,
+                                     (float)(1.0 / std::sqrt((double)d)), out.data_ptr(), need > 0 ? space.data_ptr() : nullptr, need > 0 ? need : 0,
+                                     (int32_t)n_splits, counts ? static_cast<const int64_t*>(lengths.const_data_ptr()) : nullptr,
+                                     counts ? static_cast<int32_t*>(next_len.data_ptr()) : nullptr,
+                                     counts ? static_cast<int64_t*>(next_lengths.data_ptr()) : nullptr, stream_of(q)),
+          "msa_sparse_decode_attn");
+    return counts ? std::array<Tensor, 3>{out, next_len, next_lengths} : std::array<Tensor, 3>{out, len.add(1), lengths.add(1)};
+  });
+  return py::make_tuple(r[0], r[1], r[2]);
 }
 
 }  // namespace

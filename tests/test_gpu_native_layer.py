@@ -1,4 +1,7 @@
 """The memory model's layers through native code: the bits of the pass through the modules, and that pass wherever a module is not plain."""
+import ctypes
+import subprocess
+
 import pytest
 import torch
 import torch.nn as nn
@@ -153,3 +156,43 @@ def test_a_function_put_in_the_place_of_an_op_is_called(monkeypatch, name, run):
         monkeypatch.setattr(ops, name, lambda *a, **k: calls.append(1) or real(*a, **k))
         got = run(net)
     assert calls and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+STUB = """
+int PyGILState_Check(void);
+int calls, held;
+static int seen(void) { ++calls; held += PyGILState_Check(); return 0; }
+const char* msa_last_error(void) { return "stub"; }
+long long msa_decode_workspace_bytes(void) { return 0; }
+int msa_add_rmsnorm(void) { return seen(); }
+int msa_heads_norm_rope(void) { return seen(); }
+int msa_silu_mul_parts(void) { return seen(); }
+int msa_rope_table(void) { return seen(); }
+int msa_sparse_decode_attn_next(void) { return seen(); }
+"""
+
+
+def test_python_goes_on_meanwhile(tmp_path):
+    """Allocations and launches happen without Python's lock: asked where the launches would be."""
+    from msa_b200 import _cabi as A
+    from msa_b200 import model as M
+    (tmp_path / "stub.c").write_text(STUB)
+    path = str(tmp_path / "stub.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", str(tmp_path / "stub.c"), "-o", path], check=True)
+    stub, n, net = ctypes.CDLL(path), A.native(), model()
+    of = lambda *s: torch.ones(*s, device=DEV, dtype=BF16)
+    count = lambda name: ctypes.c_int.in_dll(stub, name).value
+    with torch.no_grad():
+        parts = n.layers(tuple(net.layers), M.STEPPED_OVER)[0]
+        x, one, store, angle = of(1, 5, 256), of(3, 2, 1, 128), of(3, 2, 90, 128), of(1, 5, 128)
+        rows = of(1, 5, net.layers[0].self_attn.o_proj.weight.shape[1])
+        pos, ints = torch.zeros(1, 5, device=DEV, dtype=torch.int64), torch.ones(3, device=DEV, dtype=torch.int32)
+        calls = [lambda: n.add_norm(x, x, net.norm, M.Qwen3RMSNorm), lambda: n.front(parts, x, x, angle, angle), lambda: n.back(parts, x, rows),
+                 lambda: n.angles(pos, net.rotary_emb.inv_freq, 1.0), lambda: n.decode(one, one, one, store, store, ints, ints, ints.long(), 1)]
+        n.bind(path)
+        try:
+            for call in calls:
+                before = count("calls")
+                assert call() is not None and count("calls") > before and count("held") == 0
+        finally:
+            n.bind(A.LIB_PATH)
