@@ -6,8 +6,8 @@
 // product is therefore summed over 64 channels at a time and the parts are added in registers, rounded to nearest; the five small
 // ones go over all channels, two rows' planes side by side where the key's plane is the same (a product costs some 70 cycles,
 // whatever its columns: four per 16 channels, not six).  Against 64 bits (16,000 chunks x 64 rows x 1024) that is no further off than chains of fp32
-// multiply-adds.  Numbers for which the split is not exact or a part could overflow (not finite, 2^60 and more, below 2^-100 but
-// not zero) send the block's scores to such chains (slow; not met by keys and queries that stand for anything).
+// multiply-adds.  Rows and chunks with a number for which the split is not exact or a part could overflow (not finite, 2^60 and more, below
+// 2^-100 but not zero) get their scores from such chains (redo_odd); rows without a token are not looked at.
 //
 // 128 chunks (TMEM lanes) x up to 64 query rows per block, warps by role: 0-3 and 4-7 turn the keys' 32-channel boxes (TMA ring)
 // into three planes of bf16 in TMEM, where the products read them as their A operand; 8-10 turn the query rows into planes in shared
@@ -27,6 +27,9 @@ namespace msa {
 constexpr int kRfChunks = 128, kRfRows = 64, kRfStages = 8, kRfBox = kRfChunks * 128;       // a box: 32 channels of 128 chunks
 constexpr int kRfThreads = 16 * 32, kRfQThreads = 3 * 32, kRfSmem = kRfStages * kRfBox + 2 * 3 * kRfRows * 128 + 1024;
 constexpr uint32_t kRfLead = 0, kRfSmall = 2 * kRfRows, kRfLast = 4 * kRfRows, kRfPlanes = 5 * kRfRows;      // TMEM columns
+// redo_odd: channels at a time, floats of their row (16-byte reads without conflicts), of one buffer
+constexpr int kRfSlab = 64, kRfPitch = kRfSlab + 4, kRfSlabFloats = (kRfChunks + kRfRows) * kRfPitch;
+static_assert((2 * kRfSlabFloats + kRfRows * kRfChunks) * 4 <= kRfSmem - 1024, "redo_odd's memory");
 constexpr float kRfTop = 0x1p60f, kRfLow = 0x1p-100f;
 
 struct RouteFp32Params {
@@ -49,8 +52,8 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& h, uint32_t& 
   y -= __uint_as_float(m & 0xffff0000u);
   l = pack2_bf16(x, y);
 }
-// Denormal operands count (the file is compiled with them flushed).
-__device__ __forceinline__ void fma_exact(float& c, float a, float b) { asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(c) : "f"(a), "f"(b)); }
+// Denormal operands count (the file is compiled with them flushed), in fma_f32x2 too.
+__device__ __forceinline__ void add_exact(float& c, float a) { asm("add.rn.f32 %0, %0, %1;" : "+f"(c) : "f"(a)); }
 // Whether some of the numbers is outside what split3 takes.
 template <int N>
 __device__ __forceinline__ bool outside(const float (&x)[N]) {
@@ -68,12 +71,98 @@ __device__ __forceinline__ bool outside(const float (&x)[N]) {
   return bad;
 }
 
+// Four rows and the 32s of chunks I0 .. I1 - 1 of redo_odd; sums over the even and the odd channels.
+template <int I0, int I1>
+__device__ __forceinline__ void redo_add(unsigned long long (&sum)[4][4], const float* key, const float* row) {
+#pragma unroll 2
+  for (int k = 0; k < kRfSlab; k += 4) {
+    ulonglong2 q[4], c[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = *reinterpret_cast<const ulonglong2*>(row + j * kRfPitch + k);
+#pragma unroll
+    for (int i = I0; i < I1; ++i) c[i] = *reinterpret_cast<const ulonglong2*>(key + i * 32 * kRfPitch + k);
+#pragma unroll
+    for (int i = I0; i < I1; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[i][j] = fma_f32x2(c[i].x, q[j].x, sum[i][j]);
+#pragma unroll
+    for (int i = I0; i < I1; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[i][j] = fma_f32x2(c[i].y, q[j].y, sum[i][j]);
+  }
+}
+// Scores of the rows and chunks with a number that split3 does not take, as two chains of fp32 multiply-adds in the order of the channels: 64
+// channels of the block's 128 chunks and 64 rows at a time through shared memory, the next ones on their way, four rows per warp, four
+// chunks per lane.  A warp works on 32 chunks only where one of its rows or one of those chunks is such; the others' scores stay as the
+// products gave them.  Bound by the latency of its steps: 64 rows x 16,000 chunks x 1024 from a cold L2, table reset included, take 43 us, 84
+// with one such row, 105 with one such chunk, 135 with nothing but such rows (84 with multiply-adds throughout, and 2120 for any of them
+// when a thread per chunk read its key from memory row after row).
+__device__ __forceinline__ void redo_odd(const RouteFp32Params& p, int c0, int r0, float* tiles, float* scores, unsigned long long odd_rows,
+                                         const uint32_t* odd_chunks) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, n_steps = (p.kdim + kRfSlab - 1) / kRfSlab;
+  const uint32_t mine = (uint32_t)(odd_rows >> (4 * warp)) & 15u;
+  uint32_t groups = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) groups |= mine || odd_chunks[i] ? 1u << i : 0u;
+  unsigned long long sum[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum[i][j] = 0ull;
+  auto fetch = [&](int step) {
+    constexpr int kVecs = kRfSlab / 4;
+    const uint32_t dst = smem_u32(tiles + step % 2 * kRfSlabFloats);
+    for (int item = threadIdx.x; item < (kRfChunks + kRfRows) * kVecs; item += kRfThreads) {
+      const int r = item / kVecs, v = item % kVecs, k = step * kRfSlab + v * 4, row = r0 + r - kRfChunks;
+      const bool on = k < p.kdim && (r < kRfChunks ? c0 + r < p.n_chunks : r - kRfChunks < p.bn && row < p.n_rows);
+      const float* src = r < kRfChunks ? p.rk + (long long)(c0 + r) * p.rk_stride + k : p.qf + (long long)row * p.kdim + k;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (r * kRfPitch + v * 4) * 4), "l"(on ? src : p.qf), "r"(on ? 16u : 0u)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0);
+  for (int step = 0; step < n_steps; ++step) {
+    if (step + 1 < n_steps) {
+      fetch(step + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const float* key = tiles + step % 2 * kRfSlabFloats + lane * kRfPitch;
+    const float* row = tiles + step % 2 * kRfSlabFloats + (kRfChunks + 4 * warp) * kRfPitch;
+    if (groups == 15u) {
+      redo_add<0, 4>(sum, key, row);
+    } else {
+      if (groups & 1u) redo_add<0, 1>(sum, key, row);
+      if (groups & 2u) redo_add<1, 2>(sum, key, row);
+      if (groups & 4u) redo_add<2, 3>(sum, key, row);
+      if (groups & 8u) redo_add<3, 4>(sum, key, row);
+    }
+    __syncthreads();                                        // read before the step after the next lands there
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if ((mine >> j & 1u) || (odd_chunks[i] >> lane & 1u)) {
+        float even, odd;
+        f32x2_split(sum[i][j], even, odd);
+        add_exact(even, odd);
+        scores[(4 * warp + j) * kRfChunks + 32 * i + lane] = even;
+      }
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(kRfThreads, 1)
 route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Params p) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ uint64_t s_full[kRfStages], s_t_full[2], s_t_empty[2], s_b_full[2], s_b_empty[2], s_d_full[2], s_d_empty[2], s_drain;
   __shared__ uint32_t s_tmem_base;
-  __shared__ int s_abort, s_outside;
+  __shared__ int s_abort;
+  __shared__ unsigned long long s_odd_rows;                 // query rows and chunks with a number that split3 does not take
+  __shared__ uint32_t s_odd_chunks[kRfChunks / 32];
   __shared__ float s_bias[kRfRows];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int c0 = blockIdx.x * kRfChunks, r0 = blockIdx.y * p.bn;
@@ -89,7 +178,9 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
       mbar_init(&s_d_full[i], 1); mbar_init(&s_d_empty[i], 4);
     }
     mbar_init(&s_drain, 1);
-    s_abort = s_outside = 0;
+    s_abort = 0;
+    s_odd_rows = 0ull;
+    for (int i = 0; i < kRfChunks / 32; ++i) s_odd_chunks[i] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 11) {
@@ -140,13 +231,13 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_t_full[group]);
     }
-    if (bad) s_outside = 1;
+    if (bad) atomicOr(&s_odd_chunks[row / 32], 1u << (row % 32));
   } else if (warp < 11) {
     // ---- query rows: 64 channels at a time, eight per item
     const int t = threadIdx.x - 256, n_items = p.bn * 8;
     constexpr int kItems = (kRfRows * 8 + kRfQThreads - 1) / kRfQThreads;
     float x[kItems][8];
-    bool bad = false;
+    uint32_t bad = 0u;                                      // by item: its row is the same throughout
     auto load = [&](int kb) {
 #pragma unroll
       for (int i = 0; i < kItems; ++i) {
@@ -169,7 +260,7 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
       for (int i = 0; i < kItems; ++i) {
         const int item = t + i * kRfQThreads, r = item / 8, c = item % 8;
         if (item >= n_items) break;
-        bad |= outside(x[i]);
+        bad |= (uint32_t)outside(x[i]) << i;
         uint4 h, m, l;
         split3(x[i][0], x[i][1], h.x, m.x, l.x);
         split3(x[i][2], x[i][3], h.y, m.y, l.y);
@@ -185,7 +276,11 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
       if (lane == 0) mbar_arrive(&s_b_full[kb & 1]);
       if (kb + 1 < n_kb) load(kb + 1);
     }
-    if (bad) s_outside = 1;
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const int r = (t + i * kRfQThreads) / 8;
+      if ((bad >> i & 1u) && s_bias[r] != -INFINITY) atomicOr(&s_odd_rows, 1ull << r);       // what stands in a row without a token is not asked for
+    }
   } else if (warp == 11) {
     if (lane == 0) {
       auto fetch = [&](int box) {
@@ -264,24 +359,22 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
   __syncthreads();
   tc_fence_after();
   if (warp == 11) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-  if (warp < 12 || s_abort) return;
-  const int chunk = c0 + (warp - 12) * 32 + lane;
-  if (chunk >= p.n_chunks) return;
-  if (s_outside) {
-    const float* key = p.rk + chunk * p.rk_stride;
+  if (s_abort) return;
+  const bool some = s_odd_rows || s_odd_chunks[0] || s_odd_chunks[1] || s_odd_chunks[2] || s_odd_chunks[3];
+  float* scores = reinterpret_cast<float*>(ring) + 2 * kRfSlabFloats;                  // [row][chunk]
+  if (some) {
+    if (warp >= 12) {
 #pragma unroll
-    for (int j = 0; j < kRfRows; ++j) acc[j] = 0.f;
-    for (int k = 0; k < p.kdim; k += 4) {
-      const float4 c = *reinterpret_cast<const float4*>(key + k);
-#pragma unroll
-      for (int j = 0; j < kRfRows; ++j) {
-        if (j < p.bn && r0 + j < p.n_rows) {
-          const float4 q = *reinterpret_cast<const float4*>(p.qf + (long long)(r0 + j) * p.kdim + k);
-          fma_exact(acc[j], c.x, q.x); fma_exact(acc[j], c.y, q.y);
-          fma_exact(acc[j], c.z, q.z); fma_exact(acc[j], c.w, q.w);
-        }
-      }
+      for (int j = 0; j < kRfRows; ++j) scores[j * kRfChunks + threadIdx.x - 384] = acc[j];
     }
+    redo_odd(p, c0, r0, reinterpret_cast<float*>(ring), scores, s_odd_rows, s_odd_chunks);
+  }
+  if (warp < 12) return;
+  const int in_block = (warp - 12) * 32 + lane, chunk = c0 + in_block;
+  if (chunk >= p.n_chunks) return;
+  if (some) {
+#pragma unroll
+    for (int j = 0; j < kRfRows; ++j) acc[j] = scores[j * kRfChunks + in_block];
   }
   const int doc = p.chunk_doc[chunk];
   const bool known = doc >= 1 && doc <= p.n_docs;

@@ -67,3 +67,33 @@ def test_all_small_numbers_keep_their_digits():
     doc = torch.arange(1, 151, device=DEV, dtype=torch.int32)
     ref, got = want(q, rk, torch.float64), route(q, rk, doc).double()
     assert float((got - ref).norm() / ref.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 1e30, 1e-40])
+def test_such_numbers_leave_the_other_scores_alone(value):
+    """Two questions in one tile of rows, two tiles of chunks: what has no split costs its own row or chunk another kind of sum, no other."""
+    g = torch.Generator(device=DEV).manual_seed(7)
+    q = torch.randn(2, 4, 20, 32, generator=g, device=DEV)
+    rk = torch.randn(200, 128, generator=g, device=DEV)
+    doc = torch.arange(1, 201, device=DEV, dtype=torch.int32)
+    plain = route(q, rk, doc)
+    odd = q.clone()
+    odd[0, 2, 9, 3] = value
+    assert torch.equal(route(odd, rk, doc)[1], plain[1])
+    key = rk.clone()
+    key[131, 77] = value
+    others = torch.arange(200, device=DEV) != 131
+    assert torch.equal(route(q, key, doc)[:, others], plain[:, others])
+
+
+@pytest.mark.parametrize("kdim", [4, 124, 1024, 1100])
+def test_every_row_and_chunk_without_a_split(kdim):
+    g = torch.Generator(device=DEV).manual_seed(8)
+    q = torch.randn(3, kdim // 4, 70, 4, generator=g, device=DEV)
+    rk = torch.randn(150, kdim, generator=g, device=DEV)
+    q[..., 0] = 1e-33
+    rk[:, -1] *= 2.0 ** 61
+    doc = torch.arange(1, 151, device=DEV, dtype=torch.int32)
+    ref, got = want(q, rk, torch.float64), route(q, rk, doc).double()
+    # chains of kdim multiply-adds, each off by 2^-24 of the sum of absolute products
+    assert bool(((got - ref).abs() <= kdim * 2.0 ** -24 * want(q.abs(), rk.abs(), torch.float64)).all())
