@@ -148,8 +148,9 @@ class MSAService(Memory, MemoryClientBase):
         self._longest = 0             # chunks of the longest document that was published
         self._report = torch.zeros(3, dtype=torch.int64).pin_memory()      # total and status words of a plan, written by the kernel
 
-    #: up to how much storage the fetch of a call may allocate ahead of its read-back (see ``fetch``)
-    early_gather_bytes = 64 << 20
+    #: from and up to how much storage the fetch of a call allocates ahead of its read-back (see ``fetch``).  Small calls are bound by the
+    #: host, which the copies cost 20 us: one of 4 questions (3.9 MB) takes 124 us without and 146 with them, of 8 (7.9 MB) 183 and 168.
+    early_gather_from, early_gather_bytes = 6 << 20, 64 << 20
 
     def setup_memory_client(self, model):
         """Inject this service into every module that has ``set_memory_client`` (:1057-1067)."""
@@ -333,9 +334,10 @@ class MSAService(Memory, MemoryClientBase):
             return k, v, n_sel, total
         # The plan writes its total and the status words of this layer's routing to host memory; waiting for it sizes the result.  The
         # gather needs not wait with the host: it takes the total on the device, into storage for as many entries as the winners can
-        # have, of which the result is the front (32 questions against 16,000 chunks 507 -> 479 us).
+        # have, and what it found is copied from there into storage of its own size, which is what a caller may keep (32 questions against
+        # 16,000 chunks 506 us when it waits and 488 so).
         capacity = winner_local.numel() * self._longest
-        early = 0 < capacity * chunk_bytes <= self.early_gather_bytes
+        early = 0 < capacity and self.early_gather_from <= capacity * chunk_bytes <= self.early_gather_bytes
         planned = torch.cuda.Event()
         planned.record(torch.cuda.current_stream(self.device))
         if early:
@@ -345,6 +347,8 @@ class MSAService(Memory, MemoryClientBase):
         n = int(self._report[0])
         if early and n <= capacity:      # (a directory that was put in by hand may hold longer documents than the published one)
             k, v = (ops.packed_entries(t, g.num_key_value_heads, g.head_dim, n) for t in stores)
+            if n < capacity:
+                k, v = k.clone(), v.clone()
         else:
             k, v = ops.gather_run(plan, blk.kv.dtype, g.num_key_value_heads, g.head_dim, n, max_ctas)
         return k, v, n_sel

@@ -16,6 +16,7 @@ def service(n_docs, longest, dtype, top_k=4):
     rnd = lambda: torch.randn(sum(lens), 2, 64, generator=g, device=DEV).to(dtype)
     svc.load_pooled([Document(doc_id=10 + i, num_chunks=n) for i, n in enumerate(lens)], {0: (rnd(), rnd(), rnd())})
     svc.publish_directory()
+    svc.early_gather_from = 0                               # small calls too
     return svc, lens
 
 
@@ -37,3 +38,14 @@ def test_the_same_entries(n_docs, longest, batch, dtype):
     svc.early_gather_bytes = 1 << 30
     svc._longest = 1                                        # less room than the winners need
     assert all(torch.equal(a, b) for a, b in zip(query(svc, batch, dtype), late))
+
+
+@pytest.mark.parametrize("early_from", [0, 6 << 20])
+def test_results_hold_no_more_than_they_show(early_from):
+    """One long document in the bank sizes the storage that the gather writes to, not what a caller keeps."""
+    svc, lens = service(60, 40, torch.bfloat16)
+    svc.early_gather_from = early_from
+    k, v = query(svc, 7, torch.bfloat16)[:2]
+    assert k.shape[1] < 7 * 4 * max(lens) and k.shape == v.shape
+    for t in (k, v):
+        assert t.untyped_storage().nbytes() == t.numel() * t.element_size() and t.storage_offset() == 0
