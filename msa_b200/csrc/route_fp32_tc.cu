@@ -37,6 +37,7 @@ struct RouteFp32Params {
   const float* rk; long long rk_stride;
   const int32_t* chunk_doc;
   int n_rows, s_pad, bn, n_chunks, kdim, n_docs;
+  int first_row;                                            // of this launch: a grid has 65535 tiles of rows at most
   float alpha;
   uint32_t* keys; long long table_stride;
   int32_t* status;
@@ -165,7 +166,7 @@ route_fp32_kernel(const __grid_constant__ CUtensorMap tmap_k, const RouteFp32Par
   __shared__ uint32_t s_odd_chunks[kRfChunks / 32];
   __shared__ float s_bias[kRfRows];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int c0 = blockIdx.x * kRfChunks, r0 = blockIdx.y * p.bn;
+  const int c0 = blockIdx.x * kRfChunks, r0 = p.first_row + blockIdx.y * p.bn;
   unsigned char* ring = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   unsigned char* planes = ring + kRfStages * kRfBox;
   const int b_bytes = 3 * p.bn * 128;
@@ -403,13 +404,15 @@ int launch_route_fp32(const float* qf, const float* row_bias, int n_rows, int s_
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   MSA_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code %d", (int)r);
   const int blocks = n_rows / 16, tiles = (blocks + kRfRows / 16 - 1) / (kRfRows / 16), bn = (blocks + tiles - 1) / tiles * 16;
-  const int grid_y = (n_rows + bn - 1) / bn;
-  MSA_REQUIRE(grid_y <= 65535, "route (fp32): too many query rows (%d)", n_rows);
   static DeviceSmem state{};
   MSA_OK_OR_RETURN(ensure_dynamic_smem(route_fp32_kernel, kRfSmem, state));
-  const RouteFp32Params p{qf, row_bias, rk, rk_stride, chunk_doc, n_rows, s_pad, bn, n_chunks, kdim, n_docs, alpha, keys, table_stride, status};
-  route_fp32_kernel<<<dim3((n_chunks + kRfChunks - 1) / kRfChunks, grid_y), kRfThreads, kRfSmem, stream>>>(map, p);
-  MSA_LAUNCH_OK("route_fp32_kernel");
+  RouteFp32Params p{qf, row_bias, rk, rk_stride, chunk_doc, n_rows, s_pad, bn, n_chunks, kdim, n_docs, 0, alpha, keys, table_stride, status};
+  for (long long first = 0; first < n_rows; first += 65535ll * bn) {
+    p.first_row = (int)first;
+    const long long left = (n_rows - first + bn - 1) / bn;
+    route_fp32_kernel<<<dim3((n_chunks + kRfChunks - 1) / kRfChunks, (unsigned)(left < 65535 ? left : 65535)), kRfThreads, kRfSmem, stream>>>(map, p);
+    MSA_LAUNCH_OK("route_fp32_kernel");
+  }
   return MSA_OK;
 }
 

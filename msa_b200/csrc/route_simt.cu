@@ -199,7 +199,9 @@ int launch_route_simt_t(const void* qf, const float* row_bias, int n_seq, int s_
 int launch_route_simt(int32_t dtype, const void* qf, const float* row_bias, int n_seq, int s_pad, const void* rk,
                       int64_t rk_stride, int n_chunks, int kdim, const int32_t* chunk_doc, int n_docs, float alpha,
                       uint32_t* keys, int64_t table_stride, int32_t* status, cudaStream_t stream) {
-  if (dtype == MSA_F32 && s_pad % 16 == 0 && kdim % 4 == 0 && rk_stride % 4 == 0 && aligned16(qf) && aligned16(rk) && n_seq > 0 && n_chunks > 0)
+  // a tensor map takes rows up to 2^40 bytes apart, and none that share memory (an expanded key)
+  if (dtype == MSA_F32 && s_pad % 16 == 0 && kdim % 4 == 0 && rk_stride % 4 == 0 && rk_stride >= kdim && rk_stride < (1ll << 38) && aligned16(qf) &&
+      aligned16(rk) && n_seq > 0 && n_chunks > 0)
     return launch_route_fp32((const float*)qf, row_bias, n_seq * s_pad, s_pad, (const float*)rk, rk_stride, n_chunks, kdim, chunk_doc, n_docs, alpha,
                              keys, table_stride, status, stream);
   return dtype == MSA_BF16

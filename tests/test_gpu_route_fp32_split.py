@@ -97,3 +97,25 @@ def test_every_row_and_chunk_without_a_split(kdim):
     ref, got = want(q, rk, torch.float64), route(q, rk, doc).double()
     # chains of kdim multiply-adds, each off by 2^-24 of the sum of absolute products
     assert bool(((got - ref).abs() <= kdim * 2.0 ** -24 * want(q.abs(), rk.abs(), torch.float64)).all())
+
+
+def test_more_rows_than_a_grid_has_tiles():
+    from msa_b200 import ops
+    rows = 65535 * 64 + 80
+    g = torch.Generator(device=DEV).manual_seed(9)
+    qf, rk = torch.randn(rows, 4, generator=g, device=DEV), torch.randn(3, 4, generator=g, device=DEV)
+    qf[-1] = 50 * rk[1]                           # the best row of the second chunk is the last one
+    keys, status = ops.route_scores(qf, torch.zeros(rows, device=DEV), 1, rows, rk, torch.arange(1, 4, device=DEV, dtype=torch.int32), 3, 1.0)
+    got, ref = ops.keys_to_scores(keys)[0, 1:].double(), (qf.double() @ rk.double().t()).amax(0)
+    assert status.tolist() == [0, 0, 0, 0] and bool(((got - ref).abs() <= 4 * 2.0 ** -24 * (qf.double().abs() @ rk.double().abs().t()).amax(0)).all())
+
+
+@pytest.mark.parametrize("form", ["expanded", "overlapping"])
+def test_keys_that_share_memory(form):
+    """A bank of views: rows that a tensor map does not take."""
+    g = torch.Generator(device=DEV).manual_seed(10)
+    flat = torch.randn(128 + 4 * 40, generator=g, device=DEV)
+    rk = flat[:128].expand(40, 128) if form == "expanded" else flat.as_strided((40, 128), (4, 1))
+    q, doc = torch.randn(1, 4, 20, 32, generator=g, device=DEV), torch.arange(1, 41, device=DEV, dtype=torch.int32)
+    bound = 128 * 2.0 ** -24 * want(q.abs(), rk.abs(), torch.float64)
+    assert bool(((route(q, rk, doc).double() - want(q, rk, torch.float64)).abs() <= bound).all())
