@@ -7,7 +7,9 @@ pointers, sizes and the current CUDA stream to the C ABI.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
+import threading
 
 import torch
 
@@ -121,20 +123,31 @@ def lib() -> C.CDLL:
     return _lib
 
 
-_native = None
+_native, _native_lock = None, threading.Lock()
 
 
 def native():
     """The native host side of the memory model's layers (``csrc/host_layer.cpp``)."""
+    return _native or _load_native()
+
+
+def _load_native():
     global _native
-    if _native is None:
-        lib()
-        try:
-            from . import _native as n
-        except ImportError as e:
-            raise MsaError(f"msa_b200/_native.so cannot be loaded: build it with `python -m msa_b200.build` ({e})") from e
-        n.bind(LIB_PATH)
-        _native = n
+    lib()
+    from .build import native_path
+    path = native_path()
+    if not os.path.exists(path):
+        raise MsaError(f"{path} is missing: build it for this torch and Python with `python -m msa_b200.build`")
+    with _native_lock:                      # its classes can be registered once
+        if _native is None:
+            spec = importlib.util.spec_from_file_location("msa_b200._native", path)
+            try:
+                n = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(n)
+            except ImportError as e:
+                raise MsaError(f"{path} cannot be loaded: build it with `python -m msa_b200.build --force` ({e})") from e
+            n.bind(LIB_PATH)
+            _native = n
     return _native
 
 

@@ -5,7 +5,7 @@
 
 Two libraries, each built only when it is asked for or stale: ``libmsa_b200.so`` (memory routing and sparse attention,
 ``include/msa_b200.h``) and ``libmsa_b200_lm.so`` (the layered decoder designs, ``include/msa_b200_lm.h``); and with g++ the
-extension ``_native.so`` (host side of the memory model's layers).
+extension ``_native`` (host side of the memory model's layers), whose file is named by the versions of torch and Python that it is for.
 """
 from __future__ import annotations
 
@@ -30,9 +30,21 @@ LIBRARIES = {
 }
 
 
-# The native host side of the memory model's layers: an extension of torch, which binds the first library when it is used.
-LIB_NATIVE, NATIVE_SOURCE = os.path.join(HERE, "_native.so"), "host_layer.cpp"
-LIBRARIES["native"] = (LIB_NATIVE, [NATIVE_SOURCE], [], ["msa_b200.h"])
+NATIVE_SOURCE = "host_layer.cpp"
+LIBRARIES["native"] = (None, [NATIVE_SOURCE], [], ["msa_b200.h"])      # the path: native_path()
+
+
+def native_path() -> str:
+    """The native host side of the memory model's layers: an extension of torch, which binds the first library when it is used.  It is
+    compiled against one torch's classes and one Python's, so both are part of its name: after either changes it is built anew."""
+    import sysconfig
+
+    import torch
+    return os.path.join(HERE, f"_native.torch-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
+def _path(name: str) -> str:
+    return native_path() if name == "native" else LIBRARIES[name][0]
 
 
 def _nvcc() -> str:
@@ -41,7 +53,7 @@ def _nvcc() -> str:
 
 
 def _stale(name: str) -> bool:
-    path, sources, _, headers = LIBRARIES[name]
+    path, (_, sources, _, headers) = _path(name), LIBRARIES[name]
     if not os.path.exists(path):
         return True
     t = os.path.getmtime(path)
@@ -54,7 +66,8 @@ def _build_native() -> None:
     import sysconfig
 
     from torch.utils import cpp_extension as ext
-    part = f"{LIB_NATIVE}.{os.getpid()}"
+    path = native_path()
+    part = f"{path}.{os.getpid()}"
     paths = [a for p in ext.include_paths() for a in ("-isystem", p)]
     cuda = os.path.dirname(os.path.dirname(_nvcc())) or "/usr/local/cuda"
     libs = [f"-L{p}" for p in ext.library_paths()] + ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
@@ -63,7 +76,7 @@ def _build_native() -> None:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for {NATIVE_SOURCE}:\n{r.stdout}\n{r.stderr}")
-    os.replace(part, LIB_NATIVE)
+    os.replace(part, path)
 
 
 def _build_one(name: str, verbose: bool) -> None:
@@ -102,7 +115,7 @@ def build(force: bool = False, verbose: bool = False, only: str | None = None) -
     for name in ([only] if only else LIBRARIES):
         if force or _stale(name):
             _build_one(name, verbose)
-    return LIBRARIES[only or "msa"][0]
+    return _path(only or "msa")
 
 
 if __name__ == "__main__":
