@@ -148,9 +148,10 @@ class MSAService(Memory, MemoryClientBase):
         self._longest = 0             # chunks of the longest document that was published
         self._report = torch.zeros(3, dtype=torch.int64).pin_memory()      # total and status words of a plan, written by the kernel
 
-    #: from and up to how much storage the fetch of a call allocates ahead of its read-back (see ``fetch``).  Small calls are bound by the
-    #: host, which the copies cost 20 us: one of 4 questions (3.9 MB) takes 124 us without and 146 with them, of 8 (7.9 MB) 183 and 168.
-    early_gather_from, early_gather_bytes = 6 << 20, 64 << 20
+    #: from and up to how much storage the fetch of a call allocates ahead of its read-back (see ``fetch``).  Smaller calls are bound by the
+    #: host, which the copies cost 15 to 20 us: 3.8 MiB 119 us without and 139 so, 5.0 MiB 134 and 138 (2,100 chunks) or 252 and 238
+    #: (72,000), 5.6 MiB 160 and 150, 7.2 MiB 165 and 151, 15 MiB 280 and 264.
+    early_gather_from, early_gather_bytes = 5 << 20, 64 << 20
 
     def setup_memory_client(self, model):
         """Inject this service into every module that has ``set_memory_client`` (:1057-1067)."""
