@@ -1,8 +1,9 @@
 // The host side of a decoder layer of the memory model in bf16 inference, in native code.
 //
-// A decode token of two layers (32 sequences) is 34 launches of 300 us in all, and took 714 us: what bounded it was Python between
-// them (module calls, attribute look-ups through nn.Module.__getattr__, ctypes); 371 us now, and 16 questions of 96 tokens 1361 us
-// instead of 1566.  Here a layer is two calls around the attention of its stage:
+// A decode token of two layers (32 sequences), then 34 launches of 300 us in all, took 714 us through the modules: what bounded it was Python
+// between them (module calls, attribute look-ups through nn.Module.__getattr__, ctypes).  The same launches took 371 us from here (30 of
+// them 350, since the one that appends a token advances the lengths), 16 questions of 96 tokens 1361 us instead of 1566.  A layer is two
+// calls around the attention of its stage:
 // `front` (residual add and norm, q / k / v, head norm and rotation) and `back` (output product, residual add and norm, gated
 // feed-forward), and a third for the attention of a single token.  Products are the library calls
 // that nn.Linear comes to.

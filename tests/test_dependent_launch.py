@@ -50,7 +50,6 @@ def test_a_library_product_is_not_let_in_early():
     always = {"fold_kernel",                                        # route_dec_kernel (any other waits for its end)
               "live_blocks_kernel",                                  # pack_rows_kernel
               "moe_topk_kernel", "moe_sort_kernel", "moe_gemm_tc_kernel",
-              "group_decode_kernel", "latent_decode_kernel",         # merge_partials_kernel
               "rows_gemm_kernel"}
     assert {name for name, _, body in kernels() if re.search(r"(?<!\) )grid_launch_dependents\(\);", body)} <= always
     assert "if (rows <= kEarlyRows) grid_launch_dependents();" in open(os.path.join(CSRC, "lm_common.cuh")).read()
